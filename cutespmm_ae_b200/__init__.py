@@ -70,6 +70,8 @@ def _load() -> C.CDLL:
         "cutespmm_plan_destroy": (C.c_int, [vp]),
         "cutespmm_plan_save": (C.c_int, [vp, C.c_char_p]),
         "cutespmm_plan_load": (C.c_int, [C.POINTER(vp), C.c_char_p, C.c_int]),
+        "cutespmm_plan_dims": (C.c_int, [vp, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]),
+        "cutespmm_release_memory": (C.c_int, []),
         "cutespmm_plan_info": (C.c_int, [vp, C.POINTER(PlanInfo)]),
         "cutespmm_plan_blocked_row_ptr": (C.c_int, [vp, vp]),
         "cutespmm_plan_active_cols": (C.c_int, [vp, vp]),
@@ -166,7 +168,9 @@ class Plan:
         _check(lib.cutespmm_plan_create_device(C.byref(self._h), M, K, row_ptr.data_ptr(), cols.data_ptr(), vals.data_ptr(),
                                                C.byref(opts), st))
         self.M, self.K = M, K
-        self.nnz = self.info()["nnz"]
+        nnz = C.c_uint64()
+        _check(lib.cutespmm_plan_dims(self._h, None, None, C.byref(nnz)))
+        self.nnz = nnz.value
         return self
 
     def save(self, path) -> None:

@@ -85,6 +85,7 @@ static int build_common(cutespmm_plan_t **out, uint64_t M, uint64_t K, const uin
         delete p;
         return fail(st, err);
     }
+    p->note_list_sizes();
     *out = p;
     return CUTESPMM_OK;
 }
@@ -93,21 +94,6 @@ int cutespmm_plan_build_host(cutespmm_plan_t **plan, uint64_t M, uint64_t K, con
                              const uint32_t *cols, const float *vals, const cutespmm_options_t *opts)
 {
     return build_common(plan, M, K, rowPtr, cols, vals, opts);
-}
-
-// The current device, checked to be one this library runs on.
-static int usable_device(int *dev, int *sm_count)
-{
-    cudaError_t e = cudaGetDevice(dev);
-    if (e != cudaSuccess) return fail_cuda(e, "cudaGetDevice (libcutespmm needs a CUDA device; there is no CPU path)");
-    cudaDeviceProp prop;
-    e = cudaGetDeviceProperties(&prop, *dev);
-    if (e != cudaSuccess) return fail_cuda(e, "cudaGetDeviceProperties");
-    if (prop.major < 10)
-        return fail(CUTESPMM_EUNSUPPORTED, "this library is built for sm_100a (B200) only; found compute capability " +
-                                               std::to_string(prop.major) + "." + std::to_string(prop.minor));
-    *sm_count = prop.multiProcessorCount;
-    return CUTESPMM_OK;
 }
 
 // What the row kernel needs to finish long rows inside the launch: per scratch slot the long row it belongs to (for
@@ -201,7 +187,7 @@ static int upload_plan(cutespmm_plan *p, int dev, int sm_count)
 int cutespmm_internal_upload_plan(cutespmm_plan *p)
 {
     int dev = -1, sms = 0;
-    const int st = usable_device(&dev, &sms);
+    const int st = cutespmm_internal_usable_device(&dev, &sms);
     return st != CUTESPMM_OK ? st : upload_plan(p, dev, sms);
 }
 
@@ -212,7 +198,7 @@ int cutespmm_plan_create(cutespmm_plan_t **plan, uint64_t M, uint64_t K, const u
 {
     // fail before the (possibly long) host build when there is no usable device
     int dev = -1, sms = 0;
-    int st = usable_device(&dev, &sms);
+    int st = cutespmm_internal_usable_device(&dev, &sms);
     if (st != CUTESPMM_OK) return st;
     NvtxRange range("cutespmm: plan creation");
     if ((st = build_common(plan, M, K, rowPtr, cols, vals, opts)) != CUTESPMM_OK) return st;
@@ -221,154 +207,6 @@ int cutespmm_plan_create(cutespmm_plan_t **plan, uint64_t M, uint64_t K, const u
         *plan = nullptr;
     }
     return st;
-}
-
-int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M, uint64_t K, const uint32_t *rowPtr_dev, const uint32_t *cols_dev,
-                                const float *vals_dev, const cutespmm_options_t *opts, void *stream)
-{
-    if (!plan) return fail(CUTESPMM_EINVAL, "plan is NULL");
-    *plan = nullptr;
-    if (!rowPtr_dev) return fail(CUTESPMM_EINVAL, "rowPtr is NULL");
-    if (M >= (1ull << 32) - kPanelRows || K >= (1ull << 32)) return fail(CUTESPMM_EUNSUPPORTED, "M and K must be below 2^32");
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    NvtxRange range("cutespmm: plan creation (device CSR)");
-    int dev = -1;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return fail_cuda(e, "cudaGetDevice (libcutespmm needs a CUDA device; there is no CPU path)");
-    cudaDeviceProp prop;
-    if ((e = cudaGetDeviceProperties(&prop, dev)) != cudaSuccess) return fail_cuda(e, "cudaGetDeviceProperties");
-    if (prop.major < 10)
-        return fail(CUTESPMM_EUNSUPPORTED, "this library is built for sm_100a (B200) only; found compute capability " +
-                                               std::to_string(prop.major) + "." + std::to_string(prop.minor));
-    // the row pointers come to the host (4 bytes per row): tiles, chunks and the list of long rows are cut from them alone
-    std::vector<uint32_t> rp;
-    try {
-        rp.resize(M + 1);
-    } catch (const std::bad_alloc &) {
-        return fail(CUTESPMM_ENOMEM, "host allocation failed");
-    }
-    if ((e = cudaMemcpyAsync(rp.data(), rowPtr_dev, (M + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(s)) != cudaSuccess)
-        return fail_cuda(e, "reading the row pointers");
-    cutespmm_plan *p = new (std::nothrow) cutespmm_plan();
-    if (!p) return fail(CUTESPMM_ENOMEM, "host allocation failed");
-    std::string err;
-    int st;
-    try {
-        st = build_rows_plan_from_row_ptr(p->host, M, K, std::move(rp), opts, err);
-    } catch (const std::bad_alloc &) {
-        st = CUTESPMM_ENOMEM;
-        err = "host allocation failed while building the plan";
-    }
-    if (st != CUTESPMM_OK) { delete p; return fail(st, err); }
-    HostPlan &h = p->host;
-    if (h.nnz && (!cols_dev || !vals_dev)) { delete p; return fail(CUTESPMM_EINVAL, "cols/vals is NULL"); }
-    p->device = dev;
-    p->sm_count = prop.multiProcessorCount;
-    p->on_device = true;
-    uint64_t &by = p->device_bytes;
-    auto bail = [&](cudaError_t ce, const char *what) { delete p; return fail_cuda(ce, what); };
-    // row pointers: device-to-device, with the slack the tile copies may read behind the end
-    if ((e = cudaMalloc(&p->d_row_ptr, (M + 1 + 8) * sizeof(uint32_t))) != cudaSuccess) return bail(e, "row pointers");
-    by += (M + 1 + 8) * sizeof(uint32_t);
-    const uint32_t tail[8] = {h.row_ptr[M], h.row_ptr[M], h.row_ptr[M], h.row_ptr[M], h.row_ptr[M], h.row_ptr[M], h.row_ptr[M], h.row_ptr[M]};
-    if ((e = cudaMemcpyAsync(p->d_row_ptr, rowPtr_dev, (M + 1) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(static_cast<uint32_t *>(p->d_row_ptr) + M + 1, tail, sizeof(tail), cudaMemcpyHostToDevice, s)) != cudaSuccess)
-        return bail(e, "row pointers");
-    if ((e = cudaMalloc(&p->d_status, 256)) != cudaSuccess || (e = cudaMemsetAsync(p->d_status, 0, 256, s)) != cudaSuccess)
-        return bail(e, "status word");
-    by += 256;
-    // nonzeros: packed on the device; the second status word collects the column-range check
-    if ((e = cudaMalloc(&p->d_pairs, (h.nnz + 2) * sizeof(Pair))) != cudaSuccess) return bail(e, "packed nonzeros");
-    by += (h.nnz + 2) * sizeof(Pair);
-    e = launch_pack_pairs(cols_dev, vals_dev, p->d_pairs, h.nnz, (uint32_t)K, p->d_status + 1, p->sm_count, s);
-    if (e != cudaSuccess) return bail(e, "packing the nonzeros");
-    {   // largest column of every panel (4 bytes per panel to the host): what the row-block host-buffer call schedules by
-        const uint64_t P = h.num_panels();
-        uint32_t *d_max = nullptr;
-        try {
-            h.panel_max_col.assign(P, 0u);
-        } catch (const std::bad_alloc &) {
-            delete p;
-            return fail(CUTESPMM_ENOMEM, "host allocation failed");
-        }
-        if (P && h.nnz) {
-            if ((e = cudaMalloc(&d_max, P * sizeof(uint32_t))) != cudaSuccess ||
-                (e = launch_panel_max_col(static_cast<const uint32_t *>(p->d_row_ptr), p->d_pairs, (uint32_t)M, (uint32_t)P, d_max, p->sm_count, s)) != cudaSuccess ||
-                (e = cudaMemcpyAsync(h.panel_max_col.data(), d_max, P * sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-                (e = cudaStreamSynchronize(s)) != cudaSuccess) {
-                if (d_max) cudaFree(d_max);
-                return bail(e, "panel column ranges");
-            }
-            cudaFree(d_max);
-        }
-    }
-    // panel analysis and brick packing on the device (paths auto and brick); the per-panel column counts visit the host,
-    // where each panel's kernel is chosen and the brick slots and work lists are laid out
-    uint32_t *d_ncols = nullptr, *d_acols = nullptr, *d_which = nullptr;
-    auto drop_temps = [&]() {
-        for (uint32_t *t : {d_ncols, d_acols, d_which})
-            if (t) cudaFree(t);
-        d_ncols = d_acols = d_which = nullptr;
-    };
-    try {
-        if (h.opts.path != CUTESPMM_PATH_ROWS && h.nnz) {
-            const uint64_t P = h.num_panels();
-            std::vector<uint32_t> ncols(P);
-            if ((e = cudaMalloc(&d_ncols, P * sizeof(uint32_t))) != cudaSuccess || (e = cudaMalloc(&d_acols, h.nnz * sizeof(uint32_t))) != cudaSuccess ||
-                (e = launch_panel_columns(static_cast<const uint32_t *>(p->d_row_ptr), p->d_pairs, (uint32_t)M, (uint32_t)P, d_ncols, d_acols,
-                                          p->sm_count, s)) != cudaSuccess ||
-                (e = cudaMemcpyAsync(ncols.data(), d_ncols, P * sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-                (e = cudaStreamSynchronize(s)) != cudaSuccess) {
-                drop_temps();
-                return bail(e, "panel analysis");
-            }
-            if (h.opts.path == CUTESPMM_PATH_BRICK && std::find(ncols.begin(), ncols.end(), kPanelTooLarge) != ncols.end()) {
-                drop_temps();
-                delete p;
-                return fail(CUTESPMM_EUNSUPPORTED, "path brick on the device: a 16-row panel holds more than " + std::to_string(kDevPanelMax) +
-                                                       " nonzeros; use path auto (such panels run on the row kernel) or the host builder");
-            }
-            finish_device_plan(h, &ncols);
-            if (h.brick_panels) {
-                const uint64_t col_words = h.brick_slots * kBrickCols + 96, rec_words = h.brick_slots * kBrickRecWords;
-                if ((e = cudaMalloc(&p->d_bcols, col_words * 4)) != cudaSuccess || (e = cudaMalloc(&p->d_brecs, rec_words * 4)) != cudaSuccess ||
-                    (e = cudaMemsetAsync(p->d_bcols, 0, col_words * 4, s)) != cudaSuccess || (e = cudaMemsetAsync(p->d_brecs, 0, rec_words * 4, s)) != cudaSuccess ||
-                    (e = cudaMalloc(&d_which, h.brick_panels * sizeof(uint32_t))) != cudaSuccess ||
-                    (e = cudaMemcpyAsync(d_which, h.brick_panel_ids.data(), h.brick_panels * sizeof(uint32_t), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-                    (e = upload(h.panel_first_brick, &p->d_panel_first, by)) != cudaSuccess || (e = upload(h.panel_last_brick, &p->d_panel_last, by)) != cudaSuccess ||
-                    (e = launch_brick_fill(static_cast<const uint32_t *>(p->d_row_ptr), p->d_pairs, (uint32_t)M, d_which,
-                                           static_cast<const uint32_t *>(p->d_panel_first), static_cast<const uint32_t *>(p->d_panel_last),
-                                           (uint32_t)h.brick_panels, d_ncols, d_acols, static_cast<uint32_t *>(p->d_bcols),
-                                           static_cast<uint32_t *>(p->d_brecs), p->sm_count, s)) != cudaSuccess ||
-                    (e = cudaStreamSynchronize(s)) != cudaSuccess) {
-                    drop_temps();
-                    return bail(e, "brick packing");
-                }
-                by += (col_words + rec_words) * 4;
-            }
-            drop_temps();
-        } else {
-            finish_device_plan(h, nullptr);
-        }
-    } catch (const std::bad_alloc &) {
-        drop_temps();
-        delete p;
-        return fail(CUTESPMM_ENOMEM, "host allocation failed while building the plan");
-    }
-    if ((e = upload(h.tiles, &p->d_tiles, by)) != cudaSuccess || (e = upload(h.chunks, &p->d_chunks, by)) != cudaSuccess ||
-        (e = upload(h.long_rows, &p->d_long_rows, by)) != cudaSuccess || (e = upload(h.tiles_all, &p->d_tiles_all, by)) != cudaSuccess ||
-        (e = upload(h.chunks_all, &p->d_chunks_all, by)) != cudaSuccess || (e = upload(h.long_rows_all, &p->d_long_rows_all, by)) != cudaSuccess)
-        return bail(e, "uploading the work lists");
-    const char *what = "";
-    if ((e = reserve_long_row_state(p, by, &what)) != cudaSuccess) return bail(e, what);
-    uint32_t bad = 0;
-    if ((e = cudaMemcpyAsync(&bad, p->d_status + 1, sizeof(bad), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(s)) != cudaSuccess)
-        return bail(e, "packing the nonzeros");
-    if (bad) { delete p; return fail(CUTESPMM_EINVAL, "column index out of range (>= K)"); }
-    *plan = p;
-    return CUTESPMM_OK;
 }
 
 int cutespmm_plan_create_u32(cutespmm_plan_t **plan, uint32_t M, uint32_t K, const uint32_t *rowPtr,
@@ -393,14 +231,25 @@ int cutespmm_plan_info(const cutespmm_plan_t *p, cutespmm_plan_info_t *info)
     std::memset(info, 0, sizeof(*info));
     info->M = h.M; info->K = h.K; info->nnz = h.nnz;
     info->num_panels = h.num_panels();
+    const int st = cutespmm_internal_fetch_views(p, nullptr, nullptr);
+    if (st != CUTESPMM_OK) return st;
     info->num_blocks = h.blocked_row_ptr.empty() ? 0 : h.blocked_row_ptr.back();
-    info->num_tiles = h.tiles.size();
-    info->num_long_rows = h.long_rows.size();
-    info->num_chunks = h.chunks.size();
+    info->num_tiles = p->own.tiles;
+    info->num_long_rows = p->own.long_rows;
+    info->num_chunks = p->own.chunks;
     info->brick_panels = h.brick_panels;
     info->num_bricks = h.num_bricks;
     info->device_bytes = p->device_bytes;
-    info->scratch_bytes_per_col = std::max(h.chunks.size(), h.chunks_all.size()) * sizeof(float);
+    info->scratch_bytes_per_col = std::max(p->own.chunks, p->every.chunks) * sizeof(float);
+    return CUTESPMM_OK;
+}
+
+int cutespmm_plan_dims(const cutespmm_plan_t *p, uint64_t *M, uint64_t *K, uint64_t *nnz)
+{
+    if (!p) return fail(CUTESPMM_EINVAL, "plan is NULL");
+    if (M) *M = p->host.M;
+    if (K) *K = p->host.K;
+    if (nnz) *nnz = p->host.nnz;
     return CUTESPMM_OK;
 }
 
@@ -408,44 +257,37 @@ static const char *kNoViews =
     "this plan was built on the device without the panel analysis (path rows, or a panel beyond the device sort): "
     "the panel views come with path auto / brick, or from the host builder";
 
-static bool device_plan_has_views(const cutespmm_plan *p)
+static int need_views(const cutespmm_plan *p, std::vector<uint32_t> *ncols = nullptr, std::vector<uint32_t> *acols = nullptr)
 {
-    return !p->host.device_built || p->host.blocked_row_ptr.size() == p->host.num_panels() + 1;
+    const int st = cutespmm_internal_fetch_views(p, ncols, acols);
+    if (st != CUTESPMM_OK) return st;
+    if (p->host.device_built && p->host.blocked_row_ptr.size() != p->host.num_panels() + 1) return fail(CUTESPMM_EUNSUPPORTED, kNoViews);
+    return CUTESPMM_OK;
 }
 
 int cutespmm_plan_blocked_row_ptr(const cutespmm_plan_t *p, uint32_t *out)
 {
     if (!p || !out) return fail(CUTESPMM_EINVAL, "null argument");
-    if (!device_plan_has_views(p)) return fail(CUTESPMM_EUNSUPPORTED, kNoViews);
+    const int st = need_views(p);
+    if (st != CUTESPMM_OK) return st;
     std::memcpy(out, p->host.blocked_row_ptr.data(), p->host.blocked_row_ptr.size() * sizeof(uint32_t));
     return CUTESPMM_OK;
 }
 int cutespmm_plan_active_cols(const cutespmm_plan_t *p, uint32_t *out)
 {
     if (!p || !out) return fail(CUTESPMM_EINVAL, "null argument");
-    if (!device_plan_has_views(p)) return fail(CUTESPMM_EUNSUPPORTED, kNoViews);
     const HostPlan &h = p->host;
     if (!h.device_built) {
         std::memcpy(out, h.active_cols.data(), h.active_cols.size() * sizeof(uint32_t));
         return CUTESPMM_OK;
     }
-    // a device-built plan does not keep the column lists: run the panel analysis again and bring them back
+    // a device-built plan does not keep the column lists: run the panel analysis and bring them back
+    std::vector<uint32_t> ncols, acols;
+    int st = need_views(p, &ncols, &acols);
+    if (st == CUTESPMM_OK) st = cutespmm_internal_fetch_lists(p);
+    if (st != CUTESPMM_OK) return st;
     const uint64_t P = h.num_panels();
     if (h.nnz == 0 || P == 0) return CUTESPMM_OK;
-    int cur = -1;
-    cudaGetDevice(&cur);
-    if (cur != p->device) cudaSetDevice(p->device);
-    uint32_t *d_ncols = nullptr, *d_acols = nullptr;
-    std::vector<uint32_t> ncols(P), acols(h.nnz);
-    cudaError_t e;
-    if ((e = cudaMalloc(&d_ncols, P * sizeof(uint32_t))) == cudaSuccess && (e = cudaMalloc(&d_acols, h.nnz * sizeof(uint32_t))) == cudaSuccess &&
-        (e = launch_panel_columns(static_cast<const uint32_t *>(p->d_row_ptr), p->d_pairs, (uint32_t)h.M, (uint32_t)P, d_ncols, d_acols, p->sm_count, nullptr)) == cudaSuccess &&
-        (e = cudaMemcpy(ncols.data(), d_ncols, P * sizeof(uint32_t), cudaMemcpyDeviceToHost)) == cudaSuccess)
-        e = cudaMemcpy(acols.data(), d_acols, h.nnz * sizeof(uint32_t), cudaMemcpyDeviceToHost);
-    if (d_ncols) cudaFree(d_ncols);
-    if (d_acols) cudaFree(d_acols);
-    if (cur != p->device && cur >= 0) cudaSetDevice(cur);
-    if (e != cudaSuccess) return fail_cuda(e, "panel analysis");
     for (uint64_t q = 0; q < P; ++q) {  // per panel: its columns, zero-padded to a multiple of 16 (data.cu:160,204-209)
         uint32_t *dst = out + (uint64_t)h.blocked_row_ptr[q] * kBlockCols;
         const uint32_t width = (h.blocked_row_ptr[q + 1] - h.blocked_row_ptr[q]) * kBlockCols;
@@ -458,6 +300,8 @@ int cutespmm_plan_decode_csr(const cutespmm_plan_t *p, uint64_t *rowPtr, uint32_
 {
     if (!p || !rowPtr || (p->host.nnz && (!cols || !vals))) return fail(CUTESPMM_EINVAL, "null argument");
     if ((p->host.device_built || p->host.values_on_device) && p->on_device) {  // the current pairs live on the device, in CSR order
+        const int st = cutespmm_internal_fetch_lists(p);
+        if (st != CUTESPMM_OK) return st;
         const HostPlan &h = p->host;
         for (uint64_t r = 0; r <= h.M; ++r) rowPtr[r] = h.row_ptr[r];
         std::vector<Pair> pr(h.nnz);
@@ -485,8 +329,8 @@ static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B,
     a.tiles = all_rows ? p->d_tiles_all : p->d_tiles;
     a.chunks = all_rows ? p->d_chunks_all : p->d_chunks;
     a.long_rows = all_rows ? p->d_long_rows_all : p->d_long_rows;
-    a.num_tiles = (uint32_t)(all_rows ? h.tiles_all.size() : h.tiles.size());
-    a.num_chunks = (uint32_t)(all_rows ? h.chunks_all.size() : h.chunks.size());
+    a.num_tiles = all_rows ? p->every.tiles : p->own.tiles;
+    a.num_chunks = all_rows ? p->every.chunks : p->own.chunks;
     a.chunk_owner = static_cast<const uint32_t *>(all_rows ? p->d_chunk_owner_all : p->d_chunk_owner);
     a.arrivals = p->d_arrivals;
     a.split_nnz = h.opts.split_nnz;
@@ -569,13 +413,15 @@ static bool use_brick(const cutespmm_plan *p, const float *B, uint64_t ldb, cons
 
 // Kernels of one column window of width nw (bit 0 row kernel, bit 1 brick kernel, bit 2 slab kernel).  The alignment of
 // the caller's pointers is unknown here: the aligned case is assumed.
-static int window_kernels(const HostPlan &h, uint32_t nw)
+static int window_kernels(const cutespmm_plan *p, uint32_t nw)
 {
+    const HostPlan &h = p->host;
     const bool brick = brick_wanted(h, nw) && nw % 32 == 0;
     const bool slab = h.slab_panels && nw % 128 == 0;
     const bool all_rows = (!brick && h.num_bricks) || (!slab && h.slab_panels);
     int mask = (brick ? 2 : 0) | (slab ? 4 : 0);
-    if (all_rows ? (!h.tiles_all.empty() || !h.chunks_all.empty()) : (!h.tiles.empty() || !h.chunks.empty())) mask |= 1;
+    const cutespmm_list_sizes &rows = all_rows ? p->every : p->own;
+    if (rows.tiles || rows.chunks) mask |= 1;
     return mask;
 }
 
@@ -583,7 +429,7 @@ int cutespmm_spmm_kernels(const cutespmm_plan_t *p, uint32_t N)
 {
     if (!p || N == 0 || p->host.M == 0) return 0;
     int mask = 0;
-    for (uint32_t n0 = 0; n0 < N; n0 += kScratchCols) mask |= window_kernels(p->host, N - n0 < kScratchCols ? N - n0 : kScratchCols);
+    for (uint32_t n0 = 0; n0 < N; n0 += kScratchCols) mask |= window_kernels(p, N - n0 < kScratchCols ? N - n0 : kScratchCols);
     return mask;
 }
 
@@ -592,7 +438,7 @@ int cutespmm_spmm_launch_count(const cutespmm_plan_t *p, uint32_t N)
     if (!p || N == 0 || p->host.M == 0) return 0;
     int total = 0;
     for (uint32_t n0 = 0; n0 < N; n0 += kScratchCols) {
-        const int mask = window_kernels(p->host, N - n0 < kScratchCols ? N - n0 : kScratchCols);
+        const int mask = window_kernels(p, N - n0 < kScratchCols ? N - n0 : kScratchCols);
         total += (mask & 1) + ((mask >> 1) & 1) + ((mask >> 2) & 1);
     }
     return total;
@@ -605,6 +451,12 @@ int cutespmm_spmm(const cutespmm_plan_t *p, const float *B, uint64_t ldb, float 
 }
 
 }  // extern "C"
+
+// A plan that ran on another stream than the default one is dropped with a wait for the device (its memory may be in use there).
+static void note_stream(const cutespmm_plan *p, cudaStream_t s)
+{
+    if (s != nullptr && s != cudaStreamLegacy && !p->used_elsewhere.load(std::memory_order_relaxed)) p->used_elsewhere = true;
+}
 
 int cutespmm_internal_spmm_range(const cutespmm_plan *p, const float *B, uint64_t ldb, float *C, uint64_t ldc, uint32_t N, void *stream,
                                  const cutespmm_item_range *rg)
@@ -623,6 +475,7 @@ int cutespmm_internal_spmm_range(const cutespmm_plan *p, const float *B, uint64_
     if (cudaGetDevice(&cur) != cudaSuccess || cur != p->device)
         return fail(CUTESPMM_EINVAL, "the current CUDA device (" + std::to_string(cur) + ") is not the one the plan was created on (" +
                                          std::to_string(p->device) + "): call cudaSetDevice first");
+    note_stream(p, s);
     for (uint32_t n0 = 0; n0 < N; n0 += kScratchCols) {
         const uint32_t nw = N - n0 < kScratchCols ? N - n0 : kScratchCols;
         cudaError_t e;
@@ -664,6 +517,7 @@ int cutespmm_sddmm(const cutespmm_plan_t *p, const float *X, uint64_t ldx, const
     if (cudaGetDevice(&cur) != cudaSuccess || cur != p->device)
         return fail(CUTESPMM_EINVAL, "the current CUDA device is not the one the plan was created on");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    note_stream(p, s);
     if (N == 0) {  // an empty sum
         cudaError_t e = cudaMemsetAsync(out, 0, h.nnz * sizeof(float), s);
         return e == cudaSuccess ? CUTESPMM_OK : fail_cuda(e, "cudaMemsetAsync");
@@ -674,8 +528,8 @@ int cutespmm_sddmm(const cutespmm_plan_t *p, const float *X, uint64_t ldx, const
     a.pairs = p->d_pairs;
     a.tiles = all ? p->d_tiles_all : p->d_tiles;
     a.chunks = all ? p->d_chunks_all : p->d_chunks;
-    a.num_tiles = (uint32_t)(all ? h.tiles_all.size() : h.tiles.size());
-    a.num_chunks = (uint32_t)(all ? h.chunks_all.size() : h.chunks.size());
+    a.num_tiles = all ? p->every.tiles : p->own.tiles;
+    a.num_chunks = all ? p->every.chunks : p->own.chunks;
     a.X = X; a.Y = Y; a.ldx = ldx; a.ldy = ldy; a.out = out; a.N = N;
     a.scale = scale_by_values ? 1u : 0u;
     a.status = p->d_status;
@@ -698,6 +552,7 @@ int cutespmm_plan_set_values(cutespmm_plan_t *p, const float *vals_dev, void *st
     int cur = -1;
     if (cudaGetDevice(&cur) != cudaSuccess || cur != p->device)
         return fail(CUTESPMM_EINVAL, "the current CUDA device is not the one the plan was created on");
+    note_stream(p, static_cast<cudaStream_t>(stream));
     const cudaError_t e = launch_set_values(p->d_pairs, vals_dev, h.nnz, p->sm_count, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail_cuda(e, "replacing the values");
     p->host.values_on_device = true;

@@ -101,21 +101,67 @@ struct SlabArgs {
 cudaError_t launch_slab(const SlabArgs &a, int sm_count, cudaStream_t s);
 bool slab_supports(uint32_t N, uint64_t ldb, uint64_t ldc, const void *B, const void *C);
 
-// pairs[j] = (cols[j], bits of vals[j]) for j < nnz, two zero pairs behind; *bad |= 1 when a column is >= K
-cudaError_t launch_pack_pairs(const uint32_t *cols, const float *vals, void *pairs, uint64_t nnz, uint32_t K, uint32_t *bad, int sm_count,
-                              cudaStream_t s);
-// Device side of the panel analysis and of the brick packing (device_build.cu).  kDevPanelMax: nonzeros of a panel the
-// shared-memory sort takes (32 KB of column indices); 16 rows of at most kMaxSplitNnz nonzeros fit, so every panel
-// left out holds a long row and runs on the row kernel whatever its density.
-constexpr uint32_t kDevPanelMax = 8192;
+// ---- device side of plan creation (device_build.cu; device_plan.cu runs it) ----
+struct Tile;
+struct Chunk;
+struct LongRow;
+constexpr uint32_t kRowPtrSlack = 8;  // row pointers repeated behind the last one: a tile's copy starts and ends on 16-byte boundaries
+// kDevPanelMax: nonzeros of a panel the shared-memory sort (and the largest hash set) takes.  kMaxCensusNnz: the same for
+// the census of path auto, which looks at panels without long rows only: 16 rows of at most kMaxSplitNnz nonzeros.
+constexpr uint32_t kDevPanelMax = 8192, kMaxCensusNnz = 6144;
+
+constexpr uint32_t kTileSegmentRows = 2048;  // rows a block of the list kernels looks at; a multiple of kPanelRows
+constexpr uint32_t kSegmentEntries = 257;    // kMaxTileRows + 1: rows of a segment its first tile can start at
+
+struct BuildTotals {  // one per plan creation, read by the host after the counting kernels
+    uint32_t nnz, bad_rows, bad_cols, too_large;
+    uint32_t tiles;
+    uint32_t chunks, long_rows, brick_panels, brick_slots;  // in the order of the per-segment counters
+    uint32_t brick_nnz_max, brick_cols_max, pad;
+    unsigned long long bricks, brick_cost;
+};
+struct ListArgs {
+    uint32_t M, num_segments;
+    uint32_t split_nnz, tile_nnz, adaptive;
+    uint32_t total_known;   // 1: `total` is the cost of the listed rows; 0: every row is listed, nnz + kRowCost * M
+    uint64_t total;
+    const uint8_t *path;    // per panel: 1 = not listed (nullptr: every row is)
+    uint16_t *exits, *tile_counts;  // per segment and entry row: entry row of the next segment, tiles
+    uint32_t *seg_entry, *seg_tiles;   // per segment: the entry row, its first tile
+    uint32_t *seg_chunks, *seg_longs;  // per segment: counts, then offsets
+    BuildTotals *totals;
+    Tile *tiles;
+    Chunk *chunks;
+    LongRow *long_rows;
+    uint32_t *owners;
+};
+struct CensusArgs {
+    uint32_t M, num_panels;
+    uint32_t force;         // 1: path brick, every panel that fits
+    uint32_t split_nnz;
+    float density;
+    uint32_t most, table_words;
+    uint32_t *ncols;        // per panel: distinct columns (of candidates)
+    uint8_t *path;          // per panel: 1 = brick
+    uint32_t *seg_panels, *seg_slots;
+    BuildTotals *totals;
+};
+cudaError_t launch_lists_count(const uint32_t *row_ptr, const ListArgs &a, cudaStream_t s);
+cudaError_t launch_lists_scan(const uint32_t *row_ptr, const ListArgs &a, uint32_t *counters, uint32_t how_many, cudaStream_t s);
+cudaError_t launch_lists_write(const uint32_t *row_ptr, const ListArgs &a, cudaStream_t s);
+cudaError_t launch_panel_census(const uint32_t *row_ptr, const uint32_t *cols, CensusArgs a, int sm_count, cudaStream_t s);
+cudaError_t launch_brick_layout(uint32_t num_panels, const uint8_t *path, const uint32_t *ncols, const uint32_t *seg_panels, const uint32_t *seg_slots,
+                                uint32_t num_segments, uint32_t *ids, uint32_t *first, uint32_t *last, cudaStream_t s);
+cudaError_t launch_brick_fill(const uint32_t *row_ptr, const void *pairs, uint32_t M, const uint32_t *ids, const uint32_t *first_slot,
+                              uint32_t num_brick_panels, const uint32_t *ncols, uint32_t nnz_max, uint32_t cols_max, uint32_t *bcols, uint32_t *brecs,
+                              int sm_count, cudaStream_t s);
+cudaError_t launch_pack(const uint32_t *row_ptr, const uint32_t *cols, const float *vals, uint32_t M, uint32_t K, uint32_t nnz, uint32_t *row_ptr_out,
+                        void *pairs, uint32_t *bad, int sm_count, cudaStream_t s);
 cudaError_t launch_set_values(void *pairs, const float *vals, uint64_t nnz, int sm_count, cudaStream_t s);
+// the panel views (distinct columns per panel, ascending) and column ranges, when somebody asks for them
 cudaError_t launch_panel_columns(const uint32_t *row_ptr, const void *pairs, uint32_t M, uint32_t num_panels, uint32_t *ncols,
                                  uint32_t *acols, int sm_count, cudaStream_t s);
 cudaError_t launch_panel_max_col(const uint32_t *row_ptr, const void *pairs, uint32_t M, uint32_t num_panels, uint32_t *maxcol, int sm_count,
                                  cudaStream_t s);
-cudaError_t launch_brick_fill(const uint32_t *row_ptr, const void *pairs, uint32_t M, const uint32_t *which,
-                              const uint32_t *first_slot, const uint32_t *last_slot, uint32_t num_brick_panels, const uint32_t *ncols,
-                              const uint32_t *acols, uint32_t *bcols, uint32_t *brecs, int sm_count, cudaStream_t s);
-
 
 }  // namespace cutespmm

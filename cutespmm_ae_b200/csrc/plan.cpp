@@ -93,42 +93,20 @@ static std::vector<uint32_t> analyze_panels(HostPlan &p)
 
 // Cuts the rows that the row kernel executes into tiles of about equal cost (nonzeros + kRowCost per
 // row).  A tile is a run of consecutive rows inside one stretch of row-kernel panels, bounded so that
-// its row pointers and pairs fit the kernel's shared-memory stage.  A long row ends the running
+// its row pointers and pairs fit the kernel's shared-memory stage (device_build.cu cuts the same tiles in parallel).  A
+// long row ends the running
 // tile and is not part of any: its nonzeros are executed as chunks.
 static void build_tiles(const HostPlan &p, bool all_rows, std::vector<Tile> &tiles, std::vector<Chunk> &chunks,
                         std::vector<LongRow> &long_rows)
 {
     const uint64_t P = p.num_panels();
-    uint32_t split = p.opts.split_nnz;
-    uint64_t target = p.opts.tile_nnz;
-    bool latency_bound = false;
-    if (p.adaptive_tiling) {
-        // The default sizes (tiles of cost 512, chunks of 256 nonzeros) keep the per-item overhead small when the grid is
-        // many waves long.  A small job is a handful of memory latencies long, and then the longest chain of dependent
-        // gathers of one warp IS the run time: a 256-nonzero chunk is 64 steps of four loads, about 30 us, when the
-        // rest of a 200 000-nonzero matrix is done in 10.  So the work is cut finer the smaller the job: tiles so that
-        // one resident wave of blocks holds them all, rows cut from a shorter length on (not below 128: a piece costs
-        // about eight latencies of its own -- descriptor, pairs, arrival count, the sum -- so shorter rows are quicker
-        // whole), and a cut row into pieces of about sqrt(length / 2) nonzeros: the chain is a piece's gathers followed
-        // by the sum of the pieces, the sum runs a few slots per step, and that length makes the two about equal.
-        uint64_t total = 0;
-        for (uint64_t q = 0; q < P; ++q) {
-            if (!all_rows && p.row_path[q]) continue;
-            const uint64_t r0 = q * kPanelRows, r1 = std::min<uint64_t>(p.M, r0 + kPanelRows);
-            total += (p.row_ptr[r1] - p.row_ptr[r0]) + (r1 - r0) * kRowCost;
-        }
-        if (total / kResidentTiles <= kMaxAdaptiveTileCost) target = std::max<uint64_t>(kMinAdaptiveTileCost, total / kResidentTiles);
-        if (total / kAdaptiveSplitDivisor < split) {
-            latency_bound = true;
-            split = (uint32_t)std::max<uint64_t>(kMinAdaptiveSplitNnz, total / kAdaptiveSplitDivisor);
-        }
+    uint64_t total = 0;
+    for (uint64_t q = 0; q < P; ++q) {
+        if (!all_rows && p.row_path[q]) continue;
+        const uint64_t r0 = q * kPanelRows, r1 = std::min<uint64_t>(p.M, r0 + kPanelRows);
+        total += (p.row_ptr[r1] - p.row_ptr[r0]) + (r1 - r0) * kRowCost;
     }
-    auto piece_of = [&](uint32_t len) {  // nonzeros per chunk of a row of `len` nonzeros that is being cut
-        if (!latency_bound) return split;
-        uint32_t s = 1;
-        while ((uint64_t)s * s * 2 < len) ++s;  // ceil(sqrt(len / 2)): a latency-bound job has fewer than 2.1 M nonzeros, about 1 000 steps at most
-        return std::min(split, std::max(kMinChunkNnz, s));
-    };
+    const ItemSizes sizes = item_sizes(total, p.opts.split_nnz, p.opts.tile_nnz, p.adaptive_tiling);
     tiles.clear();
     chunks.clear();
     long_rows.clear();
@@ -147,11 +125,11 @@ static void build_tiles(const HostPlan &p, bool all_rows, std::vector<Tile> &til
         };
         for (; r < r_end; ++r) {
             const uint32_t len = p.row_ptr[r + 1] - p.row_ptr[r];
-            if (len > split) {
+            if (len > sizes.split) {
                 close(r);
                 begin = r + 1;
                 LongRow lr{p.row_map.empty() ? (uint32_t)r : p.row_map[r], (uint32_t)chunks.size(), 0, 0};  // the row of C the sum goes to
-                const uint32_t piece = piece_of(len);
+                const uint32_t piece = piece_length(sizes, len);
                 for (uint32_t j = p.row_ptr[r]; j < p.row_ptr[r + 1]; j += piece)
                     chunks.push_back(Chunk{(uint32_t)r, j, std::min<uint32_t>(j + piece, p.row_ptr[r + 1]),
                                            (uint32_t)chunks.size()});
@@ -164,7 +142,7 @@ static void build_tiles(const HostPlan &p, bool all_rows, std::vector<Tile> &til
                 begin = r;
             }
             cost += len + kRowCost;
-            if (cost >= target) {
+            if (cost >= sizes.target) {
                 close(r + 1);
                 begin = r + 1;
             }
@@ -342,12 +320,9 @@ void choose_panel_paths(HostPlan &p, const std::vector<uint32_t> &panel_ncols)
     }
 }
 
-int build_rows_plan_from_row_ptr(HostPlan &p, uint64_t M, uint64_t K, std::vector<uint32_t> &&row_ptr,
-                                 const cutespmm_options_t *opts, std::string &err)
+int check_device_options(HostPlan &p, uint64_t M, uint64_t K, const cutespmm_options_t *opts, std::string &err)
 {
     if (M >= (1ull << 32) - kPanelRows || K >= (1ull << 32)) { err = "M and K must be below 2^32"; return CUTESPMM_EUNSUPPORTED; }
-    if (row_ptr.size() != M + 1) { err = "rowPtr must have M+1 entries"; return CUTESPMM_EINVAL; }
-    if (row_ptr[0] != 0) { err = "rowPtr[0] must be 0"; return CUTESPMM_EINVAL; }
     if (opts && opts->path == CUTESPMM_PATH_SLAB) {
         err = "the slab path is built by the host builder only (cutespmm_plan_create)";
         return CUTESPMM_EUNSUPPORTED;
@@ -355,36 +330,9 @@ int build_rows_plan_from_row_ptr(HostPlan &p, uint64_t M, uint64_t K, std::vecto
     if (opts && opts->path > CUTESPMM_PATH_SLAB) { err = "unknown path"; return CUTESPMM_EINVAL; }
     p.adaptive_tiling = fill_default_options(p.opts, opts);
     if (p.opts.reorder) { err = "row reordering is done by the host builder only (cutespmm_plan_create)"; return CUTESPMM_EUNSUPPORTED; }
-    int bad = 0;
-#pragma omp parallel for schedule(static) reduction(| : bad)
-    for (int64_t r = 0; r < (int64_t)M; ++r) bad |= row_ptr[r + 1] < row_ptr[r];
-    if (bad) { err = "rowPtr is not non-decreasing"; return CUTESPMM_EINVAL; }
-    p.M = M; p.K = K; p.nnz = row_ptr[M];
-    p.row_ptr = std::move(row_ptr);
+    p.M = M; p.K = K;
     p.device_built = true;
-    p.row_path.assign(p.num_panels(), 0);
-    p.slab_path.assign((M + kSlabRows - 1) / kSlabRows, 0);
     return CUTESPMM_OK;
-}
-
-void finish_device_plan(HostPlan &p, const std::vector<uint32_t> *panel_ncols)
-{
-    if (panel_ncols) {
-        choose_panel_paths(p, *panel_ncols);
-        // the HRPB view blockedRowPtr follows from the counts -- unless a panel was left out of the analysis
-        bool complete = true;
-        p.blocked_row_ptr.assign(p.num_panels() + 1, 0);
-        for (uint64_t q = 0; q < p.num_panels(); ++q) {
-            complete &= (*panel_ncols)[q] != kPanelTooLarge;
-            p.blocked_row_ptr[q + 1] = p.blocked_row_ptr[q] + (complete ? ((*panel_ncols)[q] + kBlockCols - 1) / kBlockCols : 0);
-        }
-        if (!complete) p.blocked_row_ptr.clear();
-        std::vector<uint32_t> which;
-        layout_brick_slots(p, *panel_ncols, which);
-        p.brick_panel_ids = std::move(which);
-    }
-    build_tiles(p, false, p.tiles, p.chunks, p.long_rows);
-    if (p.brick_panels) build_tiles(p, true, p.tiles_all, p.chunks_all, p.long_rows_all);
 }
 
 int build_host_plan(HostPlan &p, uint64_t M, uint64_t K, const uint64_t *rowPtr, const uint32_t *cols,

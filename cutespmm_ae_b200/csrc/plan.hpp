@@ -8,6 +8,12 @@
 
 #include "../../include/cutespmm.h"
 
+#ifdef __CUDACC__
+#define CUTESPMM_HD __host__ __device__
+#else
+#define CUTESPMM_HD
+#endif
+
 namespace cutespmm {
 
 constexpr uint32_t kPanelRows = 16;   // row-panel height; HRPB's TM (inc.h:18-20)
@@ -40,6 +46,47 @@ struct Pair {
 struct Tile {
     uint32_t row_begin, row_end, pair_begin, pair_end;
 };
+
+// Sizes of the row kernel's work items for a list whose rows cost `total` (nonzeros + kRowCost per row): used as they
+// are by the host builder and by the device builder's kernels.
+//
+// The default sizes (tiles of cost 512, chunks of 256 nonzeros) keep the per-item overhead small when the grid is
+// many waves long.  A small job is a handful of memory latencies long, and then the longest chain of dependent
+// gathers of one warp IS the run time: a 256-nonzero chunk is 64 steps of four loads, about 30 us, when the
+// rest of a 200 000-nonzero matrix is done in 10.  So the work is cut finer the smaller the job: tiles so that
+// one resident wave of blocks holds them all, rows cut from a shorter length on (not below 128: a piece costs
+// about eight latencies of its own -- descriptor, pairs, arrival count, the sum -- so shorter rows are quicker
+// whole), and a cut row into pieces of about sqrt(length / 2) nonzeros: the chain is a piece's gathers followed
+// by the sum of the pieces, the sum runs a few slots per step, and that length makes the two about equal.
+struct ItemSizes {
+    uint32_t split;      // rows longer than this are cut into chunks
+    uint32_t target;     // cost at which a tile is closed
+    bool latency_bound;  // pieces of sqrt(length / 2)
+};
+CUTESPMM_HD inline ItemSizes item_sizes(uint64_t total, uint32_t split_nnz, uint32_t tile_nnz, bool adaptive)
+{
+    ItemSizes s{split_nnz, tile_nnz, false};
+    if (!adaptive) return s;
+    if (total / kResidentTiles <= kMaxAdaptiveTileCost) {
+        const uint64_t t = total / kResidentTiles;
+        s.target = (uint32_t)(t > kMinAdaptiveTileCost ? t : kMinAdaptiveTileCost);
+    }
+    if (total / kAdaptiveSplitDivisor < s.split) {
+        s.latency_bound = true;
+        const uint64_t t = total / kAdaptiveSplitDivisor;
+        s.split = (uint32_t)(t > kMinAdaptiveSplitNnz ? t : kMinAdaptiveSplitNnz);
+    }
+    return s;
+}
+// nonzeros per chunk of a row of `len` nonzeros that is being cut
+CUTESPMM_HD inline uint32_t piece_length(const ItemSizes &s, uint32_t len)
+{
+    if (!s.latency_bound) return s.split;
+    uint32_t r = 1;
+    while ((uint64_t)r * r * 2 < len) ++r;  // ceil(sqrt(len / 2)): a latency-bound job has fewer than 2.1 M nonzeros, about 1 000 steps at most
+    if (r < kMinChunkNnz) r = kMinChunkNnz;
+    return r < s.split ? r : s.split;
+}
 
 constexpr uint32_t kMinBrickPanels = 4440;  // path auto: fewer dense panels than two per warp of a full brick grid go to the row kernel
 constexpr uint32_t kPanelTooLarge = 0xffffffffu;  // column count of a panel the device builder did not analyse
@@ -147,16 +194,8 @@ struct HostPlan {
 int build_host_plan(HostPlan &p, uint64_t M, uint64_t K, const uint64_t *rowPtr, const uint32_t *cols,
                     const float *vals, const cutespmm_options_t *opts, std::string &err);
 
-// The row-kernel part of a plan from the row pointers alone (tiles, chunks of long rows, fix-up list): what a plan
-// needs on the host when the nonzeros themselves stay on the device.  p.pairs stays empty and p.device_built is
-// set: the HRPB views and the host-side decode are not available for such a plan.
-int build_rows_plan_from_row_ptr(HostPlan &p, uint64_t M, uint64_t K, std::vector<uint32_t> &&row_ptr,
-                                 const cutespmm_options_t *opts, std::string &err);
-
-// Second half of a device-built plan: with the per-panel distinct-column counts (nullptr: row kernel only) chooses
-// each panel's kernel, lays out the brick slots and cuts the work lists.
-void finish_device_plan(HostPlan &p, const std::vector<uint32_t> *panel_ncols);
-void choose_panel_paths(HostPlan &p, const std::vector<uint32_t> &panel_ncols);
+// The options of a plan that is built on the device, checked and with the defaults filled in (p.opts, p.adaptive_tiling).
+int check_device_options(HostPlan &p, uint64_t M, uint64_t K, const cutespmm_options_t *opts, std::string &err);
 
 // Rebuilds CSR from the packed arrays (rows-kernel part from pairs, brick part from maps + values).
 void decode_host_plan(const HostPlan &p, uint64_t *rowPtr, uint32_t *cols, float *vals);

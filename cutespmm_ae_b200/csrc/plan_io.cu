@@ -80,6 +80,9 @@ extern "C" {
 int cutespmm_plan_save(const cutespmm_plan_t *plan, const char *path)
 {
     if (!plan || !path) return fail_status(CUTESPMM_EINVAL, "null argument");
+    int st = cutespmm_internal_fetch_views(plan, nullptr, nullptr);
+    if (st == CUTESPMM_OK) st = cutespmm_internal_fetch_lists(plan);
+    if (st != CUTESPMM_OK) return st;
     HostPlan h;  // a copy: a device-built plan gets its device-only arrays filled in below
     try {
         h = plan->host;
@@ -199,6 +202,7 @@ int cutespmm_plan_load(cutespmm_plan_t **plan, const char *path, int host_only)
         delete p;
         return fail_status(CUTESPMM_EIO, std::string(path) + ": inconsistent plan");
     }
+    p->note_list_sizes();
     if (!host_only) {
         const int st = cutespmm_internal_upload_plan(p);
         if (st != CUTESPMM_OK) {

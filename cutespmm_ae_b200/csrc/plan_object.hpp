@@ -3,7 +3,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -24,8 +26,22 @@ struct cutespmm_row_block {
     cutespmm_item_range items;
 };
 
+// How long the row kernel's lists are (the lists themselves may be on the device only).
+struct cutespmm_list_sizes {
+    uint32_t tiles = 0, chunks = 0, long_rows = 0;
+};
+
+// Gives the memory of a device-built plan back.  device_plan.cu
+void cutespmm_internal_free_block(void *block, bool used_elsewhere);
+
 struct cutespmm_plan {
     cutespmm::HostPlan host;
+    cutespmm_list_sizes own, every;  // of the list of the rows outside the tensor-core panels / of the list of every row
+    // device-built plans: one block holds every array; the lists come to the host on demand
+    void *d_block = nullptr;
+    bool lists_on_host = true, views_tried = false;
+    std::mutex fetch_mutex;
+    mutable std::atomic<bool> used_elsewhere{false};  // ran on a stream that is not the default stream
     bool on_device = false;
     int device = -1;
     int sm_count = 0;
@@ -33,7 +49,7 @@ struct cutespmm_plan {
     // device arrays
     void *d_row_ptr = nullptr, *d_pairs = nullptr, *d_tiles = nullptr, *d_chunks = nullptr, *d_long_rows = nullptr;
     void *d_tiles_all = nullptr, *d_chunks_all = nullptr, *d_long_rows_all = nullptr;
-    void *d_bcols = nullptr, *d_brecs = nullptr, *d_panel_first = nullptr, *d_panel_last = nullptr;
+    void *d_bcols = nullptr, *d_brecs = nullptr, *d_panel_first = nullptr, *d_panel_last = nullptr, *d_panel_ids = nullptr;
     void *d_scols = nullptr, *d_srecs = nullptr, *d_srec_off = nullptr, *d_sfirst = nullptr, *d_slast = nullptr, *d_sids = nullptr;
     void *d_row_map = nullptr;
     void *d_chunk_owner = nullptr, *d_chunk_owner_all = nullptr;  // per scratch slot: its long row
@@ -57,15 +73,25 @@ struct cutespmm_plan {
     uint32_t row_blocks_n = 0;                   // the N they were cut for
     cudaEvent_t rb_in[kMaxRowBlocks] = {}, rb_k0[kMaxRowBlocks] = {}, rb_k1[kMaxRowBlocks] = {};
 
+    void note_list_sizes()  // from the lists on the host
+    {
+        own = {(uint32_t)host.tiles.size(), (uint32_t)host.chunks.size(), (uint32_t)host.long_rows.size()};
+        every = {(uint32_t)host.tiles_all.size(), (uint32_t)host.chunks_all.size(), (uint32_t)host.long_rows_all.size()};
+    }
+
     ~cutespmm_plan()
     {
         if (!on_device) return;
         int cur = -1;
         cudaGetDevice(&cur);
         if (cur != device) cudaSetDevice(device);
-        for (void *p : {d_row_ptr, d_pairs, d_tiles, d_chunks, d_long_rows, d_tiles_all, d_chunks_all, d_long_rows_all,
-                        d_bcols, d_brecs, d_panel_first, d_panel_last, d_scols, d_srecs, d_srec_off, d_sfirst,
-                        d_slast, d_sids, d_row_map, d_chunk_owner, d_chunk_owner_all, (void *)d_arrivals, (void *)d_scratch, (void *)d_status, (void *)d_B, (void *)d_C})
+        if (d_block) cutespmm_internal_free_block(d_block, used_elsewhere);
+        else if (!host.device_built || lists_on_host)
+            for (void *p : {d_row_ptr, d_pairs, d_tiles, d_chunks, d_long_rows, d_tiles_all, d_chunks_all, d_long_rows_all,
+                            d_bcols, d_brecs, d_panel_first, d_panel_last, d_scols, d_srecs, d_srec_off, d_sfirst,
+                            d_slast, d_sids, d_row_map, d_chunk_owner, d_chunk_owner_all, (void *)d_arrivals, (void *)d_scratch, (void *)d_status})
+                if (p) cudaFree(p);
+        for (void *p : {(void *)d_B, (void *)d_C})
             if (p) cudaFree(p);
         for (cudaEvent_t ev : {ev_entry, ev_done})
             if (ev) cudaEventDestroy(ev);
@@ -87,6 +113,11 @@ namespace cutespmm {
 int fail_status(int status, const std::string &msg);          // records the message, returns status
 int fail_cuda_status(cudaError_t e, const char *what);        // same for a CUDA error
 }  // namespace cutespmm
+
+// device_plan.cu
+int cutespmm_internal_usable_device(int *dev, int *sm_count);
+int cutespmm_internal_fetch_lists(const cutespmm_plan *p);
+int cutespmm_internal_fetch_views(const cutespmm_plan *p, std::vector<uint32_t> *ncols, std::vector<uint32_t> *acols);
 
 // cutespmm_spmm restricted to a range of work items (nullptr: everything).  capi.cu
 int cutespmm_internal_spmm_range(const cutespmm_plan *p, const float *B, uint64_t ldb, float *C, uint64_t ldc, uint32_t N, void *stream,

@@ -245,6 +245,7 @@ bool cut_row_blocks(cutespmm_plan *p, uint32_t N)
 {
     const HostPlan &h = p->host;
     p->row_blocks.clear();
+    if (h.M >= 4096 && cutespmm_internal_fetch_lists(p) != CUTESPMM_OK) return false;
     if (!h.row_map.empty() || h.slab_panels || h.panel_max_col.size() != h.num_panels() || h.M < 4096) return false;
     const uint64_t c_bytes = h.M * (uint64_t)N * sizeof(float);
     // blocks of about 16 MiB of C: every block costs about 40 us of hand-over between the copy engines and its kernel

@@ -137,13 +137,14 @@ int cutespmm_plan_build_host(cutespmm_plan_t **plan, uint64_t M, uint64_t K, con
                              const uint32_t *cols, const float *vals, const cutespmm_options_t *opts);
 
 /* A plan for a matrix that already lives on the device (rowPtr: M+1 x u32, cols: nnz x u32, vals: nnz x f32, all
- * device pointers): the nonzeros are packed by a kernel and never visit the host; only the row pointers do, because
- * the work lists are cut from them.  The reference preprocesses on the host only (data.cu:80-335) and its caller
- * uploads the result (data.cu:318-333); this is the entry point for a caller that has no host copy.  The plan runs
- * on the row kernel (opts->path auto or rows; brick and slab need the host builder's column analysis and are refused
- * with CUTESPMM_EUNSUPPORTED); rows need not be sorted.  The panel views (blocked_row_ptr, active_cols) are not
- * available for such a plan; plan_decode_csr reads the packed nonzeros back.  Work is queued on `stream`, which is
- * synchronised before the call returns (the column-range check is read back). */
+ * device pointers): work lists, panel analysis, bricks and packed nonzeros are all made by kernels; the host reads
+ * sizes only.  The reference preprocesses on the host only (data.cu:80-335) and its caller uploads the result
+ * (data.cu:318-333); this is the entry point for a caller that has no host copy, or whose matrix changes from step to
+ * step.  opts->path auto, rows or brick (the slab path needs the host builder: CUTESPMM_EUNSUPPORTED); rows need not be
+ * sorted.  The panel views (blocked_row_ptr, active_cols) are computed when asked for (not for path rows, nor when a panel
+ * holds more than 8192 nonzeros); plan_decode_csr reads the packed nonzeros back.  Work is queued on `stream`, which is
+ * synchronised before the call returns.  The plan's memory comes from a stream-ordered pool of the library's own, which
+ * keeps up to 512 MiB per device for the next such plan (cutespmm_release_memory gives that back). */
 int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M, uint64_t K, const uint32_t *rowPtr_dev,
                                 const uint32_t *cols_dev, const float *vals_dev, const cutespmm_options_t *opts,
                                 void *stream);
@@ -156,6 +157,10 @@ int cutespmm_plan_save(const cutespmm_plan_t *plan, const char *path);
 int cutespmm_plan_load(cutespmm_plan_t **plan, const char *path, int host_only);
 
 int cutespmm_plan_destroy(cutespmm_plan_t *plan);
+/* Returns the device memory the library keeps for future plans to the driver (all devices). */
+int cutespmm_release_memory(void);
+/* The matrix's sizes alone (any pointer may be NULL): cutespmm_plan_info may have to run the panel analysis first. */
+int cutespmm_plan_dims(const cutespmm_plan_t *plan, uint64_t *M, uint64_t *K, uint64_t *nnz);
 int cutespmm_plan_info(const cutespmm_plan_t *plan, cutespmm_plan_info_t *info);
 
 /* HRPB::blockedRowPtr (data.cu:65,145,176-185): prefix sum over 16-row panels of

@@ -159,3 +159,48 @@ def test_saved_plan_gives_the_same_product_after_loading(tmp_path, how):
     assert torch.equal(C0, C1)
     for a, b in zip(p.decode_csr(), q.decode_csr()):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("M,lengths,path,min_bricks", [
+    (2047, "short", cs.PATH_ROWS, 0), (2048, "short", cs.PATH_ROWS, 0), (2049, "short", cs.PATH_ROWS, 0),   # edges of a segment of rows
+    (4096 + 17, "empty", cs.PATH_ROWS, 0),     # 256-row tiles that reach into the next segment, runs of empty rows
+    (6000, "long", cs.PATH_ROWS, 0),           # long rows on both sides of every segment edge, next to each other
+    (2048 * 33 + 5, "short", cs.PATH_ROWS, 0),  # more segments than one batch of the walk through them
+    (5000, "mixed", cs.PATH_AUTO, 1),          # tensor-core panels between row-kernel panels, duplicates inside
+])
+def test_device_cut_work_lists_equal_the_host_builder_s(oracle_mod, M, lengths, path, min_bricks):
+    rng = np.random.default_rng(M)
+    K = 700
+    ln = rng.integers(0, 6, M)
+    if lengths == "empty":
+        ln[rng.random(M) < 0.9] = 0
+        ln[1000:3000] = 0
+    if lengths == "long":
+        for at in (0, 1, 2046, 2047, 2048, 2049, 4095, 4096, M - 1):
+            ln[at] = 300 + at % 7
+    rp = np.concatenate([[0], np.cumsum(ln)])
+    cols = rng.integers(0, K, rp[-1])
+    if lengths == "mixed":  # every third group of 16 rows names the same eight columns, some of them twice
+        rows = np.repeat(np.arange(M), ln)
+        dense = (rows // 16) % 3 == 0
+        cols[dense] = cols[dense] % 8
+    A = g.CsrMatrix(M, K, torch.from_numpy(rp), torch.from_numpy(cols.astype(np.int32)), torch.from_numpy(rng.standard_normal(rp[-1]).astype(np.float32)))
+    order = np.lexsort((np.arange(rp[-1]), cols, np.repeat(np.arange(M), ln)))  # the host builder sorts rows: give both the sorted order
+    A.cols, A.vals = A.cols[order].contiguous(), A.vals[order].contiguous()
+    kw = dict(path=path, min_brick_panels=min_bricks)
+    pd, ph = cs.Plan.from_device_csr(A.M, A.K, *_dev(A), **kw), cs.Plan.from_csr(A, **kw)
+    id_, ih = pd.info(), ph.info()
+    for k in ("nnz", "num_tiles", "num_long_rows", "num_chunks", "brick_panels", "num_bricks", "num_blocks"):
+        assert path == cs.PATH_ROWS and k == "num_blocks" or id_[k] == ih[k], k
+    assert (id_["num_bricks"] > 0) == (lengths == "mixed")
+    for N in (64, 33):
+        B = g.dense_operand(A.K, N, 3, device="cuda")
+        Cd, Ch = pd.spmm(B), ph.spmm(B)
+        assert torch.equal(Cd, Ch)
+        ref = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.cpu().numpy(), A.M, A.K)
+        assert oracle_mod.rel_fro(ref, Cd.cpu().numpy()) <= (1e-3 if lengths == "mixed" else 2e-6)
+    assert pd.device_status() == 0
+    # dropped while its product may still run, and made again from the memory that came back
+    del pd
+    again = cs.Plan.from_device_csr(A.M, A.K, *_dev(A), **kw)
+    assert torch.equal(again.spmm(B), Ch)
