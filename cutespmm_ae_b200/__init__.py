@@ -16,6 +16,8 @@ fails, and executing a plan without a CUDA device returns an error.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 from pathlib import Path
 
 import numpy as np
@@ -81,6 +83,7 @@ def _load() -> C.CDLL:
         "cutespmm_spmm_launch_count": (C.c_int, [vp, C.c_uint32]),
         "cutespmm_spmm_kernels": (C.c_int, [vp, C.c_uint32]),
         "cutespmm_plan_set_values": (C.c_int, [vp, vp, vp]),
+        "cutespmm_plan_csr_device": (C.c_int, [vp, vp, vp, vp, vp]),
         "cutespmm_spmm_csr_noalloc": (C.c_int, [C.c_uint32, C.c_uint32, C.c_uint32, vp, vp, vp, vp, C.c_uint64, vp,
                                                 C.c_uint64, C.c_uint32, vp]),
         "cutespmm_plan_device_status": (C.c_int, [vp, u32p]),
@@ -110,6 +113,21 @@ def _load() -> C.CDLL:
 
 
 lib = _load()
+_bind = None  # the native binding on torch tensors (csrc/torch_bind.cpp), loaded with the first call that needs it
+
+
+def _native():
+    global _bind
+    if _bind is None:
+        import torch  # noqa: F401 -- its libraries first
+
+        path = _build.build_bind()
+        loader = importlib.machinery.ExtensionFileLoader("_torch_bind", str(path))
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_torch_bind", loader))
+        loader.exec_module(mod)
+        mod.set_error_class(CuteSpmmError)
+        _bind = mod
+    return _bind
 
 
 def _check(status: int) -> None:
@@ -189,6 +207,8 @@ class Plan:
 
     def close(self) -> None:
         if getattr(self, "_h", None) and self._h.value and lib is not None:  # lib is None at interpreter shutdown
+            for i in self.__dict__.get("_op_ids", ()):  # operators hold the handle: they end with the plan
+                _bind.unregister_op(i)
             lib.cutespmm_plan_destroy(self._h)
             self._h = C.c_void_p()
 
@@ -233,21 +253,7 @@ class Plan:
     def spmm(self, B, Cout=None, stream=None):
         """C = A @ B with B, C CUDA fp32 torch tensors (row-major, last stride 1).  Runs on
         `stream` (a torch.cuda.Stream) or on torch's current stream."""
-        import torch
-
-        if not B.is_cuda or B.dtype != torch.float32 or B.dim() != 2 or B.stride(1) != 1:
-            raise ValueError("B must be a 2-D CUDA fp32 tensor with unit column stride")
-        if B.shape[0] != self.K:
-            raise ValueError(f"B has {B.shape[0]} rows, A has {self.K} columns")
-        N = B.shape[1]
-        if Cout is None:
-            Cout = torch.empty((self.M, N), dtype=torch.float32, device=B.device)
-        if not Cout.is_cuda or Cout.dtype != torch.float32 or Cout.shape != (self.M, N) or Cout.stride(1) != 1:
-            raise ValueError("C must be an M x N CUDA fp32 tensor with unit column stride")
-        st = (stream or torch.cuda.current_stream(B.device)).cuda_stream
-        _check(lib.cutespmm_spmm(self._h, B.data_ptr(), B.stride(0) if B.shape[0] > 1 else max(N, 1), Cout.data_ptr(),
-                                 Cout.stride(0) if self.M > 1 else max(N, 1), N, st))
-        return Cout
+        return (_bind or _native()).spmm(self._h.value, self.M, self.K, B, Cout, None if stream is None else stream.cuda_stream)
 
     def spmm_host(self, B, Cout=None, stream=None):
         """Host buffers in, host buffers out (numpy arrays or CPU torch tensors; pin them for full
@@ -270,32 +276,24 @@ class Plan:
     def sddmm(self, X, Y, out=None, *, scale_by_values: bool = False, stream=None):
         """out[j] = (A_j if scale_by_values else 1) * <X[row of j], Y[column of j]> for every stored nonzero j, in the
         plan's storage order (cutespmm_sddmm).  X: M x N, Y: K x N CUDA fp32 tensors with unit column stride."""
-        import torch
-
-        for t, rows, name in ((X, self.M, "X"), (Y, self.K, "Y")):
-            if not t.is_cuda or t.dtype != torch.float32 or t.dim() != 2 or t.stride(1) != 1 or t.shape[0] != rows:
-                raise ValueError(f"{name} must be a {rows} x N CUDA fp32 tensor with unit column stride")
-        if X.shape[1] != Y.shape[1]:
-            raise ValueError("X and Y must have the same number of columns")
-        N = X.shape[1]
-        if out is None:
-            out = torch.empty(self.nnz, dtype=torch.float32, device=X.device)
-        if not out.is_cuda or out.dtype != torch.float32 or out.numel() != self.nnz or not out.is_contiguous():
-            raise ValueError("out must be a contiguous CUDA fp32 tensor with one element per nonzero")
-        st = (stream or torch.cuda.current_stream(X.device)).cuda_stream
-        _check(lib.cutespmm_sddmm(self._h, X.data_ptr(), X.stride(0) if self.M > 1 else max(N, 1), Y.data_ptr(),
-                                  Y.stride(0) if self.K > 1 else max(N, 1), N, 1 if scale_by_values else 0, out.data_ptr(), st))
-        return out
+        return (_bind or _native()).sddmm(self._h.value, self.M, self.K, self.nnz, X, Y, out, scale_by_values,
+                                          None if stream is None else stream.cuda_stream)
 
     def set_values(self, vals, stream=None):
         """New values for the same pattern (cutespmm_plan_set_values): vals is a CUDA fp32 tensor with one element per
         nonzero in the plan's storage order, e.g. normalised output of `sddmm`."""
+        (_bind or _native()).set_values(self._h.value, self.nnz, vals, None if stream is None else stream.cuda_stream)
+
+    def csr_device(self):
+        """The plan's matrix as CSR tensors on its GPU (row_ptr and cols int32, vals float32), in storage order."""
         import torch
 
-        if not vals.is_cuda or vals.dtype != torch.float32 or vals.numel() != self.nnz or not vals.is_contiguous():
-            raise ValueError("vals must be a contiguous CUDA fp32 tensor with one element per nonzero")
-        st = (stream or torch.cuda.current_stream(vals.device)).cuda_stream
-        _check(lib.cutespmm_plan_set_values(self._h, vals.data_ptr(), st))
+        dev = torch.device("cuda", torch.cuda.current_device())
+        rp = torch.empty(self.M + 1, dtype=torch.int32, device=dev)
+        cols = torch.empty(self.nnz, dtype=torch.int32, device=dev)
+        vals = torch.empty(self.nnz, dtype=torch.float32, device=dev)
+        _check(lib.cutespmm_plan_csr_device(self._h, rp.data_ptr(), cols.data_ptr(), vals.data_ptr(), torch.cuda.current_stream(dev).cuda_stream))
+        return rp, cols, vals
 
     def spmm_sharded(self, comm: "Comm", B, Cout=None, *, b_mode: int = B_RESIDENT, root: int = 0, b_bounds=None, stream=None):
         """This rank's rows of A @ B through cutespmm_spmm_sharded: B (K x N, contiguous, on this rank's GPU) is
@@ -411,30 +409,7 @@ def spmm_csr_noalloc(M: int, K: int, row_ptr, cols, vals, B, Cout, stream=None):
     """C = A @ B from CSR tensors that already live on the GPU (row_ptr/cols int32, vals/B/C fp32),
     through the entry point that allocates nothing (cutespmm_spmm_csr_noalloc): for callers that
     may not allocate device memory when they call.  The caller provides C."""
-    import torch
-
-    for t, dt in ((row_ptr, torch.int32), (cols, torch.int32), (vals, torch.float32), (B, torch.float32), (Cout, torch.float32)):
-        if not t.is_cuda or t.dtype != dt:
-            raise ValueError("all operands must be CUDA tensors: row_ptr/cols int32, vals/B/C float32")
-    if B.dim() != 2 or Cout.dim() != 2:
-        raise ValueError("B and C must be 2-D")
-    if not (row_ptr.is_contiguous() and cols.is_contiguous() and vals.is_contiguous()) or B.stride(1) != 1 or Cout.stride(1) != 1:
-        raise ValueError("CSR arrays must be contiguous; B and C need unit column stride")
-    N = B.shape[1]
-    # the call itself cannot see the sizes of the buffers behind the pointers: check them here, as Plan.spmm does
-    if row_ptr.numel() != M + 1 or cols.numel() != vals.numel():
-        raise ValueError("row_ptr must have M+1 entries; cols and vals the same length")
-    if B.shape[0] != K:
-        raise ValueError(f"B has {B.shape[0]} rows, A has {K} columns")
-    if tuple(Cout.shape) != (M, N):
-        raise ValueError(f"C must be {M} x {N}, got {tuple(Cout.shape)}")
-    if len({t.device for t in (row_ptr, cols, vals, B, Cout)}) != 1:
-        raise ValueError("all operands must live on one device")
-    st = (stream or torch.cuda.current_stream(B.device)).cuda_stream
-    _check(lib.cutespmm_spmm_csr_noalloc(M, K, cols.numel(), row_ptr.data_ptr(), cols.data_ptr(), vals.data_ptr(), B.data_ptr(),
-                                         B.stride(0) if K > 1 else max(N, 1), Cout.data_ptr(),
-                                         Cout.stride(0) if M > 1 else max(N, 1), N, st))
-    return Cout
+    return (_bind or _native()).spmm_csr_noalloc(M, K, row_ptr, cols, vals, B, Cout, None if stream is None else stream.cuda_stream)
 
 
 def partition_rows(row_ptr, nparts: int, align_rows: int = 16, row_cost: int = 2) -> np.ndarray:

@@ -37,13 +37,18 @@ FLAGS = [
 ]
 
 
+# The binding on torch tensors (needs torch's headers and libraries; the C ABI library needs neither).
+BIND = LIBDIR / "_torch_bind.so"
+BIND_SOURCE = CSRC / "torch_bind.cpp"
+
+
 def _sources():
     return [CSRC / s for s in SOURCES if (CSRC / s).exists()]
 
 
 def _stamp() -> str:
     h = hashlib.sha256()
-    for f in sorted(list(CSRC.glob("*")) + [HERE.parent / "include" / "cutespmm.h"]):
+    for f in sorted([f for f in CSRC.glob("*") if f != BIND_SOURCE] + [HERE.parent / "include" / "cutespmm.h"]):
         if f.is_file():
             h.update(f.name.encode())
             h.update(f.read_bytes())
@@ -77,6 +82,39 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     return LIB
 
 
+def _bind_stamp() -> str:
+    import torch
+
+    h = hashlib.sha256(torch.__version__.encode())
+    for f in (BIND_SOURCE, HERE.parent / "include" / "cutespmm.h"):
+        h.update(f.read_bytes())
+    return h.hexdigest()
+
+
+def build_bind(force: bool = False) -> Path:
+    """The torch binding next to the library it calls (found through its own folder at load time)."""
+    import sysconfig
+
+    import torch
+
+    stamp_file = LIBDIR / (BIND.name + ".stamp")
+    stamp = _bind_stamp()
+    if not force and BIND.exists() and stamp_file.exists() and stamp_file.read_text() == stamp:
+        return BIND
+    build()
+    troot = Path(torch.__file__).resolve().parent
+    include = [troot / "include", troot / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"], CUDA_HOME / "include"]
+    # libstdc++ by its shared name: a static copy would not unwind the exceptions torch's libraries throw
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", *[f"-isystem{d}" for d in include], "-o", str(BIND), str(BIND_SOURCE),
+           f"-L{LIBDIR}", f"-L{troot / 'lib'}", "-l:" + LIB.name, "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-l:libstdc++.so.6", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("building the torch binding failed:\n" + res.stderr)
+    stamp_file.write_text(stamp)
+    return BIND
+
+
 if __name__ == "__main__":
     build(force="--force" in sys.argv, verbose=True)
     print(LIB)
+    print(build_bind(force="--force" in sys.argv))

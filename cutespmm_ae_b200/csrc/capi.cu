@@ -538,7 +538,7 @@ int cutespmm_sddmm(const cutespmm_plan_t *p, const float *X, uint64_t ldx, const
     return e == cudaSuccess ? CUTESPMM_OK : fail_cuda(e, "SDDMM kernel launch");
 }
 
-int cutespmm_plan_set_values(cutespmm_plan_t *p, const float *vals_dev, void *stream)
+int cutespmm_plan_set_values_gathered(cutespmm_plan_t *p, const float *vals_dev, const uint32_t *order_dev, void *stream)
 {
     if (!p) return fail(CUTESPMM_EINVAL, "plan is NULL");
     if (!p->on_device) return fail(CUTESPMM_EUNSUPPORTED, "host-only plan has no device arrays");
@@ -548,15 +548,36 @@ int cutespmm_plan_set_values(cutespmm_plan_t *p, const float *vals_dev, void *st
     if (!h.row_map.empty()) return fail(CUTESPMM_EUNSUPPORTED, "values cannot be replaced in a plan with row reordering");
     if (h.nnz == 0) return CUTESPMM_OK;
     if (!vals_dev) return fail(CUTESPMM_EINVAL, "vals is NULL");
-    if (reinterpret_cast<uintptr_t>(vals_dev) & 3) return fail(CUTESPMM_EINVAL, "vals must be 4-byte aligned");
+    if ((reinterpret_cast<uintptr_t>(vals_dev) | reinterpret_cast<uintptr_t>(order_dev)) & 3) return fail(CUTESPMM_EINVAL, "vals must be 4-byte aligned");
     int cur = -1;
     if (cudaGetDevice(&cur) != cudaSuccess || cur != p->device)
         return fail(CUTESPMM_EINVAL, "the current CUDA device is not the one the plan was created on");
     note_stream(p, static_cast<cudaStream_t>(stream));
-    const cudaError_t e = launch_set_values(p->d_pairs, vals_dev, h.nnz, p->sm_count, static_cast<cudaStream_t>(stream));
+    const cudaError_t e = launch_set_values(p->d_pairs, vals_dev, order_dev, h.nnz, p->sm_count, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail_cuda(e, "replacing the values");
     p->host.values_on_device = true;
     return CUTESPMM_OK;
+}
+
+int cutespmm_plan_set_values(cutespmm_plan_t *p, const float *vals_dev, void *stream)
+{
+    return cutespmm_plan_set_values_gathered(p, vals_dev, nullptr, stream);
+}
+
+int cutespmm_plan_csr_device(const cutespmm_plan_t *p, uint32_t *rowPtr_dev, uint32_t *cols_dev, float *vals_dev, void *stream)
+{
+    if (!p || !rowPtr_dev) return fail(CUTESPMM_EINVAL, "null argument");
+    if (!p->on_device) return fail(CUTESPMM_EUNSUPPORTED, "host-only plan has no device arrays");
+    if (!p->host.row_map.empty()) return fail(CUTESPMM_EUNSUPPORTED, "not available for a plan with row reordering");
+    if (p->host.nnz && !cols_dev) return fail(CUTESPMM_EINVAL, "null argument");
+    int cur = -1;
+    if (cudaGetDevice(&cur) != cudaSuccess || cur != p->device)
+        return fail(CUTESPMM_EINVAL, "the current CUDA device is not the one the plan was created on");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    note_stream(p, s);
+    cudaError_t e = cudaMemcpyAsync(rowPtr_dev, p->d_row_ptr, (p->host.M + 1) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
+    if (e == cudaSuccess) e = launch_unpack(p->d_pairs, cols_dev, vals_dev, p->host.nnz, p->sm_count, s);
+    return e == cudaSuccess ? CUTESPMM_OK : fail_cuda(e, "reading the packed nonzeros");
 }
 
 int cutespmm_plan_device_status(const cutespmm_plan_t *p, uint32_t *status)

@@ -541,21 +541,42 @@ __global__ void __launch_bounds__(256) pack_kernel(const uint32_t *__restrict__ 
     if (__any_sync(kFullMask, out_of_range) && (threadIdx.x & 31) == 0) atomicOr(bad, 1u);
 }
 
-// pairs[j].value = vals[j]: new values for an unchanged pattern.
-__global__ void __launch_bounds__(256) set_values_kernel(uint2 *__restrict__ pairs, const float *__restrict__ vals, uint64_t nnz)
+// pairs[j].value = vals[order[j]] (order may be absent): new values for an unchanged pattern.
+template <bool ORDER>
+__global__ void __launch_bounds__(256) set_values_kernel(uint2 *__restrict__ pairs, const float *__restrict__ vals, const uint32_t *__restrict__ order,
+                                                         uint64_t nnz)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nnz; j += stride) pairs[j].y = __float_as_uint(__ldcs(vals + j));
+    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nnz; j += stride)
+        pairs[j].y = __float_as_uint(ORDER ? __ldg(vals + __ldcs(order + j)) : __ldcs(vals + j));
+}
+
+__global__ void __launch_bounds__(256) unpack_kernel(const uint2 *__restrict__ pairs, uint32_t *__restrict__ cols, float *__restrict__ vals, uint64_t nnz)
+{
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nnz; j += stride) {
+        const uint2 pr = __ldcs(pairs + j);
+        cols[j] = pr.x;
+        if (vals) vals[j] = __uint_as_float(pr.y);
+    }
 }
 
 }  // namespace
 
-cudaError_t launch_set_values(void *pairs, const float *vals, uint64_t nnz, int sm_count, cudaStream_t s)
+cudaError_t launch_set_values(void *pairs, const float *vals, const uint32_t *order, uint64_t nnz, int sm_count, cudaStream_t s)
 {
     if (nnz == 0) return cudaSuccess;
-    const uint64_t want = (nnz + 255) / 256;
-    const uint32_t blocks = (uint32_t)(want < (uint64_t)sm_count * 8 ? want : (uint64_t)sm_count * 8);
-    set_values_kernel<<<blocks, 256, 0, s>>>(static_cast<uint2 *>(pairs), vals, nnz);
+    const uint32_t blocks = (uint32_t)std::min<uint64_t>((nnz + 255) / 256, (uint64_t)sm_count * 8);
+    if (order) set_values_kernel<true><<<blocks, 256, 0, s>>>(static_cast<uint2 *>(pairs), vals, order, nnz);
+    else set_values_kernel<false><<<blocks, 256, 0, s>>>(static_cast<uint2 *>(pairs), vals, order, nnz);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_unpack(const void *pairs, uint32_t *cols, float *vals, uint64_t nnz, int sm_count, cudaStream_t s)
+{
+    if (nnz == 0) return cudaSuccess;
+    const uint32_t blocks = (uint32_t)std::min<uint64_t>((nnz + 255) / 256, (uint64_t)sm_count * 8);
+    unpack_kernel<<<blocks, 256, 0, s>>>(static_cast<const uint2 *>(pairs), cols, vals, nnz);
     return cudaGetLastError();
 }
 

@@ -157,7 +157,8 @@ cudaError_t launch_brick_fill(const uint32_t *row_ptr, const void *pairs, uint32
                               int sm_count, cudaStream_t s);
 cudaError_t launch_pack(const uint32_t *row_ptr, const uint32_t *cols, const float *vals, uint32_t M, uint32_t K, uint32_t nnz, uint32_t *row_ptr_out,
                         void *pairs, uint32_t *bad, int sm_count, cudaStream_t s);
-cudaError_t launch_set_values(void *pairs, const float *vals, uint64_t nnz, int sm_count, cudaStream_t s);
+cudaError_t launch_set_values(void *pairs, const float *vals, const uint32_t *order, uint64_t nnz, int sm_count, cudaStream_t s);
+cudaError_t launch_unpack(const void *pairs, uint32_t *cols, float *vals, uint64_t nnz, int sm_count, cudaStream_t s);
 // the panel views (distinct columns per panel, ascending) and column ranges, when somebody asks for them
 cudaError_t launch_panel_columns(const uint32_t *row_ptr, const void *pairs, uint32_t M, uint32_t num_panels, uint32_t *ncols,
                                  uint32_t *acols, int sm_count, cudaStream_t s);

@@ -3,7 +3,7 @@
 The reference tree ships its graph-layer operators as a pybind extension of the TC-GNN baseline
 (TC-GNN_ATC23/TCGNN_conv/TCGNN.cpp:260-271: forward / backward are the same SpMM on the symmetric
 adjacency, forward_ef is SDDMM).  Here the same two operators are `torch.library` custom ops on top of
-libcutespmm, so they work under autograd, `torch.compile` (through the registered fake kernels) and on
+libcutespmm, registered from native code, so they work under autograd, `torch.compile` (through the registered fake kernels) and on
 any stream:
 
     op = SparseOperator(plan)          # registers the plan, gives it an integer id
@@ -26,7 +26,10 @@ import weakref
 import numpy as np
 import torch
 
-from . import Plan
+from . import PATH_SLAB, CuteSpmmError, Plan
+from . import _native as _load_native
+
+_native = _load_native()
 
 __all__ = ["SparseOperator", "register_plan", "unregister_plan", "transpose_csr"]
 
@@ -54,46 +57,74 @@ class SparseOperator:
         self.M, self.K, self.nnz = plan.M, plan.K, plan.nnz
         self._plan_kwargs = plan_kwargs or {}
         self._transposed: Plan | None = None
-        self._t_perm: torch.Tensor | None = None  # storage position in A of every stored position of A^T
+        self._t_perm: torch.Tensor | None = None  # storage position in A of every stored position of A^T (int32)
         self.id = next(_ids)
         _plans[self.id] = self
         weakref.finalize(self, _plans.pop, self.id, None)
+        _native.register_op(self.id, plan._h.value, self.M, self.K, self.nnz, self._make_transposed)
+        plan.__dict__.setdefault("_op_ids", []).append(self.id)
 
     def transposed(self) -> Plan:
         if self._transposed is None:
-            rp, cols, vals = self.plan.decode_csr()
-            t_rp, t_cols, t_vals = transpose_csr(self.M, self.K, rp, cols, vals)
-            self._transposed = Plan(self.K, self.M, t_rp, t_cols, t_vals, **self._plan_kwargs)
+            self._make_transposed(False)
         return self._transposed
 
+    def _make_transposed(self, with_order: bool) -> None:
+        """Builds what is missing of the plan of A^T and the order its stored positions have in A, and hands both to the
+        native operators.  On the device where the plan's options and layout allow it."""
+        on_device = self._plan_kwargs.get("path", 0) != PATH_SLAB and not set(self._plan_kwargs) - {"path", "split_nnz", "tile_nnz", "min_brick_panels"}
+        csr = None
+        if on_device:
+            try:
+                csr = self.plan.csr_device()
+            except CuteSpmmError:  # rows reordered, or a host-only plan
+                csr = None
+        if csr is not None:
+            rp, cols, vals = csr
+            _, order = torch.sort(cols.to(torch.int64) & 0xFFFFFFFF, stable=True)
+            if self._transposed is None:
+                rows = torch.repeat_interleave(torch.arange(self.M, dtype=torch.int32, device=cols.device), (rp[1:] - rp[:-1]).to(torch.int64), output_size=self.nnz)
+                t_rp = torch.zeros(self.K + 1, dtype=torch.int64, device=cols.device)
+                torch.cumsum(torch.bincount(cols.to(torch.int64) & 0xFFFFFFFF, minlength=self.K), 0, out=t_rp[1:])
+                self._transposed = Plan.from_device_csr(self.K, self.M, t_rp.to(torch.int32), rows[order], vals[order], **self._plan_kwargs)
+            if with_order and self._t_perm is None:
+                self._t_perm = order.to(torch.int32)
+        else:
+            rp, cols, vals = self.plan.decode_csr()
+            if self._transposed is None:
+                t_rp, t_cols, t_vals = transpose_csr(self.M, self.K, rp, cols, vals)
+                self._transposed = Plan(self.K, self.M, t_rp, t_cols, t_vals, **self._plan_kwargs)
+            if with_order and self._t_perm is None:
+                self._t_perm = torch.from_numpy(np.argsort(np.asarray(cols, dtype=np.int64), kind="stable").astype(np.uint32).view(np.int32)).cuda()
+        _native.set_transposed(self.id, self._transposed._h.value, self._t_perm)
+
     def __call__(self, B: torch.Tensor) -> torch.Tensor:
-        return torch.ops.cutespmm.spmm(self.id, B)
+        if torch.compiler.is_compiling():
+            return torch.ops.cutespmm.spmm(self.id, B)
+        return _native.op_spmm(self.id, B)
 
     def sddmm(self, X: torch.Tensor, Y: torch.Tensor, scale_by_values: bool = False) -> torch.Tensor:
-        return torch.ops.cutespmm.sddmm(self.id, X, Y, scale_by_values)
+        if torch.compiler.is_compiling():
+            return torch.ops.cutespmm.sddmm(self.id, X, Y, scale_by_values)
+        return _native.op_sddmm(self.id, X, Y, scale_by_values)
 
     def weighted(self, w: torch.Tensor, B: torch.Tensor) -> torch.Tensor:
-        return torch.ops.cutespmm.spmm_weighted(self.id, w, B)
-
-    def _transposed_with(self, w: torch.Tensor) -> Plan:
-        """The plan of A^T carrying the weights w (given in this plan's storage order)."""
-        if self._t_perm is None:
-            rp, cols, _ = self.plan.decode_csr()
-            self._t_perm = torch.from_numpy(np.argsort(np.asarray(cols, dtype=np.int64), kind="stable")).to(w.device)
-        t = self.transposed()
-        t.set_values(w.detach().contiguous()[self._t_perm])
-        return t
+        if torch.compiler.is_compiling():
+            return torch.ops.cutespmm.spmm_weighted(self.id, w, B)
+        return _native.op_weighted(self.id, w, B)
 
     def set_values(self, vals: torch.Tensor) -> None:
         """New values for the same pattern (Plan.set_values), e.g. normalised `sddmm` scores as attention weights.  The
         plan of A^T, if a backward pass has built one, is dropped and rebuilt from the new values on next use."""
         self.plan.set_values(vals)
         if self._transposed is not None:
+            _native.set_transposed(self.id, None, self._t_perm)
             self._transposed.close()
             self._transposed = None
 
     def close(self) -> None:
         _plans.pop(self.id, None)
+        _native.unregister_op(self.id)
         for p in (self.plan, self._transposed):
             if p is not None:
                 p.close()
@@ -122,90 +153,27 @@ def _get(plan_id: int) -> SparseOperator:
         raise RuntimeError(f"cutespmm: no plan registered under id {plan_id}") from None
 
 
-@torch.library.custom_op("cutespmm::spmm", mutates_args=())
-def _spmm(plan_id: int, B: torch.Tensor) -> torch.Tensor:
-    op = _get(plan_id)
-    Bc = B if B.stride(-1) == 1 else B.contiguous()
-    return op.plan.spmm(Bc)
-
-
-@_spmm.register_fake
+# The operators and their gradients are native (csrc/torch_bind.cpp); the fake kernels give shapes to tracing.
+@torch.library.register_fake("cutespmm::spmm")
 def _(plan_id: int, B: torch.Tensor) -> torch.Tensor:
     return B.new_empty((_get(plan_id).M, B.shape[1]))
 
 
-@torch.library.custom_op("cutespmm::spmm_transposed", mutates_args=())
-def _spmm_t(plan_id: int, G: torch.Tensor) -> torch.Tensor:
-    op = _get(plan_id)
-    Gc = G if G.stride(-1) == 1 else G.contiguous()
-    return op.transposed().spmm(Gc)
-
-
-@_spmm_t.register_fake
+@torch.library.register_fake("cutespmm::spmm_transposed")
 def _(plan_id: int, G: torch.Tensor) -> torch.Tensor:
     return G.new_empty((_get(plan_id).K, G.shape[1]))
 
 
-def _spmm_backward(ctx, grad_C):
-    return None, torch.ops.cutespmm.spmm_transposed(ctx.plan_id, grad_C)
-
-
-def _spmm_setup(ctx, inputs, output):
-    ctx.plan_id = inputs[0]
-
-
-_spmm.register_autograd(_spmm_backward, setup_context=_spmm_setup)
-_spmm_t.register_autograd(lambda ctx, g: (None, torch.ops.cutespmm.spmm(ctx.plan_id, g)), setup_context=_spmm_setup)
-
-
-@torch.library.custom_op("cutespmm::spmm_weighted", mutates_args=())
-def _spmm_w(plan_id: int, w: torch.Tensor, B: torch.Tensor) -> torch.Tensor:
-    op = _get(plan_id)
-    op.plan.set_values(w.detach().contiguous())
-    Bc = B if B.stride(-1) == 1 else B.contiguous()
-    return op.plan.spmm(Bc)
-
-
-@_spmm_w.register_fake
+@torch.library.register_fake("cutespmm::spmm_weighted")
 def _(plan_id: int, w: torch.Tensor, B: torch.Tensor) -> torch.Tensor:
     return B.new_empty((_get(plan_id).M, B.shape[1]))
 
 
-@torch.library.custom_op("cutespmm::spmm_weighted_transposed", mutates_args=())
-def _spmm_wt(plan_id: int, w: torch.Tensor, G: torch.Tensor) -> torch.Tensor:
-    op = _get(plan_id)
-    Gc = G if G.stride(-1) == 1 else G.contiguous()
-    return op._transposed_with(w).spmm(Gc)
-
-
-@_spmm_wt.register_fake
+@torch.library.register_fake("cutespmm::spmm_weighted_transposed")
 def _(plan_id: int, w: torch.Tensor, G: torch.Tensor) -> torch.Tensor:
     return G.new_empty((_get(plan_id).K, G.shape[1]))
 
 
-def _spmm_w_setup(ctx, inputs, output):
-    ctx.plan_id = inputs[0]
-    ctx.save_for_backward(inputs[1], inputs[2])
-
-
-def _spmm_w_backward(ctx, grad_C):
-    w, B = ctx.saved_tensors
-    grad_w = torch.ops.cutespmm.sddmm(ctx.plan_id, grad_C, B, False) if ctx.needs_input_grad[1] else None
-    grad_B = torch.ops.cutespmm.spmm_weighted_transposed(ctx.plan_id, w, grad_C) if ctx.needs_input_grad[2] else None
-    return None, grad_w, grad_B
-
-
-_spmm_w.register_autograd(_spmm_w_backward, setup_context=_spmm_w_setup)
-
-
-@torch.library.custom_op("cutespmm::sddmm", mutates_args=())
-def _sddmm(plan_id: int, X: torch.Tensor, Y: torch.Tensor, scale_by_values: bool) -> torch.Tensor:
-    op = _get(plan_id)
-    Xc = X if X.stride(-1) == 1 else X.contiguous()
-    Yc = Y if Y.stride(-1) == 1 else Y.contiguous()
-    return op.plan.sddmm(Xc, Yc, scale_by_values=scale_by_values)
-
-
-@_sddmm.register_fake
+@torch.library.register_fake("cutespmm::sddmm")
 def _(plan_id: int, X: torch.Tensor, Y: torch.Tensor, scale_by_values: bool) -> torch.Tensor:
     return X.new_empty((_get(plan_id).nnz,))

@@ -212,6 +212,12 @@ int cutespmm_sddmm(const cutespmm_plan_t *plan, const float *X_dev, uint64_t ldx
  * afterwards see the new values.  For plans whose rows all run on the row kernel (path rows, or auto without dense
  * panels) and without row reordering; CUTESPMM_EUNSUPPORTED otherwise. */
 int cutespmm_plan_set_values(cutespmm_plan_t *plan, const float *vals_dev, void *stream);
+/* The same through an order: the value of stored position j becomes vals[order[j]] (order: nnz x u32 on the device).  The
+ * plan of A^T takes weights given in A's storage order this way, without a permuted copy of them. */
+int cutespmm_plan_set_values_gathered(cutespmm_plan_t *plan, const float *vals_dev, const uint32_t *order_dev, void *stream);
+/* The plan's matrix as CSR into device buffers (rowPtr: M+1, cols and vals: nnz; vals may be NULL), in the plan's storage
+ * order; not for a plan with row reordering. */
+int cutespmm_plan_csr_device(const cutespmm_plan_t *plan, uint32_t *rowPtr_dev, uint32_t *cols_dev, float *vals_dev, void *stream);
 
 /* ---- product without any allocation ------------------------------------------------------------
  * No counterpart in the reference.  For callers that must not allocate device memory when they
