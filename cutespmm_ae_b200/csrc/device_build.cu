@@ -100,8 +100,9 @@ __global__ void __launch_bounds__(256) panel_max_col_kernel(const uint32_t *__re
 // it starts, so the tiles of a segment of rows depend on the row its first tile starts at -- but a tile has at most
 // kMaxTileRows rows, so there are only kMaxTileRows + 1 such rows.  The counting kernel follows the chain of tiles from
 // each of them at once (a thread per entry row), which gives the row the next segment is entered at and the number of
-// tiles; a single block then walks the segments through these tables, and the writing kernel cuts every segment again
-// from the one entry row that is real.  (The row pointers used to visit the host, which cut the lists there: for
+// tiles; the tables of 32 segments are composed into one, a single block walks those, and the writing kernel cuts every
+// segment again from the one entry row that is real.  512 rows per segment: 2048 gave R-MAT 2^17 64 blocks and 76 us for
+// counting and writing.  (The row pointers used to visit the host, which cut the lists there: for
 // R-MAT 2^17, 1.9 M nonzeros, copies and host loops of 2-6 ms against 20 us.)
 constexpr int kListThreads = 288;  // >= kEntries
 constexpr uint32_t kEntries = kSegmentEntries;
@@ -219,27 +220,53 @@ __global__ void __launch_bounds__(kListThreads) lists_count_kernel(const uint32_
     }
 }
 
-// Block 0 walks the segments: the row each is really entered at and the number of its first tile.  Block 1 + i turns the
+// One block per group of kGroup segments, a thread per entry row of the group's first: the entry row of every segment
+// and the tiles in front of it, were the group entered there; and the group's own exit and tiles.
+constexpr uint32_t kGroup = 32;
+__global__ void __launch_bounds__(kListThreads) lists_compose_kernel(ListArgs a)
+{
+    __shared__ uint16_t exits[kGroup * kEntries], counts[kGroup * kEntries];
+    const uint32_t s0 = blockIdx.x * kGroup, n = min(kGroup, a.num_segments - s0);
+    for (uint32_t i = threadIdx.x; i < n * kEntries; i += kListThreads) {
+        exits[i] = a.exits[(size_t)s0 * kEntries + i];
+        counts[i] = a.tile_counts[(size_t)s0 * kEntries + i];
+    }
+    __syncthreads();
+    const uint32_t e = threadIdx.x;
+    if (e >= kEntries) return;
+    uint32_t at = e, tiles = 0;
+    for (uint32_t k = 0; k < n; ++k) {
+        a.path_entry[(size_t)(s0 + k) * kEntries + e] = (uint16_t)at;
+        a.path_tiles[(size_t)(s0 + k) * kEntries + e] = tiles;
+        tiles += counts[k * kEntries + at];
+        at = exits[k * kEntries + at];
+    }
+    a.group_exit[(size_t)blockIdx.x * kEntries + e] = (uint16_t)at;
+    a.group_tiles[(size_t)blockIdx.x * kEntries + e] = tiles;
+}
+
+// Block 0 walks the groups: the row each is really entered at and the number of its first tile.  Block 1 + i turns the
 // i-th per-segment counter into exclusive sums, in place.  The sums go to the totals.
-constexpr uint32_t kChainBatch = 32;  // segments whose tables are in shared memory at a time
+constexpr uint32_t kChainBatch = 16;  // groups whose tables are in shared memory at a time
 __global__ void __launch_bounds__(1024) lists_scan_kernel(const uint32_t *__restrict__ row_ptr, ListArgs a, uint32_t *__restrict__ counters)
 {
     __shared__ uint32_t sums[32];
-    __shared__ uint16_t exits[kChainBatch * kEntries], counts[kChainBatch * kEntries];
+    __shared__ uint16_t exits[kChainBatch * kEntries];
+    __shared__ uint32_t counts[kChainBatch * kEntries];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (blockIdx.x == 0) {
         uint32_t entry = 0, tiles = 0;
-        for (uint32_t s0 = 0; s0 < a.num_segments; s0 += kChainBatch) {
-            const uint32_t n = min(kChainBatch, a.num_segments - s0);
+        const uint32_t groups = (a.num_segments + kGroup - 1) / kGroup;
+        for (uint32_t g0 = 0; g0 < groups; g0 += kChainBatch) {
+            const uint32_t n = min(kChainBatch, groups - g0);
             for (uint32_t i = tid; i < n * kEntries; i += 1024) {
-                exits[i] = a.exits[(size_t)s0 * kEntries + i];
-                counts[i] = a.tile_counts[(size_t)s0 * kEntries + i];
+                exits[i] = a.group_exit[(size_t)g0 * kEntries + i];
+                counts[i] = a.group_tiles[(size_t)g0 * kEntries + i];
             }
             __syncthreads();
             if (tid == 0)
                 for (uint32_t k = 0; k < n; ++k) {
-                    a.seg_entry[s0 + k] = entry;
-                    a.seg_tiles[s0 + k] = tiles;
+                    a.group_entry[g0 + k] = make_uint2(entry, tiles);
                     tiles += counts[k * kEntries + entry];
                     entry = exits[k * kEntries + entry];
                 }
@@ -288,9 +315,10 @@ __global__ void __launch_bounds__(kListThreads) lists_write_kernel(const uint32_
     const ItemSizes sizes = list_sizes(a, nnz);
     load_segment(v, row_ptr, a, sizes, seg, nnz);
     const uint32_t rows = min(v.n, kTileSegmentRows);
+    const uint2 group = a.group_entry[seg / kGroup];  // the group's real entry row, tiles in front of the group
     if (tid == 0) {
         uint32_t k = 0;
-        for (uint32_t r = __ldg(a.seg_entry + seg); r < rows; r = v.next[r])
+        for (uint32_t r = a.path_entry[(size_t)seg * kEntries + group.x]; r < rows; r = v.next[r])
             if (!is_special(v, r)) starts[k++] = (uint16_t)r;
         num_starts = k;
     }
@@ -324,7 +352,7 @@ __global__ void __launch_bounds__(kListThreads) lists_write_kernel(const uint32_
         lr += lt;
         __syncthreads();
     }
-    const uint32_t t0 = __ldg(a.seg_tiles + seg);
+    const uint32_t t0 = group.y + a.path_tiles[(size_t)seg * kEntries + group.x];
     for (uint32_t k = tid; k < num_starts; k += kListThreads) {
         const uint32_t r = starts[k], e = v.next[r];
         a.tiles[t0 + k] = Tile{first + r, first + e, v.rp[r], v.rp[e]};
@@ -334,73 +362,111 @@ __global__ void __launch_bounds__(kListThreads) lists_write_kernel(const uint32_
 // ---- panel census: which panels the tensor-core kernel takes ------------------------------------------------------
 // Distinct columns of a panel, counted with a hash set in shared memory (open addressing; a 16-row panel holds a few
 // hundred nonzeros, so the set is a few KB and a count costs one shared atomic per nonzero, where sorting the panel
-// costs 36-91 passes over it: 590 us -> 25 us on R-MAT 2^17 with 1.9 M nonzeros).  Runs on row pointers nobody has checked
-// yet: every position is clamped to nnz = row_ptr[M], and the host drops the result when the check fails.
+// costs 36-91 passes over it: 590 us for R-MAT 2^17 with 1.9 M nonzeros).  A panel is a chain of five latencies, so a
+// warp takes one on its own (four at a time per block; a block per panel took 35 us there, with 7 blocks per SM by their
+// shared memory); panels of more than kWarpPanelNnz are left to the whole block.  Runs on row pointers nobody
+// has checked yet: every position is clamped to nnz = row_ptr[M], and the host drops the result when the check fails.
 constexpr int kCensusThreads = 128;
+constexpr uint32_t kCensusWarps = kCensusThreads / 32;
+constexpr uint32_t kWarpPanelNnz = 512;  // panels up to this are a warp's: four batches of loads
 
-// Inserts the columns of pairs/cols [j0, j0 + n) into `table` (size a power of two > n); returns through `emit(slot)`
-// every slot a new column landed in.  Whole block; the table must be clear.
+// Inserts the columns col_at(0 .. n-1) into `table` (size a power of two > n, clear): `threads` threads, of which this
+// is number `me`; emit(slot) for every slot a new column lands in.
 template <class ColAt, class Emit>
-__device__ __forceinline__ void hash_insert(uint32_t *table, uint32_t size, uint32_t n, ColAt col_at, Emit emit)
+__device__ __forceinline__ void hash_insert(uint32_t *table, uint32_t size, uint32_t n, uint32_t me, uint32_t threads, ColAt col_at, Emit emit)
 {
-    for (uint32_t i = threadIdx.x; i < n; i += kCensusThreads) {
-        const uint32_t c = col_at(i);
-        uint32_t h = (c * 2654435761u) >> 7 & (size - 1);
-        for (;;) {
-            const uint32_t old = atomicCAS(&table[h], 0xffffffffu, c);  // 0xffffffff is no column: K < 2^32
-            if (old == 0xffffffffu) { emit(h); break; }
-            if (old == c) break;
-            h = (h + 1) & (size - 1);
+    const uint32_t shift = 1 + __clz(size);  // the product's top bits: its low ones see only the column's low bits
+    constexpr uint32_t kAhead = 4;  // columns loaded together: the inserts do not wait for one load each
+    for (uint32_t i = me; i < n; i += threads * kAhead) {
+        uint32_t c[kAhead];
+#pragma unroll
+        for (uint32_t u = 0; u < kAhead; ++u) c[u] = i + u * threads < n ? col_at(i + u * threads) : 0u;
+#pragma unroll
+        for (uint32_t u = 0; u < kAhead; ++u) {
+            if (i + u * threads >= n) break;
+            uint32_t h = (c[u] * 2654435761u) >> shift;
+            for (;;) {
+                const uint32_t old = atomicCAS(&table[h], 0xffffffffu, c[u]);  // 0xffffffff is no column: K < 2^32
+                if (old == 0xffffffffu) { emit(h); break; }
+                if (old == c[u]) break;
+                h = (h + 1) & (size - 1);
+            }
         }
     }
 }
-__device__ __forceinline__ uint32_t hash_size(uint32_t n, uint32_t most)
+// entries of a set for n columns: half full, or up to three quarters where `most` entries are there
+__host__ __device__ __forceinline__ uint32_t hash_size(uint32_t n, uint32_t most)
 {
-    uint32_t size = 128;
-    while (size < n + n / 3) size <<= 1;
-    return size < most ? size : most;
+    uint32_t size = 64;
+    while (size < 2 * n && size < most) size <<= 1;
+    return size;
+}
+
+// What the census decides about panel q with n nonzeros and nc distinct columns; one thread.
+__device__ __forceinline__ void census_result(const CensusArgs &a, uint32_t q, uint32_t n, uint32_t nc, bool candidate)
+{
+    const uint32_t r0 = q * kPanelRows, r1 = min(a.M, r0 + kPanelRows), padded = (nc + kBrickCols - 1) / kBrickCols * kBrickCols;
+    // fill of the panel's 16 x padded dense image, the expression of choose_panel_paths (plan.cpp)
+    const bool brick = candidate && (a.force || (float)n / (float)(kPanelRows * padded) >= a.density);
+    a.ncols[q] = nc;
+    a.path[q] = brick ? 1 : 0;
+    if (!brick) return;
+    const uint32_t nb = padded / kBrickCols;
+    atomicAdd(&a.seg_panels[r0 / kTileSegmentRows], 1u);
+    atomicAdd(&a.seg_slots[r0 / kTileSegmentRows], (nb + 3) / 4 * 4);
+    atomicAdd(&a.totals->bricks, (unsigned long long)nb);
+    atomicAdd(&a.totals->brick_cost, (unsigned long long)n + (r1 - r0) * kRowCost);
+    atomicMax(&a.totals->brick_nnz_max, n);
+    atomicMax(&a.totals->brick_cols_max, nc);
 }
 
 __global__ void __launch_bounds__(kCensusThreads) panel_census_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ cols, CensusArgs a)
 {
     extern __shared__ uint32_t table[];
-    __shared__ uint32_t distinct, longest;
-    const uint32_t nnz = __ldg(row_ptr + a.M);
-    for (uint32_t q = blockIdx.x; q < a.num_panels; q += gridDim.x) {
-        const uint32_t r0 = q * kPanelRows, r1 = min(a.M, r0 + kPanelRows);
-        const uint32_t j0 = min(__ldg(row_ptr + r0), nnz), j1 = min(max(__ldg(row_ptr + r1), j0), nnz), n = j1 - j0;
-        if (threadIdx.x == 0) distinct = longest = 0;
-        __syncthreads();
-        if (threadIdx.x < r1 - r0) {
-            const uint32_t b = __ldg(row_ptr + r0 + threadIdx.x), e = __ldg(row_ptr + r0 + threadIdx.x + 1);
-            atomicMax(&longest, e > b ? e - b : 0u);
-        }
-        const bool fits = n <= a.most;
-        const uint32_t size = hash_size(n, a.table_words);
-        if (fits) for (uint32_t i = threadIdx.x; i < size; i += kCensusThreads) table[i] = 0xffffffffu;
-        __syncthreads();
-        const bool candidate = n != 0 && fits && (a.force || longest <= a.split_nnz);
-        uint32_t mine = 0;
-        if (candidate) hash_insert(table, size, n, [&](uint32_t i) { return __ldg(cols + j0 + i); }, [&](uint32_t) { ++mine; });
-        mine = __reduce_add_sync(kFullMask, mine);
-        if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&distinct, mine);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const uint32_t nc = distinct, padded = (nc + kBrickCols - 1) / kBrickCols * kBrickCols;
-            // fill of the panel's 16 x padded dense image, the expression of choose_panel_paths (plan.cpp)
-            const bool brick = candidate && (a.force || (float)n / (float)(kPanelRows * padded) >= a.density);
-            a.ncols[q] = nc;
-            a.path[q] = brick ? 1 : 0;
-            if (!fits) atomicAdd(&a.totals->too_large, 1u);
-            if (brick) {
-                const uint32_t nb = padded / kBrickCols;
-                atomicAdd(&a.seg_panels[r0 / kTileSegmentRows], 1u);
-                atomicAdd(&a.seg_slots[r0 / kTileSegmentRows], (nb + 3) / 4 * 4);
-                atomicAdd(&a.totals->bricks, (unsigned long long)nb);
-                atomicAdd(&a.totals->brick_cost, (unsigned long long)n + (r1 - r0) * kRowCost);
-                atomicMax(&a.totals->brick_nnz_max, n);
-                atomicMax(&a.totals->brick_cols_max, nc);
+    __shared__ uint32_t distinct, big[kCensusWarps];
+    const uint32_t nnz = __ldg(row_ptr + a.M), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t quarter = a.table_words / kCensusWarps;
+    uint32_t *mine = table + warp * quarter;
+    for (uint32_t q0 = blockIdx.x * kCensusWarps; q0 < a.num_panels; q0 += gridDim.x * kCensusWarps) {
+        const uint32_t q = q0 + warp, r0 = q * kPanelRows;
+        bool large = false;
+        if (q < a.num_panels) {  // uniform across the warp
+            const uint32_t r1 = min(a.M, r0 + kPanelRows);
+            const uint32_t p = __ldg(row_ptr + min(r0 + lane, r1)), p_next = __shfl_down_sync(kFullMask, p, 1);
+            const uint32_t longest = __reduce_max_sync(kFullMask, lane < r1 - r0 && p_next > p ? p_next - p : 0u);
+            const uint32_t j0 = min(__shfl_sync(kFullMask, p, 0), nnz), j1 = min(max(__shfl_sync(kFullMask, p, (int)(r1 - r0)), j0), nnz), n = j1 - j0;
+            const bool candidate = n != 0 && n <= a.most && (a.force || longest <= a.split_nnz);
+            if (n > a.most && lane == 0) atomicAdd(&a.totals->too_large, 1u);
+            const uint32_t size = hash_size(n, quarter);
+            large = candidate && n > kWarpPanelNnz;
+            if (!large) {
+                uint32_t got = 0;
+                if (candidate) {
+                    for (uint32_t i = lane; i < size; i += 32) mine[i] = 0xffffffffu;
+                    __syncwarp();
+                    hash_insert(mine, size, n, lane, 32, [&](uint32_t i) { return __ldg(cols + j0 + i); }, [&](uint32_t) { ++got; });
+                }
+                got = __reduce_add_sync(kFullMask, got);
+                if (lane == 0) census_result(a, q, n, got, candidate);
+                __syncwarp();
             }
+        }
+        if (lane == 0) big[warp] = large;
+        __syncthreads();
+        for (uint32_t w = 0; w < kCensusWarps; ++w) {
+            if (!big[w]) continue;  // uniform across the block
+            const uint32_t qq = q0 + w, j0 = min(__ldg(row_ptr + qq * kPanelRows), nnz),
+                           j1 = min(max(__ldg(row_ptr + min(a.M, qq * kPanelRows + kPanelRows)), j0), nnz), n = j1 - j0, size = hash_size(n, a.table_words);
+            if (tid == 0) distinct = 0;
+            for (uint32_t i = tid; i < size; i += kCensusThreads) table[i] = 0xffffffffu;
+            __syncthreads();
+            uint32_t got = 0;
+            hash_insert(table, size, n, tid, kCensusThreads, [&](uint32_t i) { return __ldg(cols + j0 + i); }, [&](uint32_t) { ++got; });
+            got = __reduce_add_sync(kFullMask, got);
+            if (lane == 0 && got) atomicAdd(&distinct, got);
+            __syncthreads();
+            if (tid == 0) census_result(a, qq, n, distinct, true);
+            __syncthreads();
         }
         __syncthreads();
     }
@@ -470,7 +536,7 @@ __global__ void __launch_bounds__(kCensusThreads) brick_fill_kernel(const uint32
         uint4 *rec4 = reinterpret_cast<uint4 *>(brecs + (size_t)f * kBrickRecWords);
         for (uint32_t k = tid; k < nslots * (kBrickRecWords / 4); k += kCensusThreads) rec4[k] = make_uint4(0u, 0u, 0u, 0u);
         __syncthreads();
-        hash_insert(table, size, n, [&](uint32_t k) { return __ldg(&pairs[j0 + k].x); }, [&](uint32_t h) { list[atomicAdd(&count, 1u)] = table[h]; });
+        hash_insert(table, size, n, tid, kCensusThreads, [&](uint32_t k) { return __ldg(&pairs[j0 + k].x); }, [&](uint32_t h) { list[atomicAdd(&count, 1u)] = table[h]; });
         __syncthreads();
         for (uint32_t k = 2; k <= sorted; k <<= 1)
             for (uint32_t j = k >> 1; j > 0; j >>= 1) {
@@ -598,6 +664,7 @@ cudaError_t launch_lists_count(const uint32_t *row_ptr, const ListArgs &a, cudaS
 
 cudaError_t launch_lists_scan(const uint32_t *row_ptr, const ListArgs &a, uint32_t *counters, uint32_t how_many, cudaStream_t s)
 {
+    if (a.num_segments) lists_compose_kernel<<<(a.num_segments + kGroup - 1) / kGroup, kListThreads, 0, s>>>(a);
     lists_scan_kernel<<<1 + how_many, 1024, 0, s>>>(row_ptr, a, counters);
     return cudaGetLastError();
 }
@@ -618,7 +685,7 @@ cudaError_t launch_panel_census(const uint32_t *row_ptr, const uint32_t *cols, C
     const int smem = (int)a.table_words * 4;
     cudaError_t e = allow_dynamic_smem<panel_census_kernel>(16384 * 4);
     if (e != cudaSuccess) return e;
-    const uint32_t blocks = std::min(a.num_panels, (uint32_t)sm_count * 16);
+    const uint32_t blocks = std::min((a.num_panels + kCensusWarps - 1) / kCensusWarps, (uint32_t)sm_count * 16);
     panel_census_kernel<<<blocks, kCensusThreads, smem, s>>>(row_ptr, cols, a);
     return cudaGetLastError();
 }
@@ -655,8 +722,7 @@ cudaError_t launch_brick_fill(const uint32_t *row_ptr, const void *pairs, uint32
                               int sm_count, cudaStream_t s)
 {
     if (num_brick_panels == 0) return cudaSuccess;
-    uint32_t table = 128, list = 1;
-    while (table < nnz_max + nnz_max / 3) table <<= 1;
+    uint32_t table = hash_size(nnz_max, 16384), list = 1;
     while (list < cols_max) list <<= 1;
     list = (list + 3) / 4 * 4;
     const uint32_t map = (cols_max + kBrickCols - 1) / kBrickCols * 4;

@@ -23,15 +23,26 @@ namespace {
 // ---- memory of device-built plans ----------------------------------------------------------------------------------
 // A program whose graph changes from step to step makes and drops a plan per step; cudaMalloc and cudaFree (which waits
 // for the whole device) would be most of its time.  So these plans' memory comes from a stream-ordered pool of the
-// library's own, one per device, thread-safe in the driver.  The pool keeps at most kPoolKeeps bytes it does not need
-// across a synchronisation (larger plans go back to the driver), and everything when an allocation fails or
-// cutespmm_release_memory is called.
-constexpr uint64_t kPoolKeeps = 512ull << 20;
+// library's own, one per device, thread-safe in the driver.  The pool keeps at most kPoolKeeps bytes beyond what
+// living plans hold across a synchronisation (the rest goes back to the driver), and gives them up when an allocation
+// fails or cutespmm_release_memory is called.
+constexpr uint64_t kPoolKeeps = 512ull << 20, kPoolStep = 128ull << 20;
 constexpr int kMaxDevices = 64;
 
 std::mutex g_device_mutex;
 cudaMemPool_t g_pool[kMaxDevices] = {};
+uint64_t g_pool_live[kMaxDevices] = {}, g_pool_threshold[kMaxDevices] = {};
 int g_sm_count[kMaxDevices] = {};
+
+// Bytes of living plans changed: the driver's threshold counts them too, so it moves along (in steps, to be set rarely).
+void note_live(int dev, int64_t change)
+{
+    std::lock_guard<std::mutex> lock(g_device_mutex);
+    g_pool_live[dev] += (uint64_t)change;
+    uint64_t want = (g_pool_live[dev] + kPoolStep - 1) / kPoolStep * kPoolStep + kPoolKeeps - kPoolStep;
+    if (g_pool[dev] && want != g_pool_threshold[dev] && cudaMemPoolSetAttribute(g_pool[dev], cudaMemPoolAttrReleaseThreshold, &want) == cudaSuccess)
+        g_pool_threshold[dev] = want;
+}
 
 cudaError_t device_pool(int dev, cudaMemPool_t *pool)
 {
@@ -43,8 +54,6 @@ cudaError_t device_pool(int dev, cudaMemPool_t *pool)
         props.location.id = dev;
         cudaError_t e = cudaMemPoolCreate(&g_pool[dev], &props);
         if (e != cudaSuccess) { g_pool[dev] = nullptr; return e; }
-        uint64_t keep = kPoolKeeps;
-        if ((e = cudaMemPoolSetAttribute(g_pool[dev], cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) return e;
     }
     *pool = g_pool[dev];
     return cudaSuccess;
@@ -108,13 +117,14 @@ int cutespmm_internal_usable_device(int *dev, int *sm_count)
 // The block of a device-built plan goes back to the pool.  cudaFree waited for everything on the device; here the block
 // is handed back in the order of the default stream, which is enough for a plan that ran on no other (stream handles
 // of a caller may be gone by now, so nothing can be recorded on them), and after a wait for the device otherwise.
-void cutespmm_internal_free_block(void *block, bool used_elsewhere)
+void cutespmm_internal_free_block(void *block, uint64_t bytes, int dev, bool used_elsewhere)
 {
     if (used_elsewhere) cudaDeviceSynchronize();
     if (cudaFreeAsync(block, nullptr) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(block);
     }
+    note_live(dev, -(int64_t)bytes);
 }
 
 namespace {
@@ -274,8 +284,9 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
     cudaError_t e;
     Temp temp(s);
     BuildTotals *d_totals = nullptr, *d_totals2 = nullptr;
-    uint32_t *counters = nullptr, *counters2 = nullptr, *where = nullptr, *where2 = nullptr, *ncols = nullptr;
-    uint16_t *tables = nullptr;  // shared by the two lists: the first is through with them when the second counts
+    uint32_t *counters = nullptr, *counters2 = nullptr, *path_tiles = nullptr, *group_tiles = nullptr, *ncols = nullptr;
+    uint2 *group_entry = nullptr;
+    uint16_t *tables = nullptr, *path_entry = nullptr, *group_exit = nullptr;
     uint8_t *path = nullptr;
     auto carve_temp = [&](Carver &c) {
         c.take(d_totals, 1);
@@ -283,9 +294,14 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
         c.take(counters, 4ull * segments);  // chunks, long rows, brick panels, brick slots
         const uint64_t zeroed = c.used;
         c.take(counters2, census ? 2ull * segments : 0);
-        c.take(where, 2ull * segments);
-        c.take(where2, census ? 2ull * segments : 0);
-        c.take(tables, 2ull * segments * kSegmentEntries);
+        // the tables of both lists (the second only where there may be one)
+        const uint64_t lists = census ? 2 : 1, entries = lists * segments * kSegmentEntries, groups = lists * (segments / 32 + 1);
+        c.take(tables, 2 * entries);
+        c.take(path_entry, entries);
+        c.take(path_tiles, entries);
+        c.take(group_exit, groups * kSegmentEntries);
+        c.take(group_tiles, groups * kSegmentEntries);
+        c.take(group_entry, groups);
         c.take(ncols, census ? P : 0);
         c.take(path, census ? P : 0);
         return zeroed;
@@ -299,8 +315,14 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
     ListArgs la{};
     la.M = M; la.num_segments = segments;
     la.split_nnz = h.opts.split_nnz; la.tile_nnz = h.opts.tile_nnz; la.adaptive = h.adaptive_tiling ? 1u : 0u;
-    la.exits = tables; la.tile_counts = tables + (uint64_t)segments * kSegmentEntries;
-    la.seg_entry = where; la.seg_tiles = where + segments;
+    auto set_tables = [&](ListArgs &l, uint64_t list) {
+        const uint64_t entries = (uint64_t)segments * kSegmentEntries, groups = segments / 32 + 1;
+        l.exits = tables + 2 * list * entries; l.tile_counts = l.exits + entries;
+        l.path_entry = path_entry + list * entries; l.path_tiles = path_tiles + list * entries;
+        l.group_exit = group_exit + list * groups * kSegmentEntries; l.group_tiles = group_tiles + list * groups * kSegmentEntries;
+        l.group_entry = group_entry + list * groups;
+    };
+    set_tables(la, 0);
     la.seg_chunks = counters; la.seg_longs = counters + segments;
     la.totals = d_totals;
     CensusArgs ca{};
@@ -332,7 +354,7 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
         la2.path = path;
         la2.total_known = 1;
         la2.total = h.nnz + (uint64_t)kRowCost * M - t.brick_cost;
-        la2.seg_entry = where2; la2.seg_tiles = where2 + segments;
+        set_tables(la2, 1);
         la2.seg_chunks = counters2; la2.seg_longs = counters2 + segments;
         la2.totals = d_totals2;
         BuildTotals t2{};
@@ -378,6 +400,8 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
     Carver need;
     carve(need);
     if ((e = pool_alloc(&p->d_block, need.used, dev, s)) != cudaSuccess) return fail_cuda_status(e, "memory of the plan");
+    p->block_bytes = need.used;
+    note_live(dev, (int64_t)need.used);
     Carver c;
     c.base = static_cast<char *>(p->d_block);
     const uint64_t zero = carve(c);

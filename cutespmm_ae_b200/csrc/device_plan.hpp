@@ -110,7 +110,7 @@ constexpr uint32_t kRowPtrSlack = 8;  // row pointers repeated behind the last o
 // the census of path auto, which looks at panels without long rows only: 16 rows of at most kMaxSplitNnz nonzeros.
 constexpr uint32_t kDevPanelMax = 8192, kMaxCensusNnz = 6144;
 
-constexpr uint32_t kTileSegmentRows = 2048;  // rows a block of the list kernels looks at; a multiple of kPanelRows
+constexpr uint32_t kTileSegmentRows = 512;   // rows a block of the list kernels looks at; a multiple of kPanelRows
 constexpr uint32_t kSegmentEntries = 257;    // kMaxTileRows + 1: rows of a segment its first tile can start at
 
 struct BuildTotals {  // one per plan creation, read by the host after the counting kernels
@@ -125,9 +125,13 @@ struct ListArgs {
     uint32_t split_nnz, tile_nnz, adaptive;
     uint32_t total_known;   // 1: `total` is the cost of the listed rows; 0: every row is listed, nnz + kRowCost * M
     uint64_t total;
-    const uint8_t *path;    // per panel: 1 = not listed (nullptr: every row is)
+    const uint8_t *path;   // per panel: 1 = not listed (nullptr: every row is)
     uint16_t *exits, *tile_counts;  // per segment and entry row: entry row of the next segment, tiles
-    uint32_t *seg_entry, *seg_tiles;   // per segment: the entry row, its first tile
+    uint16_t *path_entry;   // per segment and entry row of its group: entry row of the segment ...
+    uint32_t *path_tiles;   // ... and tiles of the group in front of it
+    uint16_t *group_exit;   // per group and entry row: entry row of the next group, tiles
+    uint32_t *group_tiles;
+    uint2 *group_entry;     // per group: real entry row, its first tile
     uint32_t *seg_chunks, *seg_longs;  // per segment: counts, then offsets
     BuildTotals *totals;
     Tile *tiles;

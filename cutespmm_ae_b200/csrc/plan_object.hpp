@@ -32,13 +32,14 @@ struct cutespmm_list_sizes {
 };
 
 // Gives the memory of a device-built plan back.  device_plan.cu
-void cutespmm_internal_free_block(void *block, bool used_elsewhere);
+void cutespmm_internal_free_block(void *block, uint64_t bytes, int dev, bool used_elsewhere);
 
 struct cutespmm_plan {
     cutespmm::HostPlan host;
     cutespmm_list_sizes own, every;  // of the list of the rows outside the tensor-core panels / of the list of every row
     // device-built plans: one block holds every array; the lists come to the host on demand
     void *d_block = nullptr;
+    uint64_t block_bytes = 0;
     bool lists_on_host = true, views_tried = false;
     std::mutex fetch_mutex;
     mutable std::atomic<bool> used_elsewhere{false};  // ran on a stream that is not the default stream
@@ -85,7 +86,7 @@ struct cutespmm_plan {
         int cur = -1;
         cudaGetDevice(&cur);
         if (cur != device) cudaSetDevice(device);
-        if (d_block) cutespmm_internal_free_block(d_block, used_elsewhere);
+        if (d_block) cutespmm_internal_free_block(d_block, block_bytes, device, used_elsewhere);
         else if (!host.device_built || lists_on_host)
             for (void *p : {d_row_ptr, d_pairs, d_tiles, d_chunks, d_long_rows, d_tiles_all, d_chunks_all, d_long_rows_all,
                             d_bcols, d_brecs, d_panel_first, d_panel_last, d_scols, d_srecs, d_srec_off, d_sfirst,

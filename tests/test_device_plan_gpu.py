@@ -162,10 +162,10 @@ def test_saved_plan_gives_the_same_product_after_loading(tmp_path, how):
 
 
 @pytest.mark.parametrize("M,lengths,path,min_bricks", [
-    (2047, "short", cs.PATH_ROWS, 0), (2048, "short", cs.PATH_ROWS, 0), (2049, "short", cs.PATH_ROWS, 0),   # edges of a segment of rows
+    (511, "short", cs.PATH_ROWS, 0), (512, "short", cs.PATH_ROWS, 0), (2049, "short", cs.PATH_ROWS, 0),   # edges of a segment of rows
     (4096 + 17, "empty", cs.PATH_ROWS, 0),     # 256-row tiles that reach into the next segment, runs of empty rows
     (6000, "long", cs.PATH_ROWS, 0),           # long rows on both sides of every segment edge, next to each other
-    (2048 * 33 + 5, "short", cs.PATH_ROWS, 0),  # more segments than one batch of the walk through them
+    (512 * 16 * 33 + 5, "short", cs.PATH_ROWS, 0),  # more groups of segments than one batch of the walk through them
     (5000, "mixed", cs.PATH_AUTO, 1),          # tensor-core panels between row-kernel panels, duplicates inside
 ])
 def test_device_cut_work_lists_equal_the_host_builder_s(oracle_mod, M, lengths, path, min_bricks):
@@ -176,7 +176,7 @@ def test_device_cut_work_lists_equal_the_host_builder_s(oracle_mod, M, lengths, 
         ln[rng.random(M) < 0.9] = 0
         ln[1000:3000] = 0
     if lengths == "long":
-        for at in (0, 1, 2046, 2047, 2048, 2049, 4095, 4096, M - 1):
+        for at in (0, 1, 510, 511, 512, 513, 2047, 2048, 4096, M - 1):
             ln[at] = 300 + at % 7
     rp = np.concatenate([[0], np.cumsum(ln)])
     cols = rng.integers(0, K, rp[-1])
