@@ -127,3 +127,22 @@ def test_set_values_is_refused_where_the_values_live_in_tensor_core_records_or_r
     p = cs.Plan.from_csr(S, path=cs.PATH_ROWS)
     with pytest.raises(ValueError):
         p.set_values(torch.ones(S.nnz + 1, device="cuda"))
+
+
+@pytest.mark.parametrize("N", [1, 3, 4, 15, 16, 17, 28, 32, 33, 60, 64, 65, 68, 96, 97, 124, 128, 132, 256])
+@pytest.mark.parametrize("per_row", [3, 21])
+def test_sddmm_at_the_edges_of_every_span(oracle_mod, N, per_row):
+    """Spans of 16, 32, 64, 96 and 128 columns, whole and ragged, aligned and not; rows short enough for the flat form and
+    long enough for a warp per row; a hub row beside them and tiles whose last claim is a part of 32 nonzeros."""
+    ln = np.full(230, per_row)
+    ln[7], ln[100:110] = 400, 0
+    rng = np.random.default_rng(N)
+    rp = np.concatenate([[0], np.cumsum(ln)])
+    A = g.CsrMatrix(230, 500, torch.from_numpy(rp), torch.from_numpy(rng.integers(0, 500, rp[-1]).astype(np.int32)),
+                    torch.from_numpy(rng.standard_normal(rp[-1]).astype(np.float32)))
+    p = cs.Plan.from_device_csr(A.M, A.K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS)
+    X, Y = g.dense_operand(A.M, N, 62, device="cuda"), g.dense_operand(A.K, N, 63, device="cuda")
+    out = torch.full((A.nnz,), float("nan"), device="cuda")
+    p.sddmm(X, Y, out, scale_by_values=True)
+    want = oracle_mod.sddmm_csr(A.row_ptr, A.cols, A.vals, X.cpu().numpy(), Y.cpu().numpy())
+    assert rel(want, out.cpu().numpy()) <= TOL and p.device_status() == 0
