@@ -320,7 +320,7 @@ int cutespmm_plan_decode_csr(const cutespmm_plan_t *p, uint64_t *rowPtr, uint32_
 }
 
 static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B, uint64_t ldb, float *C, uint64_t ldc,
-                          uint32_t N, const cutespmm_item_range *rg = nullptr)
+                          uint32_t N, bool b_padded, const cutespmm_item_range *rg = nullptr)
 {
     const HostPlan &h = p->host;
     RowsArgs a{};
@@ -340,6 +340,7 @@ static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B,
     a.N = N;
     a.status = p->d_status;
     a.row_map = static_cast<const uint32_t *>(p->d_row_map);
+    a.b_padded = b_padded ? 1u : 0u;
     if (rg) {  // a sub-range of the lists: 16-byte tiles and chunks (a chunk names its scratch slot and, through it, its long row)
         const uint32_t t0 = all_rows ? rg->ta0 : rg->t0, t1 = all_rows ? rg->ta1 : rg->t1;
         const uint32_t c0 = all_rows ? rg->ca0 : rg->c0, c1 = all_rows ? rg->ca1 : rg->c1;
@@ -447,7 +448,7 @@ int cutespmm_spmm_launch_count(const cutespmm_plan_t *p, uint32_t N)
 int cutespmm_spmm(const cutespmm_plan_t *p, const float *B, uint64_t ldb, float *C, uint64_t ldc, uint32_t N,
                   void *stream)
 {
-    return cutespmm_internal_spmm_range(p, B, ldb, C, ldc, N, stream, nullptr);
+    return cutespmm_internal_spmm_range(p, B, ldb, C, ldc, N, stream, nullptr, false);
 }
 
 }  // extern "C"
@@ -458,8 +459,29 @@ static void note_stream(const cutespmm_plan *p, cudaStream_t s)
     if (s != nullptr && s != cudaStreamLegacy && !p->used_elsewhere.load(std::memory_order_relaxed)) p->used_elsewhere = true;
 }
 
+// Rows of B that are not 16-byte aligned (N not a multiple of four columns, a view) cost the row kernel four times the
+// load instructions, each for a quarter of the bytes, and there is no form for several rows per warp.  Where the matrix
+// names a row of B often enough it pays to copy B once into rows of N rounded up to four (the copy lives on the stream):
+// measured, the row kernel gains about 12 ps per nonzero up to 64 columns and 0.4 ps per nonzero and column beyond (R-MAT
+// 2^18 N = 47: 186 -> 139 us, uniform 7 per row N = 201: 211 -> 125 us), the copy costs a launch and 8 bytes per element at
+// 6.4 TB/s.  Even widths above 32 are read two columns per lane and gain nothing.  Not while the stream is being captured
+// (a graph should not own memory).
+static bool worth_padding(const HostPlan &h, const float *B, uint64_t ldb, const float *C, uint64_t ldc, uint32_t N, cudaStream_t s)
+{
+    const bool two = !((reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 7) && !((ldb | ldc | N) & 1);
+    if (two && N > 32) return false;
+    const uint64_t gain = h.nnz * (N <= 64 ? 12 : N * 2 / 5), cost = 3000000 + h.K * N * 5 / 4;  // picoseconds
+    if (gain < cost) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return cap == cudaStreamCaptureStatusNone;
+}
+
 int cutespmm_internal_spmm_range(const cutespmm_plan *p, const float *B, uint64_t ldb, float *C, uint64_t ldc, uint32_t N, void *stream,
-                                 const cutespmm_item_range *rg)
+                                 const cutespmm_item_range *rg, bool b_padded)
 {
     if (!p) return fail(CUTESPMM_EINVAL, "plan is NULL");
     if (!p->on_device) return fail(CUTESPMM_EUNSUPPORTED, "host-only plan: build it with cutespmm_plan_create on a CUDA device to execute it");
@@ -492,8 +514,27 @@ int cutespmm_internal_spmm_range(const cutespmm_plan *p, const float *B, uint64_
         }
         // brick panels whose shape the brick kernel does not take (N not a multiple of 32, unaligned
         // operands) are executed by the row kernel from its all-rows work list
-        RowsArgs ra = rows_args(p, (!brick && p->host.num_bricks) || (!slab && p->host.slab_panels), B + n0, ldb, C + n0, ldc, nw, rg);
-        if ((e = launch_rows(ra, p->sm_count, s)) != cudaSuccess) return fail_cuda(e, "row kernel launch");
+        const bool all_rows = (!brick && p->host.num_bricks) || (!slab && p->host.slab_panels);
+        const float *Bw = B + n0;
+        uint64_t ldw = ldb;
+        float *copy = nullptr;
+        const cutespmm_list_sizes &list = all_rows ? p->every : p->own;
+        const bool aligned = !(reinterpret_cast<uintptr_t>(Bw) & 15) && !(ldb & 3) && (!(nw & 3) || b_padded);
+        if (!aligned && (list.tiles || list.chunks) && !rg && worth_padding(p->host, Bw, ldb, C + n0, ldc, nw, s)) {
+            ldw = (nw + 3) / 4 * 4;
+            if (cutespmm_internal_pool_alloc(reinterpret_cast<void **>(&copy), p->host.K * ldw * sizeof(float), p->device, s) == cudaSuccess) {
+                if ((e = launch_pad_rows(Bw, ldb, copy, p->host.K, nw, p->sm_count, s)) != cudaSuccess) return fail_cuda(e, "padding the rows of B");
+                Bw = copy;
+            } else {  // no memory for the copy: the kernel reads B as it is
+                cudaGetLastError();
+                copy = nullptr;
+                ldw = ldb;
+            }
+        }
+        RowsArgs ra = rows_args(p, all_rows, Bw, ldw, C + n0, ldc, nw, copy || b_padded, rg);
+        e = launch_rows(ra, p->sm_count, s);
+        if (copy) cudaFreeAsync(copy, s);
+        if (e != cudaSuccess) return fail_cuda(e, "row kernel launch");
     }
     return CUTESPMM_OK;
 }

@@ -46,6 +46,7 @@ void note_live(int dev, int64_t change)
 
 cudaError_t device_pool(int dev, cudaMemPool_t *pool)
 {
+    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lock(g_device_mutex);
     if (!g_pool[dev]) {
         cudaMemPoolProps props{};
@@ -57,18 +58,6 @@ cudaError_t device_pool(int dev, cudaMemPool_t *pool)
     }
     *pool = g_pool[dev];
     return cudaSuccess;
-}
-
-cudaError_t pool_alloc(void **p, uint64_t bytes, int dev, cudaStream_t s)
-{
-    cudaMemPool_t pool = nullptr;
-    cudaError_t e = device_pool(dev, &pool);
-    if (e != cudaSuccess) return e;
-    if ((e = cudaMallocFromPoolAsync(p, bytes, pool, s)) != cudaErrorMemoryAllocation) return e;
-    cudaGetLastError();
-    cudaStreamSynchronize(s);
-    cudaMemPoolTrimTo(pool, 0);
-    return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
 
 // Hands out 256-byte aligned parts of one block.
@@ -90,6 +79,18 @@ struct Temp {  // stream-ordered scratch of one call
 };
 
 }  // namespace
+
+cudaError_t cutespmm_internal_pool_alloc(void **p, uint64_t bytes, int dev, cudaStream_t s)
+{
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = device_pool(dev, &pool);
+    if (e != cudaSuccess) return e;
+    if ((e = cudaMallocFromPoolAsync(p, bytes, pool, s)) != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    cudaStreamSynchronize(s);
+    cudaMemPoolTrimTo(pool, 0);
+    return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
 
 // The current device, checked to be one this library runs on (the properties are read once per device).
 int cutespmm_internal_usable_device(int *dev, int *sm_count)
@@ -308,7 +309,7 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
     };
     Carver sizes;
     carve_temp(sizes);
-    if ((e = pool_alloc(&temp.p, sizes.used, dev, s)) != cudaSuccess) return fail_cuda_status(e, "scratch of the plan creation");
+    if ((e = cutespmm_internal_pool_alloc(&temp.p, sizes.used, dev, s)) != cudaSuccess) return fail_cuda_status(e, "scratch of the plan creation");
     Carver at;
     at.base = static_cast<char *>(temp.p);
     const uint64_t zeroed = carve_temp(at);
@@ -399,7 +400,7 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
     };
     Carver need;
     carve(need);
-    if ((e = pool_alloc(&p->d_block, need.used, dev, s)) != cudaSuccess) return fail_cuda_status(e, "memory of the plan");
+    if ((e = cutespmm_internal_pool_alloc(&p->d_block, need.used, dev, s)) != cudaSuccess) return fail_cuda_status(e, "memory of the plan");
     p->block_bytes = need.used;
     note_live(dev, (int64_t)need.used);
     Carver c;

@@ -39,11 +39,15 @@ struct RowsArgs {
     float *scratch;            // partial sums, leading dimension ld_scratch
     uint64_t ldb, ldc, ld_scratch;
     uint32_t N;
+    uint32_t b_padded;         // 1: a row of B can be read up to N rounded up to four columns
+    uint32_t c_scalar;         // set by launch_rows: C is written column by column
     uint32_t *status;          // device status word: set to 1 when a bounded wait gives up
     const uint32_t *row_map;   // reordered plan: row r of the work lists is row row_map[r] of C (nullptr: identity)
 };
 
 cudaError_t launch_rows(const RowsArgs &a, int sm_count, cudaStream_t s);
+// dst: rows x (N rounded up to 4) floats, 16-byte aligned
+cudaError_t launch_pad_rows(const float *src, uint64_t ld_src, float *dst, uint64_t rows, uint32_t N, int sm_count, cudaStream_t s);
 int rows_kernel_count(const RowsArgs &a);
 
 // Arguments of the SDDMM kernel (sddmm_kernel.cu): out[j] = (scale ? value of nonzero j : 1) * <X[row of j], Y[column of j]>.

@@ -120,6 +120,10 @@ int cutespmm_internal_usable_device(int *dev, int *sm_count);
 int cutespmm_internal_fetch_lists(const cutespmm_plan *p);
 int cutespmm_internal_fetch_views(const cutespmm_plan *p, std::vector<uint32_t> *ncols, std::vector<uint32_t> *acols);
 
-// cutespmm_spmm restricted to a range of work items (nullptr: everything).  capi.cu
+// Memory of the library's pool on `dev` in the order of stream s (cudaFreeAsync gives it back).
+cudaError_t cutespmm_internal_pool_alloc(void **p, uint64_t bytes, int dev, cudaStream_t s);
+
+// cutespmm_spmm restricted to a range of work items (nullptr: everything).  b_padded: rows of B can be read up to N rounded up
+// to four columns.  capi.cu
 int cutespmm_internal_spmm_range(const cutespmm_plan *p, const float *B, uint64_t ldb, float *C, uint64_t ldc, uint32_t N, void *stream,
-                                 const cutespmm_item_range *range);
+                                 const cutespmm_item_range *range, bool b_padded);

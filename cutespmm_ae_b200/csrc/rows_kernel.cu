@@ -66,9 +66,22 @@ __device__ __forceinline__ void zero_vec(float4 &a) { a = make_float4(0.f, 0.f, 
 __device__ __forceinline__ void zero_vec(float2 &a) { a = make_float2(0.f, 0.f); }
 __device__ __forceinline__ void zero_vec(float &a) { a = 0.f; }
 
-__device__ __forceinline__ void store_stream(float4 *p, const float4 &v) { __stcs(p, v); }
-__device__ __forceinline__ void store_stream(float2 *p, const float2 &v) { __stcs(p, v); }
-__device__ __forceinline__ void store_stream(float *p, const float &v) { __stcs(p, v); }
+// This lane's columns of a row of C: one vector store where C allows it, single columns up to N otherwise (C with rows that
+// are not 16-byte aligned under a padded copy of B).
+template <bool FULL>
+__device__ __forceinline__ void store_row(float *p, const float4 &v, bool scalar, uint32_t cols)
+{
+    if (FULL || !scalar) {
+        __stcs(reinterpret_cast<float4 *>(p), v);
+    } else {
+        __stcs(p, v.x);
+        if (cols > 1) __stcs(p + 1, v.y);
+        if (cols > 2) __stcs(p + 2, v.z);
+        if (cols > 3) __stcs(p + 3, v.w);
+    }
+}
+template <bool FULL> __device__ __forceinline__ void store_row(float *p, const float2 &v, bool, uint32_t) { __stcs(reinterpret_cast<float2 *>(p), v); }
+template <bool FULL> __device__ __forceinline__ void store_row(float *p, const float &v, bool, uint32_t) { __stcs(p, v); }
 
 // acc[ch] += sum over nonzeros [j0, j1) of val * B[col][lane's columns].  `bl` points at this lane's
 // first column of row 0 of B; ok[ch] says whether the lane's ch-th column group exists (ragged N).
@@ -200,6 +213,7 @@ struct ChunkArgs {
     float *scratch, *C;
     uint64_t ldb, ld_scratch, ldc;
     uint32_t num_chunks, N, col0;
+    bool c_scalar;
 };
 
 // A chunk's partial sum goes to its slot of the scratch matrix; the warp (or group) that completes a row's last
@@ -274,7 +288,7 @@ __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
                 float *crow = a.C + (uint64_t)lr_row * a.ldc;
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch)
-                    if (FULL || ok[ch]) store_stream(reinterpret_cast<V *>(crow + ch * 32 * VEC), acc[ch]);
+                    if (FULL || ok[ch]) store_row<FULL>(crow + ch * 32 * VEC, acc[ch], a.c_scalar, a.N - a.col0 - ch * 32 * VEC);
             }
         } else {
             // The whole warp adds the slots of every row one of its groups completed: group h takes slots h, h+G, ...
@@ -296,7 +310,7 @@ __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
                         acc[0].z += __shfl_xor_sync(kFull, acc[0].z, off);
                         acc[0].w += __shfl_xor_sync(kFull, acc[0].w, off);
                     }
-                    if (grp == 0 && (FULL || ok[0])) store_stream(reinterpret_cast<V *>(a.C + (uint64_t)row * a.ldc), acc[0]);
+                    if (grp == 0 && (FULL || ok[0])) store_row<FULL>(a.C + (uint64_t)row * a.ldc, acc[0], a.c_scalar, a.N - a.col0);
                 }
             }
         }
@@ -332,7 +346,7 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::kMinBlocks) spmm_ro
     if (a.num_chunks)
         run_chunks<VEC, CH, FULL, DEEP, G>(ChunkArgs{pairs, reinterpret_cast<const uint4 *>(a.chunks), reinterpret_cast<const uint4 *>(a.long_rows),
                                                      a.chunk_owner, a.arrivals, bl, a.scratch + col0, a.C + col0, a.ldb, a.ld_scratch, a.ldc,
-                                                     a.num_chunks, a.N, col0});
+                                                     a.num_chunks, a.N, col0, a.c_scalar != 0});
 
     for (uint32_t i = 0;; ++i) {
         const uint64_t t = blockIdx.x + (uint64_t)i * gridDim.x;
@@ -367,7 +381,7 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::kMinBlocks) spmm_ro
                 float *out = a.C + (uint64_t)r_out * a.ldc + col0;
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch)
-                    if (FULL || ok[ch]) store_stream(reinterpret_cast<V *>(out + ch * 32 * VEC), acc[ch]);
+                    if (FULL || ok[ch]) store_row<FULL>(out + ch * 32 * VEC, acc[ch], a.c_scalar != 0, a.N - col0 - ch * 32 * VEC);
             }
             if constexpr (G > 1) __syncwarp();
         }
@@ -395,38 +409,78 @@ cudaError_t launch_rows_t(const RowsArgs &a, uint32_t slabs, int sm_count, cudaS
     return cudaGetLastError();
 }
 
+// dst (rows x quads float4, 16-byte aligned) = src (rows x N, leading dimension ld_src), padding zeroed.  Bound by memory
+// (each byte once in and once out); a thread keeps its four columns and walks the rows, four in flight.
+__global__ void __launch_bounds__(256) pad_rows_kernel(const float *__restrict__ src, uint64_t ld_src, float4 *__restrict__ dst, uint32_t quads, uint32_t N,
+                                                       uint64_t rows)
+{
+    const uint32_t per_block = 256 / quads, mine = threadIdx.x / quads, c = (threadIdx.x - mine * quads) * 4;
+    if (mine >= per_block) return;
+    const uint64_t step = (uint64_t)gridDim.x * per_block;
+    for (uint64_t r = (uint64_t)blockIdx.x * per_block + mine; r < rows; r += 4 * step) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r + u * step < rows) {
+                const float *p = src + (r + u * step) * ld_src + c;
+                v[u].x = __ldg(p);
+                if (c + 1 < N) v[u].y = __ldg(p + 1);
+                if (c + 2 < N) v[u].z = __ldg(p + 2);
+                if (c + 3 < N) v[u].w = __ldg(p + 3);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (r + u * step < rows) dst[(r + u * step) * quads + c / 4] = v[u];
+    }
+}
+
 }  // namespace
+
+cudaError_t launch_pad_rows(const float *src, uint64_t ld_src, float *dst, uint64_t rows, uint32_t N, int sm_count, cudaStream_t s)
+{
+    const uint32_t quads = (N + 3) / 4;
+    if (rows == 0 || N == 0) return cudaSuccess;
+    const uint64_t per_block = 256 / quads, want = (rows + 4 * per_block - 1) / (4 * per_block), cap = (uint64_t)sm_count * 8;
+    pad_rows_kernel<<<(uint32_t)(want < cap ? want : cap), 256, 0, s>>>(src, ld_src, reinterpret_cast<float4 *>(dst), quads, N, rows);
+    return cudaGetLastError();
+}
 
 int rows_kernel_count(const RowsArgs &a) { return (a.num_tiles || a.num_chunks) ? 1 : 0; }
 
 // Picks the widest vector the pointers, leading dimensions and N allow.
-cudaError_t launch_rows(const RowsArgs &a, int sm_count, cudaStream_t s)
+cudaError_t launch_rows(const RowsArgs &args, int sm_count, cudaStream_t s)
 {
+    RowsArgs a = args;
     if (a.num_tiles == 0 && a.num_chunks == 0) return cudaSuccess;
     const uintptr_t pb = reinterpret_cast<uintptr_t>(a.B), pc = reinterpret_cast<uintptr_t>(a.C),
                     ps = reinterpret_cast<uintptr_t>(a.scratch);
-    const bool v4 = !((pb | pc | ps) & 15) && !((a.ldb | a.ldc | a.ld_scratch | a.N) & 3);
+    // four columns per lane need B's rows aligned and readable to the end of the last four; C is written as it allows
+    const bool v4 = !((pb | ps) & 15) && !((a.ldb | a.ld_scratch) & 3) && ((a.N & 3) == 0 || a.b_padded);
     const bool v2 = !((pb | pc | ps) & 7) && !((a.ldb | a.ldc | a.ld_scratch | a.N) & 1);
+    a.c_scalar = (pc & 15) || ((a.ldc | a.N) & 3);
     const uint32_t N = a.N;
     // deep: at most one resident wave of tiles, or long rows (measured on shards of R-MAT 2^24: 300 nonzeros per row
     // 2.19 vs 2.38 ms, 21 per row 1.88 vs 1.93 ms in favour of deep; 15 per row (R-MAT 2^20) 0.645 vs 0.611 ms and
     // 3.4 per row 1.50 vs 1.48 ms in favour of shallow)
     const bool deep = (uint64_t)a.num_tiles <= (uint64_t)sm_count * 6 || a.avg_row_nnz >= 20;
+    auto full = [&](uint32_t w) { return N % w == 0 && !(v4 && a.c_scalar); };
 #define CUTESPMM_GO(VEC, CH)                                                                   \
     do {                                                                                       \
         const uint32_t w = 32 * VEC * CH, slabs = (N + w - 1) / w;                             \
         if (deep)                                                                              \
-            return (N % w == 0) ? launch_rows_t<VEC, CH, true, true>(a, slabs, sm_count, s)    \
+            return full(w) ? launch_rows_t<VEC, CH, true, true>(a, slabs, sm_count, s)          \
                                 : launch_rows_t<VEC, CH, false, true>(a, slabs, sm_count, s);  \
-        return (N % w == 0) ? launch_rows_t<VEC, CH, true, false>(a, slabs, sm_count, s)       \
+        return full(w) ? launch_rows_t<VEC, CH, true, false>(a, slabs, sm_count, s)             \
                             : launch_rows_t<VEC, CH, false, false>(a, slabs, sm_count, s);     \
     } while (0)
     if (v4 && N <= 64) {  // narrow products: G rows of A per warp, a group of 32/G float4 lanes spans the row of B
 #define CUTESPMM_GROUPS(G)                                                                              \
     do {                                                                                                \
-        if (deep) return (N == 128 / G) ? launch_rows_t<4, 1, true, true, G>(a, 1, sm_count, s)         \
+        if (deep) return full(128 / G) ? launch_rows_t<4, 1, true, true, G>(a, 1, sm_count, s)         \
                                         : launch_rows_t<4, 1, false, true, G>(a, 1, sm_count, s);       \
-        return (N == 128 / G) ? launch_rows_t<4, 1, true, false, G>(a, 1, sm_count, s)                  \
+        return full(128 / G) ? launch_rows_t<4, 1, true, false, G>(a, 1, sm_count, s)                  \
                               : launch_rows_t<4, 1, false, false, G>(a, 1, sm_count, s);                \
     } while (0)
         if (N <= 16) CUTESPMM_GROUPS(8);
@@ -435,14 +489,14 @@ cudaError_t launch_rows(const RowsArgs &a, int sm_count, cudaStream_t s)
 #undef CUTESPMM_GROUPS
     }
     if (v4) {
-        if (N >= 256) CUTESPMM_GO(4, 2);
+        if (N > 128) CUTESPMM_GO(4, 2);
         CUTESPMM_GO(4, 1);
     }
     if (v2 && N > 32) {
-        if (N >= 128) CUTESPMM_GO(2, 2);
+        if (N > 64) CUTESPMM_GO(2, 2);
         CUTESPMM_GO(2, 1);
     }
-    if (N >= 64) CUTESPMM_GO(1, 2);
+    if (N > 32) CUTESPMM_GO(1, 2);
     CUTESPMM_GO(1, 1);
 #undef CUTESPMM_GO
 }

@@ -350,7 +350,7 @@ int run_row_blocks(cutespmm_plan *p, const float *B_host, uint64_t ldb, float *C
         const cutespmm_row_block &b = p->row_blocks[i];
         cudaStreamWaitEvent(s, p->rb_in[i], 0);
         cudaEventRecord(p->rb_k0[i], s);
-        const int st = cutespmm_internal_spmm_range(p, p->d_B, ldd, p->d_C, ldd, N, s, &b.items);
+        const int st = cutespmm_internal_spmm_range(p, p->d_B, ldd, p->d_C, ldd, N, s, &b.items, true);
         if (st != CUTESPMM_OK) {
             drain();
             return st;
@@ -629,7 +629,7 @@ int cutespmm_spmm_sharded_host(cutespmm_plan_t *p, cutespmm_comm_t *comm, const 
             cudaStreamWaitEvent(s, p->ev_in[w], 0);
         }
         cudaEventRecord(p->ev_k0[w], s);
-        st = cutespmm_spmm(p, dB, ldd, dC, ldd, cw, s);
+        st = cutespmm_internal_spmm_range(p, dB, ldd, dC, ldd, cw, s, nullptr, ldd >= (cw + 3) / 4 * 4);
         if (st != CUTESPMM_OK) {
             drain();
             return st;

@@ -384,3 +384,32 @@ def test_host_call_in_blocks_of_rows_on_banded_matrices(oracle_mod, N, pad, path
     Cb, _ = pb.spmm_host(Bb)
     want = oracle_mod.spmm_csr(rp.astype(np.uint64), cols.astype(np.uint32), vals, Bb.numpy(), rows, K2)
     assert oracle_mod.rel_fro(want, Cb.numpy()) <= REL_FRO_TOL
+
+
+@pytest.mark.parametrize("N", [1, 3, 13, 17, 30, 33, 47, 63, 65, 127, 129, 131, 255, 257, 301, 511, 515])
+@pytest.mark.parametrize("hub", [0, 3000])
+def test_widths_that_no_vector_divides_on_jobs_worth_a_padded_copy(oracle_mod, N, hub):
+    """N not a multiple of four columns: small jobs read B column by column, jobs that name a row of B often enough copy it
+    into aligned rows first (both sides of the rule here); C is written column by column up to N; hub rows are summed
+    from pieces.  Views with a gap between the rows and operands off the 16-byte grid take the same ways."""
+    K = 300
+    for M, per_row in ((500, 4), (20000, 40)):
+        ln = np.full(M, per_row)
+        ln[3], ln[4] = max(hub, per_row), 0
+        rng = np.random.default_rng(N)
+        rp = np.concatenate([[0], np.cumsum(ln)])
+        A = g.CsrMatrix(M, K, torch.from_numpy(rp), torch.from_numpy(rng.integers(0, K, rp[-1]).astype(np.int32)),
+                        torch.from_numpy(rng.standard_normal(rp[-1]).astype(np.float32)))
+        p = cs.Plan.from_device_csr(M, K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS)
+        B = g.dense_operand(K, N, 71)
+        want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.numpy(), M, K)
+        out = torch.full((M + 1, N), float("nan"), device="cuda")
+        p.spmm(B.cuda(), out[:M])
+        assert oracle_mod.rel_fro(want, out[:M].cpu().numpy()) <= 2e-6
+        assert torch.isnan(out[M]).all()  # nothing behind the last row
+        big, cbig = torch.zeros((K, N + 3), device="cuda"), torch.full((M, N + 5), 7.0, device="cuda")
+        big[:, 1:N + 1] = B.cuda()
+        p.spmm(big[:, 1:N + 1], cbig[:, 2:N + 2])
+        assert oracle_mod.rel_fro(want, cbig[:, 2:N + 2].cpu().numpy()) <= 2e-6
+        assert (cbig[:, :2] == 7).all() and (cbig[:, N + 2:] == 7).all()  # nothing between the rows
+        assert p.device_status() == 0
