@@ -39,7 +39,7 @@ void note_live(int dev, int64_t change)
 {
     std::lock_guard<std::mutex> lock(g_device_mutex);
     g_pool_live[dev] += (uint64_t)change;
-    uint64_t want = (g_pool_live[dev] + kPoolStep - 1) / kPoolStep * kPoolStep + kPoolKeeps - kPoolStep;
+    uint64_t want = g_pool_live[dev] / kPoolStep * kPoolStep + kPoolKeeps;
     if (g_pool[dev] && want != g_pool_threshold[dev] && cudaMemPoolSetAttribute(g_pool[dev], cudaMemPoolAttrReleaseThreshold, &want) == cudaSuccess)
         g_pool_threshold[dev] = want;
 }
@@ -55,6 +55,8 @@ cudaError_t device_pool(int dev, cudaMemPool_t *pool)
         props.location.id = dev;
         cudaError_t e = cudaMemPoolCreate(&g_pool[dev], &props);
         if (e != cudaSuccess) { g_pool[dev] = nullptr; return e; }
+        uint64_t keep = g_pool_threshold[dev] = kPoolKeeps;
+        if ((e = cudaMemPoolSetAttribute(g_pool[dev], cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) return e;
     }
     *pool = g_pool[dev];
     return cudaSuccess;

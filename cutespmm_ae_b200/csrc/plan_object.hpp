@@ -34,6 +34,8 @@ struct cutespmm_list_sizes {
 // Gives the memory of a device-built plan back.  device_plan.cu
 void cutespmm_internal_free_block(void *block, uint64_t bytes, int dev, bool used_elsewhere);
 
+void cutespmm_internal_give_status_word(uint32_t *word);  // sharded.cu
+
 struct cutespmm_plan {
     cutespmm::HostPlan host;
     cutespmm_list_sizes own, every;  // of the list of the rows outside the tensor-core panels / of the list of every row
@@ -59,6 +61,7 @@ struct cutespmm_plan {
     uint32_t *d_status = nullptr;
     // staging for the host-buffer call
     float *d_B = nullptr, *d_C = nullptr;
+    uint32_t *h_status = nullptr;  // pinned: where a call's status word arrives
     uint64_t staged_B = 0, staged_C = 0;
     // the host-buffer calls pipeline column windows: copy-in, exchange between ranks, product and copy-out each on a
     // stream of their own
@@ -94,6 +97,7 @@ struct cutespmm_plan {
                 if (p) cudaFree(p);
         for (void *p : {(void *)d_B, (void *)d_C})
             if (p) cudaFree(p);
+        if (h_status) cutespmm_internal_give_status_word(h_status);
         for (cudaEvent_t ev : {ev_entry, ev_done})
             if (ev) cudaEventDestroy(ev);
         for (int w = 0; w < kMaxWindows; ++w)

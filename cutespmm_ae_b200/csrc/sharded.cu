@@ -179,6 +179,25 @@ int new_comm(cutespmm_comm_t **out, nccl_comm_t c, int nranks, int rank, int dev
 
 namespace {
 
+// Pinned words the calls' status arrives in, one per plan that makes host-buffer calls: handed out of pages of 1024, because
+// pinning a page takes milliseconds.  Given-back words are handed out again; the pages stay (4 KB per 1024 such plans).
+std::mutex g_status_mutex;
+std::vector<uint32_t *> g_status_words;
+cudaError_t take_status_word(uint32_t **word)
+{
+    std::lock_guard<std::mutex> lock(g_status_mutex);
+    if (g_status_words.empty()) {
+        uint32_t *page = nullptr;
+        const cudaError_t e = cudaHostAlloc(&page, 1024 * sizeof(uint32_t), cudaHostAllocPortable);
+        if (e != cudaSuccess) return e;
+        for (int i = 1023; i >= 0; --i) g_status_words.push_back(page + i);
+    }
+    *word = g_status_words.back();
+    g_status_words.pop_back();
+    **word = 0;
+    return cudaSuccess;
+}
+
 // How a host-buffer call cuts N columns into windows, and the staging it needs on the device.
 struct Windows {
     uint32_t count = 1, width = 0;
@@ -196,11 +215,14 @@ int ensure_staging(cutespmm_plan *p, uint32_t N, bool sharded, Windows &w)
     const uint64_t rows_for_cut = sharded ? K : std::max(M, K);
     uint32_t nw = 1;
     if ((uint64_t)N * rows_for_cut * sizeof(float) >= (8u << 20)) nw = std::max(1u, std::min<uint32_t>(cutespmm_plan::kMaxWindows, N / 64));
-    // window width: a multiple of 64 columns (the last may be narrower); strided copies of rows shorter than 256 bytes
-    // were measured at 2/3 of the link rate, 256-byte rows at the full rate
-    w.width = ((N + nw - 1) / nw + 63) / 64 * 64;
-    w.count = (N + w.width - 1) / w.width;
-    w.ldd = w.count == 1 ? (uint64_t)(N + 3) / 4 * 4 : w.width;  // rows start 16-byte aligned
+    // window width: a multiple of 64 columns, the last takes what is left over (64 or more); strided copies of rows
+    // shorter than 256 bytes were measured at 2/3 of the link rate and far less the shorter they are, 256-byte rows at the
+    // full rate.  One window is as wide as the product, so that contiguous operands are copied in one piece (a pitch
+    // rounded up to 16 bytes made 100 000 rows of N = 43 a 12 ms copy, 0.4 ms in one piece); the kernel takes any alignment.
+    w.count = nw;
+    w.width = nw == 1 ? N : N / nw / 64 * 64;
+    const uint32_t last = N - w.width * (nw - 1);
+    w.ldd = nw == 1 ? N : (last + 3) / 4 * 4;
     const uint64_t needB = (uint64_t)w.count * K * w.ldd * sizeof(float), needC = (uint64_t)w.count * M * w.ldd * sizeof(float);
     cudaError_t e;
     if (needB > p->staged_B) {
@@ -214,6 +236,9 @@ int ensure_staging(cutespmm_plan *p, uint32_t N, bool sharded, Windows &w)
         p->d_C = nullptr; p->staged_C = 0;
         if ((e = cudaMalloc(&p->d_C, needC)) != cudaSuccess) return fail_cuda_status(e, "staging buffer for C");
         p->staged_C = needC;
+    }
+    if (!p->h_status) {
+        if ((e = take_status_word(&p->h_status)) != cudaSuccess) return fail_cuda_status(e, "status word");
     }
     if (!p->s_in) {
         if ((e = cudaStreamCreateWithFlags(&p->s_in, cudaStreamNonBlocking)) != cudaSuccess ||
@@ -248,9 +273,11 @@ bool cut_row_blocks(cutespmm_plan *p, uint32_t N)
     if (h.M >= 4096 && cutespmm_internal_fetch_lists(p) != CUTESPMM_OK) return false;
     if (!h.row_map.empty() || h.slab_panels || h.panel_max_col.size() != h.num_panels() || h.M < 4096) return false;
     const uint64_t c_bytes = h.M * (uint64_t)N * sizeof(float);
-    // blocks of about 16 MiB of C: every block costs about 40 us of hand-over between the copy engines and its kernel
-    // (measured: 6-8 blocks are best for 134 MB, 16 blocks lose what the finer overlap gains)
-    int R = (int)std::min<uint64_t>(cutespmm_plan::kMaxRowBlocks, c_bytes / (16u << 20));
+    // Blocks of 4 MiB of C up to 48 MiB (at most ten), of 16 MiB beyond: the first upload and the last download overlap
+    // nothing, so a small call wants small blocks (23 MB each way: 0.90 ms in one block, 0.71 in five; 49 MB: 1.55 ms in
+    // three, 1.43 in ten); a large one is bound by what the link carries both ways at once, and every block costs about
+    // 40 us of hand-over between the copy engines and its kernel (134 MB: 3.50 ms in eight blocks, 3.86 in sixteen)
+    int R = (int)(c_bytes <= (48u << 20) ? std::min<uint64_t>(10, c_bytes / (4u << 20)) : std::min<uint64_t>(cutespmm_plan::kMaxRowBlocks, c_bytes / (16u << 20)));
     if (R < 2) return false;
     // boundaries: near equal row counts, on 16-row panel boundaries, never inside a tile of either tile list
     auto snap = [&](uint64_t target, const std::vector<Tile> &tiles) {
@@ -316,7 +343,7 @@ cudaError_t copy_rows(void *dst, uint64_t ld_dst, const void *src, uint64_t ld_s
 int run_row_blocks(cutespmm_plan *p, const float *B_host, uint64_t ldb, float *C_host, uint64_t ldc, uint32_t N, cudaStream_t s, float *kernel_ms)
 {
     const uint64_t M = p->host.M, K = p->host.K;
-    const uint64_t ldd = (uint64_t)(N + 3) / 4 * 4;
+    const uint64_t ldd = N;  // contiguous: copies go in one piece
     cudaError_t e;
     if (!p->rb_in[0])
         for (int i = 0; i < cutespmm_plan::kMaxRowBlocks; ++i)
@@ -350,7 +377,7 @@ int run_row_blocks(cutespmm_plan *p, const float *B_host, uint64_t ldb, float *C
         const cutespmm_row_block &b = p->row_blocks[i];
         cudaStreamWaitEvent(s, p->rb_in[i], 0);
         cudaEventRecord(p->rb_k0[i], s);
-        const int st = cutespmm_internal_spmm_range(p, p->d_B, ldd, p->d_C, ldd, N, s, &b.items, true);
+        const int st = cutespmm_internal_spmm_range(p, p->d_B, ldd, p->d_C, ldd, N, s, &b.items, false);
         if (st != CUTESPMM_OK) {
             drain();
             return st;
@@ -366,6 +393,7 @@ int run_row_blocks(cutespmm_plan *p, const float *B_host, uint64_t ldb, float *C
     (void)M;
     cudaEventRecord(p->ev_done, p->s_out);
     cudaStreamWaitEvent(s, p->ev_done, 0);
+    cudaMemcpyAsync(p->h_status, p->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail_cuda_status(e, "SpMM execution");
     if (kernel_ms) {
         *kernel_ms = 0.f;
@@ -374,13 +402,19 @@ int run_row_blocks(cutespmm_plan *p, const float *B_host, uint64_t ldb, float *C
             if (cudaEventElapsedTime(&ms, p->rb_k0[i], p->rb_k1[i]) == cudaSuccess) *kernel_ms += ms;
         }
     }
-    uint32_t dev_status = 0;
-    cutespmm_plan_device_status(p, &dev_status);
+    uint32_t dev_status = *p->h_status;
+    if (dev_status) cutespmm_plan_device_status(p, &dev_status);  // reads it again and clears it
     if (dev_status) return fail_status(CUTESPMM_ETIMEOUT, "a device-side wait ran out (status " + std::to_string(dev_status) + ")");
     return CUTESPMM_OK;
 }
 
 }  // namespace
+
+void cutespmm_internal_give_status_word(uint32_t *word)
+{
+    std::lock_guard<std::mutex> lock(g_status_mutex);
+    g_status_words.push_back(word);
+}
 
 extern "C" {
 
@@ -603,17 +637,16 @@ int cutespmm_spmm_sharded_host(cutespmm_plan_t *p, cutespmm_comm_t *comm, const 
     // every upload is queued before the first download, so that no download waiting for its kernel sits in front of
     // an upload in a copy queue
     for (uint32_t w = 0; w < nw; ++w) {
-        const uint32_t c0 = w * wcols, cw = std::min(wcols, N - c0);
+        const uint32_t c0 = w * wcols, cw = w + 1 == nw ? N - c0 : wcols;
         float *dB = p->d_B + (uint64_t)w * K * ldd;
-        if (k1 > k0 && (e = cudaMemcpy2DAsync(dB + k0 * ldd, ldd * sizeof(float), B_host_rows + c0, ldb * sizeof(float),
-                                              (size_t)cw * sizeof(float), k1 - k0, cudaMemcpyHostToDevice, p->s_in)) != cudaSuccess) {
+        if (k1 > k0 && (e = copy_rows(dB + k0 * ldd, ldd, B_host_rows + c0, ldb, cw, k1 - k0, cudaMemcpyHostToDevice, p->s_in)) != cudaSuccess) {
             drain();
             return fail_cuda_status(e, "copy of B to the device");
         }
         cudaEventRecord(p->ev_in[w], p->s_in);
     }
     for (uint32_t w = 0; w < nw; ++w) {
-        const uint32_t c0 = w * wcols, cw = std::min(wcols, N - c0);
+        const uint32_t c0 = w * wcols, cw = w + 1 == nw ? N - c0 : wcols;
         float *dB = p->d_B + (uint64_t)w * K * ldd, *dC = p->d_C + (uint64_t)w * M * ldd;
         if (!unit.empty()) {  // the slices of this window meet on every rank
             cudaStreamWaitEvent(p->s_x, p->ev_in[w], 0);
@@ -636,14 +669,14 @@ int cutespmm_spmm_sharded_host(cutespmm_plan_t *p, cutespmm_comm_t *comm, const 
         }
         cudaEventRecord(p->ev_k1[w], s);
         cudaStreamWaitEvent(p->s_out, p->ev_k1[w], 0);
-        if (M && (e = cudaMemcpy2DAsync(C_host + c0, ldc * sizeof(float), dC, ldd * sizeof(float), (size_t)cw * sizeof(float), M,
-                                        cudaMemcpyDeviceToHost, p->s_out)) != cudaSuccess) {
+        if (M && (e = copy_rows(C_host + c0, ldc, dC, ldd, cw, M, cudaMemcpyDeviceToHost, p->s_out)) != cudaSuccess) {
             drain();
             return fail_cuda_status(e, "copy of C to the host");
         }
     }
     cudaEventRecord(p->ev_done, p->s_out);
     cudaStreamWaitEvent(s, p->ev_done, 0);  // later work on `stream` sees the finished call
+    cudaMemcpyAsync(p->h_status, p->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail_cuda_status(e, "SpMM execution");
     if (kernel_ms) *kernel_ms = 0.f;
     if (exchange_ms) *exchange_ms = 0.f;
@@ -653,8 +686,8 @@ int cutespmm_spmm_sharded_host(cutespmm_plan_t *p, cutespmm_comm_t *comm, const 
         if (exchange_ms && !unit.empty() && !(comm && comm->stub) && cudaEventElapsedTime(&ms, p->ev_x0[w], p->ev_x1[w]) == cudaSuccess)
             *exchange_ms += ms;
     }
-    uint32_t dev_status = 0;
-    cutespmm_plan_device_status(p, &dev_status);
+    uint32_t dev_status = *p->h_status;
+    if (dev_status) cutespmm_plan_device_status(p, &dev_status);  // reads it again and clears it
     if (dev_status) return fail_status(CUTESPMM_ETIMEOUT, "a device-side wait ran out (status " + std::to_string(dev_status) + ")");
     return CUTESPMM_OK;
 }
