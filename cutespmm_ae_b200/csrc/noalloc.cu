@@ -5,14 +5,14 @@
 // which may synchronise the device, or in a process whose memory budget was fixed at start-up.  Such
 // a caller cannot create a plan (plan creation uploads arrays and reserves the partial-sum scratch
 // with cudaMalloc).  This entry point takes plain CSR arrays that already sit in device memory and
-// computes the product with the row kernel's method -- a warp per row, long rows cut into chunks
+// computes the product with the row kernel's method -- a group of lanes per row, long rows cut into chunks
 // whose partial sums are added in a fixed order -- keeping the partial sums in a scratch array that
 // is part of the library image instead of an allocation.
 //
-// The scratch is the file-scope array g_scratch below (16 MiB).  Every GPU on which the library is
-// loaded holds it until the process exits.  All calls on one device share it, and it keeps whatever
-// the previous call left there; nothing in it has to start at zero, because every slot a call reads
-// was written earlier by the same call.  Two calls that overlap on the same GPU (different streams,
+// The scratch is the file-scope array g_scratch below (16 MiB), beside it the list of chunks and their counters
+// (2 MiB).  Every GPU on which the library is loaded holds them until the process exits.  All calls on one
+// device share them, and the scratch keeps whatever the previous call left there; nothing in it has to start at
+// zero, because every slot a call reads was written earlier by the same call.  Two calls that overlap on the same GPU (different streams,
 // or different host threads) race on it: order them on one stream or with events.
 //
 // In host code the name g_scratch is only a stand-in, not a device address.  The address the
@@ -35,25 +35,28 @@ void set_last_error(const std::string &msg);  // capi.cu
 
 namespace {
 
-constexpr uint32_t kSplit = CUTESPMM_NOALLOC_SPLIT_NNZ;          // rows longer than this are cut into chunks of this length
+constexpr uint32_t kLimitSplit = CUTESPMM_NOALLOC_SPLIT_NNZ;  // the chunk length the published limit is stated for
 constexpr uint64_t kScratchFloats = CUTESPMM_NOALLOC_SCRATCH_BYTES / 4;
+constexpr uint32_t kListSlots = 1u << 16;                       // chunks one call can list
+constexpr uint32_t kMaxSlabs = CUTESPMM_NOALLOC_MAX_N / 128;
 constexpr int kWarps = 8;
-constexpr int kSlab = 128;                                        // columns one block row covers (4 per lane)
+constexpr uint32_t kBuf = 256;  // nonzeros a warp stages at a time
+constexpr uint32_t kNoCol = 0xffffffffu;
 constexpr unsigned kFull = 0xffffffffu;
 
 static __device__ __align__(256) float g_scratch[kScratchFloats];
-static __device__ uint32_t g_next_row[CUTESPMM_NOALLOC_MAX_N / kSlab];  // row counters of the rows kernel, one per column slab
+// {row, j0, j1, slot of the row's first chunk} of chunk i, whose partial sum is row i of the scratch
+static __device__ uint4 g_list[kListSlots];
+static __device__ uint32_t g_arrivals[kListSlots * kMaxSlabs];  // per first slot of a row and column slab: chunks finished
+// All zero between calls: the last block of a call's main kernel puts it back.
+struct State {
+    uint32_t chunks, overflow, done, pad;
+    uint32_t next_row[kMaxSlabs];
+};
+static __device__ State g_state;
 
-// Slot of the chunk that starts at nonzero position `start`.  Chunks of one row start kSplit apart
-// and two long rows start more than kSplit apart, so a window of kSplit positions holds at most one
-// first chunk and one later chunk: two slots per window are enough and need no counter.
-__device__ __forceinline__ uint64_t chunk_slot(uint32_t start, bool first_of_row)
-{
-    return 2ull * (start / kSplit) + (first_of_row ? 1u : 0u);
-}
-
-// Nonzero positions [j0, j1) of row r, forced into [0, nnz] and into order: every position the kernels derive a
-// scratch slot or an array index from is then below the `nnz` the host sized its checks with, whatever rowPtr holds.
+// Nonzero positions [j0, j1) of row r, forced into [0, nnz] and into order: every position the kernels derive an array
+// index from is then below the `nnz` the host sized its checks with, whatever rowPtr holds.
 struct Range {
     uint32_t j0, j1;
 };
@@ -65,154 +68,272 @@ __device__ __forceinline__ Range row_range(const uint32_t *__restrict__ rowPtr, 
     return g;
 }
 
-// acc[i] += sum over nonzeros [j0, j1) of vals[j] * B[cols[j]][n0 + lane + 32 i].  A nonzero whose column is not
-// below K is left out (B has no such row); the call cannot report it without reading something back.
-__device__ __forceinline__ void accumulate(float (&acc)[4], const uint32_t *__restrict__ cols,
-                                           const float *__restrict__ vals, uint32_t j0, uint32_t j1,
-                                           const float *__restrict__ B, uint64_t ldb, uint32_t n0, uint32_t N, uint32_t K,
-                                           int lane)
+// Lists the chunks of the rows longer than `split`.  One pass over the row pointers (4 us at 2^18 rows); which slots a row
+// gets depends on the order of arrival, the order its chunks are added in does not.  A row that does not fit the list (row
+// pointers that claim more nonzeros than there are) raises `overflow`: the main kernel then computes long rows whole.
+__global__ void __launch_bounds__(256) noalloc_list_kernel(const uint32_t *__restrict__ rowPtr, uint32_t M, uint32_t nnz, uint32_t split,
+                                                           uint32_t capacity)
 {
-    constexpr int U = 4;  // nonzeros whose rows of B are in flight together
-    for (uint32_t j = j0; j < j1; j += 32) {
-        const uint32_t n = min(32u, j1 - j);
-        uint32_t c = 0;
-        float v = 0.f;
-        if ((uint32_t)lane < n) {
-            c = __ldg(cols + j + lane);
-            v = __ldg(vals + j + lane);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < M; r += stride) {
+        const Range g = row_range(rowPtr, r, nnz);
+        const uint32_t len = g.j1 - g.j0;
+        if (len <= split) continue;
+        const uint32_t n = (uint32_t)(((uint64_t)len + split - 1) / split);
+        const uint32_t slot0 = n <= capacity ? atomicAdd(&g_state.chunks, n) : 0u;
+        if (n > capacity || slot0 > capacity - n) {
+            g_state.overflow = 1;
+            continue;
         }
-        for (uint32_t k = 0; k < n; k += U) {
-            float vk[U], b[U][4];
+        for (uint32_t i = 0; i < n; ++i) {
+            const uint32_t j = g.j0 + i * split;
+            g_list[slot0 + i] = make_uint4((uint32_t)r, j, min(g.j1 - j, split) + j, slot0);
+        }
+        for (uint32_t y = 0; y < kMaxSlabs; ++y) g_arrivals[slot0 * kMaxSlabs + y] = 0;
+    }
+}
+
+template <int VEC> struct Vec;
+template <> struct Vec<4> { using T = float4; };
+template <> struct Vec<1> { using T = float; };
+__device__ __forceinline__ void zero(float4 &a) { a = make_float4(0.f, 0.f, 0.f, 0.f); }
+__device__ __forceinline__ void zero(float &a) { a = 0.f; }
+__device__ __forceinline__ void fma_to(float4 &a, float v, const float4 &b)
+{
+    a.x = fmaf(v, b.x, a.x); a.y = fmaf(v, b.y, a.y); a.z = fmaf(v, b.z, a.z); a.w = fmaf(v, b.w, a.w);
+}
+__device__ __forceinline__ void fma_to(float &a, float v, const float &b) { a = fmaf(v, b, a); }
+__device__ __forceinline__ void add_to(float4 &a, const float4 &b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
+__device__ __forceinline__ void add_to(float &a, const float &b) { a += b; }
+__device__ __forceinline__ float4 from_lane(const float4 &a, int o)
+{
+    return make_float4(__shfl_xor_sync(kFull, a.x, o), __shfl_xor_sync(kFull, a.y, o), __shfl_xor_sync(kFull, a.z, o), __shfl_xor_sync(kFull, a.w, o));
+}
+__device__ __forceinline__ float from_lane(const float &a, int o) { return __shfl_xor_sync(kFull, a, o); }
+
+struct MainArgs {
+    const uint32_t *rowPtr, *cols;
+    const float *vals, *B;
+    float *C, *scratch;
+    uint64_t ldb, ldc;
+    uint32_t M, K, nnz, N, lds, split, claim;
+};
+
+// The product.  A warp is G groups of 32/G lanes; a group spans a slab of 32/G * VEC * CH columns.  First the listed chunks
+// (the groups share a chunk's nonzeros; whoever finishes a row's last chunk adds the row's slots in order and writes C),
+// then the rows: a warp claims `claim` consecutive rows at a time from a counter per slab -- a fixed stride would hand the
+// rows r, r + stride, ... of a power-law graph, whose long rows sit at indices with few one-bits, to the same few warps --
+// and stages their nonzeros, up to kBuf at a time, in shared memory with one coalesced pass, columns checked; its groups
+// then take a row each (and a long one together).  Bound by the latency of the gathers of rows of B; U of them are in flight
+// per group, 40 warps per SM (U = 8 with 32 warps: 171 against 160 us below).
+// R-MAT 2^18, 3.9 M nonzeros, N = 64: 815 -> 160 us (before: a warp per row and per 1024-nonzero chunk, single-column
+// loads, three kernels one after the other); R-MAT 2^16 N = 16 474 -> 36, uniform4096 N = 32 25.6 -> 11.1.
+template <int VEC, int CH, int G>
+__global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a)
+{
+    using V = typename Vec<VEC>::T;
+    constexpr int L = 32 / G, U = (VEC == 4 ? 4 : 8) / CH;  // rows of B in flight per group
+    static_assert(U >= 2 && (G == 1 || CH == 1), "groups span one vector per lane");
+    __shared__ uint2 bufs[kWarps][kBuf];
+    __shared__ uint32_t starts[kWarps][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / L, sub = lane % L;
+    uint2 *buf = bufs[warp];
+    uint32_t *start = starts[warp];
+    const uint32_t col0 = blockIdx.y * (L * VEC * CH) + sub * VEC;
+    bool ok[CH];
+#pragma unroll
+    for (int ch = 0; ch < CH; ++ch) ok[ch] = col0 + ch * L * VEC < a.N;
+    const float *bl = a.B + col0;
+
+    auto stage = [&](uint32_t j, uint32_t n) {  // nonzeros [j, j + n) to the warp's buffer; a column that is not below K counts nothing
+        for (uint32_t t = lane; t < n; t += 32) {
+            const uint32_t c = __ldg(a.cols + j + t);
+            buf[t] = make_uint2(c < a.K ? c : kNoCol, __float_as_uint(__ldg(a.vals + j + t)));
+        }
+    };
+    // acc += the staged nonzeros from, from + step, ... below end
+    auto gather = [&](V(&acc)[CH], uint32_t from, uint32_t end, uint32_t step) {
+        for (uint32_t k = from; k < end; k += U * step) {
+            float v[U];
+            V x[U][CH];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int src = (int)min(k + u, n - 1);  // positions past the end repeat the last one and add nothing
-                const uint32_t ck = __shfl_sync(kFull, c, src);
-                vk[u] = __shfl_sync(kFull, v, src);
-                const bool use = k + u < n && ck < K;    // uniform across the warp
-                if (!use) vk[u] = 0.f;
-                const float *row = B + (uint64_t)ck * ldb + n0 + lane;
+                const bool in = k + u * step < end;
+                const uint2 pr = buf[in ? k + u * step : k];
+                v[u] = __uint_as_float(pr.y);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) b[u][i] = (use && n0 + lane + 32 * i < N) ? __ldg(row + 32 * i) : 0.f;
+                for (int ch = 0; ch < CH; ++ch) {
+                    zero(x[u][ch]);
+                    if (in && ok[ch] && pr.x != kNoCol) x[u][ch] = __ldg(reinterpret_cast<const V *>(bl + (uint64_t)pr.x * a.ldb + ch * L * VEC));
+                }
+                if (!in || pr.x == kNoCol) v[u] = 0.f;
             }
 #pragma unroll
             for (int u = 0; u < U; ++u)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) acc[i] = fmaf(vk[u], b[u][i], acc[i]);
+                for (int ch = 0; ch < CH; ++ch) fma_to(acc[ch], v[u], x[u][ch]);
+        }
+    };
+    auto over_groups = [&](V(&acc)[CH]) {  // every group ends up with the sum of all groups'
+#pragma unroll
+        for (int o = L; o < 32; o <<= 1)
+#pragma unroll
+            for (int ch = 0; ch < CH; ++ch) add_to(acc[ch], from_lane(acc[ch], o));
+    };
+    auto store = [&](uint64_t row, const V(&acc)[CH]) {
+#pragma unroll
+        for (int ch = 0; ch < CH; ++ch)
+            if (ok[ch]) __stcs(reinterpret_cast<V *>(a.C + row * a.ldc + col0 + ch * L * VEC), acc[ch]);
+    };
+    auto whole_warp = [&](V(&acc)[CH], uint32_t j0, uint32_t j1) {  // a run of nonzeros the groups share
+#pragma unroll
+        for (int ch = 0; ch < CH; ++ch) zero(acc[ch]);
+        for (uint32_t j = j0; j < j1; j += kBuf) {
+            const uint32_t n = min(kBuf, j1 - j);
+            __syncwarp();
+            stage(j, n);
+            __syncwarp();
+            gather(acc, grp, n, G);
+        }
+        over_groups(acc);
+    };
+
+    const bool overflow = g_state.overflow != 0;
+    const uint32_t chunks = overflow ? 0u : g_state.chunks;
+    for (uint32_t c = warp * gridDim.x + blockIdx.x; c < chunks; c += gridDim.x * kWarps) {
+        const uint4 ck = g_list[c];
+        V acc[CH];
+        whole_warp(acc, ck.y, ck.z);
+        if (grp == 0) {
+#pragma unroll
+            for (int ch = 0; ch < CH; ++ch)
+                if (ok[ch]) __stcg(reinterpret_cast<V *>(a.scratch + (uint64_t)c * a.lds + col0 + ch * L * VEC), acc[ch]);
+        }
+        __threadfence();
+        __syncwarp();
+        uint32_t pieces = 0;
+        if (lane == 0) {
+            const Range g = row_range(a.rowPtr, ck.x, a.nnz);
+            pieces = (uint32_t)(((uint64_t)(g.j1 - g.j0) + a.split - 1) / a.split);
+            if (atomicAdd(&g_arrivals[ck.w * kMaxSlabs + blockIdx.y], 1u) != pieces - 1) pieces = 0;
+            __threadfence();
+        }
+        pieces = __shfl_sync(kFull, pieces, 0);
+        if (pieces) {  // this warp finished the row's last chunk
+#pragma unroll
+            for (int ch = 0; ch < CH; ++ch) zero(acc[ch]);
+#pragma unroll 4
+            for (uint32_t k = grp; k < pieces; k += G)
+#pragma unroll
+                for (int ch = 0; ch < CH; ++ch)
+                    if (ok[ch]) add_to(acc[ch], __ldcg(reinterpret_cast<const V *>(a.scratch + (uint64_t)(ck.w + k) * a.lds + col0 + ch * L * VEC)));
+            over_groups(acc);
+            if (grp == 0) store(ck.x, acc);
         }
     }
-}
 
-// Rows of at most kSplit nonzeros: one warp per row, result straight to C.  Warps claim kClaim consecutive rows at a
-// time from a counter per column slab (next_row, zeroed by the host before the launch): a fixed stride would hand the
-// rows r, r + stride, ... of a power-law graph -- whose long rows sit at indices with few one-bits -- to the same few warps.
-constexpr uint32_t kClaim = 4;
-__global__ void __launch_bounds__(kWarps * 32) noalloc_rows_kernel(const uint32_t *__restrict__ rowPtr,
-                                                                   const uint32_t *__restrict__ cols,
-                                                                   const float *__restrict__ vals, uint32_t M,
-                                                                   uint32_t K, uint32_t nnz,
-                                                                   const float *__restrict__ B, uint64_t ldb,
-                                                                   float *__restrict__ C, uint64_t ldc, uint32_t N,
-                                                                   uint32_t *__restrict__ next_row)
-{
-    const int lane = threadIdx.x & 31;
-    const uint32_t n0 = blockIdx.y * kSlab;
     for (;;) {
         uint32_t first = 0;
-        if (lane == 0) first = atomicAdd(next_row + blockIdx.y, kClaim);
+        if (lane == 0) first = atomicAdd(&g_state.next_row[blockIdx.y], a.claim);
         first = __shfl_sync(kFull, first, 0);
-        if (first >= M) break;  // also ends the loop should the counter ever wrap: M < 2^32 - kClaim * warps is not assumed
-        const uint32_t last = min(M, first + kClaim);
-        for (uint64_t r = first; r < last; ++r) {
-            const Range rg = row_range(rowPtr, r, nnz);
-            const uint32_t j0 = rg.j0, j1 = rg.j1;
-            if (j1 - j0 > kSplit) continue;  // written by the fix-up kernel
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            accumulate(acc, cols, vals, j0, j1, B, ldb, n0, N, K, lane);
+        if (first >= a.M) break;
+        const uint32_t cnt = min(a.claim, a.M - first);
+        Range g{0u, 0u};
+        if ((uint32_t)lane < cnt) g = row_range(a.rowPtr, (uint64_t)first + lane, a.nnz);
+        const bool listed = !overflow && g.j1 - g.j0 > a.split;
+        for (uint32_t i0 = 0; i0 < cnt;) {
+            const uint32_t j0 = __shfl_sync(kFull, g.j0, (int)i0), j1 = __shfl_sync(kFull, g.j1, (int)i0);
+            if (__shfl_sync(kFull, listed, (int)i0)) {
+                ++i0;
+                continue;
+            }
+            V acc[CH];
+            if (j1 - j0 > kBuf) {
+                whole_warp(acc, j0, j1);
+                if (grp == 0) store((uint64_t)first + i0, acc);
+                ++i0;
+                continue;
+            }
+            // the rows from i0 on whose nonzeros fit the buffer together
+            const bool fits = (uint32_t)lane < cnt && !listed && g.j0 >= j0 && g.j1 - j0 <= kBuf && g.j1 >= g.j0;
+            const unsigned miss = __ballot_sync(kFull, (uint32_t)lane >= i0 && !fits);
+            const uint32_t i1 = miss ? __ffs(miss) - 1 : 32u;
+            const uint32_t end = __shfl_sync(kFull, g.j1, (int)i1 - 1);
+            __syncwarp();
+            stage(j0, end - j0);
+            if ((uint32_t)lane >= i0 && (uint32_t)lane < i1) start[lane] = g.j0 - j0;
+            if ((uint32_t)lane + 1 == i1) start[i1] = g.j1 - j0;
+            __syncwarp();
+            // a row of more than a few steps is shared by the groups, the others are a group's each
+            constexpr uint32_t kShared = G == 1 ? kBuf : 4 * U;
+            for (uint32_t i = i0 + grp; i < i1; i += G) {
+                const uint32_t from = start[i], to = max(start[i + 1], from);
+                if (G > 1 && to - from > kShared) continue;
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (n0 + lane + 32 * i < N) C[r * ldc + n0 + lane + 32 * i] = acc[i];
+                for (int ch = 0; ch < CH; ++ch) zero(acc[ch]);
+                gather(acc, from, to, 1);
+                store((uint64_t)first + i, acc);
+            }
+            if constexpr (G > 1) {
+                __syncwarp();
+                unsigned shared = __ballot_sync(kFull, (uint32_t)lane >= i0 && (uint32_t)lane < i1 && start[lane + 1] > start[lane] + kShared);
+                for (; shared; shared &= shared - 1) {
+                    const uint32_t i = __ffs(shared) - 1;
+#pragma unroll
+                    for (int ch = 0; ch < CH; ++ch) zero(acc[ch]);
+                    gather(acc, start[i] + grp, start[i + 1], G);
+                    over_groups(acc);
+                    if (grp == 0) store((uint64_t)first + i, acc);
+                }
+            }
+            i0 = i1;
+        }
+    }
+
+    // the last block to leave puts the counters back for the next call
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const uint32_t blocks = gridDim.x * gridDim.y;
+        __threadfence();
+        if (atomicInc(&g_state.done, blocks - 1) == blocks - 1) {
+            g_state.chunks = 0;
+            g_state.overflow = 0;
+            for (uint32_t y = 0; y < kMaxSlabs; ++y) g_state.next_row[y] = 0;
         }
     }
 }
 
-// Chunks of long rows.  A warp takes a window of kSplit nonzero positions, finds the row that holds
-// the window's first position by bisection over rowPtr, and computes every chunk that starts inside
-// the window (at most two) into its slot of the scratch.
-__global__ void __launch_bounds__(kWarps * 32) noalloc_chunks_kernel(const uint32_t *__restrict__ rowPtr,
-                                                                     const uint32_t *__restrict__ cols,
-                                                                     const float *__restrict__ vals, uint32_t M,
-                                                                     uint32_t K, uint32_t nnz, const float *__restrict__ B,
-                                                                     uint64_t ldb, float *__restrict__ scratch,
-                                                                     uint32_t lds, uint32_t N)
-{
-    const int lane = threadIdx.x & 31;
-    const uint32_t n0 = blockIdx.y * kSlab;
-    const uint32_t windows = (nnz + kSplit - 1) / kSplit;
-    const uint64_t nw = (uint64_t)gridDim.x * kWarps;
-    for (uint64_t w = (uint64_t)blockIdx.x * kWarps + (threadIdx.x >> 5); w < windows; w += nw) {
-        const uint32_t p0 = (uint32_t)w * kSplit, p1 = min(nnz, p0 + kSplit);
-        // last row r with rowPtr[r] <= p0 (rows without nonzeros share a start; take the last of them)
-        uint32_t lo = 0, hi = M;  // invariant: rowPtr[lo] <= p0 < rowPtr[hi] (rowPtr[M] = nnz > p0)
-        while (hi - lo > 1) {
-            const uint32_t mid = lo + (hi - lo) / 2;
-            if (__ldg(rowPtr + mid) <= p0) lo = mid; else hi = mid;
-        }
-        for (uint32_t r = lo; r < M; ++r) {
-            const Range rg = row_range(rowPtr, r, nnz);
-            const uint32_t j0 = rg.j0, j1 = rg.j1;
-            if (j0 >= p1) break;
-            if (j1 - j0 <= kSplit) continue;
-            // chunk starts of row r are j0, j0 + kSplit, ...; the one (if any) inside [p0, p1)
-            uint32_t i = j0 >= p0 ? 0u : (p0 - j0 + kSplit - 1) / kSplit;
-            const uint32_t start = j0 + i * kSplit;  // cannot wrap: start < j1 is checked before use below
-            if (start < p0 || start >= p1 || start >= j1) continue;
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            accumulate(acc, cols, vals, start, min(j1, start + kSplit), B, ldb, n0, N, K, lane);
-            float *out = scratch + chunk_slot(start, i == 0) * lds + n0 + lane;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (n0 + lane + 32 * k < N) out[32 * k] = acc[k];
-        }
-    }
-}
-
-// C[row] of every long row = its chunks' partial sums, added in chunk order.
-__global__ void __launch_bounds__(kWarps * 32) noalloc_fixup_kernel(const uint32_t *__restrict__ rowPtr, uint32_t M,
-                                                                    uint32_t nnz, const float *__restrict__ scratch, uint32_t lds,
-                                                                    float *__restrict__ C, uint64_t ldc, uint32_t N)
-{
-    const int lane = threadIdx.x & 31;
-    const uint32_t n0 = blockIdx.y * kSlab;
-    const uint64_t nw = (uint64_t)gridDim.x * kWarps;
-    for (uint64_t r = (uint64_t)blockIdx.x * kWarps + (threadIdx.x >> 5); r < M; r += nw) {
-        const Range rg = row_range(rowPtr, r, nnz);
-        const uint32_t j0 = rg.j0, j1 = rg.j1;
-        if (j1 - j0 <= kSplit) continue;
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-        for (uint32_t start = j0, i = 0; start < j1; start += kSplit, ++i) {
-            const float *in = scratch + chunk_slot(start, i == 0) * lds + n0 + lane;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (n0 + lane + 32 * k < N) acc[k] += in[32 * k];
-            if (j1 - start <= kSplit) break;  // last chunk (also keeps start from wrapping past 2^32)
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (n0 + lane + 32 * k < N) C[r * ldc + n0 + lane + 32 * k] = acc[k];
-    }
-}
-
-// Device address of g_scratch and the SM count, looked up once per device.
+// What a device needs to know: looked up once.
 struct DeviceSetup {
     float *scratch = nullptr;
-    uint32_t *next_row = nullptr;
     int sm_count = 0;
-    int rows_blocks_per_sm = 0;  // resident blocks of the rows kernel: its grid is one resident wave
-    int chunks_blocks_per_sm = 0;  // the same for the chunks kernel
 };
 constexpr int kMaxDevices = 64;
 DeviceSetup g_setup[kMaxDevices];
 std::mutex g_setup_mutex;
+
+template <int VEC, int CH, int G> cudaError_t launch_main(MainArgs a, int sm_count, cudaStream_t s)
+{
+    static int per_sm = 0;  // same for every device of one model; queried once
+    if (per_sm == 0) {
+        int n = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, noalloc_main_kernel<VEC, CH, G>, kWarps * 32, 0);
+        if (e != cudaSuccess) return e;
+        per_sm = n > 0 ? n : 1;
+    }
+    const uint32_t slabs = (a.N + 32 / G * VEC * CH - 1) / (32 / G * VEC * CH);
+    const uint32_t wave = (uint32_t)(sm_count * per_sm) / slabs;  // one resident wave
+    // rows per claim: about a buffer of nonzeros, at most one per lane; few rows are spread over all warps
+    const uint64_t fill = (uint64_t)kBuf * a.M / (a.nnz + 1) + 1, spread = (uint64_t)a.M / ((uint64_t)wave * kWarps) + 1;
+    uint64_t claim = fill < spread ? fill : spread;
+    if (claim < (uint64_t)G) claim = G;
+    if (claim > 32) claim = 32;
+    a.claim = (uint32_t)claim;
+    const uint64_t row_blocks = ((uint64_t)a.M + claim * kWarps - 1) / (claim * kWarps), chunk_blocks = (2ull * a.nnz / a.split + kWarps - 1) / kWarps;
+    const uint64_t want = a.nnz > a.split && chunk_blocks > row_blocks ? chunk_blocks : row_blocks;
+    noalloc_main_kernel<VEC, CH, G><<<dim3((uint32_t)(want < wave ? (want ? want : 1) : (wave ? wave : 1)), slabs), kWarps * 32, 0, s>>>(a);
+    return cudaGetLastError();
+}
 
 int fail(int status, const std::string &msg)
 {
@@ -234,11 +355,12 @@ extern "C" int cutespmm_spmm_csr_noalloc(uint32_t M, uint32_t K, uint32_t nnz, c
         return fail(CUTESPMM_EUNSUPPORTED, "cutespmm_spmm_csr_noalloc: N exceeds CUTESPMM_NOALLOC_MAX_N (" +
                                                std::to_string(CUTESPMM_NOALLOC_MAX_N) + "); call it per column window");
     const uint32_t lds = (N + 3) / 4 * 4;
-    const uint64_t slots = 2ull * ((nnz + kSplit - 1) / kSplit) + 2;
+    if (M > 0xfff00000u) return fail(CUTESPMM_EUNSUPPORTED, "cutespmm_spmm_csr_noalloc: the row counter leaves room for 2^32 - 2^20 rows");
+    const uint64_t slots = 2ull * ((nnz + kLimitSplit - 1) / kLimitSplit) + 2;
     if (slots * lds > kScratchFloats)
         return fail(CUTESPMM_EUNSUPPORTED,
                     "cutespmm_spmm_csr_noalloc: the built-in scratch (" + std::to_string(CUTESPMM_NOALLOC_SCRATCH_BYTES >> 20) +
-                        " MiB) holds (2*ceil(nnz/" + std::to_string(kSplit) + ")+2) x N partial sums; this call needs " +
+                        " MiB) holds (2*ceil(nnz/" + std::to_string(kLimitSplit) + ")+2) x N partial sums; this call needs " +
                         std::to_string((slots * lds * 4) >> 20) + " MiB. Use a plan (cutespmm_plan_create) or split the rows.");
     int dev = -1;
     cudaError_t e = cudaGetDevice(&dev);
@@ -256,48 +378,33 @@ extern "C" int cutespmm_spmm_csr_noalloc(uint32_t M, uint32_t K, uint32_t nnz, c
             e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
             if (e != cudaSuccess || sms <= 0)
                 return fail(CUTESPMM_ECUDA, std::string("cudaDeviceGetAttribute: ") + cudaGetErrorString(e));
-            uint32_t *ctr = nullptr;
-            e = cudaGetSymbolAddress(reinterpret_cast<void **>(&ctr), g_next_row);
-            if (e != cudaSuccess || !ctr)
-                return fail(CUTESPMM_ECUDA, std::string("cudaGetSymbolAddress(row counters): ") + cudaGetErrorString(e));
-            int per_sm = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, noalloc_rows_kernel, kWarps * 32, 0);
-            if (e != cudaSuccess) return fail(CUTESPMM_ECUDA, std::string("cudaOccupancyMaxActiveBlocksPerMultiprocessor: ") + cudaGetErrorString(e));
-            int per_sm_chunks = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_chunks, noalloc_chunks_kernel, kWarps * 32, 0);
-            if (e != cudaSuccess) return fail(CUTESPMM_ECUDA, std::string("cudaOccupancyMaxActiveBlocksPerMultiprocessor: ") + cudaGetErrorString(e));
             g_setup[dev].sm_count = sms;
-            g_setup[dev].rows_blocks_per_sm = per_sm > 0 ? per_sm : 1;
-            g_setup[dev].chunks_blocks_per_sm = per_sm_chunks > 0 ? per_sm_chunks : 1;
-            g_setup[dev].next_row = ctr;
             g_setup[dev].scratch = ptr;
         }
         setup = g_setup[dev];
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const uint32_t slabs = (N + kSlab - 1) / kSlab;
-    const uint32_t max_blocks = (uint32_t)setup.sm_count * 8;
-    auto blocks_for = [&](uint64_t items) {
-        const uint64_t b = (items + kWarps - 1) / kWarps;
-        return (uint32_t)(b < 1 ? 1 : (b > max_blocks ? max_blocks : b));
-    };
-    // the rows kernel: one resident wave of blocks whose warps claim rows from a counter per slab, zeroed here on the stream
-    e = cudaMemsetAsync(setup.next_row, 0, sizeof(uint32_t) * (CUTESPMM_NOALLOC_MAX_N / kSlab), s);
-    if (e != cudaSuccess) return fail(CUTESPMM_ECUDA, std::string("cutespmm_spmm_csr_noalloc: clearing the row counters: ") + cudaGetErrorString(e));
-    {
-        const uint64_t want = ((uint64_t)M + kClaim * kWarps - 1) / (kClaim * kWarps);
-        const uint64_t wave = (uint64_t)setup.sm_count * setup.rows_blocks_per_sm;
-        noalloc_rows_kernel<<<dim3((uint32_t)(want < wave ? (want ? want : 1) : wave), slabs), kWarps * 32, 0, s>>>(
-            rowPtr_dev, cols_dev, vals_dev, M, K, nnz, B_dev, ldb, C_dev, ldc, N, setup.next_row);
+    // Chunks as short as a large job (256 nonzeros) or a latency-bound one (128) wants them, longer where the scratch or the
+    // list would not hold them.
+    uint64_t split = nnz > (2u << 20) ? 256 : 128;
+    auto slots_of = [&](uint64_t len) { return 2ull * ((nnz + len - 1) / len) + 2; };
+    while (slots_of(split) * lds > kScratchFloats || slots_of(split) > kListSlots) split *= 2;
+    MainArgs a{rowPtr_dev, cols_dev, vals_dev, B_dev, C_dev, setup.scratch, ldb, ldc, M, K, nnz, N, lds, (uint32_t)split, 1};
+    if (nnz > split) {
+        const uint64_t want = ((uint64_t)M + 255) / 256, cap = (uint64_t)setup.sm_count * 8;
+        noalloc_list_kernel<<<(uint32_t)(want < cap ? want : cap), 256, 0, s>>>(rowPtr_dev, M, nnz, (uint32_t)split, (uint32_t)slots_of(split));
+        e = cudaGetLastError();
     }
-    if (nnz > kSplit) {  // a long row needs more than kSplit nonzeros
-        const uint32_t chunk_wave = (uint32_t)setup.sm_count * (uint32_t)setup.chunks_blocks_per_sm;
-        noalloc_chunks_kernel<<<dim3(std::min(blocks_for((nnz + kSplit - 1) / kSplit), chunk_wave), slabs), kWarps * 32, 0, s>>>(
-            rowPtr_dev, cols_dev, vals_dev, M, K, nnz, B_dev, ldb, setup.scratch, lds, N);
-        noalloc_fixup_kernel<<<dim3(blocks_for(M), slabs), kWarps * 32, 0, s>>>(rowPtr_dev, M, nnz, setup.scratch, lds,
-                                                                                C_dev, ldc, N);
+    // four columns per lane where the rows of B and C are 16-byte aligned; narrow products put several rows on a warp
+    const bool v4 = !((reinterpret_cast<uintptr_t>(B_dev) | reinterpret_cast<uintptr_t>(C_dev)) & 15) && !((ldb | ldc | N) & 3);
+    if (e == cudaSuccess) {
+        if (v4) e = N <= 16 ? launch_main<4, 1, 8>(a, setup.sm_count, s) : N <= 32 ? launch_main<4, 1, 4>(a, setup.sm_count, s)
+                  : N <= 64 ? launch_main<4, 1, 2>(a, setup.sm_count, s) : N <= 128 ? launch_main<4, 1, 1>(a, setup.sm_count, s)
+                                                                                   : launch_main<4, 2, 1>(a, setup.sm_count, s);
+        else e = N <= 8 ? launch_main<1, 1, 4>(a, setup.sm_count, s) : N <= 16 ? launch_main<1, 1, 2>(a, setup.sm_count, s)
+                : N <= 32 ? launch_main<1, 1, 1>(a, setup.sm_count, s) : N <= 64 ? launch_main<1, 2, 1>(a, setup.sm_count, s)
+                                                                              : launch_main<1, 4, 1>(a, setup.sm_count, s);
     }
-    e = cudaGetLastError();
     if (e != cudaSuccess) return fail(CUTESPMM_ECUDA, std::string("cutespmm_spmm_csr_noalloc launch: ") + cudaGetErrorString(e));
     return CUTESPMM_OK;
 }

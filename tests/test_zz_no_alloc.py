@@ -110,3 +110,28 @@ def test_noalloc_survives_row_pointers_and_columns_beyond_the_arrays(oracle_mod)
     cs.spmm_csr_noalloc(A.M, A.K, rp_bad.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), B, C2)
     torch.cuda.synchronize()
     assert oracle_mod.rel_fro(want2, C2.cpu().numpy()) <= REL_FRO_TOL_FP32
+
+
+@pytest.mark.parametrize("N", [1, 4, 8, 9, 16, 17, 32, 33, 64, 65, 100, 128, 132, 256, 257, 512])
+def test_noalloc_at_the_edges_of_every_width(oracle_mod, N):
+    """One form of the kernel per range of widths and alignment; rows around the staging buffer (256), the row length the
+    groups of a warp share (16), the chunk length (128); a chunk list that a claim of too many nonzeros overflows."""
+    rng = np.random.default_rng(N)
+    ln = rng.integers(0, 12, 700)
+    ln[[0, 5, 6, 7, 300, 301, 699]] = (16, 17, 127, 128, 129, 256, 1500)
+    rp = np.concatenate([[0], np.cumsum(ln)])
+    A = g.CsrMatrix(700, 400, torch.from_numpy(rp), torch.from_numpy(rng.integers(0, 400, rp[-1]).astype(np.int32)),
+                    torch.from_numpy(rng.standard_normal(rp[-1]).astype(np.float32)))
+    B = g.dense_operand(A.K, N, 99, device="cuda")
+    args = (A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), B)
+    want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.cpu().numpy(), A.M, A.K)
+    C = torch.full((A.M + 1, N), float("nan"), device="cuda")
+    for _ in range(2):  # the second call meets the counters as the first left them
+        cs.spmm_csr_noalloc(A.M, A.K, *args, C[:A.M])
+        assert oracle_mod.rel_fro(want, C[:A.M].cpu().numpy()) <= REL_FRO_TOL_FP32 and torch.isnan(C[A.M]).all()
+    bad = A.row_ptr.clone()
+    bad[1::2] = 0  # every second row claims all nonzeros up to its end: far more chunks than the nonzeros allow
+    cs.spmm_csr_noalloc(A.M, A.K, bad.to(torch.int32).cuda(), *args[1:], C[:A.M])
+    torch.cuda.synchronize()
+    cs.spmm_csr_noalloc(A.M, A.K, *args, C[:A.M])
+    assert oracle_mod.rel_fro(want, C[:A.M].cpu().numpy()) <= REL_FRO_TOL_FP32
