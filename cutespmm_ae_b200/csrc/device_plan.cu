@@ -122,6 +122,10 @@ int cutespmm_internal_usable_device(int *dev, int *sm_count)
 // of a caller may be gone by now, so nothing can be recorded on them), and after a wait for the device otherwise.
 void cutespmm_internal_free_block(void *block, uint64_t bytes, int dev, bool used_elsewhere)
 {
+    if (bytes > kPoolKeeps) {
+        cudaFree(block);  // not from the pool
+        return;
+    }
     if (used_elsewhere) cudaDeviceSynchronize();
     if (cudaFreeAsync(block, nullptr) != cudaSuccess) {
         cudaGetLastError();
@@ -402,9 +406,13 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
     };
     Carver need;
     carve(need);
-    if ((e = cutespmm_internal_pool_alloc(&p->d_block, need.used, dev, s)) != cudaSuccess) return fail_cuda_status(e, "memory of the plan");
+    // a block the pool would not keep is the driver's: mapping it into the pool takes longer than cudaMalloc (R-MAT 2^24,
+    // 3.7 GB: plan creation 130 ms longer)
+    const bool pooled = need.used <= kPoolKeeps;
+    if ((e = pooled ? cutespmm_internal_pool_alloc(&p->d_block, need.used, dev, s) : cudaMalloc(&p->d_block, need.used)) != cudaSuccess)
+        return fail_cuda_status(e, "memory of the plan");
     p->block_bytes = need.used;
-    note_live(dev, (int64_t)need.used);
+    if (pooled) note_live(dev, (int64_t)need.used);
     Carver c;
     c.base = static_cast<char *>(p->d_block);
     const uint64_t zero = carve(c);

@@ -34,6 +34,7 @@ struct RowsArgs {
     uint32_t *arrivals;        // per long row and column slab: chunks finished so far (zero between launches)
     uint32_t num_tiles, num_chunks, split_nnz;
     uint32_t avg_row_nnz;      // nonzeros per row of the whole matrix (picks the kernel's tuning)
+    uint32_t short_chunks;     // 1: a small job, its long rows are cut into pieces of tens of nonzeros
     const float *B;            // K x N window, leading dimension ldb
     float *C;                  // M x N window, leading dimension ldc
     float *scratch;            // partial sums, leading dimension ld_scratch

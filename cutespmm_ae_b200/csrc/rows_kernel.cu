@@ -202,6 +202,59 @@ __device__ __forceinline__ void accumulate_group(typename Vec<VEC>::T (&acc)[CH]
     }
 }
 
+// The same sum with the groups of a narrow warp sharing the nonzeros: group g takes nonzeros g, g + G, ... of every 32, so a
+// chunk is 1/G as many dependent steps.  The pairs come 32 at a time with one coalesced load, the next 32 while these are
+// in use.  Every group is left with its own partial sum.
+template <int VEC, int CH, bool FULL, int U, int G>
+__device__ __forceinline__ void accumulate_shared(typename Vec<VEC>::T (&acc)[CH], const uint2 *__restrict__ pairs, uint32_t j0, uint32_t j1,
+                                                  const float *__restrict__ bl, uint32_t ldb32, const bool (&ok)[CH], int lane, int grp)
+{
+    using V = typename Vec<VEC>::T;
+    constexpr int UU = U < 32 / G ? U : 32 / G;  // rows of B in flight per group and step
+    uint2 nxt = make_uint2(0u, 0u);
+    if (j0 + lane < j1) nxt = __ldcs(pairs + j0 + lane);
+    for (uint32_t j = j0; j < j1; j += 32) {
+        const uint2 pr = nxt;
+        if (j + 32 + lane < j1) nxt = __ldcs(pairs + j + 32 + lane);
+        const uint32_t n = min(32u, j1 - j);
+        for (uint32_t k = 0; k < n; k += UU * G) {
+            float v[UU];
+            V b[UU][CH];
+#pragma unroll
+            for (int u = 0; u < UU; ++u) {
+                const uint32_t at = k + u * G + grp;
+                const int src = (int)min(at, n - 1);
+                const uint32_t c = __shfl_sync(kFull, pr.x, src);
+                v[u] = __uint_as_float(__shfl_sync(kFull, pr.y, src));
+                if (at >= n) v[u] = 0.f;
+                const float *row = bl + (uint64_t)c * ldb32;
+#pragma unroll
+                for (int ch = 0; ch < CH; ++ch) {  // positions past the end load nothing and add nothing
+                    if (at < n && (FULL || ok[ch])) b[u][ch] = ldg_b(reinterpret_cast<const V *>(row + ch * 32 * VEC));
+                    else zero_vec(b[u][ch]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < UU; ++u)
+#pragma unroll
+                for (int ch = 0; ch < CH; ++ch) fma_vec(acc[ch], v[u], b[u][ch]);
+        }
+    }
+}
+
+// acc = the sum over the groups of a warp, pairwise in a fixed tree (the result depends on nothing but the group size), in
+// every lane.
+template <int L> __device__ __forceinline__ void add_groups(float4 &acc)
+{
+#pragma unroll
+    for (int off = L; off < 32; off <<= 1) {
+        acc.x += __shfl_xor_sync(kFull, acc.x, off);
+        acc.y += __shfl_xor_sync(kFull, acc.y, off);
+        acc.z += __shfl_xor_sync(kFull, acc.z, off);
+        acc.w += __shfl_xor_sync(kFull, acc.w, off);
+    }
+}
+
 // What the chunk part of the kernel needs.  The pointers bl / scratch / C already point at this lane's first column.
 struct ChunkArgs {
     const uint2 *pairs;
@@ -216,41 +269,48 @@ struct ChunkArgs {
     bool c_scalar;
 };
 
-// A chunk's partial sum goes to its slot of the scratch matrix; the warp (or group) that completes a row's last
-// outstanding chunk adds the slots in slot order -- so the sum does not depend on who that was -- and writes the row
-// of C.  Nobody waits for anybody: whoever is not last just moves on.
-template <int VEC, int CH, bool FULL, bool DEEP, int G>
+// A chunk's partial sum goes to its slot of the scratch matrix, and the warp that completes a row's last outstanding chunk
+// adds the slots in slot order -- so the sum does not depend on who that was -- and writes the row of C.  Nobody waits for
+// anybody: whoever is not last just moves on.  A warp takes a chunk at a time (SHARE, or G = 1), or one per group.
+template <int VEC, int CH, bool FULL, bool DEEP, int G, bool SHARE>
 __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
 {
     using V = typename Vec<VEC>::T;
-    constexpr int L = 32 / G;
+    constexpr int L = 32 / G, P = SHARE ? 1 : G;  // P chunks per warp
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int grp = G == 1 ? 0 : lane / L, sub = G == 1 ? lane : lane % L;
+    const int grp = G == 1 ? 0 : lane / L, sub = lane - grp * L;
+    const bool lead = P == 1 ? lane == 0 : sub == 0;
     bool ok[CH];
 #pragma unroll
     for (int ch = 0; ch < CH; ++ch) ok[ch] = FULL || (a.col0 + ch * 32 * VEC < a.N);
     // chunk (group) c goes to block c mod gridDim.x: spread over the SMs, and the warps of a block that got none
     // start on the block's tile at once (rows of a tile are claimed as they go, so they take over the others' share)
     const uint32_t gw = warp * gridDim.x + blockIdx.x, nw = gridDim.x * kWarps;
-    for (uint64_t cw = gw; cw * G < a.num_chunks; cw += nw) {
-        const uint64_t c = cw * G + grp;
-        const bool have = c < a.num_chunks;
+    for (uint64_t cw = gw; cw * P < a.num_chunks; cw += nw) {
+        const uint64_t c = P == 1 ? cw : cw * P + grp;
+        const bool have = P == 1 || c < a.num_chunks;
         uint4 ck = make_uint4(0u, 0u, 0u, 0u);
         if (have) ck = __ldg(a.chunks + c);
         // which long row the chunk belongs to.  The narrow kernels (small N: latency-bound jobs) ask now and use the
         // answer after the gathers; the wide ones ask when they need it and keep the registers for the gathers.
         uint32_t owner = 0;
         uint4 lr = make_uint4(0u, 0u, 0u, 0u);  // row of C, slot0, slot1
-        if (G > 1 && have && sub == 0) {
+        if (G > 1 && have && lead) {
             owner = __ldg(a.chunk_owner + ck.w);
             lr = __ldg(a.long_rows + owner);
         }
         V acc[CH];
 #pragma unroll
         for (int ch = 0; ch < CH; ++ch) zero_vec(acc[ch]);
-        if constexpr (G == 1) accumulate<VEC, CH, FULL, DEEP>(acc, a.pairs, ck.y, ck.z, a.bl, a.ldb, ok, lane);
-        else accumulate_group<VEC, CH, FULL, Tuning<DEEP>::kUnroll, L>(acc, a.pairs, ck.y, ck.z, a.bl, (uint32_t)a.ldb, ok, sub, (L == 32 ? kFull : ((1u << L) - 1u)) << (grp * L));
-        if (have) {
+        if constexpr (G == 1) {
+            accumulate<VEC, CH, FULL, DEEP>(acc, a.pairs, ck.y, ck.z, a.bl, a.ldb, ok, lane);
+        } else if constexpr (!SHARE) {
+            accumulate_group<VEC, CH, FULL, Tuning<DEEP>::kUnroll, L>(acc, a.pairs, ck.y, ck.z, a.bl, (uint32_t)a.ldb, ok, sub, ((1u << L) - 1u) << (grp * L));
+        } else {
+            accumulate_shared<VEC, CH, FULL, Tuning<DEEP>::kUnroll, G>(acc, a.pairs, ck.y, ck.z, a.bl, (uint32_t)a.ldb, ok, lane, grp);
+            add_groups<L>(acc[0]);
+        }
+        if (P == 1 ? (G == 1 || grp == 0) : have) {
             float *out = a.scratch + (uint64_t)ck.w * a.ld_scratch;
 #pragma unroll
             for (int ch = 0; ch < CH; ++ch)
@@ -259,7 +319,7 @@ __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
         __threadfence();  // this lane's part of the slot is visible device-wide before the arrival is counted
         __syncwarp();
         uint32_t lr_row = 0, slot0 = 0, slot1 = 0;
-        if (have && sub == 0) {
+        if (have && lead) {
             if (G == 1) {
                 owner = __ldg(a.chunk_owner + ck.w);
                 lr = __ldg(a.long_rows + owner);
@@ -271,46 +331,27 @@ __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
                 lr_row = lr.x; slot0 = lr.y; slot1 = lr.z;
             }
         }
-        constexpr int R = (VEC * CH >= 8) ? 4 : 8;  // slots in flight
-        if constexpr (G == 1) {
-            lr_row = __shfl_sync(kFull, lr_row, 0);
-            slot0 = __shfl_sync(kFull, slot0, 0);
-            slot1 = __shfl_sync(kFull, slot1, 0);
-            if (slot1 > slot0) {
+        __syncwarp();
+        // the whole warp adds the slots of every row it completed: group h takes slots h, h + G, ... in order
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+            const uint32_t s0 = __shfl_sync(kFull, slot0, q * L), s1 = __shfl_sync(kFull, slot1, q * L), row = __shfl_sync(kFull, lr_row, q * L);
+            if (s1 > s0) {  // the same for every lane of the warp
+                constexpr int R = (VEC * CH >= 8) ? 4 : 8;  // slots in flight
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch) zero_vec(acc[ch]);
 #pragma unroll R
-                for (uint32_t k = slot0; k < slot1; ++k) {
+                for (uint32_t k = s0 + grp; k < s1; k += G) {
 #pragma unroll
                     for (int ch = 0; ch < CH; ++ch)
                         if (FULL || ok[ch]) add_vec(acc[ch], __ldcg(reinterpret_cast<const V *>(a.scratch + (uint64_t)k * a.ld_scratch + ch * 32 * VEC)));
                 }
-                float *crow = a.C + (uint64_t)lr_row * a.ldc;
+                if constexpr (G > 1) add_groups<L>(acc[0]);
+                if (G == 1 || grp == 0) {
+                    float *crow = a.C + (uint64_t)row * a.ldc;
 #pragma unroll
-                for (int ch = 0; ch < CH; ++ch)
-                    if (FULL || ok[ch]) store_row<FULL>(crow + ch * 32 * VEC, acc[ch], a.c_scalar, a.N - a.col0 - ch * 32 * VEC);
-            }
-        } else {
-            // The whole warp adds the slots of every row one of its groups completed: group h takes slots h, h+G, ...
-            // in order, then the groups' sums are added pairwise (a fixed tree: the result depends on nothing but G).
-            __syncwarp();
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const uint32_t s0 = __shfl_sync(kFull, slot0, g * L), s1 = __shfl_sync(kFull, slot1, g * L);
-                const uint32_t row = __shfl_sync(kFull, lr_row, g * L);
-                if (s1 > s0) {  // the same for every lane of the warp
-                    zero_vec(acc[0]);
-#pragma unroll R
-                    for (uint32_t k = s0 + grp; k < s1; k += G)
-                        if (FULL || ok[0]) add_vec(acc[0], __ldcg(reinterpret_cast<const V *>(a.scratch + (uint64_t)k * a.ld_scratch)));
-#pragma unroll
-                    for (int off = L; off < 32; off <<= 1) {
-                        acc[0].x += __shfl_xor_sync(kFull, acc[0].x, off);
-                        acc[0].y += __shfl_xor_sync(kFull, acc[0].y, off);
-                        acc[0].z += __shfl_xor_sync(kFull, acc[0].z, off);
-                        acc[0].w += __shfl_xor_sync(kFull, acc[0].w, off);
-                    }
-                    if (grp == 0 && (FULL || ok[0])) store_row<FULL>(a.C + (uint64_t)row * a.ldc, acc[0], a.c_scalar, a.N - a.col0);
+                    for (int ch = 0; ch < CH; ++ch)
+                        if (FULL || ok[ch]) store_row<FULL>(crow + ch * 32 * VEC, acc[ch], a.c_scalar, a.N - a.col0 - ch * 32 * VEC);
                 }
             }
         }
@@ -343,10 +384,17 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::kMinBlocks) spmm_ro
     tile_ring_start(ring, src);
 
     // Chunks of long rows first (the first tiles are on their way meanwhile): they are the largest single work items.
-    if (a.num_chunks)
-        run_chunks<VEC, CH, FULL, DEEP, G>(ChunkArgs{pairs, reinterpret_cast<const uint4 *>(a.chunks), reinterpret_cast<const uint4 *>(a.long_rows),
-                                                     a.chunk_owner, a.arrivals, bl, a.scratch + col0, a.C + col0, a.ldb, a.ld_scratch, a.ldc,
-                                                     a.num_chunks, a.N, col0, a.c_scalar != 0});
+    if (a.num_chunks) {
+        const ChunkArgs ca{pairs, reinterpret_cast<const uint4 *>(a.chunks), reinterpret_cast<const uint4 *>(a.long_rows), a.chunk_owner, a.arrivals, bl,
+                           a.scratch + col0, a.C + col0, a.ldb, a.ld_scratch, a.ldc, a.num_chunks, a.N, col0, a.c_scalar != 0};
+        // Narrow products: when the warps outnumber the chunks, a chunk is shared by the groups of a warp -- it is the longest
+        // chain of the job (R-MAT 2^17: 4 500 chunks of 256, 64 steps of four gathers for a group at N = 64; N = 16 63.6 ->
+        // 39.4 us, N = 32 70.4 -> 56.5) -- otherwise a group takes one on its own and the cost of starting and finishing a
+        // chunk is paid once per G of them (R-MAT 2^20 N = 64: shared is 5 % slower).  The short pieces of a small job are shared
+        // only when they leave half of the warps to the rows (R-MAT 2^12 N = 32 12.1 -> 9.2 us, 2^14 N = 64 14.3 -> 15.2).
+        if (G == 1 || a.num_chunks <= gridDim.x * (a.short_chunks ? kWarps / 2 : kWarps)) run_chunks<VEC, CH, FULL, DEEP, G, true>(ca);
+        else if constexpr (G > 1) run_chunks<VEC, CH, FULL, DEEP, G, false>(ca);
+    }
 
     for (uint32_t i = 0;; ++i) {
         const uint64_t t = blockIdx.x + (uint64_t)i * gridDim.x;
