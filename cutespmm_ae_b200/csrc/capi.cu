@@ -341,6 +341,9 @@ static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B,
     a.N = N;
     a.status = p->d_status;
     a.row_map = static_cast<const uint32_t *>(p->d_row_map);
+    // Tiles are dealt as they are finished where there are long rows: launches of such a plan share the partial sums and must
+    // not overlap anyway; a plan without long rows may run on several streams at once and keeps nothing between launches.
+    a.counters = a.num_chunks && !rg ? p->d_status + kTileCounters : nullptr;
     a.b_padded = b_padded ? 1u : 0u;
     if (rg) {  // a sub-range of the lists: 16-byte tiles and chunks (a chunk names its scratch slot and, through it, its long row)
         const uint32_t t0 = all_rows ? rg->ta0 : rg->t0, t1 = all_rows ? rg->ta1 : rg->t1;

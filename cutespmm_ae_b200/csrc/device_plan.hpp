@@ -32,6 +32,7 @@ struct RowsArgs {
     const void *long_rows;     // the whole list of long rows {row of C, slot0, slot1, -}, indexed by chunk_owner
     const uint32_t *chunk_owner;  // per scratch slot: index of the long row the chunk belongs to
     uint32_t *arrivals;        // per long row and column slab: chunks finished so far (zero between launches)
+    uint32_t *counters;        // blocks done, then tiles dealt per column slab; zero between launches.  nullptr: tiles in fixed turns
     uint32_t num_tiles, num_chunks, split_nnz;
     uint32_t avg_row_nnz;      // nonzeros per row of the whole matrix (picks the kernel's tuning)
     uint32_t short_chunks;     // 1: a small job, its long rows are cut into pieces of tens of nonzeros

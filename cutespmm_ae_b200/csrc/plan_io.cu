@@ -3,7 +3,7 @@
 //
 // File layout (little-endian, as the machine writes it; the tag word detects the other kind):
 //     16 bytes  "CUTESPMM-PLAN\0\0\0"
-//     u32 version, u32 byte-order tag 0x01020304, u64 M, K, nnz, cutespmm_options_t, u32 device_built, u32 0
+//     u32 version, u32 byte-order tag 0x01020304, u64 M, K, nnz, cutespmm_options_t, u32 device_built, u32 adaptive_tiling
 //     u64 num_bricks, brick_panels, brick_slots, slab_steps, slab_panels
 //     sections  { u32 id, u32 element size, u64 count, count * size bytes }   one per array of the plan
 //     u32 id 0, u32 0, u64 checksum (FNV-1a over everything before this section)
@@ -116,7 +116,7 @@ int cutespmm_plan_save(const cutespmm_plan_t *plan, const char *path)
     w.pod(h.M); w.pod(h.K); w.pod(h.nnz);
     w.pod(h.opts);
     w.pod((uint32_t)(h.device_built ? 1 : 0));
-    w.pod((uint32_t)0);
+    w.pod((uint32_t)(h.adaptive_tiling ? 1 : 0));
     w.pod(h.num_bricks); w.pod(h.brick_panels); w.pod(h.brick_slots); w.pod(h.slab_steps); w.pod(h.slab_panels);
     for_each_array(h, [&](uint32_t id, auto &v) { w.section(id, v); });
     const uint64_t sum = w.hash;
@@ -147,7 +147,7 @@ int cutespmm_plan_load(cutespmm_plan_t **plan, const char *path, int host_only)
     HostPlan &h = p->host;
     Reader r{f};
     char magic[16];
-    uint32_t version = 0, tag = 0, built = 0, zero = 0;
+    uint32_t version = 0, tag = 0, built = 0, adaptive = 0;
     r.bytes(magic, sizeof(magic));
     r.pod(version);
     r.pod(tag);
@@ -157,10 +157,11 @@ int cutespmm_plan_load(cutespmm_plan_t **plan, const char *path, int host_only)
     r.pod(h.M); r.pod(h.K); r.pod(h.nnz);
     r.pod(h.opts);
     r.pod(built);
-    r.pod(zero);
+    r.pod(adaptive);
     r.pod(h.num_bricks); r.pod(h.brick_panels); r.pod(h.brick_slots); r.pod(h.slab_steps); r.pod(h.slab_panels);
     if (!r.ok || h.opts.struct_size != sizeof(cutespmm_options_t)) return bad("damaged header");
     h.device_built = built != 0;
+    h.adaptive_tiling = adaptive != 0;
     bool fine = true;
     std::string why;
     try {

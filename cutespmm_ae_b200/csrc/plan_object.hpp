@@ -11,6 +11,9 @@
 
 #include "plan.hpp"
 
+// The 256-byte status block: word 0 the status, words kTileCounters... the row kernel's counters (blocks done, tiles per slab).
+constexpr uint32_t kTileCounters = 16;
+
 // A contiguous range of the plan's work items (tiles and chunks of the row kernel -- of its own list and
 // of the list over every row -- and panels of the brick kernel): what one launch covers when a product is issued in
 // blocks of rows.

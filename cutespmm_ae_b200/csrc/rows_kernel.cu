@@ -362,7 +362,7 @@ __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
 // G = rows of A (or chunks) a warp works on at the same time.  G = 1: the 32 lanes span 32*VEC*CH columns of B.
 // G = 2, 4, 8 (narrow products, N <= 64, float4 lanes): the warp is G groups of 32/G lanes, a group spans the whole
 // row of B and owns a row of A of its own, so a warp keeps G times as many gathers in flight and no lane idles.
-template <int VEC, int CH, bool FULL, bool DEEP, int G>
+template <int VEC, int CH, bool FULL, bool DEEP, int G, bool DYN>
 __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::kMinBlocks) spmm_rows_kernel(RowsArgs a)
 {
     using V = typename Vec<VEC>::T;
@@ -380,8 +380,8 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::kMinBlocks) spmm_ro
 
     // ---- tiles: descriptor, row pointers and pairs arrive in shared memory by TMA, kTileStages deep ----
     __shared__ TileRing ring;
-    const TileSource src{reinterpret_cast<const uint4 *>(a.tiles), a.row_ptr, pairs, a.num_tiles};
-    tile_ring_start(ring, src);
+    const TileSource src{reinterpret_cast<const uint4 *>(a.tiles), a.row_ptr, pairs, a.num_tiles, DYN ? a.counters + 1 + blockIdx.y : nullptr};
+    tile_ring_start<DYN>(ring, src);
 
     // Chunks of long rows first (the first tiles are on their way meanwhile): they are the largest single work items.
     if (a.num_chunks) {
@@ -397,12 +397,16 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::kMinBlocks) spmm_ro
     }
 
     for (uint32_t i = 0;; ++i) {
-        const uint64_t t = blockIdx.x + (uint64_t)i * gridDim.x;
-        if (t >= a.num_tiles) break;
+        uint64_t t = blockIdx.x + (uint64_t)i * gridDim.x;
+        if (!DYN && t >= a.num_tiles) break;
         const int s = i % kTileStages;
         if (!tile_wait(ring, i)) {
             if (lane == 0) atomicExch(a.status, 1u);  // the copy never landed: report, do not hang
             break;
+        }
+        if (DYN) {
+            t = ring.tile[s];
+            if (t == kNoTile) break;
         }
         const TileStage &st = ring.stage[s];
         const uint4 d = st.desc;
@@ -433,7 +437,16 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::kMinBlocks) spmm_ro
             }
             if constexpr (G > 1) __syncwarp();
         }
-        tile_release(ring, src, i, t, lane);  // the last warp to leave the stage refills it
+        tile_release<DYN>(ring, src, i, t, lane);  // the last warp to leave the stage refills it
+    }
+    if (DYN) {  // the last block to leave puts the tile counters back for the next launch
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const uint32_t blocks = gridDim.x * gridDim.y;
+            __threadfence();
+            if (atomicInc(a.counters, blocks - 1) == blocks - 1)
+                for (uint32_t y = 0; y < gridDim.y; ++y) a.counters[1 + y] = 0;
+        }
     }
 }
 
@@ -443,17 +456,22 @@ cudaError_t launch_rows_t(const RowsArgs &a, uint32_t slabs, int sm_count, cudaS
     static int blocks_per_sm = 0;  // same for every device of one model; queried once
     if (blocks_per_sm == 0) {
         int n = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, spmm_rows_kernel<VEC, CH, FULL, DEEP, G>, kWarps * 32, 0);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, spmm_rows_kernel<VEC, CH, FULL, DEEP, G, false>, kWarps * 32, 0);
         if (e != cudaSuccess) return e;
         blocks_per_sm = n > 0 ? n : 1;
     }
     const uint64_t want = (uint64_t)sm_count * blocks_per_sm;
-    const uint64_t chunk_blocks = ((uint64_t)a.num_chunks + kWarps * G - 1) / (kWarps * G);
+    const uint64_t chunk_blocks = ((uint64_t)a.num_chunks + kWarps - 1) / kWarps;
     uint64_t work = a.num_tiles > chunk_blocks ? a.num_tiles : chunk_blocks;
     uint32_t gx = (uint32_t)(work < want ? work : want);
     if (slabs > 1) gx = (gx + slabs - 1) / slabs;  // keep the whole grid about one resident wave
     if (gx == 0) gx = 1;
-    spmm_rows_kernel<VEC, CH, FULL, DEEP, G><<<dim3(gx, slabs), kWarps * 32, 0, s>>>(a);
+    if constexpr (VEC == 4)  // tiles dealt by a counter: where there are counters and enough tiles to deal
+        if (a.counters && a.num_tiles >= 8ull * gx) {
+            spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true><<<dim3(gx, slabs), kWarps * 32, 0, s>>>(a);
+            return cudaGetLastError();
+        }
+    spmm_rows_kernel<VEC, CH, FULL, DEEP, G, false><<<dim3(gx, slabs), kWarps * 32, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, FLAT || V < 3 ? 4 : 3) sddmm_
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % LANES;
     const uint2 *pairs = reinterpret_cast<const uint2 *>(a.pairs);
     __shared__ TileRing ring;
-    const TileSource src{reinterpret_cast<const uint4 *>(a.tiles), a.row_ptr, pairs, a.num_tiles};
+    const TileSource src{reinterpret_cast<const uint4 *>(a.tiles), a.row_ptr, pairs, a.num_tiles, nullptr};
     tile_ring_start(ring, src);
 
     // chunks of long rows first (the tiles are on their way): chunk c goes to block c mod gridDim.x.  The pairs of a

@@ -26,6 +26,7 @@ struct __align__(16) TileStage {
 struct TileRing {
     TileStage stage[kTileStages];
     alignas(8) uint64_t full_bar[kTileStages];
+    uint32_t tile[kTileStages];        // dealt by a counter: the staged tile's index, kNoTile when there are no more
     uint32_t next_row[kTileStages];    // rows of the staged tile already claimed
     uint32_t warps_done[kTileStages];  // warps that have left the stage
 };
@@ -36,7 +37,14 @@ struct TileSource {
     const uint32_t *row_ptr;
     const uint2 *pairs;
     uint32_t num_tiles;
+    uint32_t *counter;  // DYN: tiles dealt beyond the first kTileStages per block, zero at the start
 };
+constexpr uint32_t kNoTile = 0xffffffffu;
+
+// DYN: which tiles a block gets beyond its first kTileStages.  Every gridDim.x-th (false), or the next one of a counter, which
+// evens out tiles that run unequally long (rows of very different lengths, long rows summed by some of the warps): R-MAT 2^20
+// N = 128 720 -> 671 us, 2^24 15.9 -> 14.8 ms.  Below about eight tiles per block there is nothing to even out and the
+// counter's latency shows (R-MAT 2^17 N = 64: 71 -> 73 us).
 
 // One thread: fetch tile t into stage s.
 __device__ __forceinline__ void tile_issue(TileRing &ring, const TileSource &src, uint32_t t, int s)
@@ -51,9 +59,18 @@ __device__ __forceinline__ void tile_issue(TileRing &ring, const TileSource &src
     if (je > jb) ptx::bulk_g2s(ring.stage[s].pairs, src.pairs + jb, (je - jb) * 8u, &ring.full_bar[s]);
 }
 
-// Whole block: set the ring up and ask for the block's first tiles (tile i of block b is b + i * gridDim.x).
+// One thread: tile t into stage s if there is one; with DYN the end is marked there otherwise.
+template <bool DYN> __device__ __forceinline__ void tile_issue_or_end(TileRing &ring, const TileSource &src, uint64_t t, int s)
+{
+    const bool more = t < src.num_tiles;
+    if (DYN) ring.tile[s] = more ? (uint32_t)t : kNoTile;
+    if (more) tile_issue(ring, src, (uint32_t)t, s);
+    else if (DYN) ptx::mbar_arrive(&ring.full_bar[s]);
+}
+
+// Whole block: set the ring up and ask for the block's first tiles (tile i of block b is b + i * gridDim.x, i < kTileStages).
 // Ends with a block-wide barrier.
-__device__ __forceinline__ void tile_ring_start(TileRing &ring, const TileSource &src)
+template <bool DYN = false> __device__ __forceinline__ void tile_ring_start(TileRing &ring, const TileSource &src)
 {
     if (threadIdx.x == 0) {
         for (int s = 0; s < kTileStages; ++s) {
@@ -64,7 +81,7 @@ __device__ __forceinline__ void tile_ring_start(TileRing &ring, const TileSource
         ptx::fence_mbar_init();
         for (int s = 0; s < kTileStages; ++s) {
             const uint64_t t = blockIdx.x + (uint64_t)s * gridDim.x;
-            if (t < src.num_tiles) tile_issue(ring, src, (uint32_t)t, s);
+            tile_issue_or_end<DYN>(ring, src, t, s);
         }
     }
     __syncthreads();
@@ -85,7 +102,7 @@ __device__ __forceinline__ uint32_t tile_claim_rows(TileRing &ring, int s, uint3
 }
 
 // Whole warp: this warp is finished with the block's i-th tile (tile index t); the last warp to say so refills the stage.
-__device__ __forceinline__ void tile_release(TileRing &ring, const TileSource &src, uint32_t i, uint64_t t, int lane)
+template <bool DYN = false> __device__ __forceinline__ void tile_release(TileRing &ring, const TileSource &src, uint32_t i, uint64_t t, int lane)
 {
     const int s = i % kTileStages;
     __syncwarp();
@@ -95,10 +112,10 @@ __device__ __forceinline__ void tile_release(TileRing &ring, const TileSource &s
             __threadfence_block();
             ring.warps_done[s] = 0;
             ring.next_row[s] = 0;
-            const uint64_t t2 = t + (uint64_t)kTileStages * gridDim.x;
-            if (t2 < src.num_tiles) {
+            const uint64_t t2 = DYN ? (uint64_t)kTileStages * gridDim.x + atomicAdd(src.counter, 1u) : t + (uint64_t)kTileStages * gridDim.x;
+            if (DYN || t2 < src.num_tiles) {
                 ptx::fence_async_smem();
-                tile_issue(ring, src, (uint32_t)t2, s);
+                tile_issue_or_end<DYN>(ring, src, t2, s);
             }
         }
     }

@@ -413,3 +413,25 @@ def test_widths_that_no_vector_divides_on_jobs_worth_a_padded_copy(oracle_mod, N
         assert oracle_mod.rel_fro(want, cbig[:, 2:N + 2].cpu().numpy()) <= 2e-6
         assert (cbig[:, :2] == 7).all() and (cbig[:, N + 2:] == 7).all()  # nothing between the rows
         assert p.device_status() == 0
+
+
+@pytest.mark.parametrize("N", [16, 30, 64, 128, 160])
+def test_tiles_dealt_by_a_counter(oracle_mod, N):
+    """A matrix with long rows and at least eight tiles per block has its tiles dealt as they are finished; the counters are
+    back at zero after every launch, and a plan whose long rows come from few chunks shares them between lane groups."""
+    rng = np.random.default_rng(5)
+    ln = rng.integers(0, 6, 900_000)
+    ln[[0, 400_000, 899_999]] = (5000, 300, 2000)
+    rp = np.concatenate([[0], np.cumsum(ln)])
+    A = g.CsrMatrix(ln.size, 5000, torch.from_numpy(rp), torch.from_numpy(rng.integers(0, 5000, rp[-1]).astype(np.int32)),
+                    torch.from_numpy(rng.standard_normal(rp[-1]).astype(np.float32)))
+    p = cs.Plan.from_device_csr(A.M, A.K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS)
+    assert p.info()["num_tiles"] >= 8 * 888 and p.info()["num_long_rows"] == 3
+    B = g.dense_operand(A.K, N, 6)
+    want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.numpy(), A.M, A.K)
+    Bd = B.cuda()
+    first = p.spmm(Bd)
+    assert oracle_mod.rel_fro(want, first.cpu().numpy()) <= 2e-6
+    for _ in range(3):
+        assert torch.equal(p.spmm(Bd), first)
+    assert p.device_status() == 0
