@@ -335,7 +335,7 @@ static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B,
     a.arrivals = p->d_arrivals;
     a.split_nnz = h.opts.split_nnz;
     a.avg_row_nnz = (uint32_t)(h.nnz / std::max<uint64_t>(h.M, 1));
-    a.short_chunks = item_sizes(h.nnz + kRowCost * h.M, h.opts.split_nnz, h.opts.tile_nnz, h.adaptive_tiling).latency_bound ? 1u : 0u;
+    a.short_chunks = item_sizes(h.nnz + kRowCost * h.M, h.nnz, h.M, 0, h.opts.split_nnz, h.opts.tile_nnz, h.adaptive_tiling).latency_bound ? 1u : 0u;
     a.B = B; a.C = C; a.scratch = p->d_scratch;
     a.ldb = ldb; a.ldc = ldc; a.ld_scratch = kScratchCols;
     a.N = N;

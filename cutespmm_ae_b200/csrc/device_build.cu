@@ -110,6 +110,19 @@ static_assert(kEntries == kMaxTileRows + 1 && kTileSegmentRows % kPanelRows == 0
 static_assert(kListThreads >= (int)kEntries && kListThreads % 32 == 0, "a thread per entry row");
 constexpr uint32_t kSegmentView = kTileSegmentRows + kMaxTileRows;  // rows a segment's last tile may reach
 
+// *out += nonzeros in rows longer than kDefaultSplitNnz (what item_sizes decides by; of jobs large enough to ask).
+__global__ void __launch_bounds__(256) long_share_kernel(const uint32_t *__restrict__ row_ptr, uint32_t M, unsigned long long *__restrict__ out)
+{
+    if ((uint64_t)__ldg(row_ptr + M) + (uint64_t)kRowCost * M <= (uint64_t)kMaxAdaptiveTileCost * kResidentTiles) return;
+    uint32_t mine = 0;
+    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < M; r += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t p0 = __ldg(row_ptr + r), p1 = __ldg(row_ptr + r + 1);
+        if (p1 > p0 && p1 - p0 > kDefaultSplitNnz) mine += p1 - p0;
+    }
+    mine = __reduce_add_sync(kFullMask, mine);
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(out, (unsigned long long)mine);
+}
+
 struct SegmentView {
     uint32_t rp[kSegmentView + 1];           // row pointers of rows [first, first + n]
     uint32_t special[kSegmentView / 32 + 1];  // bit r: row is long, or not in this list
@@ -173,7 +186,7 @@ __device__ __forceinline__ bool load_segment(SegmentView &v, const uint32_t *__r
 
 __device__ __forceinline__ ItemSizes list_sizes(const ListArgs &a, uint32_t nnz)
 {
-    return item_sizes(a.total_known ? a.total : (uint64_t)nnz + (uint64_t)kRowCost * a.M, a.split_nnz, a.tile_nnz, a.adaptive != 0);
+    return item_sizes(a.total_known ? a.total : (uint64_t)nnz + (uint64_t)kRowCost * a.M, nnz, a.M, *a.long_nnz, a.split_nnz, a.tile_nnz, a.adaptive != 0);
 }
 // pieces of row r when it is long and in the list
 __device__ __forceinline__ uint32_t pieces_of(const SegmentView &v, const ListArgs &a, const ItemSizes &sizes, uint32_t first, uint32_t r)
@@ -658,6 +671,8 @@ cudaError_t launch_pack(const uint32_t *row_ptr, const uint32_t *cols, const flo
 cudaError_t launch_lists_count(const uint32_t *row_ptr, const ListArgs &a, cudaStream_t s)
 {
     if (a.num_segments == 0) return cudaSuccess;
+    if (!a.total_known)  // the first list of a plan
+        long_share_kernel<<<std::min((a.M + 2047) / 2048, 1184u), 256, 0, s>>>(row_ptr, a.M, const_cast<unsigned long long *>(a.long_nnz));
     lists_count_kernel<<<a.num_segments, kListThreads, 0, s>>>(row_ptr, a);
     return cudaGetLastError();
 }

@@ -332,6 +332,7 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
     set_tables(la, 0);
     la.seg_chunks = counters; la.seg_longs = counters + segments;
     la.totals = d_totals;
+    la.long_nnz = &d_totals->long_nnz;
     CensusArgs ca{};
     ca.M = M; ca.num_panels = P; ca.force = brick_path ? 1u : 0u;
     ca.split_nnz = h.opts.split_nnz; ca.density = h.opts.brick_density;

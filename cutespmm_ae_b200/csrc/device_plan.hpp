@@ -125,13 +125,14 @@ struct BuildTotals {  // one per plan creation, read by the host after the count
     uint32_t tiles;
     uint32_t chunks, long_rows, brick_panels, brick_slots;  // in the order of the per-segment counters
     uint32_t brick_nnz_max, brick_cols_max, pad;
-    unsigned long long bricks, brick_cost;
+    unsigned long long bricks, brick_cost, long_nnz;
 };
 struct ListArgs {
     uint32_t M, num_segments;
     uint32_t split_nnz, tile_nnz, adaptive;
     uint32_t total_known;   // 1: `total` is the cost of the listed rows; 0: every row is listed, nnz + kRowCost * M
     uint64_t total;
+    const unsigned long long *long_nnz;  // nonzeros in long rows, summed by the first count
     const uint8_t *path;   // per panel: 1 = not listed (nullptr: every row is)
     uint16_t *exits, *tile_counts;  // per segment and entry row: entry row of the next segment, tiles
     uint16_t *path_entry;   // per segment and entry row of its group: entry row of the segment ...

@@ -106,7 +106,12 @@ static void build_tiles(const HostPlan &p, bool all_rows, std::vector<Tile> &til
         const uint64_t r0 = q * kPanelRows, r1 = std::min<uint64_t>(p.M, r0 + kPanelRows);
         total += (p.row_ptr[r1] - p.row_ptr[r0]) + (r1 - r0) * kRowCost;
     }
-    const ItemSizes sizes = item_sizes(total, p.opts.split_nnz, p.opts.tile_nnz, p.adaptive_tiling);
+    uint64_t long_nnz = 0;
+    for (uint64_t r = 0; r < p.M; ++r) {
+        const uint32_t len = p.row_ptr[r + 1] - p.row_ptr[r];
+        if (len > kDefaultSplitNnz) long_nnz += len;
+    }
+    const ItemSizes sizes = item_sizes(total, p.nnz, p.M, long_nnz, p.opts.split_nnz, p.opts.tile_nnz, p.adaptive_tiling);
     tiles.clear();
     chunks.clear();
     long_rows.clear();

@@ -30,6 +30,9 @@ constexpr uint32_t kMinAdaptiveTileCost = 96;     // smallest tile it makes (8 w
 constexpr uint32_t kMaxAdaptiveTileCost = 1024;   // largest: beyond it the job is not small, tiles go back to the default cost
 constexpr uint32_t kAdaptiveSplitDivisor = 8192;  // rows are cut from job cost / this nonzeros on: 256 from 2.1 M cost units
 constexpr uint32_t kMinAdaptiveSplitNnz = 128;    // ... but never from fewer than this
+constexpr uint64_t kMidJobCost = 8u << 20;        // jobs up to this with an eighth of their nonzeros in long rows: cut from 128 on
+constexpr uint32_t kWideTileRowNnz = 12;          // nonzeros per row from which a large job's tiles are larger:
+constexpr uint32_t kWideTileCost = 768, kMixedTileCost = 640;  // ... and with an eighth of the nonzeros in long rows
 constexpr uint32_t kMinChunkNnz = 32;             // smallest piece of a cut row
 constexpr uint32_t kMaxSplitNnz = 384;   // a row must fit a tile together with a part-filled one
 constexpr uint32_t kScratchCols = 512;  // widest N one launch handles; wider products run in column windows
@@ -58,23 +61,32 @@ struct Tile {
 // about eight latencies of its own -- descriptor, pairs, arrival count, the sum -- so shorter rows are quicker
 // whole), and a cut row into pieces of about sqrt(length / 2) nonzeros: the chain is a piece's gathers followed
 // by the sum of the pieces, the sum runs a few slots per step, and that length makes the two about equal.
+//
+// Larger jobs: a graph with much of its nonzeros in long rows is cut finer up to kMidJobCost (R-MAT 2^17 N = 32 56 -> 41 us,
+// 2^18 N = 64 118 -> 99: a chunk of 256 is still a visible part of the run; beyond, N = 128 loses what N = 32 gains), and
+// rows of a dozen nonzeros and more get larger tiles (elasticity40 N = 32 41 -> 37 us: fewer starts per nonzero).
 struct ItemSizes {
     uint32_t split;      // rows longer than this are cut into chunks
     uint32_t target;     // cost at which a tile is closed
     bool latency_bound;  // pieces of sqrt(length / 2)
 };
-CUTESPMM_HD inline ItemSizes item_sizes(uint64_t total, uint32_t split_nnz, uint32_t tile_nnz, bool adaptive)
+// nnz, M: of the whole matrix; long_nnz: its nonzeros in rows longer than kDefaultSplitNnz
+CUTESPMM_HD inline ItemSizes item_sizes(uint64_t total, uint64_t nnz, uint64_t M, uint64_t long_nnz, uint32_t split_nnz, uint32_t tile_nnz, bool adaptive)
 {
     ItemSizes s{split_nnz, tile_nnz, false};
     if (!adaptive) return s;
     if (total / kResidentTiles <= kMaxAdaptiveTileCost) {
         const uint64_t t = total / kResidentTiles;
         s.target = (uint32_t)(t > kMinAdaptiveTileCost ? t : kMinAdaptiveTileCost);
+    } else if (nnz >= kWideTileRowNnz * M) {
+        s.target = long_nnz * 8 >= nnz ? kMixedTileCost : kWideTileCost;
     }
     if (total / kAdaptiveSplitDivisor < s.split) {
         s.latency_bound = true;
         const uint64_t t = total / kAdaptiveSplitDivisor;
         s.split = (uint32_t)(t > kMinAdaptiveSplitNnz ? t : kMinAdaptiveSplitNnz);
+    } else if (total < kMidJobCost && long_nnz * 8 >= nnz && s.split > kMinAdaptiveSplitNnz) {
+        s.split = kMinAdaptiveSplitNnz;
     }
     return s;
 }
