@@ -71,7 +71,11 @@ __global__ void __launch_bounds__(kBrickWarps * 32, 1) spmm_brick_kernel(const _
     // (stencil512 0.0700 -> 0.0676 ms, elasticity40 0.0720 -> 0.0679 ms at N = 128).
     const uint32_t W = gridDim.x * kBrickWarps;
     uint32_t ord = warp * gridDim.x + blockIdx.x;  // this warp's current panel (ordinal among brick panels)
-    if (ord >= a.num_panels) return;  // warps never synchronise with each other, so leaving early is safe
+    if (ord >= a.num_panels) {
+        ptx::grid_wait();
+        return;
+    }
+    // (warps never synchronise with each other, so leaving early is safe)
     // A product wider than one slab of L::kSlab columns walks every panel once per slab, slab after slab, before it moves
     // to its next panel: the panel's records and column lists are then found in L2 by the second walk, and one grid of
     // persistent blocks covers all slabs.
@@ -169,6 +173,8 @@ __global__ void __launch_bounds__(kBrickWarps * 32, 1) spmm_brick_kernel(const _
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
 
+    ptx::grid_wait();  // the plan's metadata is in registers; B and C are the stream's
+    ptx::grid_release();
     for (int s0 = 1; s0 < kStages && producer_has_work(); ++s0) issue_one();  // fill the ring
     for (;;) {
         if (producer_has_work() && issued < done + kStages) issue_one();
@@ -232,9 +238,7 @@ template <int NT, bool ROUND_B> cudaError_t launch_brick_t(const BrickArgs &a, i
     CUtensorMap tmap;
     e = make_b_tensor_map(&tmap, a.B, a.N, a.K, a.ldb, L::kStride, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (e != cudaSuccess) return e;
-    if (multi) spmm_brick_kernel<NT, ROUND_B, true><<<blocks, kBrickWarps * 32, smem, s>>>(tmap, a);
-    else spmm_brick_kernel<NT, ROUND_B, false><<<blocks, kBrickWarps * 32, smem, s>>>(tmap, a);
-    return cudaGetLastError();
+    return launch_overlapped(multi ? spmm_brick_kernel<NT, ROUND_B, true> : spmm_brick_kernel<NT, ROUND_B, false>, blocks, kBrickWarps * 32, smem, s, tmap, a);
 }
 
 }  // namespace

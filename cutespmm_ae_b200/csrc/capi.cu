@@ -344,6 +344,7 @@ static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B,
     // Tiles are dealt as they are finished where there are long rows: launches of such a plan share the partial sums and must
     // not overlap anyway; a plan without long rows may run on several streams at once and keeps nothing between launches.
     a.counters = a.num_chunks && !rg ? p->d_status + kTileCounters : nullptr;
+    a.early = h.values_on_device ? 0u : 1u;
     a.b_padded = b_padded ? 1u : 0u;
     if (rg) {  // a sub-range of the lists: 16-byte tiles and chunks (a chunk names its scratch slot and, through it, its long row)
         const uint32_t t0 = all_rows ? rg->ta0 : rg->t0, t1 = all_rows ? rg->ta1 : rg->t1;
@@ -577,6 +578,7 @@ int cutespmm_sddmm(const cutespmm_plan_t *p, const float *X, uint64_t ldx, const
     a.num_chunks = all ? p->every.chunks : p->own.chunks;
     a.X = X; a.Y = Y; a.ldx = ldx; a.ldy = ldy; a.out = out; a.N = N;
     a.scale = scale_by_values ? 1u : 0u;
+    a.early = h.values_on_device ? 0u : 1u;
     a.avg_row_nnz = (uint32_t)(h.nnz / std::max<uint64_t>(h.M, 1));
     a.status = p->d_status;
     a.vec4 = !((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15) && !((ldx | ldy) & 3) ? 1u : 0u;

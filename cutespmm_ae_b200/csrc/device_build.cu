@@ -10,6 +10,7 @@
 
 #include "device_plan.hpp"
 #include "plan.hpp"
+#include "ptx.cuh"
 
 namespace cutespmm {
 
@@ -625,6 +626,8 @@ template <bool ORDER>
 __global__ void __launch_bounds__(256) set_values_kernel(uint2 *__restrict__ pairs, const float *__restrict__ vals, const uint32_t *__restrict__ order,
                                                          uint64_t nnz)
 {
+    ptx::grid_wait();
+    ptx::grid_release();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nnz; j += stride)
         pairs[j].y = __float_as_uint(ORDER ? __ldg(vals + __ldcs(order + j)) : __ldcs(vals + j));
@@ -646,9 +649,7 @@ cudaError_t launch_set_values(void *pairs, const float *vals, const uint32_t *or
 {
     if (nnz == 0) return cudaSuccess;
     const uint32_t blocks = (uint32_t)std::min<uint64_t>((nnz + 255) / 256, (uint64_t)sm_count * 8);
-    if (order) set_values_kernel<true><<<blocks, 256, 0, s>>>(static_cast<uint2 *>(pairs), vals, order, nnz);
-    else set_values_kernel<false><<<blocks, 256, 0, s>>>(static_cast<uint2 *>(pairs), vals, order, nnz);
-    return cudaGetLastError();
+    return launch_overlapped(order ? set_values_kernel<true> : set_values_kernel<false>, blocks, 256, 0, s, static_cast<uint2 *>(pairs), vals, order, nnz);
 }
 
 cudaError_t launch_unpack(const void *pairs, uint32_t *cols, float *vals, uint64_t nnz, int sm_count, cudaStream_t s)

@@ -23,6 +23,24 @@ template <auto Kernel> cudaError_t allow_dynamic_smem(int bytes)
     return e;
 }
 
+// Launches a kernel whose blocks may be set up while the kernel in front of it on the stream still runs (the kernel calls
+// ptx::grid_wait before it depends on anything): back-to-back calls of a 5-us product are a launch latency shorter each.
+template <class... Params, class... Args>
+cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args &&...args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // Arguments of the row-gather kernel.
 struct RowsArgs {
     const uint32_t *row_ptr;   // M+1 offsets into pairs
@@ -41,6 +59,7 @@ struct RowsArgs {
     float *scratch;            // partial sums, leading dimension ld_scratch
     uint64_t ldb, ldc, ld_scratch;
     uint32_t N;
+    uint32_t early;            // 1: the plan's arrays never change, its first tiles can be fetched before the kernel in front is done
     uint32_t b_padded;         // 1: a row of B can be read up to N rounded up to four columns
     uint32_t c_scalar;         // set by launch_rows: C is written column by column
     uint32_t *status;          // device status word: set to 1 when a bounded wait gives up
@@ -63,6 +82,7 @@ struct SddmmArgs {
     uint32_t N;
     uint32_t scale;                      // 1: multiply by the stored value of A
     uint32_t avg_row_nnz;                // nonzeros per row of the whole matrix (picks the kernel's form)
+    uint32_t early;                      // 1: the plan's arrays never change (RowsArgs::early)
     uint32_t vec4;                       // 1: X, Y and their leading dimensions allow 16-byte loads
     uint32_t *status;                    // device status word: set to 1 when a bounded wait gives up
 };

@@ -28,12 +28,16 @@
 #include <string>
 
 #include "../../include/cutespmm.h"
+#include "device_plan.hpp"
+#include "ptx.cuh"
 
 namespace cutespmm {
 void set_last_error(const std::string &msg);  // capi.cu
 }
 
 namespace {
+
+namespace ptx = cutespmm::ptx;
 
 constexpr uint32_t kLimitSplit = CUTESPMM_NOALLOC_SPLIT_NNZ;  // the chunk length the published limit is stated for
 constexpr uint64_t kScratchFloats = CUTESPMM_NOALLOC_SCRATCH_BYTES / 4;
@@ -74,6 +78,8 @@ __device__ __forceinline__ Range row_range(const uint32_t *__restrict__ rowPtr, 
 __global__ void __launch_bounds__(256) noalloc_list_kernel(const uint32_t *__restrict__ rowPtr, uint32_t M, uint32_t nnz, uint32_t split,
                                                            uint32_t capacity)
 {
+    ptx::grid_wait();
+    ptx::grid_release();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < M; r += stride) {
         const Range g = row_range(rowPtr, r, nnz);
@@ -198,6 +204,8 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
         over_groups(acc);
     };
 
+    ptx::grid_wait();
+    ptx::grid_release();
     const bool overflow = g_state.overflow != 0;
     const uint32_t chunks = overflow ? 0u : g_state.chunks;
     for (uint32_t c = warp * gridDim.x + blockIdx.x; c < chunks; c += gridDim.x * kWarps) {
@@ -331,8 +339,8 @@ template <int VEC, int CH, int G> cudaError_t launch_main(MainArgs a, int sm_cou
     a.claim = (uint32_t)claim;
     const uint64_t row_blocks = ((uint64_t)a.M + claim * kWarps - 1) / (claim * kWarps), chunk_blocks = (2ull * a.nnz / a.split + kWarps - 1) / kWarps;
     const uint64_t want = a.nnz > a.split && chunk_blocks > row_blocks ? chunk_blocks : row_blocks;
-    noalloc_main_kernel<VEC, CH, G><<<dim3((uint32_t)(want < wave ? (want ? want : 1) : (wave ? wave : 1)), slabs), kWarps * 32, 0, s>>>(a);
-    return cudaGetLastError();
+    return cutespmm::launch_overlapped(noalloc_main_kernel<VEC, CH, G>, dim3((uint32_t)(want < wave ? (want ? want : 1) : (wave ? wave : 1)), slabs), kWarps * 32,
+                                       0, s, a);
 }
 
 int fail(int status, const std::string &msg)
@@ -392,8 +400,8 @@ extern "C" int cutespmm_spmm_csr_noalloc(uint32_t M, uint32_t K, uint32_t nnz, c
     MainArgs a{rowPtr_dev, cols_dev, vals_dev, B_dev, C_dev, setup.scratch, ldb, ldc, M, K, nnz, N, lds, (uint32_t)split, 1};
     if (nnz > split) {
         const uint64_t want = ((uint64_t)M + 255) / 256, cap = (uint64_t)setup.sm_count * 8;
-        noalloc_list_kernel<<<(uint32_t)(want < cap ? want : cap), 256, 0, s>>>(rowPtr_dev, M, nnz, (uint32_t)split, (uint32_t)slots_of(split));
-        e = cudaGetLastError();
+        e = cutespmm::launch_overlapped(noalloc_list_kernel, (uint32_t)(want < cap ? want : cap), 256, 0, s, rowPtr_dev, M, nnz, (uint32_t)split,
+                                        (uint32_t)slots_of(split));
     }
     // four columns per lane where the rows of B and C are 16-byte aligned; narrow products put several rows on a warp
     const bool v4 = !((reinterpret_cast<uintptr_t>(B_dev) | reinterpret_cast<uintptr_t>(C_dev)) & 15) && !((ldb | ldc | N) & 3);

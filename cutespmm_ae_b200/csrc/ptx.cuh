@@ -9,6 +9,12 @@
 namespace cutespmm {
 namespace ptx {
 
+// Programmatic dependent launch (launch_overlapped in device_plan.hpp): grid_wait returns when every kernel in front of this
+// one on its stream has completed and its writes are visible; every thread of a kernel launched that way runs it before it
+// touches anything such a kernel may have written, or still reads.  grid_release lets the next such kernel be set up now.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 constexpr uint32_t kSpinLimit = 1u << 22;  // polls of try_wait (each already blocks for a hardware time slice)
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }

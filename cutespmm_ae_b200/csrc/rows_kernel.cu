@@ -381,7 +381,10 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::kMinBlocks) spmm_ro
     // ---- tiles: descriptor, row pointers and pairs arrive in shared memory by TMA, kTileStages deep ----
     __shared__ TileRing ring;
     const TileSource src{reinterpret_cast<const uint4 *>(a.tiles), a.row_ptr, pairs, a.num_tiles, DYN ? a.counters + 1 + blockIdx.y : nullptr};
+    if (!a.early) ptx::grid_wait();
     tile_ring_start<DYN>(ring, src);
+    ptx::grid_wait();
+    ptx::grid_release();
 
     // Chunks of long rows first (the first tiles are on their way meanwhile): they are the largest single work items.
     if (a.num_chunks) {
@@ -467,12 +470,9 @@ cudaError_t launch_rows_t(const RowsArgs &a, uint32_t slabs, int sm_count, cudaS
     if (slabs > 1) gx = (gx + slabs - 1) / slabs;  // keep the whole grid about one resident wave
     if (gx == 0) gx = 1;
     if constexpr (VEC == 4)  // tiles dealt by a counter: where there are counters and enough tiles to deal
-        if (a.counters && a.num_tiles >= 8ull * gx) {
-            spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true><<<dim3(gx, slabs), kWarps * 32, 0, s>>>(a);
-            return cudaGetLastError();
-        }
-    spmm_rows_kernel<VEC, CH, FULL, DEEP, G, false><<<dim3(gx, slabs), kWarps * 32, 0, s>>>(a);
-    return cudaGetLastError();
+        if (a.counters && a.num_tiles >= 8ull * gx)
+            return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true>, dim3(gx, slabs), kWarps * 32, 0, s, a);
+    return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, false>, dim3(gx, slabs), kWarps * 32, 0, s, a);
 }
 
 // dst (rows x quads float4, 16-byte aligned) = src (rows x N, leading dimension ld_src), padding zeroed.  Bound by memory
@@ -480,6 +480,8 @@ cudaError_t launch_rows_t(const RowsArgs &a, uint32_t slabs, int sm_count, cudaS
 __global__ void __launch_bounds__(256) pad_rows_kernel(const float *__restrict__ src, uint64_t ld_src, float4 *__restrict__ dst, uint32_t quads, uint32_t N,
                                                        uint64_t rows)
 {
+    ptx::grid_wait();
+    ptx::grid_release();
     const uint32_t per_block = 256 / quads, mine = threadIdx.x / quads, c = (threadIdx.x - mine * quads) * 4;
     if (mine >= per_block) return;
     const uint64_t step = (uint64_t)gridDim.x * per_block;
@@ -509,8 +511,7 @@ cudaError_t launch_pad_rows(const float *src, uint64_t ld_src, float *dst, uint6
     const uint32_t quads = (N + 3) / 4;
     if (rows == 0 || N == 0) return cudaSuccess;
     const uint64_t per_block = 256 / quads, want = (rows + 4 * per_block - 1) / (4 * per_block), cap = (uint64_t)sm_count * 8;
-    pad_rows_kernel<<<(uint32_t)(want < cap ? want : cap), 256, 0, s>>>(src, ld_src, reinterpret_cast<float4 *>(dst), quads, N, rows);
-    return cudaGetLastError();
+    return launch_overlapped(pad_rows_kernel, (uint32_t)(want < cap ? want : cap), 256, 0, s, src, ld_src, reinterpret_cast<float4 *>(dst), quads, N, rows);
 }
 
 int rows_kernel_count(const RowsArgs &a) { return (a.num_tiles || a.num_chunks) ? 1 : 0; }

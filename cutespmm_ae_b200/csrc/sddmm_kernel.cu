@@ -167,7 +167,10 @@ __global__ void __launch_bounds__(kTileWarps * 32, FLAT || V < 3 ? 4 : 3) sddmm_
     const uint2 *pairs = reinterpret_cast<const uint2 *>(a.pairs);
     __shared__ TileRing ring;
     const TileSource src{reinterpret_cast<const uint4 *>(a.tiles), a.row_ptr, pairs, a.num_tiles, nullptr};
+    if (!a.early) ptx::grid_wait();
     tile_ring_start(ring, src);
+    ptx::grid_wait();
+    ptx::grid_release();
 
     // chunks of long rows first (the tiles are on their way): chunk c goes to block c mod gridDim.x.  The pairs of a
     // chunk come 32 at a time with one coalesced load, the next 32 while these are in use.
@@ -249,8 +252,7 @@ template <int LANES, int V, bool VEC4, bool FULL, bool FLAT> cudaError_t launch_
     uint32_t blocks = a.num_tiles > chunk_blocks ? a.num_tiles : chunk_blocks;
     const uint32_t cap = (uint32_t)(sm_count * per_sm);  // one resident wave
     if (blocks > cap) blocks = cap;
-    sddmm_kernel<LANES, V, VEC4, FULL, FLAT><<<blocks, kTileWarps * 32, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_overlapped(sddmm_kernel<LANES, V, VEC4, FULL, FLAT>, blocks, kTileWarps * 32, 0, s, a);
 }
 template <int LANES, int V> cudaError_t launch_sddmm_v(const SddmmArgs &a, int sm_count, cudaStream_t s)
 {
