@@ -1,0 +1,147 @@
+// Row kernel for matrices whose rows come in runs of R with the same columns: the degrees of freedom of a node in a
+// finite-element matrix (R = 3 in 3-D elasticity).  A group of lanes takes a run at a time: a row of B is loaded once and
+// multiplied into R accumulators, where the row kernel loads it R times.  The row kernel is bound by the L1 data pipe on such
+// matrices (80 % busy on elasticity40 at N = 32, half of its requests hits), and that is what a shared load relieves.
+// fp32, storage order: a row's result is the row kernel's, bit for bit.  Tiles and their staging are the row kernel's too
+// (tile_stage.cuh); a run that a tile boundary cuts is computed in two parts.  The reference has no counterpart (its bricks
+// share loads between the rows of a panel on the tensor cores, kernel.cu:119-288).
+// Row kernel -> here: elasticity40 N = 32 35.1 -> 25.7 us, N = 27 48.7 -> 34.2; elasticity20 N = 128 20.4 -> 12.8.
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "device_plan.hpp"
+#include "plan.hpp"
+#include "ptx.cuh"
+#include "tile_stage.cuh"
+
+namespace cutespmm {
+
+namespace {
+
+constexpr int kUnroll = 6;  // rows of B in flight per group: 4 / 6 / 8 took 27.2 / 25.7 / 28.5 us on elasticity40 at N = 32
+
+__device__ __forceinline__ void fma4(float4 &a, float v, const float4 &b)
+{
+    a.x = fmaf(v, b.x, a.x); a.y = fmaf(v, b.y, a.y); a.z = fmaf(v, b.z, a.z); a.w = fmaf(v, b.w, a.w);
+}
+
+// U columns of a run, the pairs of its rows at first[0 .. R-1] + i: U rows of B in flight.  TAIL: only the first cnt count.
+template <int R, int U, bool TAIL>
+__device__ __forceinline__ void run_step(float4 (&acc)[R], const uint2 *pairs, const uint32_t (&first)[R], uint32_t i, uint32_t cnt, const float *bl, uint32_t ldb,
+                                         bool ok)
+{
+    float4 b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const uint32_t c = pairs[first[0] + i + (TAIL ? min((uint32_t)u, cnt - 1) : u)].x;
+        b[u] = ok ? __ldg(reinterpret_cast<const float4 *>(bl + (uint64_t)c * ldb)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (!TAIL || (uint32_t)u < cnt) {
+#pragma unroll
+            for (int k = 0; k < R; ++k) fma4(acc[k], __uint_as_float(pairs[first[k] + i + u].y), b[u]);
+        }
+}
+
+template <int R, int G>
+__global__ void __launch_bounds__(kTileWarps * 32, 4) spmm_block_rows_kernel(RowsArgs a)
+{
+    constexpr int L = 32 / G, U = kUnroll;
+    const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
+    const uint32_t col0 = blockIdx.y * 128 + sub * 4;
+    const bool ok = col0 < a.N;
+    const float *bl = a.B + col0;
+    const uint32_t ldb = (uint32_t)a.ldb;
+
+    __shared__ TileRing ring;
+    const TileSource src{reinterpret_cast<const uint4 *>(a.tiles), a.row_ptr, reinterpret_cast<const uint2 *>(a.pairs), a.num_tiles, nullptr};
+    if (!a.early) ptx::grid_wait();
+    tile_ring_start(ring, src);
+    ptx::grid_wait();
+    ptx::grid_release();
+
+    for (uint32_t i = 0;; ++i) {
+        const uint64_t t = blockIdx.x + (uint64_t)i * gridDim.x;
+        if (t >= a.num_tiles) break;
+        const int s = i % kTileStages;
+        if (!tile_wait(ring, i)) {
+            if (lane == 0) atomicExch(a.status, 1u);  // the copy never landed: report, do not hang
+            break;
+        }
+        const TileStage &st = ring.stage[s];
+        const uint4 d = st.desc;
+        const uint32_t rb = d.x & ~3u, jb = d.z & ~1u, run0 = d.x / R, runs = (d.y + R - 1) / R - run0;
+        for (;;) {
+            const uint32_t claimed = tile_claim_rows(ring, s, (uint32_t)G, lane);
+            if (claimed >= runs) break;
+            const uint32_t run = claimed + grp;
+            if (run < runs) {
+                const uint32_t r0 = (run0 + run) * R, lo = max(r0, d.x), hi = min(r0 + R, d.y);
+                // rows of the run outside the tile stand in for a row inside it; they are not stored
+                uint32_t first[R];
+#pragma unroll
+                for (int k = 0; k < R; ++k) first[k] = st.row_ptr[min(max(r0 + k, lo), hi - 1) - rb] - jb;
+                const uint32_t len = st.row_ptr[lo + 1 - rb] - st.row_ptr[lo - rb];
+                float4 acc[R];
+#pragma unroll
+                for (int k = 0; k < R; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                uint32_t j = 0;
+                for (; j + U <= len; j += U) run_step<R, U, false>(acc, st.pairs, first, j, U, bl, ldb, ok);
+                if (const uint32_t rem = len - j) {
+                    if (rem > U / 2) run_step<R, U, true>(acc, st.pairs, first, j, rem, bl, ldb, ok);
+                    else run_step<R, U / 2, true>(acc, st.pairs, first, j, rem, bl, ldb, ok);
+                }
+#pragma unroll
+                for (int k = 0; k < R; ++k) {
+                    if (r0 + k < lo || r0 + k >= hi || !ok) continue;
+                    float *p = a.C + (uint64_t)(r0 + k) * a.ldc + col0;
+                    if (!a.c_scalar) {
+                        __stcs(reinterpret_cast<float4 *>(p), acc[k]);
+                    } else {
+                        __stcs(p, acc[k].x);
+                        if (col0 + 1 < a.N) __stcs(p + 1, acc[k].y);
+                        if (col0 + 2 < a.N) __stcs(p + 2, acc[k].z);
+                        if (col0 + 3 < a.N) __stcs(p + 3, acc[k].w);
+                    }
+                }
+            }
+            if constexpr (G > 1) __syncwarp();
+        }
+        tile_release(ring, src, i, t, lane);
+    }
+}
+
+template <int R, int G> cudaError_t launch_t(const RowsArgs &a, int sm_count, cudaStream_t s)
+{
+    static int per_sm = 0;  // same for every device of one model; queried once
+    if (per_sm == 0) {
+        int n = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, spmm_block_rows_kernel<R, G>, kTileWarps * 32, 0);
+        if (e != cudaSuccess) return e;
+        per_sm = n > 0 ? n : 1;
+    }
+    const uint32_t slabs = (a.N + 127) / 128, wave = (uint32_t)(sm_count * per_sm);
+    uint32_t gx = a.num_tiles < wave ? a.num_tiles : wave;
+    if (slabs > 1) gx = (gx + slabs - 1) / slabs;
+    return launch_overlapped(spmm_block_rows_kernel<R, G>, dim3(gx, slabs), kTileWarps * 32, 0, s, a);
+}
+template <int R> cudaError_t launch_r(const RowsArgs &a, int sm_count, cudaStream_t s)
+{
+    if (a.N <= 16) return launch_t<R, 8>(a, sm_count, s);
+    if (a.N <= 32) return launch_t<R, 4>(a, sm_count, s);
+    if (a.N <= 64) return launch_t<R, 2>(a, sm_count, s);
+    return launch_t<R, 1>(a, sm_count, s);
+}
+
+}  // namespace
+
+// Called by launch_rows for operands it reads four columns per lane (a.c_scalar is set), a list without chunks and a plan
+// whose rows come in runs of a.run_rows.
+cudaError_t launch_block_rows(const RowsArgs &a, int sm_count, cudaStream_t s)
+{
+    return a.run_rows == 3 ? launch_r<3>(a, sm_count, s) : launch_r<2>(a, sm_count, s);
+}
+
+}  // namespace cutespmm

@@ -345,6 +345,8 @@ static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B,
     // not overlap anyway; a plan without long rows may run on several streams at once and keeps nothing between launches.
     a.counters = a.num_chunks && !rg ? p->d_status + kTileCounters : nullptr;
     a.early = h.values_on_device ? 0u : 1u;
+    a.run_rows = h.run_rows;
+    a.num_rows = (uint32_t)h.M;
     a.b_padded = b_padded ? 1u : 0u;
     if (rg) {  // a sub-range of the lists: 16-byte tiles and chunks (a chunk names its scratch slot and, through it, its long row)
         const uint32_t t0 = all_rows ? rg->ta0 : rg->t0, t1 = all_rows ? rg->ta1 : rg->t1;

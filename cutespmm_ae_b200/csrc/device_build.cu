@@ -486,6 +486,31 @@ __global__ void __launch_bounds__(kCensusThreads) panel_census_kernel(const uint
     }
 }
 
+// ---- rows in runs of the same columns (find_row_runs, plan.cpp) ----------------------------------------------------
+// A thread per row compares it with the row in front.  What is ruled out already is not looked at again: for most matrices that
+// is everything after each block's first rows, so the grid is one block per SM at most and a warp reports once.  Positions are
+// clamped to nnz (nobody has checked the row pointers yet).
+__global__ void __launch_bounds__(1024) row_runs_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ cols, uint32_t M,
+                                                        volatile uint32_t *uneven)
+{
+    const uint32_t nnz = __ldg(row_ptr + M), lane = threadIdx.x & 31;
+    for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); b < M; b += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t known = __shfl_sync(kFullMask, *uneven, 0);
+        if (known == 3) return;
+        const uint64_t r = b + lane;
+        const uint32_t asks = r < M ? ((r % 2 ? 1u : 0u) | (r % 3 ? 2u : 0u)) & ~known : 0u;
+        uint32_t found = 0;
+        if (asks) {
+            const uint32_t i = min(__ldg(row_ptr + r - 1), nnz), j = min(__ldg(row_ptr + r), nnz), e = min(__ldg(row_ptr + r + 1), nnz);
+            bool same = i <= j && j <= e && j - i == e - j;
+            for (uint32_t k = 0; same && j + k < e; ++k) same = __ldg(cols + i + k) == __ldg(cols + j + k);
+            if (!same) found = asks;
+        }
+        found = __reduce_or_sync(kFullMask, found);
+        if (found && lane == 0) atomicOr(const_cast<uint32_t *>(uneven), found);
+    }
+}
+
 // ---- slots of the brick stream ------------------------------------------------------------------------------------
 // One warp per segment of kTileSegmentRows rows: its panels' slot ranges, from the segment's offsets (lists_scan_kernel).
 __global__ void __launch_bounds__(128) brick_layout_kernel(uint32_t num_panels, const uint8_t *__restrict__ path, const uint32_t *__restrict__ ncols,
@@ -703,6 +728,13 @@ cudaError_t launch_panel_census(const uint32_t *row_ptr, const uint32_t *cols, C
     if (e != cudaSuccess) return e;
     const uint32_t blocks = std::min((a.num_panels + kCensusWarps - 1) / kCensusWarps, (uint32_t)sm_count * 16);
     panel_census_kernel<<<blocks, kCensusThreads, smem, s>>>(row_ptr, cols, a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_row_runs(const uint32_t *row_ptr, const uint32_t *cols, uint32_t M, uint32_t *uneven, int sm_count, cudaStream_t s)
+{
+    if (M < 2) return cudaSuccess;
+    row_runs_kernel<<<std::min((M + 1023) / 1024, (uint32_t)sm_count), 1024, 0, s>>>(row_ptr, cols, M, uneven);
     return cudaGetLastError();
 }
 

@@ -341,11 +341,13 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
     ca.totals = d_totals;
     BuildTotals t{};
     if ((e = cudaMemsetAsync(temp.p, 0, zeroed, s)) != cudaSuccess || (e = launch_lists_count(rowPtr_dev, la, s)) != cudaSuccess ||
+        (cols_dev && (M % 2 == 0 || M % 3 == 0) && (e = launch_row_runs(rowPtr_dev, cols_dev, M, &d_totals->uneven, sms, s)) != cudaSuccess) ||
         (census && cols_dev && (e = launch_panel_census(rowPtr_dev, cols_dev, ca, sms, s)) != cudaSuccess) ||
         (e = launch_lists_scan(rowPtr_dev, la, counters, census ? 4 : 2, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(&t, d_totals, sizeof(t), cudaMemcpyDeviceToHost, s)) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)
         return fail_cuda_status(e, "reading the row pointers");
     h.nnz = t.nnz;
+    h.run_rows = M < 2 || !t.nnz ? 0 : M % 3 == 0 && !(t.uneven & 2) ? 3 : M % 2 == 0 && !(t.uneven & 1) ? 2 : 0;
     if (t.bad_rows || (M == 0 && t.nnz)) return fail_status(CUTESPMM_EINVAL, "rowPtr must start at 0 and be non-decreasing");
     if (h.nnz && (!cols_dev || !vals_dev)) return fail_status(CUTESPMM_EINVAL, "cols/vals is NULL");
     if (brick_path && t.too_large)

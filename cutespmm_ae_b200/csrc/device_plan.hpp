@@ -59,6 +59,8 @@ struct RowsArgs {
     float *scratch;            // partial sums, leading dimension ld_scratch
     uint64_t ldb, ldc, ld_scratch;
     uint32_t N;
+    uint32_t num_rows;         // of the whole matrix
+    uint32_t run_rows;         // rows come in aligned runs of this many (2 or 3) with the same columns; 0: they do not
     uint32_t early;            // 1: the plan's arrays never change, its first tiles can be fetched before the kernel in front is done
     uint32_t b_padded;         // 1: a row of B can be read up to N rounded up to four columns
     uint32_t c_scalar;         // set by launch_rows: C is written column by column
@@ -66,6 +68,7 @@ struct RowsArgs {
     const uint32_t *row_map;   // reordered plan: row r of the work lists is row row_map[r] of C (nullptr: identity)
 };
 
+cudaError_t launch_block_rows(const RowsArgs &a, int sm_count, cudaStream_t s);
 cudaError_t launch_rows(const RowsArgs &a, int sm_count, cudaStream_t s);
 // dst: rows x (N rounded up to 4) floats, 16-byte aligned
 cudaError_t launch_pad_rows(const float *src, uint64_t ld_src, float *dst, uint64_t rows, uint32_t N, int sm_count, cudaStream_t s);
@@ -144,7 +147,8 @@ struct BuildTotals {  // one per plan creation, read by the host after the count
     uint32_t nnz, bad_rows, bad_cols, too_large;
     uint32_t tiles;
     uint32_t chunks, long_rows, brick_panels, brick_slots;  // in the order of the per-segment counters
-    uint32_t brick_nnz_max, brick_cols_max, pad;
+    uint32_t brick_nnz_max, brick_cols_max;
+    uint32_t uneven;  // bit 0: some odd row has other columns than the row in front of it, bit 1: some row not divisible by 3
     unsigned long long bricks, brick_cost, long_nnz;
 };
 struct ListArgs {
@@ -181,6 +185,7 @@ struct CensusArgs {
 cudaError_t launch_lists_count(const uint32_t *row_ptr, const ListArgs &a, cudaStream_t s);
 cudaError_t launch_lists_scan(const uint32_t *row_ptr, const ListArgs &a, uint32_t *counters, uint32_t how_many, cudaStream_t s);
 cudaError_t launch_lists_write(const uint32_t *row_ptr, const ListArgs &a, cudaStream_t s);
+cudaError_t launch_row_runs(const uint32_t *row_ptr, const uint32_t *cols, uint32_t M, uint32_t *uneven, int sm_count, cudaStream_t s);
 cudaError_t launch_panel_census(const uint32_t *row_ptr, const uint32_t *cols, CensusArgs a, int sm_count, cudaStream_t s);
 cudaError_t launch_brick_layout(uint32_t num_panels, const uint8_t *path, const uint32_t *ncols, const uint32_t *seg_panels, const uint32_t *seg_slots,
                                 uint32_t num_segments, uint32_t *ids, uint32_t *first, uint32_t *last, cudaStream_t s);

@@ -325,6 +325,24 @@ void choose_panel_paths(HostPlan &p, const std::vector<uint32_t> &panel_ncols)
     }
 }
 
+uint32_t find_row_runs(const HostPlan &p)
+{
+    if (p.M < 2 || p.nnz == 0) return 0;
+    bool two = p.M % 2 == 0, three = p.M % 3 == 0;
+    for (uint64_t r = 1; r < p.M && (two || three); ++r) {
+        const bool asked = (two && r % 2) || (three && r % 3);
+        if (!asked) continue;
+        const uint32_t j = p.row_ptr[r], len = p.row_ptr[r + 1] - j, i = p.row_ptr[r - 1];
+        bool same = j - i == len;
+        for (uint32_t k = 0; same && k < len; ++k) same = p.pairs[i + k].col == p.pairs[j + k].col;
+        if (!same) {
+            if (r % 2) two = false;
+            if (r % 3) three = false;
+        }
+    }
+    return three ? 3 : two ? 2 : 0;
+}
+
 int check_device_options(HostPlan &p, uint64_t M, uint64_t K, const cutespmm_options_t *opts, std::string &err)
 {
     if (M >= (1ull << 32) - kPanelRows || K >= (1ull << 32)) { err = "M and K must be below 2^32"; return CUTESPMM_EUNSUPPORTED; }
@@ -395,6 +413,7 @@ int build_host_plan(HostPlan &p, uint64_t M, uint64_t K, const uint64_t *rowPtr,
     if (p.opts.reorder == CUTESPMM_REORDER_CLUSTER_ROWS) cluster_rows(p);
     if (p.opts.reorder == CUTESPMM_REORDER_SIMILAR_ROWS) group_similar_rows(p);
 
+    p.run_rows = find_row_runs(p);
     const std::vector<uint32_t> panel_ncols = analyze_panels(p);
 
     choose_panel_paths(p, panel_ncols);

@@ -156,6 +156,8 @@ struct HostPlan {
     std::vector<Chunk> chunks;
     std::vector<LongRow> long_rows;
 
+    uint32_t run_rows = 0;               // rows come in aligned runs of 3 or 2 with the same columns (0: they do not)
+
     // ---- panel analysis (HRPB-compatible view) ----
     std::vector<uint32_t> blocked_row_ptr;  // num_panels+1
     std::vector<uint32_t> active_cols;      // per panel ascending distinct columns, zero-padded to x16
@@ -208,6 +210,9 @@ int build_host_plan(HostPlan &p, uint64_t M, uint64_t K, const uint64_t *rowPtr,
 
 // The options of a plan that is built on the device, checked and with the defaults filled in (p.opts, p.adaptive_tiling).
 int check_device_options(HostPlan &p, uint64_t M, uint64_t K, const cutespmm_options_t *opts, std::string &err);
+
+// HostPlan::run_rows of a matrix whose pairs are on the host.
+uint32_t find_row_runs(const HostPlan &p);
 
 // Rebuilds CSR from the packed arrays (rows-kernel part from pairs, brick part from maps + values).
 void decode_host_plan(const HostPlan &p, uint64_t *rowPtr, uint32_t *cols, float *vals);

@@ -204,6 +204,7 @@ int cutespmm_plan_load(cutespmm_plan_t **plan, const char *path, int host_only)
         return fail_status(CUTESPMM_EIO, std::string(path) + ": inconsistent plan");
     }
     p->note_list_sizes();
+    h.run_rows = find_row_runs(h);
     if (!host_only) {
         const int st = cutespmm_internal_upload_plan(p);
         if (st != CUTESPMM_OK) {

@@ -528,6 +528,12 @@ cudaError_t launch_rows(const RowsArgs &args, int sm_count, cudaStream_t s)
     const bool v2 = !((pb | pc | ps) & 7) && !((a.ldb | a.ldc | a.ld_scratch | a.N) & 1);
     a.c_scalar = (pc & 15) || ((a.ldc | a.N) & 3);
     const uint32_t N = a.N;
+    // Rows in runs of the same columns: one load for a run (a row map writes rows elsewhere, chunks are single rows).  Jobs with
+    // fewer runs than a block per SM has lane groups keep the row kernel: they need the rows to fill the machine
+    // (elasticity12 at N = 64: 4.1 us, 4.3 by runs).
+    const uint64_t groups = (uint64_t)sm_count * kWarps * (N <= 16 ? 8 : N <= 32 ? 4 : N <= 64 ? 2 : 1);
+    if (a.run_rows && v4 && a.num_chunks == 0 && !a.row_map && a.num_rows / a.run_rows * ((N + 127) / 128) >= groups)
+        return launch_block_rows(a, sm_count, s);
     // deep: at most one resident wave of tiles, or long rows (measured on shards of R-MAT 2^24: 300 nonzeros per row
     // 2.19 vs 2.38 ms, 21 per row 1.88 vs 1.93 ms in favour of deep; 15 per row (R-MAT 2^20) 0.645 vs 0.611 ms and
     // 3.4 per row 1.50 vs 1.48 ms in favour of shallow)

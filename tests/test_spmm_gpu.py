@@ -435,3 +435,33 @@ def test_tiles_dealt_by_a_counter(oracle_mod, N):
     for _ in range(3):
         assert torch.equal(p.spmm(Bd), first)
     assert p.device_status() == 0
+
+
+@pytest.mark.parametrize("N", [4, 16, 17, 32, 47, 64, 100, 128, 130, 256, 515])
+@pytest.mark.parametrize("run", [2, 3])
+def test_rows_in_runs_of_the_same_columns(oracle_mod, run, N):
+    """Runs of two and three rows with the same columns share their loads: tiles that cut a run (tile sizes no run divides),
+    runs of empty rows, lengths around a step's eight columns; one row that differs sends the matrix back to the row kernel."""
+    rng = np.random.default_rng(10 * N + run)
+    nodes, K = 10000, 300  # more runs than a block per SM has lane groups at every width
+    ln = rng.integers(0, 20, nodes)
+    ln[[0, 7, 8, nodes - 1]] = (1, 0, 0, 9)
+    rows = [np.sort(rng.choice(K, n, replace=False)) for n in ln]
+    rp = np.concatenate([[0], np.cumsum(np.repeat(ln, run))])
+    cols = np.concatenate([c for c in rows for _ in range(run)]).astype(np.int32)
+    vals = torch.from_numpy(rng.standard_normal(rp[-1]).astype(np.float32))
+    B = g.dense_operand(K, N, 81)
+    for cut in (0, 64):
+        for differ in (False, True):
+            c = cols.copy()
+            if differ:  # the last row of a long run names another last column
+                at = int(rp[run * int(np.argmax(ln)) + run]) - 1
+                c[at] = K - 1 if c[at] < K - 1 else 0
+            A = g.CsrMatrix(nodes * run, K, torch.from_numpy(rp), torch.from_numpy(c), vals)
+            want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.numpy(), A.M, K)
+            for p in (cs.Plan.from_device_csr(A.M, K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS, tile_nnz=cut),
+                      cs.Plan.from_csr(A, path=cs.PATH_ROWS, tile_nnz=cut)):
+                out = torch.full((A.M + 1, N), float("nan"), device="cuda")
+                p.spmm(B.cuda(), out[:A.M])
+                assert oracle_mod.rel_fro(want, out[:A.M].cpu().numpy()) <= 2e-6
+                assert torch.isnan(out[A.M]).all() and p.device_status() == 0
