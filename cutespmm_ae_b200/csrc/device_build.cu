@@ -111,19 +111,6 @@ static_assert(kEntries == kMaxTileRows + 1 && kTileSegmentRows % kPanelRows == 0
 static_assert(kListThreads >= (int)kEntries && kListThreads % 32 == 0, "a thread per entry row");
 constexpr uint32_t kSegmentView = kTileSegmentRows + kMaxTileRows;  // rows a segment's last tile may reach
 
-// *out += nonzeros in rows longer than kDefaultSplitNnz (what item_sizes decides by; of jobs large enough to ask).
-__global__ void __launch_bounds__(256) long_share_kernel(const uint32_t *__restrict__ row_ptr, uint32_t M, unsigned long long *__restrict__ out)
-{
-    if ((uint64_t)__ldg(row_ptr + M) + (uint64_t)kRowCost * M <= (uint64_t)kMaxAdaptiveTileCost * kResidentTiles) return;
-    uint32_t mine = 0;
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < M; r += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t p0 = __ldg(row_ptr + r), p1 = __ldg(row_ptr + r + 1);
-        if (p1 > p0 && p1 - p0 > kDefaultSplitNnz) mine += p1 - p0;
-    }
-    mine = __reduce_add_sync(kFullMask, mine);
-    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(out, (unsigned long long)mine);
-}
-
 struct SegmentView {
     uint32_t rp[kSegmentView + 1];           // row pointers of rows [first, first + n]
     uint32_t special[kSegmentView / 32 + 1];  // bit r: row is long, or not in this list
@@ -200,6 +187,8 @@ __device__ __forceinline__ uint32_t pieces_of(const SegmentView &v, const ListAr
 
 __global__ void __launch_bounds__(kListThreads) lists_count_kernel(const uint32_t *__restrict__ row_ptr, ListArgs a)
 {
+    ptx::grid_wait();
+    ptx::grid_release();
     __shared__ SegmentView v;
     __shared__ uint32_t chunks, longs, wrong;
     const uint32_t seg = blockIdx.x, first = seg * kTileSegmentRows, nnz = __ldg(row_ptr + a.M);
@@ -239,6 +228,8 @@ __global__ void __launch_bounds__(kListThreads) lists_count_kernel(const uint32_
 constexpr uint32_t kGroup = 32;
 __global__ void __launch_bounds__(kListThreads) lists_compose_kernel(ListArgs a)
 {
+    ptx::grid_wait();
+    ptx::grid_release();
     __shared__ uint16_t exits[kGroup * kEntries], counts[kGroup * kEntries];
     const uint32_t s0 = blockIdx.x * kGroup, n = min(kGroup, a.num_segments - s0);
     for (uint32_t i = threadIdx.x; i < n * kEntries; i += kListThreads) {
@@ -264,6 +255,8 @@ __global__ void __launch_bounds__(kListThreads) lists_compose_kernel(ListArgs a)
 constexpr uint32_t kChainBatch = 16;  // groups whose tables are in shared memory at a time
 __global__ void __launch_bounds__(1024) lists_scan_kernel(const uint32_t *__restrict__ row_ptr, ListArgs a, uint32_t *__restrict__ counters)
 {
+    ptx::grid_wait();
+    ptx::grid_release();
     __shared__ uint32_t sums[32];
     __shared__ uint16_t exits[kChainBatch * kEntries];
     __shared__ uint32_t counts[kChainBatch * kEntries];
@@ -321,6 +314,8 @@ __global__ void __launch_bounds__(1024) lists_scan_kernel(const uint32_t *__rest
 
 __global__ void __launch_bounds__(kListThreads) lists_write_kernel(const uint32_t *__restrict__ row_ptr, ListArgs a)
 {
+    ptx::grid_wait();
+    ptx::grid_release();
     __shared__ SegmentView v;
     __shared__ uint16_t starts[kTileSegmentRows];
     __shared__ uint32_t num_starts, warp_longs[kListThreads / 32], warp_chunks[kListThreads / 32];
@@ -436,6 +431,8 @@ __device__ __forceinline__ void census_result(const CensusArgs &a, uint32_t q, u
 
 __global__ void __launch_bounds__(kCensusThreads) panel_census_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ cols, CensusArgs a)
 {
+    ptx::grid_wait();
+    ptx::grid_release();
     extern __shared__ uint32_t table[];
     __shared__ uint32_t distinct, big[kCensusWarps];
     const uint32_t nnz = __ldg(row_ptr + a.M), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -486,29 +483,41 @@ __global__ void __launch_bounds__(kCensusThreads) panel_census_kernel(const uint
     }
 }
 
-// ---- rows in runs of the same columns (find_row_runs, plan.cpp) ----------------------------------------------------
-// A thread per row compares it with the row in front.  What is ruled out already is not looked at again: for most matrices that
-// is everything after each block's first rows, so the grid is one block per SM at most and a warp reports once.  Positions are
-// clamped to nnz (nobody has checked the row pointers yet).
-__global__ void __launch_bounds__(1024) row_runs_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ cols, uint32_t M,
-                                                        volatile uint32_t *uneven)
+// ---- what the whole matrix looks like --------------------------------------------------------------------------------
+// A thread per row.  (1) The nonzeros in rows longer than kDefaultSplitNnz, which item_sizes decides by, of jobs large enough
+// to ask.  (2) Whether rows come in runs of the same columns (find_row_runs, plan.cpp): a row is compared with the row in
+// front; what is ruled out already is not looked at again, which for most matrices is everything after each block's first
+// rows, so the grid is one block per SM at most and a warp reports once.  Positions are clamped to nnz (nobody has checked
+// the row pointers yet).  cols may be missing: no runs are looked for then.
+__global__ void __launch_bounds__(1024) row_survey_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ cols, uint32_t M, BuildTotals *totals)
 {
+    ptx::grid_wait();
+    ptx::grid_release();
+    volatile uint32_t *uneven = &totals->uneven;
     const uint32_t nnz = __ldg(row_ptr + M), lane = threadIdx.x & 31;
+    const bool share = (uint64_t)nnz + (uint64_t)kRowCost * M > (uint64_t)kMaxAdaptiveTileCost * kResidentTiles;
+    const uint32_t never = (M % 2 ? 1u : 0u) | (M % 3 ? 2u : 0u);
+    uint32_t in_long = 0;
     for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); b < M; b += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t known = __shfl_sync(kFullMask, *uneven, 0);
-        if (known == 3) return;
+        const uint32_t known = cols ? __shfl_sync(kFullMask, *uneven | never, 0) : 3u;
+        if (known == 3 && !share) return;
         const uint64_t r = b + lane;
         const uint32_t asks = r < M ? ((r % 2 ? 1u : 0u) | (r % 3 ? 2u : 0u)) & ~known : 0u;
+        const uint32_t j = min(__ldg(row_ptr + min(r, (uint64_t)M)), nnz), e = min(__ldg(row_ptr + min(r + 1, (uint64_t)M)), nnz);
+        if (e > j && e - j > kDefaultSplitNnz) in_long += e - j;
         uint32_t found = 0;
         if (asks) {
-            const uint32_t i = min(__ldg(row_ptr + r - 1), nnz), j = min(__ldg(row_ptr + r), nnz), e = min(__ldg(row_ptr + r + 1), nnz);
+            const uint32_t i = min(__ldg(row_ptr + r - 1), nnz);
             bool same = i <= j && j <= e && j - i == e - j;
             for (uint32_t k = 0; same && j + k < e; ++k) same = __ldg(cols + i + k) == __ldg(cols + j + k);
             if (!same) found = asks;
         }
         found = __reduce_or_sync(kFullMask, found);
-        if (found && lane == 0) atomicOr(const_cast<uint32_t *>(uneven), found);
+        if (found && lane == 0) atomicOr(&totals->uneven, found);
     }
+    if (!share) return;
+    in_long = __reduce_add_sync(kFullMask, in_long);
+    if (lane == 0 && in_long) atomicAdd(&totals->long_nnz, (unsigned long long)in_long);
 }
 
 // ---- slots of the brick stream ------------------------------------------------------------------------------------
@@ -518,6 +527,8 @@ __global__ void __launch_bounds__(128) brick_layout_kernel(uint32_t num_panels, 
                                                            uint32_t num_segments, uint32_t *__restrict__ ids, uint32_t *__restrict__ first,
                                                            uint32_t *__restrict__ last)
 {
+    ptx::grid_wait();
+    ptx::grid_release();
     constexpr uint32_t kPanels = kTileSegmentRows / kPanelRows;
     const uint32_t lane = threadIdx.x & 31, seg = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (seg >= num_segments) return;
@@ -556,6 +567,8 @@ __global__ void __launch_bounds__(kCensusThreads) brick_fill_kernel(const uint32
                                                                     uint32_t num_brick_panels, const uint32_t *__restrict__ ncols, uint32_t table_words,
                                                                     uint32_t list_words, uint32_t *__restrict__ bcols, uint32_t *__restrict__ brecs)
 {
+    ptx::grid_wait();
+    ptx::grid_release();
     extern __shared__ uint32_t table[];
     uint32_t *list = table + table_words;   // the panel's distinct columns, ascending
     uint32_t *map = list + list_words;      // occupancy: 4 words per brick
@@ -632,6 +645,8 @@ __global__ void __launch_bounds__(256) pack_kernel(const uint32_t *__restrict__ 
                                                    uint32_t M, uint32_t K, uint32_t nnz, uint32_t *__restrict__ row_ptr_out, uint2 *__restrict__ pairs,
                                                    uint32_t *__restrict__ bad)
 {
+    ptx::grid_wait();
+    ptx::grid_release();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool out_of_range = false;
     for (uint64_t j = t0; j < (uint64_t)nnz + 2; j += stride) {
@@ -690,31 +705,28 @@ cudaError_t launch_pack(const uint32_t *row_ptr, const uint32_t *cols, const flo
 {
     const uint64_t items = std::max<uint64_t>((uint64_t)nnz + 2, (uint64_t)M + 1 + kRowPtrSlack);
     const uint32_t blocks = (uint32_t)std::min<uint64_t>((items + 255) / 256, (uint64_t)sm_count * 8);
-    pack_kernel<<<blocks, 256, 0, s>>>(row_ptr, cols, vals, M, K, nnz, row_ptr_out, static_cast<uint2 *>(pairs), bad);
-    return cudaGetLastError();
+    return launch_overlapped(pack_kernel, blocks, 256, 0, s, row_ptr, cols, vals, M, K, nnz, row_ptr_out, static_cast<uint2 *>(pairs), bad);
 }
 
 cudaError_t launch_lists_count(const uint32_t *row_ptr, const ListArgs &a, cudaStream_t s)
 {
     if (a.num_segments == 0) return cudaSuccess;
-    if (!a.total_known)  // the first list of a plan
-        long_share_kernel<<<std::min((a.M + 2047) / 2048, 1184u), 256, 0, s>>>(row_ptr, a.M, const_cast<unsigned long long *>(a.long_nnz));
-    lists_count_kernel<<<a.num_segments, kListThreads, 0, s>>>(row_ptr, a);
-    return cudaGetLastError();
+    return launch_overlapped(lists_count_kernel, a.num_segments, kListThreads, 0, s, row_ptr, a);
 }
 
 cudaError_t launch_lists_scan(const uint32_t *row_ptr, const ListArgs &a, uint32_t *counters, uint32_t how_many, cudaStream_t s)
 {
-    if (a.num_segments) lists_compose_kernel<<<(a.num_segments + kGroup - 1) / kGroup, kListThreads, 0, s>>>(a);
-    lists_scan_kernel<<<1 + how_many, 1024, 0, s>>>(row_ptr, a, counters);
-    return cudaGetLastError();
+    if (a.num_segments) {
+        const cudaError_t e = launch_overlapped(lists_compose_kernel, (a.num_segments + kGroup - 1) / kGroup, kListThreads, 0, s, a);
+        if (e != cudaSuccess) return e;
+    }
+    return launch_overlapped(lists_scan_kernel, 1 + how_many, 1024, 0, s, row_ptr, a, counters);
 }
 
 cudaError_t launch_lists_write(const uint32_t *row_ptr, const ListArgs &a, cudaStream_t s)
 {
     if (a.num_segments == 0) return cudaSuccess;
-    lists_write_kernel<<<a.num_segments, kListThreads, 0, s>>>(row_ptr, a);
-    return cudaGetLastError();
+    return launch_overlapped(lists_write_kernel, a.num_segments, kListThreads, 0, s, row_ptr, a);
 }
 
 cudaError_t launch_panel_census(const uint32_t *row_ptr, const uint32_t *cols, CensusArgs a, int sm_count, cudaStream_t s)
@@ -727,22 +739,19 @@ cudaError_t launch_panel_census(const uint32_t *row_ptr, const uint32_t *cols, C
     cudaError_t e = allow_dynamic_smem<panel_census_kernel>(16384 * 4);
     if (e != cudaSuccess) return e;
     const uint32_t blocks = std::min((a.num_panels + kCensusWarps - 1) / kCensusWarps, (uint32_t)sm_count * 16);
-    panel_census_kernel<<<blocks, kCensusThreads, smem, s>>>(row_ptr, cols, a);
-    return cudaGetLastError();
+    return launch_overlapped(panel_census_kernel, blocks, kCensusThreads, smem, s, row_ptr, cols, a);
 }
 
-cudaError_t launch_row_runs(const uint32_t *row_ptr, const uint32_t *cols, uint32_t M, uint32_t *uneven, int sm_count, cudaStream_t s)
+cudaError_t launch_row_survey(const uint32_t *row_ptr, const uint32_t *cols, uint32_t M, BuildTotals *totals, int sm_count, cudaStream_t s)
 {
-    if (M < 2) return cudaSuccess;
-    row_runs_kernel<<<std::min((M + 1023) / 1024, (uint32_t)sm_count), 1024, 0, s>>>(row_ptr, cols, M, uneven);
-    return cudaGetLastError();
+    if (M == 0) return cudaSuccess;
+    return launch_overlapped(row_survey_kernel, std::min((M + 1023) / 1024, (uint32_t)sm_count), 1024, 0, s, row_ptr, cols, M, totals);
 }
 
 cudaError_t launch_brick_layout(uint32_t num_panels, const uint8_t *path, const uint32_t *ncols, const uint32_t *seg_panels, const uint32_t *seg_slots,
                                 uint32_t num_segments, uint32_t *ids, uint32_t *first, uint32_t *last, cudaStream_t s)
 {
-    brick_layout_kernel<<<(num_segments + 3) / 4, 128, 0, s>>>(num_panels, path, ncols, seg_panels, seg_slots, num_segments, ids, first, last);
-    return cudaGetLastError();
+    return launch_overlapped(brick_layout_kernel, (num_segments + 3) / 4, 128, 0, s, num_panels, path, ncols, seg_panels, seg_slots, num_segments, ids, first, last);
 }
 
 cudaError_t launch_panel_columns(const uint32_t *row_ptr, const void *pairs, uint32_t M, uint32_t num_panels, uint32_t *ncols,
@@ -776,9 +785,8 @@ cudaError_t launch_brick_fill(const uint32_t *row_ptr, const void *pairs, uint32
     const uint32_t map = (cols_max + kBrickCols - 1) / kBrickCols * 4;
     cudaError_t e = allow_dynamic_smem<brick_fill_kernel>((16384 + kDevPanelMax + kDevPanelMax / kBrickCols * 4) * 4);
     if (e != cudaSuccess) return e;
-    brick_fill_kernel<<<std::min(num_brick_panels, (uint32_t)sm_count * 16), kCensusThreads, (table + list + map) * 4, s>>>(
-        row_ptr, static_cast<const uint2 *>(pairs), M, ids, first_slot, num_brick_panels, ncols, table, list, bcols, brecs);
-    return cudaGetLastError();
+    return launch_overlapped(brick_fill_kernel, std::min(num_brick_panels, (uint32_t)sm_count * 16), kCensusThreads, (table + list + map) * 4, s,
+                             row_ptr, static_cast<const uint2 *>(pairs), M, ids, first_slot, num_brick_panels, ncols, table, list, bcols, brecs);
 }
 
 }  // namespace cutespmm

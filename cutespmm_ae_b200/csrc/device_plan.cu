@@ -73,6 +73,23 @@ struct Carver {
     }
 };
 
+// A pinned slot device words arrive in (a copy to pageable memory costs a staging pass more).
+struct Landing {
+    uint32_t *slot = nullptr;
+    cudaStream_t s;
+    explicit Landing(cudaStream_t stream) : s(stream) {}
+    ~Landing() { if (slot) cutespmm_internal_give_status_word(slot); }
+    template <class T> cudaError_t fetch(T &out, const T *device)  // waits for the stream
+    {
+        static_assert(sizeof(T) <= kStatusSlotBytes, "one slot");
+        cudaError_t e = slot ? cudaSuccess : cutespmm_internal_take_status_word(&slot);
+        if (e != cudaSuccess || (e = cudaMemcpyAsync(slot, device, sizeof(T), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+        e = cudaStreamSynchronize(s);
+        std::memcpy(&out, slot, sizeof(T));
+        return e;
+    }
+};
+
 struct Temp {  // stream-ordered scratch of one call
     void *p = nullptr;
     cudaStream_t s;
@@ -339,12 +356,13 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
     ca.ncols = ncols; ca.path = path;
     ca.seg_panels = counters + 2ull * segments; ca.seg_slots = counters + 3ull * segments;
     ca.totals = d_totals;
+    Landing landing(s);
     BuildTotals t{};
-    if ((e = cudaMemsetAsync(temp.p, 0, zeroed, s)) != cudaSuccess || (e = launch_lists_count(rowPtr_dev, la, s)) != cudaSuccess ||
-        (cols_dev && (M % 2 == 0 || M % 3 == 0) && (e = launch_row_runs(rowPtr_dev, cols_dev, M, &d_totals->uneven, sms, s)) != cudaSuccess) ||
+    if ((e = cudaMemsetAsync(temp.p, 0, zeroed, s)) != cudaSuccess || (e = launch_row_survey(rowPtr_dev, cols_dev, M, d_totals, sms, s)) != cudaSuccess ||
+        (e = launch_lists_count(rowPtr_dev, la, s)) != cudaSuccess ||
         (census && cols_dev && (e = launch_panel_census(rowPtr_dev, cols_dev, ca, sms, s)) != cudaSuccess) ||
         (e = launch_lists_scan(rowPtr_dev, la, counters, census ? 4 : 2, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(&t, d_totals, sizeof(t), cudaMemcpyDeviceToHost, s)) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)
+        (e = landing.fetch(t, d_totals)) != cudaSuccess)
         return fail_cuda_status(e, "reading the row pointers");
     h.nnz = t.nnz;
     h.run_rows = M < 2 || !t.nnz ? 0 : M % 3 == 0 && !(t.uneven & 2) ? 3 : M % 2 == 0 && !(t.uneven & 1) ? 2 : 0;
@@ -370,7 +388,7 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
         BuildTotals t2{};
         if ((e = launch_lists_count(rowPtr_dev, la2, s)) != cudaSuccess ||
             (e = launch_lists_scan(rowPtr_dev, la2, counters2, 2, s)) != cudaSuccess ||
-            (e = cudaMemcpyAsync(&t2, d_totals2, sizeof(t2), cudaMemcpyDeviceToHost, s)) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)
+            (e = landing.fetch(t2, d_totals2)) != cudaSuccess)
             return fail_cuda_status(e, "counting the work lists");
         p->own = {t2.tiles, t2.chunks, t2.long_rows};
     }
@@ -445,8 +463,7 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
                                    sms, s)) != cudaSuccess)
             return fail_cuda_status(e, "packing the bricks");
     }
-    if ((e = cudaMemcpyAsync(&bad_cols, &d_totals->bad_cols, sizeof(bad_cols), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(s)) != cudaSuccess)
+    if ((e = landing.fetch(bad_cols, &d_totals->bad_cols)) != cudaSuccess)
         return fail_cuda_status(e, "packing the nonzeros");
     if (bad_cols) return fail_status(CUTESPMM_EINVAL, "column index out of range (>= K)");
     p->used_elsewhere = false;

@@ -156,7 +156,7 @@ struct ListArgs {
     uint32_t split_nnz, tile_nnz, adaptive;
     uint32_t total_known;   // 1: `total` is the cost of the listed rows; 0: every row is listed, nnz + kRowCost * M
     uint64_t total;
-    const unsigned long long *long_nnz;  // nonzeros in long rows, summed by the first count
+    const unsigned long long *long_nnz;  // nonzeros in long rows, summed by the survey
     const uint8_t *path;   // per panel: 1 = not listed (nullptr: every row is)
     uint16_t *exits, *tile_counts;  // per segment and entry row: entry row of the next segment, tiles
     uint16_t *path_entry;   // per segment and entry row of its group: entry row of the segment ...
@@ -185,7 +185,7 @@ struct CensusArgs {
 cudaError_t launch_lists_count(const uint32_t *row_ptr, const ListArgs &a, cudaStream_t s);
 cudaError_t launch_lists_scan(const uint32_t *row_ptr, const ListArgs &a, uint32_t *counters, uint32_t how_many, cudaStream_t s);
 cudaError_t launch_lists_write(const uint32_t *row_ptr, const ListArgs &a, cudaStream_t s);
-cudaError_t launch_row_runs(const uint32_t *row_ptr, const uint32_t *cols, uint32_t M, uint32_t *uneven, int sm_count, cudaStream_t s);
+cudaError_t launch_row_survey(const uint32_t *row_ptr, const uint32_t *cols, uint32_t M, BuildTotals *totals, int sm_count, cudaStream_t s);
 cudaError_t launch_panel_census(const uint32_t *row_ptr, const uint32_t *cols, CensusArgs a, int sm_count, cudaStream_t s);
 cudaError_t launch_brick_layout(uint32_t num_panels, const uint8_t *path, const uint32_t *ncols, const uint32_t *seg_panels, const uint32_t *seg_slots,
                                 uint32_t num_segments, uint32_t *ids, uint32_t *first, uint32_t *last, cudaStream_t s);

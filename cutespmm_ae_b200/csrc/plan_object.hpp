@@ -37,7 +37,11 @@ struct cutespmm_list_sizes {
 // Gives the memory of a device-built plan back.  device_plan.cu
 void cutespmm_internal_free_block(void *block, uint64_t bytes, int dev, bool used_elsewhere);
 
-void cutespmm_internal_give_status_word(uint32_t *word);  // sharded.cu
+// Pinned slots that status words and sizes arrive in: handed out of pages of 256, because pinning takes milliseconds.
+// Given-back slots are handed out again; the pages stay (32 KB for 256 plans that make host-buffer calls).  sharded.cu
+constexpr uint32_t kStatusSlotBytes = 128;
+cudaError_t cutespmm_internal_take_status_word(uint32_t **slot);
+void cutespmm_internal_give_status_word(uint32_t *slot);
 
 struct cutespmm_plan {
     cutespmm::HostPlan host;

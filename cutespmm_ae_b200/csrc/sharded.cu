@@ -28,6 +28,33 @@
 using namespace cutespmm;
 
 namespace {
+std::mutex g_status_mutex;
+std::vector<uint32_t *> g_status_slots;
+}  // namespace
+
+cudaError_t cutespmm_internal_take_status_word(uint32_t **slot)
+{
+    constexpr uint32_t kWords = kStatusSlotBytes / 4, kSlots = 256;
+    std::lock_guard<std::mutex> lock(g_status_mutex);
+    if (g_status_slots.empty()) {
+        uint32_t *page = nullptr;
+        const cudaError_t e = cudaHostAlloc(&page, kSlots * kStatusSlotBytes, cudaHostAllocPortable);
+        if (e != cudaSuccess) return e;
+        for (uint32_t i = kSlots; i-- > 0;) g_status_slots.push_back(page + i * kWords);
+    }
+    *slot = g_status_slots.back();
+    g_status_slots.pop_back();
+    **slot = 0;
+    return cudaSuccess;
+}
+
+void cutespmm_internal_give_status_word(uint32_t *slot)
+{
+    std::lock_guard<std::mutex> lock(g_status_mutex);
+    g_status_slots.push_back(slot);
+}
+
+namespace {
 
 // ---- the slice of NCCL's ABI this file uses -------------------------------------------------------
 using nccl_comm_t = void *;
@@ -179,25 +206,6 @@ int new_comm(cutespmm_comm_t **out, nccl_comm_t c, int nranks, int rank, int dev
 
 namespace {
 
-// Pinned words the calls' status arrives in, one per plan that makes host-buffer calls: handed out of pages of 1024, because
-// pinning a page takes milliseconds.  Given-back words are handed out again; the pages stay (4 KB per 1024 such plans).
-std::mutex g_status_mutex;
-std::vector<uint32_t *> g_status_words;
-cudaError_t take_status_word(uint32_t **word)
-{
-    std::lock_guard<std::mutex> lock(g_status_mutex);
-    if (g_status_words.empty()) {
-        uint32_t *page = nullptr;
-        const cudaError_t e = cudaHostAlloc(&page, 1024 * sizeof(uint32_t), cudaHostAllocPortable);
-        if (e != cudaSuccess) return e;
-        for (int i = 1023; i >= 0; --i) g_status_words.push_back(page + i);
-    }
-    *word = g_status_words.back();
-    g_status_words.pop_back();
-    **word = 0;
-    return cudaSuccess;
-}
-
 // How a host-buffer call cuts N columns into windows, and the staging it needs on the device.
 struct Windows {
     uint32_t count = 1, width = 0;
@@ -238,7 +246,7 @@ int ensure_staging(cutespmm_plan *p, uint32_t N, bool sharded, Windows &w)
         p->staged_C = needC;
     }
     if (!p->h_status) {
-        if ((e = take_status_word(&p->h_status)) != cudaSuccess) return fail_cuda_status(e, "status word");
+        if ((e = cutespmm_internal_take_status_word(&p->h_status)) != cudaSuccess) return fail_cuda_status(e, "status word");
     }
     if (!p->s_in) {
         if ((e = cudaStreamCreateWithFlags(&p->s_in, cudaStreamNonBlocking)) != cudaSuccess ||
@@ -409,12 +417,6 @@ int run_row_blocks(cutespmm_plan *p, const float *B_host, uint64_t ldb, float *C
 }
 
 }  // namespace
-
-void cutespmm_internal_give_status_word(uint32_t *word)
-{
-    std::lock_guard<std::mutex> lock(g_status_mutex);
-    g_status_words.push_back(word);
-}
 
 extern "C" {
 
