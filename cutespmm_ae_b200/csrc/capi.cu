@@ -471,14 +471,16 @@ static void note_stream(const cutespmm_plan *p, cudaStream_t s)
 // names a row of B often enough it pays to copy B once into rows of N rounded up to four (the copy lives on the stream):
 // measured, the row kernel gains about 12 ps per nonzero up to 64 columns and 0.4 ps per nonzero and column beyond (R-MAT
 // 2^18 N = 47: 186 -> 139 us, uniform 7 per row N = 201: 211 -> 125 us), the copy costs a launch and 8 bytes per element at
-// 6.4 TB/s.  Even widths above 32 are read two columns per lane and gain nothing.  Not while the stream is being captured
+// 6.4 TB/s.  Copies above kMaxPadBytes are not made: the pool would give them back at every synchronisation and map them anew
+// (1.8 GB: 4.6 -> 5.6 ms per product); wide products of large matrices go in narrower windows instead.  Even widths above 32 are read two columns per lane and gain nothing.  Not while the stream is being captured
 // (a graph should not own memory).
+constexpr uint64_t kMaxPadBytes = 512ull << 20;
 static bool worth_padding(const HostPlan &h, const float *B, uint64_t ldb, const float *C, uint64_t ldc, uint32_t N, cudaStream_t s)
 {
     const bool two = !((reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 7) && !((ldb | ldc | N) & 1);
     if (two && N > 32) return false;
     const uint64_t gain = h.nnz * (N <= 64 ? 12 : N * 2 / 5), cost = 3000000 + h.K * N * 5 / 4;  // picoseconds
-    if (gain < cost) return false;
+    if (gain < cost || h.K * ((uint64_t)N + 3) * sizeof(float) > kMaxPadBytes) return false;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
         cudaGetLastError();
@@ -505,8 +507,14 @@ int cutespmm_internal_spmm_range(const cutespmm_plan *p, const float *B, uint64_
         return fail(CUTESPMM_EINVAL, "the current CUDA device (" + std::to_string(cur) + ") is not the one the plan was created on (" +
                                          std::to_string(p->device) + "): call cudaSetDevice first");
     note_stream(p, s);
-    for (uint32_t n0 = 0; n0 < N; n0 += kScratchCols) {
-        const uint32_t nw = N - n0 < kScratchCols ? N - n0 : kScratchCols;
+    uint32_t nw = 0;
+    for (uint32_t n0 = 0; n0 < N; n0 += nw) {
+        nw = N - n0 < kScratchCols ? N - n0 : kScratchCols;
+        // rows of B off the 16-byte grid: a window is narrowed until a padded copy of it may be made
+        if (((reinterpret_cast<uintptr_t>(B) & 15) || (ldb & 3)) && p->host.K * ((uint64_t)nw + 3) * sizeof(float) > kMaxPadBytes) {
+            const uint64_t fit = kMaxPadBytes / (p->host.K * sizeof(float)) / 128 * 128;
+            if (fit && fit < nw && worth_padding(p->host, B, ldb, C, ldc, (uint32_t)fit, s)) nw = (uint32_t)fit;
+        }
         cudaError_t e;
         const bool slab = p->host.slab_panels && slab_supports(nw, ldb, ldc, B + n0, C + n0);
         if (slab && rg) return fail(CUTESPMM_EUNSUPPORTED, "a plan with slab panels runs whole");

@@ -26,7 +26,7 @@ namespace {
 // library's own, one per device, thread-safe in the driver.  The pool keeps at most kPoolKeeps bytes beyond what
 // living plans hold across a synchronisation (the rest goes back to the driver), and gives them up when an allocation
 // fails or cutespmm_release_memory is called.
-constexpr uint64_t kPoolKeeps = 512ull << 20, kPoolStep = 128ull << 20;
+constexpr uint64_t kPoolKeeps = 1ull << 30, kPoolStep = 128ull << 20;
 constexpr int kMaxDevices = 64;
 
 std::mutex g_device_mutex;

@@ -144,7 +144,7 @@ int cutespmm_plan_build_host(cutespmm_plan_t **plan, uint64_t M, uint64_t K, con
  * sorted.  The panel views (blocked_row_ptr, active_cols) are computed when asked for (not for path rows, nor when a panel
  * holds more than 8192 nonzeros); plan_decode_csr reads the packed nonzeros back.  Work is queued on `stream`, which is
  * synchronised before the call returns.  The plan's memory comes from a stream-ordered pool of the library's own, which
- * keeps up to 512 MiB per device for the next such plan (cutespmm_release_memory gives that back). */
+ * keeps up to 1 GiB per device for the next such plan (cutespmm_release_memory gives that back). */
 int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M, uint64_t K, const uint32_t *rowPtr_dev,
                                 const uint32_t *cols_dev, const float *vals_dev, const cutespmm_options_t *opts,
                                 void *stream);

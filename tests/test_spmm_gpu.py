@@ -465,3 +465,16 @@ def test_rows_in_runs_of_the_same_columns(oracle_mod, run, N):
                 p.spmm(B.cuda(), out[:A.M])
                 assert oracle_mod.rel_fro(want, out[:A.M].cpu().numpy()) <= 2e-6
                 assert torch.isnan(out[A.M]).all() and p.device_status() == 0
+
+
+def test_wide_unaligned_products_of_large_matrices_go_in_windows(oracle_mod):
+    """A padded copy of B above 512 MiB is made window by window; rows in runs take the run kernel in every window."""
+    A = g.elasticity3d(48, 3, 9)  # 331776 rows: 409 columns are 543 MB
+    N = 409
+    p = cs.Plan.from_device_csr(A.M, A.K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS)
+    B = torch.randn((A.K, N), generator=torch.Generator("cuda").manual_seed(3), device="cuda")
+    C = p.spmm(B)
+    for cols in (slice(0, 8), slice(380, 388), slice(401, 409)):  # both sides of the window edges
+        want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B[:, cols].contiguous().cpu().numpy(), A.M, A.K)
+        assert oracle_mod.rel_fro(want, C[:, cols].cpu().numpy()) <= 2e-6
+    assert p.device_status() == 0
