@@ -187,8 +187,8 @@ __device__ __forceinline__ uint32_t pieces_of(const SegmentView &v, const ListAr
 
 __global__ void __launch_bounds__(kListThreads) lists_count_kernel(const uint32_t *__restrict__ row_ptr, ListArgs a)
 {
+    ptx::grid_release();  // the census, next on the stream, needs nothing of this kernel: it runs beside it
     ptx::grid_wait();
-    ptx::grid_release();
     __shared__ SegmentView v;
     __shared__ uint32_t chunks, longs, wrong;
     const uint32_t seg = blockIdx.x, first = seg * kTileSegmentRows, nnz = __ldg(row_ptr + a.M);
@@ -314,8 +314,7 @@ __global__ void __launch_bounds__(1024) lists_scan_kernel(const uint32_t *__rest
 
 __global__ void __launch_bounds__(kListThreads) lists_write_kernel(const uint32_t *__restrict__ row_ptr, ListArgs a)
 {
-    ptx::grid_wait();
-    ptx::grid_release();
+    ptx::grid_release();  // reads the counts the host has waited for and writes lists nobody else touches: runs beside pack_kernel
     __shared__ SegmentView v;
     __shared__ uint16_t starts[kTileSegmentRows];
     __shared__ uint32_t num_starts, warp_longs[kListThreads / 32], warp_chunks[kListThreads / 32];
@@ -366,6 +365,7 @@ __global__ void __launch_bounds__(kListThreads) lists_write_kernel(const uint32_
         const uint32_t r = starts[k], e = v.next[r];
         a.tiles[t0 + k] = Tile{first + r, first + e, v.rp[r], v.rp[e]};
     }
+    ptx::grid_wait();
 }
 
 // ---- panel census: which panels the tensor-core kernel takes ------------------------------------------------------
@@ -431,7 +431,6 @@ __device__ __forceinline__ void census_result(const CensusArgs &a, uint32_t q, u
 
 __global__ void __launch_bounds__(kCensusThreads) panel_census_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ cols, CensusArgs a)
 {
-    ptx::grid_wait();
     ptx::grid_release();
     extern __shared__ uint32_t table[];
     __shared__ uint32_t distinct, big[kCensusWarps];
@@ -481,6 +480,7 @@ __global__ void __launch_bounds__(kCensusThreads) panel_census_kernel(const uint
         }
         __syncthreads();
     }
+    ptx::grid_wait();  // what follows waits for this kernel, and through it for the lists
 }
 
 // ---- what the whole matrix looks like --------------------------------------------------------------------------------
@@ -645,8 +645,8 @@ __global__ void __launch_bounds__(256) pack_kernel(const uint32_t *__restrict__ 
                                                    uint32_t M, uint32_t K, uint32_t nnz, uint32_t *__restrict__ row_ptr_out, uint2 *__restrict__ pairs,
                                                    uint32_t *__restrict__ bad)
 {
-    ptx::grid_wait();
     ptx::grid_release();
+    ptx::grid_wait();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool out_of_range = false;
     for (uint64_t j = t0; j < (uint64_t)nnz + 2; j += stride) {
