@@ -249,17 +249,42 @@ bool brick_supports(uint32_t N, uint64_t ldb, uint64_t ldc, const void *B, const
     return N % 32 == 0 && N > 0 && !((pb | pc) & 15) && !((ldb | ldc) & 3);
 }
 
-cudaError_t launch_brick(const BrickArgs &a, int sm_count, cudaStream_t s)
+// Columns of the next launch of a product with N (a multiple of 32) columns left: spans of 128, 96 and 64 columns, so that no
+// product is walked in spans of 32 (N = 96 was three walks of 32 columns: stencil512 92 -> 60 us, elasticity40 110 -> 62; N = 160
+// was five: 148 -> 108).  192 columns are two spans of 96, not three of 64 (stencil512 126 -> 115).
+static uint32_t brick_span(uint32_t N)
 {
-    if (a.num_bricks == 0 || a.num_panels == 0) return cudaSuccess;
-    if (a.round_b) {
-        if (a.N % 128 == 0) return launch_brick_t<16, true>(a, sm_count, s);
-        if (a.N % 64 == 0) return launch_brick_t<8, true>(a, sm_count, s);
-        return launch_brick_t<4, true>(a, sm_count, s);
+    switch (N % 128) {
+        case 0: return N;
+        case 96: return 96;
+        case 64: return N >= 192 ? 192 : 64;
+        default: return N >= 160 ? 96 : 32;
     }
-    if (a.N % 128 == 0) return launch_brick_t<16, false>(a, sm_count, s);
-    if (a.N % 64 == 0) return launch_brick_t<8, false>(a, sm_count, s);
-    return launch_brick_t<4, false>(a, sm_count, s);
+}
+
+int brick_launches(uint32_t N)
+{
+    int n = 0;
+    for (; N; N -= brick_span(N)) ++n;
+    return n;
+}
+
+cudaError_t launch_brick(const BrickArgs &args, int sm_count, cudaStream_t s)
+{
+    if (args.num_bricks == 0 || args.num_panels == 0) return cudaSuccess;
+    BrickArgs a = args;
+    for (uint32_t left = args.N; left; left -= a.N, a.B += a.N, a.C += a.N) {
+        a.N = brick_span(left);
+        cudaError_t e;
+#define CUTESPMM_BRICK(NT) e = a.round_b ? launch_brick_t<NT, true>(a, sm_count, s) : launch_brick_t<NT, false>(a, sm_count, s)
+        if (a.N % 128 == 0) CUTESPMM_BRICK(16);
+        else if (a.N % 96 == 0) CUTESPMM_BRICK(12);
+        else if (a.N % 64 == 0) CUTESPMM_BRICK(8);
+        else CUTESPMM_BRICK(4);
+#undef CUTESPMM_BRICK
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace cutespmm

@@ -409,14 +409,18 @@ static SlabArgs slab_args(const cutespmm_plan *p, const float *B, uint64_t ldb, 
 // Path auto leaves products narrower than 64 columns to the row kernel even where the plan has brick panels: with a
 // group of N/4 lanes per row it is the faster of the two there (stencil512 at N = 32: 0.035 against 0.041 ms,
 // elasticity40: 0.045 against 0.047 ms; at N = 64 the brick kernel wins, 0.048 / 0.053 against 0.057 / 0.070 ms).
+// Rows in runs of the same columns take one load per run there, and win at 64 columns too (elasticity40: 0.0405 against
+// 0.0458 ms); wider, B no longer stays near the SM and the bricks win (N = 128: 0.068 against 0.063 ms).
 // A plan created with path brick runs its bricks at every width the brick kernel takes.
-static bool brick_wanted(const HostPlan &h, uint32_t N)
+static bool brick_wanted(const cutespmm_plan *p, uint32_t N)
 {
-    return h.num_bricks && (N >= 64 || h.opts.path == CUTESPMM_PATH_BRICK);
+    const HostPlan &h = p->host;
+    const bool runs = h.run_rows && h.row_map.empty() && p->every.chunks == 0;
+    return h.num_bricks && (N > 64 || (N == 64 && !runs) || h.opts.path == CUTESPMM_PATH_BRICK);
 }
 static bool use_brick(const cutespmm_plan *p, const float *B, uint64_t ldb, const float *C, uint64_t ldc, uint32_t N)
 {
-    return brick_wanted(p->host, N) && brick_supports(N, ldb, ldc, B, C);
+    return brick_wanted(p, N) && brick_supports(N, ldb, ldc, B, C);
 }
 
 // Kernels of one column window of width nw (bit 0 row kernel, bit 1 brick kernel, bit 2 slab kernel).  The alignment of
@@ -424,7 +428,7 @@ static bool use_brick(const cutespmm_plan *p, const float *B, uint64_t ldb, cons
 static int window_kernels(const cutespmm_plan *p, uint32_t nw)
 {
     const HostPlan &h = p->host;
-    const bool brick = brick_wanted(h, nw) && nw % 32 == 0;
+    const bool brick = brick_wanted(p, nw) && nw % 32 == 0;
     const bool slab = h.slab_panels && nw % 128 == 0;
     const bool all_rows = (!brick && h.num_bricks) || (!slab && h.slab_panels);
     int mask = (brick ? 2 : 0) | (slab ? 4 : 0);
@@ -447,7 +451,7 @@ int cutespmm_spmm_launch_count(const cutespmm_plan_t *p, uint32_t N)
     int total = 0;
     for (uint32_t n0 = 0; n0 < N; n0 += kScratchCols) {
         const int mask = window_kernels(p, N - n0 < kScratchCols ? N - n0 : kScratchCols);
-        total += (mask & 1) + ((mask >> 1) & 1) + ((mask >> 2) & 1);
+        total += (mask & 1) + (mask & 2 ? brick_launches(N - n0 < kScratchCols ? N - n0 : kScratchCols) : 0) + ((mask >> 2) & 1);
     }
     return total;
 }

@@ -110,6 +110,7 @@ struct BrickArgs {
 };
 
 cudaError_t launch_brick(const BrickArgs &a, int sm_count, cudaStream_t s);
+int brick_launches(uint32_t N);  // kernels launch_brick queues for N columns
 bool brick_supports(uint32_t N, uint64_t ldb, uint64_t ldc, const void *B, const void *C);
 
 // Arguments of the tcgen05 slab kernel (128-row panels).

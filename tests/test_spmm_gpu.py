@@ -478,3 +478,19 @@ def test_wide_unaligned_products_of_large_matrices_go_in_windows(oracle_mod):
         want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B[:, cols].contiguous().cpu().numpy(), A.M, A.K)
         assert oracle_mod.rel_fro(want, C[:, cols].cpu().numpy()) <= 2e-6
     assert p.device_status() == 0
+
+
+@pytest.mark.parametrize("N", [32, 64, 96, 128, 160, 192, 224, 256, 288, 320, 352, 480, 512, 608])
+@pytest.mark.parametrize("make", [lambda: g.stencil9(100), lambda: g.elasticity3d(14, 3, 5)])
+def test_brick_spans(oracle_mod, make, N):
+    """Every composition of 128-, 96- and 64-column spans, on path brick and on path auto (whose widths up to 64 run by rows)."""
+    A = make()
+    B = g.dense_operand(A.K, N, 91)
+    want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.numpy(), A.M, A.K)
+    for kw in (dict(path=cs.PATH_BRICK), dict(round_b_nearest=True)):
+        p = cs.Plan.from_csr(A, **kw)
+        out = torch.full((A.M + 1, N), float("nan"), device="cuda")
+        p.spmm(B.cuda(), out[:A.M])
+        assert oracle_mod.rel_fro(want, out[:A.M].cpu().numpy()) <= 1e-3
+        assert torch.isnan(out[A.M]).all() and p.device_status() == 0
+    assert cs.Plan.from_csr(A, path=cs.PATH_BRICK).launch_count(N) == {160: 2, 224: 2, 288: 2, 320: 2, 352: 2, 480: 2, 608: 2}.get(N, 1)
