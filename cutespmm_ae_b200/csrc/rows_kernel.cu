@@ -28,13 +28,16 @@ namespace cutespmm {
 namespace {
 
 // Two tunings of the row kernel, chosen per launch (measured on R-MAT graphs and the 512x512 stencil at N = 128):
-//   DEEP = false  4 rows of B in flight per warp, 6 blocks (48 warps) per SM: more warps hide the gather latency
+//   DEEP = false  4 rows of B in flight per warp, 5 blocks (40 warps) per SM: more warps hide the gather latency
 //                 better than more loads per warp when rows are short and the grid is several waves of tiles long;
 //   DEEP = true   8 rows in flight, 4 blocks per SM: fewer dependent steps per row, better for long rows and when
 //                 the whole job is a single wave of tiles and the time is a handful of latencies.
 template <bool DEEP> struct Tuning {
     static constexpr int kUnroll = DEEP ? 8 : 4;
-    static constexpr int kMinBlocks = DEEP ? 4 : 6;
+    // 48 registers, 40 warps per SM (the lane-group kernels spill 200 bytes at 40 registers and 48 warps: R-MAT 2^17 N = 64
+    // 55.8 -> 50.8 us, 800 000 rows of 4 at N = 32 74 -> 65, R-MAT 2^20 N = 128 662 -> 647); the narrow kernels that deal
+    // tiles by a counter have long rows to hide and keep 48 warps (R-MAT 2^20 N = 32: 266 us, 281 with 40)
+    static constexpr int min_blocks(bool dyn, int G) { return DEEP ? 4 : dyn && G >= 4 ? 6 : 5; }
 };
 constexpr int kWarps = kTileWarps;
 constexpr unsigned kFull = 0xffffffffu;
@@ -363,7 +366,7 @@ __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
 // G = 2, 4, 8 (narrow products, N <= 64, float4 lanes): the warp is G groups of 32/G lanes, a group spans the whole
 // row of B and owns a row of A of its own, so a warp keeps G times as many gathers in flight and no lane idles.
 template <int VEC, int CH, bool FULL, bool DEEP, int G, bool DYN>
-__global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::kMinBlocks) spmm_rows_kernel(RowsArgs a)
+__global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DYN, G)) spmm_rows_kernel(RowsArgs a)
 {
     using V = typename Vec<VEC>::T;
     static_assert(G == 1 || (VEC == 4 && CH == 1), "row groups are for float4 lanes and one column group");
@@ -453,26 +456,40 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::kMinBlocks) spmm_ro
     }
 }
 
+template <int VEC, int CH, bool FULL, bool DEEP, int G, bool DYN>
+cudaError_t blocks_per_sm(int &n)
+{
+    static int known = 0;  // same for every device of one model; queried once
+    if (known == 0) {
+        int got = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&got, spmm_rows_kernel<VEC, CH, FULL, DEEP, G, DYN>, kWarps * 32, 0);
+        if (e != cudaSuccess) return e;
+        known = got > 0 ? got : 1;
+    }
+    n = known;
+    return cudaSuccess;
+}
+
 template <int VEC, int CH, bool FULL, bool DEEP, int G = 1>
 cudaError_t launch_rows_t(const RowsArgs &a, uint32_t slabs, int sm_count, cudaStream_t s)
 {
-    static int blocks_per_sm = 0;  // same for every device of one model; queried once
-    if (blocks_per_sm == 0) {
-        int n = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, spmm_rows_kernel<VEC, CH, FULL, DEEP, G, false>, kWarps * 32, 0);
-        if (e != cudaSuccess) return e;
-        blocks_per_sm = n > 0 ? n : 1;
-    }
-    const uint64_t want = (uint64_t)sm_count * blocks_per_sm;
     const uint64_t chunk_blocks = ((uint64_t)a.num_chunks + kWarps - 1) / kWarps;
-    uint64_t work = a.num_tiles > chunk_blocks ? a.num_tiles : chunk_blocks;
-    uint32_t gx = (uint32_t)(work < want ? work : want);
-    if (slabs > 1) gx = (gx + slabs - 1) / slabs;  // keep the whole grid about one resident wave
-    if (gx == 0) gx = 1;
-    if constexpr (VEC == 4)  // tiles dealt by a counter: where there are counters and enough tiles to deal
-        if (a.counters && a.num_tiles >= 8ull * gx)
-            return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true>, dim3(gx, slabs), kWarps * 32, 0, s, a);
-    return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, false>, dim3(gx, slabs), kWarps * 32, 0, s, a);
+    const uint64_t work = a.num_tiles > chunk_blocks ? a.num_tiles : chunk_blocks;
+    auto grid = [&](int per_sm) {  // about one resident wave over all slabs
+        const uint64_t want = (uint64_t)sm_count * per_sm;
+        const uint64_t gx = ((work < want ? work : want) + slabs - 1) / slabs;
+        return (uint32_t)(gx ? gx : 1);
+    };
+    int n = 0;
+    cudaError_t e;
+    if constexpr (VEC == 4)
+        if (a.counters) {  // tiles dealt by a counter: where there are enough to deal
+            if ((e = blocks_per_sm<VEC, CH, FULL, DEEP, G, true>(n)) != cudaSuccess) return e;
+            if (a.num_tiles >= 8ull * grid(n)) 
+                return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true>, dim3(grid(n), slabs), kWarps * 32, 0, s, a);
+        }
+    if ((e = blocks_per_sm<VEC, CH, FULL, DEEP, G, false>(n)) != cudaSuccess) return e;
+    return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, false>, dim3(grid(n), slabs), kWarps * 32, 0, s, a);
 }
 
 // dst (rows x quads float4, 16-byte aligned) = src (rows x N, leading dimension ld_src), padding zeroed.  Bound by memory
@@ -534,10 +551,11 @@ cudaError_t launch_rows(const RowsArgs &args, int sm_count, cudaStream_t s)
     const uint64_t groups = (uint64_t)sm_count * kWarps * (N <= 16 ? 8 : N <= 32 ? 4 : N <= 64 ? 2 : 1);
     if (a.run_rows && v4 && a.num_chunks == 0 && !a.row_map && a.num_rows / a.run_rows * ((N + 127) / 128) >= groups)
         return launch_block_rows(a, sm_count, s);
-    // deep: at most one resident wave of tiles, or long rows (measured on shards of R-MAT 2^24: 300 nonzeros per row
-    // 2.19 vs 2.38 ms, 21 per row 1.88 vs 1.93 ms in favour of deep; 15 per row (R-MAT 2^20) 0.645 vs 0.611 ms and
-    // 3.4 per row 1.50 vs 1.48 ms in favour of shallow)
-    const bool deep = (uint64_t)a.num_tiles <= (uint64_t)sm_count * 6 || a.avg_row_nnz >= 20;
+    // deep: at most one resident wave of tiles, or long rows (R-MAT 2^24 with 300 nonzeros per row 2.19 against 2.38 ms, with 21
+    // 1.88 against 1.93; with 15 R-MAT 2^20 0.652 against 0.647 and 3.4 per row 1.50 against 1.48 in favour of shallow).  Two
+    // column groups per lane halve the rows in flight, and deep pays from shorter rows on: N = 256, R-MAT 2^18 (15 per row) 275
+    // against 293 us, uniform with 7 per row 122.5 against 121.6.
+    const bool deep = (uint64_t)a.num_tiles <= (uint64_t)sm_count * 6 || a.avg_row_nnz >= (v4 && N > 128 ? 10u : 20u);
     auto full = [&](uint32_t w) { return N % w == 0 && !(v4 && a.c_scalar); };
 #define CUTESPMM_GO(VEC, CH)                                                                   \
     do {                                                                                       \
