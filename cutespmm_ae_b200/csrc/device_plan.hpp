@@ -63,6 +63,7 @@ struct RowsArgs {
     uint32_t run_rows;         // rows come in aligned runs of this many (2 or 3) with the same columns; 0: they do not
     uint32_t early;            // 1: the plan's arrays never change, its first tiles can be fetched before the kernel in front is done
     uint32_t b_padded;         // 1: a row of B can be read up to N rounded up to four columns
+    uint32_t slab_cols;        // set by launch_rows: columns per slab of blocks (a multiple of 4)
     uint32_t c_scalar;         // set by launch_rows: C is written column by column
     uint32_t *status;          // device status word: set to 1 when a bounded wait gives up
     const uint32_t *row_map;   // reordered plan: row r of the work lists is row row_map[r] of C (nullptr: identity)

@@ -268,7 +268,7 @@ struct ChunkArgs {
     const float *bl;
     float *scratch, *C;
     uint64_t ldb, ld_scratch, ldc;
-    uint32_t num_chunks, N, col0;
+    uint32_t num_chunks, N, col0;  // N: the end of the slab
     bool c_scalar;
 };
 
@@ -373,10 +373,11 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DYN, G))
     constexpr int L = 32 / G;  // lanes of a group
     const int lane = threadIdx.x & 31;
     const int grp = G == 1 ? 0 : lane / L, sub = G == 1 ? lane : lane % L;
-    const uint32_t col0 = blockIdx.y * (32 * VEC * CH) + sub * VEC;  // this lane's first column
+    const uint32_t col0 = blockIdx.y * a.slab_cols + sub * VEC;          // this lane's first column
+    const uint32_t end = min(a.N, (blockIdx.y + 1) * a.slab_cols);       // ... and the end of the block's slab
     bool ok[CH];
 #pragma unroll
-    for (int ch = 0; ch < CH; ++ch) ok[ch] = FULL || (col0 + ch * 32 * VEC < a.N);
+    for (int ch = 0; ch < CH; ++ch) ok[ch] = FULL || (col0 + ch * 32 * VEC < end);
     const float *bl = a.B + col0;
     const uint32_t ldb32 = (uint32_t)a.ldb;  // < 2^32 (checked by the caller): one 32x32->64 multiply per address
     const uint2 *pairs = reinterpret_cast<const uint2 *>(a.pairs);
@@ -392,7 +393,7 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DYN, G))
     // Chunks of long rows first (the first tiles are on their way meanwhile): they are the largest single work items.
     if (a.num_chunks) {
         const ChunkArgs ca{pairs, reinterpret_cast<const uint4 *>(a.chunks), reinterpret_cast<const uint4 *>(a.long_rows), a.chunk_owner, a.arrivals, bl,
-                           a.scratch + col0, a.C + col0, a.ldb, a.ld_scratch, a.ldc, a.num_chunks, a.N, col0, a.c_scalar != 0};
+                           a.scratch + col0, a.C + col0, a.ldb, a.ld_scratch, a.ldc, a.num_chunks, end, col0, a.c_scalar != 0};
         // Narrow products: when the warps outnumber the chunks, a chunk is shared by the groups of a warp -- it is the longest
         // chain of the job (R-MAT 2^17: 4 500 chunks of 256, 64 steps of four gathers for a group at N = 64; N = 16 63.6 ->
         // 39.4 us, N = 32 70.4 -> 56.5) -- otherwise a group takes one on its own and the cost of starting and finishing a
@@ -439,7 +440,7 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DYN, G))
                 float *out = a.C + (uint64_t)r_out * a.ldc + col0;
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch)
-                    if (FULL || ok[ch]) store_row<FULL>(out + ch * 32 * VEC, acc[ch], a.c_scalar != 0, a.N - col0 - ch * 32 * VEC);
+                    if (FULL || ok[ch]) store_row<FULL>(out + ch * 32 * VEC, acc[ch], a.c_scalar != 0, end - col0 - ch * 32 * VEC);
             }
             if constexpr (G > 1) __syncwarp();
         }
@@ -471,7 +472,7 @@ cudaError_t blocks_per_sm(int &n)
 }
 
 template <int VEC, int CH, bool FULL, bool DEEP, int G = 1>
-cudaError_t launch_rows_t(const RowsArgs &a, uint32_t slabs, int sm_count, cudaStream_t s)
+cudaError_t launch_rows_t(RowsArgs a, uint32_t slabs, int sm_count, cudaStream_t s)
 {
     const uint64_t chunk_blocks = ((uint64_t)a.num_chunks + kWarps - 1) / kWarps;
     const uint64_t work = a.num_tiles > chunk_blocks ? a.num_tiles : chunk_blocks;
@@ -480,6 +481,10 @@ cudaError_t launch_rows_t(const RowsArgs &a, uint32_t slabs, int sm_count, cudaS
         const uint64_t gx = ((work < want ? work : want) + slabs - 1) / slabs;
         return (uint32_t)(gx ? gx : 1);
     };
+    // Slabs get equal shares of the grid, so a small job's are of equal width (uniform 15727 x 13804 at N = 260: 33.4 us as 256 + 4
+    // columns, 24.5 as 132 + 128); large ones are bound by the gathers' bytes and keep whole lines (170003 x 99991 at N = 384:
+    // 225 us as 256 + 128, 256 as 192 + 192).
+    a.slab_cols = (uint64_t)a.num_tiles <= (uint64_t)sm_count * 6 ? ((a.N + slabs - 1) / slabs + 3) & ~3u : 32 / G * VEC * CH;
     int n = 0;
     cudaError_t e;
     if constexpr (VEC == 4)
@@ -554,8 +559,9 @@ cudaError_t launch_rows(const RowsArgs &args, int sm_count, cudaStream_t s)
     // deep: at most one resident wave of tiles, or long rows (R-MAT 2^24 with 300 nonzeros per row 2.19 against 2.38 ms, with 21
     // 1.88 against 1.93; with 15 R-MAT 2^20 0.652 against 0.647 and 3.4 per row 1.50 against 1.48 in favour of shallow).  Two
     // column groups per lane halve the rows in flight, and deep pays from shorter rows on: N = 256, R-MAT 2^18 (15 per row) 275
-    // against 293 us, uniform with 7 per row 122.5 against 121.6.
-    const bool deep = (uint64_t)a.num_tiles <= (uint64_t)sm_count * 6 || a.avg_row_nnz >= (v4 && N > 128 ? 10u : 20u);
+    // against 293 us, uniform with 7 per row 122.5 against 121.6; with two slabs of such groups always (7 per row, N = 260: 180
+    // against 208 us, N = 384: 221 against 244).
+    const bool deep = (uint64_t)a.num_tiles <= (uint64_t)sm_count * 6 || a.avg_row_nnz >= (!v4 || N <= 128 ? 20u : N <= 256 ? 10u : 0u);
     auto full = [&](uint32_t w) { return N % w == 0 && !(v4 && a.c_scalar); };
 #define CUTESPMM_GO(VEC, CH)                                                                   \
     do {                                                                                       \
