@@ -12,6 +12,7 @@
 #include "plan.hpp"
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <numeric>
 
@@ -328,18 +329,22 @@ void choose_panel_paths(HostPlan &p, const std::vector<uint32_t> &panel_ncols)
 uint32_t find_row_runs(const HostPlan &p)
 {
     if (p.M < 2 || p.nnz == 0) return 0;
-    bool two = p.M % 2 == 0, three = p.M % 3 == 0;
-    for (uint64_t r = 1; r < p.M && (two || three); ++r) {
-        const bool asked = (two && r % 2) || (three && r % 3);
-        if (!asked) continue;
-        const uint32_t j = p.row_ptr[r], len = p.row_ptr[r + 1] - j, i = p.row_ptr[r - 1];
-        bool same = j - i == len;
-        for (uint32_t k = 0; same && k < len; ++k) same = p.pairs[i + k].col == p.pairs[j + k].col;
-        if (!same) {
-            if (r % 2) two = false;
-            if (r % 3) three = false;
+    // bit 0: runs of two are ruled out, bit 1: runs of three; blocks of rows, so that most matrices are done after the first few
+    std::atomic<uint32_t> ruled_out{(p.M % 2 ? 1u : 0u) | (p.M % 3 ? 2u : 0u)};
+    constexpr uint64_t kRows = 4096;
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int64_t b = 0; b < (int64_t)((p.M + kRows - 1) / kRows); ++b) {
+        for (uint64_t r = std::max<uint64_t>(1, b * kRows); r < std::min<uint64_t>(p.M, (b + 1) * kRows); ++r) {
+            const uint32_t known = ruled_out.load(std::memory_order_relaxed), asks = ((r % 2 ? 1u : 0u) | (r % 3 ? 2u : 0u)) & ~known;
+            if (known == 3) break;
+            if (!asks) continue;
+            const uint32_t j = p.row_ptr[r], len = p.row_ptr[r + 1] - j, i = p.row_ptr[r - 1];
+            bool same = j - i == len;
+            for (uint32_t k = 0; same && k < len; ++k) same = p.pairs[i + k].col == p.pairs[j + k].col;
+            if (!same) ruled_out.fetch_or(asks);
         }
     }
+    const bool two = !(ruled_out & 1), three = !(ruled_out & 2);
     return three ? 3 : two ? 2 : 0;
 }
 
