@@ -29,6 +29,7 @@
 
 #include "../../include/cutespmm.h"
 #include "device_plan.hpp"
+#include "noalloc_rows.hpp"
 #include "ptx.cuh"
 
 namespace cutespmm {
@@ -38,6 +39,7 @@ void set_last_error(const std::string &msg);  // capi.cu
 namespace {
 
 namespace ptx = cutespmm::ptx;
+using cutespmm::RowRange;
 
 constexpr uint32_t kLimitSplit = CUTESPMM_NOALLOC_SPLIT_NNZ;  // the chunk length the published limit is stated for
 constexpr uint64_t kScratchFloats = CUTESPMM_NOALLOC_SCRATCH_BYTES / 4;
@@ -59,17 +61,9 @@ struct State {
 };
 static __device__ State g_state;
 
-// Nonzero positions [j0, j1) of row r, forced into [0, nnz] and into order: every position the kernels derive an array
-// index from is then below the `nnz` the host sized its checks with, whatever rowPtr holds.
-struct Range {
-    uint32_t j0, j1;
-};
-__device__ __forceinline__ Range row_range(const uint32_t *__restrict__ rowPtr, uint64_t r, uint32_t nnz)
+__device__ __forceinline__ RowRange load_range(const uint32_t *__restrict__ rowPtr, uint64_t r, uint32_t nnz)
 {
-    Range g;
-    g.j0 = min(__ldg(rowPtr + r), nnz);
-    g.j1 = min(max(__ldg(rowPtr + r + 1), g.j0), nnz);
-    return g;
+    return cutespmm::row_range(__ldg(rowPtr + r), __ldg(rowPtr + r + 1), nnz);
 }
 
 // Lists the chunks of the rows longer than `split`.  One pass over the row pointers (4 us at 2^18 rows); which slots a row
@@ -82,7 +76,7 @@ __global__ void __launch_bounds__(256) noalloc_list_kernel(const uint32_t *__res
     ptx::grid_release();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < M; r += stride) {
-        const Range g = row_range(rowPtr, r, nnz);
+        const RowRange g = load_range(rowPtr, r, nnz);
         const uint32_t len = g.j1 - g.j0;
         if (len <= split) continue;
         const uint32_t n = (uint32_t)(((uint64_t)len + split - 1) / split);
@@ -221,7 +215,7 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
         __syncwarp();
         uint32_t pieces = 0;
         if (lane == 0) {
-            const Range g = row_range(a.rowPtr, ck.x, a.nnz);
+            const RowRange g = load_range(a.rowPtr, ck.x, a.nnz);
             pieces = (uint32_t)(((uint64_t)(g.j1 - g.j0) + a.split - 1) / a.split);
             if (atomicAdd(&g_arrivals[ck.w * kMaxSlabs + blockIdx.y], 1u) != pieces - 1) pieces = 0;
             __threadfence();
@@ -246,8 +240,9 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
         first = __shfl_sync(kFull, first, 0);
         if (first >= a.M) break;
         const uint32_t cnt = min(a.claim, a.M - first);
-        Range g{0u, 0u};
-        if ((uint32_t)lane < cnt) g = row_range(a.rowPtr, (uint64_t)first + lane, a.nnz);
+        RowRange g{0u, 0u};
+        if ((uint32_t)lane < cnt) g = load_range(a.rowPtr, (uint64_t)first + lane, a.nnz);
+        const RowRange before{__shfl_up_sync(kFull, g.j0, 1), __shfl_up_sync(kFull, g.j1, 1)};
         const bool listed = !overflow && g.j1 - g.j0 > a.split;
         for (uint32_t i0 = 0; i0 < cnt;) {
             const uint32_t j0 = __shfl_sync(kFull, g.j0, (int)i0), j1 = __shfl_sync(kFull, g.j1, (int)i0);
@@ -262,9 +257,10 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
                 ++i0;
                 continue;
             }
-            // the rows from i0 on whose nonzeros fit the buffer together
-            const bool fits = (uint32_t)lane < cnt && !listed && g.j0 >= j0 && g.j1 - j0 <= kBuf && g.j1 >= g.j0;
-            const unsigned miss = __ballot_sync(kFull, (uint32_t)lane >= i0 && !fits);
+            // the rows from i0 on whose nonzeros follow one another and fit the buffer together: what is staged up to the last
+            // one's end holds all of them, so nothing below reads a position of the buffer that this batch has not written
+            const bool fits = (uint32_t)lane < cnt && !listed && cutespmm::joins_batch(before, g, j0, kBuf);
+            const unsigned miss = __ballot_sync(kFull, (uint32_t)lane > i0 && !fits);
             const uint32_t i1 = miss ? __ffs(miss) - 1 : 32u;
             const uint32_t end = __shfl_sync(kFull, g.j1, (int)i1 - 1);
             __syncwarp();
@@ -275,7 +271,7 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
             // a row of more than a few steps is shared by the groups, the others are a group's each
             constexpr uint32_t kShared = G == 1 ? kBuf : 4 * U;
             for (uint32_t i = i0 + grp; i < i1; i += G) {
-                const uint32_t from = start[i], to = max(start[i + 1], from);
+                const uint32_t from = start[i], to = start[i + 1];
                 if (G > 1 && to - from > kShared) continue;
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch) zero(acc[ch]);

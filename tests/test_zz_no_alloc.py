@@ -135,3 +135,25 @@ def test_noalloc_at_the_edges_of_every_width(oracle_mod, N):
     torch.cuda.synchronize()
     cs.spmm_csr_noalloc(A.M, A.K, *args, C[:A.M])
     assert oracle_mod.rel_fro(want, C[:A.M].cpu().numpy()) <= REL_FRO_TOL_FP32
+
+
+@pytest.mark.parametrize("N", [1, 16, 33, 64, 128, 132, 256])
+def test_noalloc_with_row_pointers_that_go_down(oracle_mod, N):
+    """Row ends that decrease among rows that a warp takes together: every row is the sum over its own range, cut to the
+    stated nnz and empty where it ends before it begins, and nothing else is read."""
+    rng = np.random.default_rng(N + 1)
+    M, K, nnz = 500, 300, 4000
+    rp = np.sort(rng.integers(0, nnz, M + 1))
+    rp[:4] = (0, 100, 10, 20)
+    at = rng.choice(np.arange(4, M + 1), 120, replace=False)
+    rp[at] = np.clip(rp[at] + rng.integers(-60, 61, 120), 0, nnz + 50)
+    cols, vals = rng.integers(0, K, nnz).astype(np.int32), rng.standard_normal(nnz).astype(np.float32)
+    begin, end = np.minimum(rp[:-1], nnz), np.minimum(rp[1:], nnz)
+    own = [np.arange(b, max(b, e)) for b, e in zip(begin, end)]
+    pos = np.concatenate(own)
+    want_rp = np.concatenate([[0], np.cumsum([len(o) for o in own])]).astype(np.uint64)
+    B = g.dense_operand(K, N, 101, device="cuda")
+    want = oracle_mod.spmm_csr(want_rp, cols[pos].astype(np.uint32), vals[pos], B.cpu().numpy(), M, K)
+    C = torch.full((M, N), float("nan"), device="cuda")
+    cs.spmm_csr_noalloc(M, K, torch.from_numpy(rp.astype(np.int32)).cuda(), torch.from_numpy(cols).cuda(), torch.from_numpy(vals).cuda(), B, C)
+    assert oracle_mod.rel_fro(want, C.cpu().numpy()) <= REL_FRO_TOL_FP32
