@@ -12,8 +12,10 @@
 // The scratch is the file-scope array g_scratch below (16 MiB), beside it the list of chunks and their counters
 // (2 MiB).  Every GPU on which the library is loaded holds them until the process exits.  All calls on one
 // device share them, and the scratch keeps whatever the previous call left there; nothing in it has to start at
-// zero, because every slot a call reads was written earlier by the same call.  Two calls that overlap on the same GPU (different streams,
-// or different host threads) race on it: order them on one stream or with events.
+// zero, because every slot a call reads was written earlier by the same call; the counters are put back to zero by the last
+// block of a call.  Two calls that overlap on the same GPU (different streams, or different host threads) race on all of it
+// and their results are undefined -- order them on one stream or with events -- but they stay inside their own arrays, and
+// the next call that overlaps with none starts from zero counters (last_block.cuh).
 //
 // In host code the name g_scratch is only a stand-in, not a device address.  The address the
 // kernels receive comes from cudaGetSymbolAddress, looked up once per device, with that device
@@ -29,6 +31,7 @@
 
 #include "../../include/cutespmm.h"
 #include "device_plan.hpp"
+#include "last_block.cuh"
 #include "noalloc_rows.hpp"
 #include "ptx.cuh"
 
@@ -54,9 +57,11 @@ static __device__ __align__(256) float g_scratch[kScratchFloats];
 // {row, j0, j1, slot of the row's first chunk} of chunk i, whose partial sum is row i of the scratch
 static __device__ uint4 g_list[kListSlots];
 static __device__ uint32_t g_arrivals[kListSlots * kMaxSlabs];  // per first slot of a row and column slab: chunks finished
-// All zero between calls: the last block of a call's main kernel puts it back.
+// All zero between calls: the last block of a call's main kernel puts it back, and the host where that kernel could not be
+// launched behind the list.  (Clearing it on the stream in front of every call instead gives up the overlap of launches: 65 000
+// nonzeros at N = 32 7.5 -> 10.3 us, R-MAT 2^16 N = 16 30.9 -> 32.9.)
 struct State {
-    uint32_t chunks, overflow, done, pad;
+    uint32_t chunks, overflow, balance, pad;
     uint32_t next_row[kMaxSlabs];
 };
 static __device__ State g_state;
@@ -116,7 +121,7 @@ struct MainArgs {
     const float *vals, *B;
     float *C, *scratch;
     uint64_t ldb, ldc;
-    uint32_t M, K, nnz, N, lds, split, claim;
+    uint32_t M, K, nnz, N, lds, split, capacity, claim;  // capacity: chunks the scratch and the list hold for this call
 };
 
 // The product.  A warp is G groups of 32/G lanes; a group spans a slab of 32/G * VEC * CH columns.  First the listed chunks
@@ -201,9 +206,11 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
     ptx::grid_wait();
     ptx::grid_release();
     const bool overflow = g_state.overflow != 0;
-    const uint32_t chunks = overflow ? 0u : g_state.chunks;
+    const uint32_t chunks = overflow ? 0u : min(g_state.chunks, a.capacity);
     for (uint32_t c = warp * gridDim.x + blockIdx.x; c < chunks; c += gridDim.x * kWarps) {
         const uint4 ck = g_list[c];
+        // a call that overlaps this one may have written the list: what it names has to lie inside this call's arrays
+        if (ck.x >= a.M || ck.y > ck.z || ck.z > a.nnz || ck.w > c) continue;
         V acc[CH];
         whole_warp(acc, ck.y, ck.z);
         if (grp == 0) {
@@ -217,7 +224,7 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
         if (lane == 0) {
             const RowRange g = load_range(a.rowPtr, ck.x, a.nnz);
             pieces = (uint32_t)(((uint64_t)(g.j1 - g.j0) + a.split - 1) / a.split);
-            if (atomicAdd(&g_arrivals[ck.w * kMaxSlabs + blockIdx.y], 1u) != pieces - 1) pieces = 0;
+            if (atomicAdd(&g_arrivals[ck.w * kMaxSlabs + blockIdx.y], 1u) != pieces - 1 || pieces > a.capacity - ck.w) pieces = 0;
             __threadfence();
         }
         pieces = __shfl_sync(kFull, pieces, 0);
@@ -294,22 +301,18 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
         }
     }
 
-    // the last block to leave puts the counters back for the next call
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t blocks = gridDim.x * gridDim.y;
-        __threadfence();
-        if (atomicInc(&g_state.done, blocks - 1) == blocks - 1) {
-            g_state.chunks = 0;
-            g_state.overflow = 0;
-            for (uint32_t y = 0; y < kMaxSlabs; ++y) g_state.next_row[y] = 0;
-        }
+    if (threadIdx.x == 0 && cutespmm::last_block_out(&g_state.balance)) {
+        g_state.chunks = 0;
+        g_state.overflow = 0;
+        for (uint32_t y = 0; y < kMaxSlabs; ++y) g_state.next_row[y] = 0;
     }
 }
 
 // What a device needs to know: looked up once.
 struct DeviceSetup {
     float *scratch = nullptr;
+    void *state = nullptr;
     int sm_count = 0;
 };
 constexpr int kMaxDevices = 64;
@@ -375,14 +378,16 @@ extern "C" int cutespmm_spmm_csr_noalloc(uint32_t M, uint32_t K, uint32_t nnz, c
         std::lock_guard<std::mutex> lock(g_setup_mutex);
         if (!g_setup[dev].scratch) {  // first call on this device: resolve the symbol with this device current
             float *ptr = nullptr;
-            e = cudaGetSymbolAddress(reinterpret_cast<void **>(&ptr), g_scratch);
-            if (e != cudaSuccess || !ptr)
-                return fail(CUTESPMM_ECUDA, std::string("cudaGetSymbolAddress(scratch): ") + cudaGetErrorString(e));
+            void *state = nullptr;
+            if ((e = cudaGetSymbolAddress(reinterpret_cast<void **>(&ptr), g_scratch)) != cudaSuccess || !ptr ||
+                (e = cudaGetSymbolAddress(&state, g_state)) != cudaSuccess || !state)
+                return fail(CUTESPMM_ECUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
             int sms = 0;
             e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
             if (e != cudaSuccess || sms <= 0)
                 return fail(CUTESPMM_ECUDA, std::string("cudaDeviceGetAttribute: ") + cudaGetErrorString(e));
             g_setup[dev].sm_count = sms;
+            g_setup[dev].state = state;
             g_setup[dev].scratch = ptr;
         }
         setup = g_setup[dev];
@@ -393,11 +398,11 @@ extern "C" int cutespmm_spmm_csr_noalloc(uint32_t M, uint32_t K, uint32_t nnz, c
     uint64_t split = nnz > (2u << 20) ? 256 : 128;
     auto slots_of = [&](uint64_t len) { return 2ull * ((nnz + len - 1) / len) + 2; };
     while (slots_of(split) * lds > kScratchFloats || slots_of(split) > kListSlots) split *= 2;
-    MainArgs a{rowPtr_dev, cols_dev, vals_dev, B_dev, C_dev, setup.scratch, ldb, ldc, M, K, nnz, N, lds, (uint32_t)split, 1};
+    MainArgs a{rowPtr_dev, cols_dev, vals_dev, B_dev, C_dev, setup.scratch, ldb, ldc, M, K, nnz, N, lds, (uint32_t)split, (uint32_t)slots_of(split), 1};
     if (nnz > split) {
         const uint64_t want = ((uint64_t)M + 255) / 256, cap = (uint64_t)setup.sm_count * 8;
-        e = cutespmm::launch_overlapped(noalloc_list_kernel, (uint32_t)(want < cap ? want : cap), 256, 0, s, rowPtr_dev, M, nnz, (uint32_t)split,
-                                        (uint32_t)slots_of(split));
+        e = cutespmm::launch_overlapped(noalloc_list_kernel, (uint32_t)(want < cap ? want : cap), 256, 0, s, rowPtr_dev, M, nnz, a.split,
+                                        a.capacity);
     }
     // four columns per lane where the rows of B and C are 16-byte aligned; narrow products put several rows on a warp
     const bool v4 = !((reinterpret_cast<uintptr_t>(B_dev) | reinterpret_cast<uintptr_t>(C_dev)) & 15) && !((ldb | ldc | N) & 3);
@@ -409,6 +414,7 @@ extern "C" int cutespmm_spmm_csr_noalloc(uint32_t M, uint32_t K, uint32_t nnz, c
                 : N <= 32 ? launch_main<1, 1, 1>(a, setup.sm_count, s) : N <= 64 ? launch_main<1, 2, 1>(a, setup.sm_count, s)
                                                                               : launch_main<1, 4, 1>(a, setup.sm_count, s);
     }
+    if (e != cudaSuccess) cudaMemsetAsync(setup.state, 0, sizeof(State), s);  // a list without its product
     if (e != cudaSuccess) return fail(CUTESPMM_ECUDA, std::string("cutespmm_spmm_csr_noalloc launch: ") + cudaGetErrorString(e));
     return CUTESPMM_OK;
 }

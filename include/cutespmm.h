@@ -232,9 +232,9 @@ int cutespmm_plan_csr_device(const cutespmm_plan_t *plan, uint32_t *rowPtr_dev, 
  * Limits, checked before anything is launched (CUTESPMM_EUNSUPPORTED with a message otherwise):
  *   N <= CUTESPMM_NOALLOC_MAX_N   and   (2*ceil(nnz/SPLIT_NNZ) + 2) * roundup(N, 4) * 4 <= SCRATCH_BYTES
  *   (16.7 M nonzeros at N = 128).
- * All calls on a device share the scratch, which keeps the previous call's contents; nothing in it
- * needs clearing, but calls that overlap on the same GPU race on it -- keep them on one stream or
- * order them with events.  The first call on each device looks up the device address of the scratch
+ * All calls on a device share the scratch and its counters.  Calls that overlap on the same GPU race on them and their
+ * results are undefined -- keep them on one stream or order them with events; they stay inside their own operands, and later
+ * calls that overlap with none are not affected.  The first call on each device looks up the device address of the scratch
  * (cudaGetSymbolAddress) and the kernels' occupancy; make that first call outside any stream capture. */
 #define CUTESPMM_NOALLOC_SCRATCH_BYTES (16u << 20)
 #define CUTESPMM_NOALLOC_SPLIT_NNZ 1024u

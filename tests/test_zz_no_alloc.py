@@ -157,3 +157,27 @@ def test_noalloc_with_row_pointers_that_go_down(oracle_mod, N):
     C = torch.full((M, N), float("nan"), device="cuda")
     cs.spmm_csr_noalloc(M, K, torch.from_numpy(rp.astype(np.int32)).cuda(), torch.from_numpy(cols).cuda(), torch.from_numpy(vals).cuda(), B, C)
     assert oracle_mod.rel_fro(want, C.cpu().numpy()) <= REL_FRO_TOL_FP32
+
+
+def test_noalloc_calls_after_overlapping_ones_are_whole(oracle_mod):
+    """Calls that overlap on two streams race on the scratch, the list of chunks and the counters: what they write is not
+    defined, but they stay inside their own operands, and the ordered calls after them compute every row."""
+    A, S = g.rmat(16, 8, seed=103, values="uniform"), g.rmat(11, 8, seed=104, values="uniform")
+    dev = [(m.M, m.K, m.row_ptr.to(torch.int32).cuda(), m.cols.cuda(), m.vals.cuda()) for m in (A, S)]
+    want, ops = [], []
+    for m, N in ((A, 64), (S, 160)):
+        B = g.dense_operand(m.K, N, 105, device="cuda")
+        ops.append((B, torch.full((m.M + 64, N), float("nan"), device="cuda")))
+        want.append(oracle_mod.spmm_csr(m.row_ptr, m.cols, m.vals, B.cpu().numpy(), m.M, m.K))
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for d, (B, C), s in zip(dev, ops, streams):
+            cs.spmm_csr_noalloc(*d, B, C[: d[0]], stream=s)
+    torch.cuda.synchronize()
+    for d, (B, C), w in zip(dev, ops, want):
+        assert torch.isnan(C[d[0]:]).all()  # nothing behind the last row
+        C.fill_(float("nan"))
+        for _ in range(2):
+            cs.spmm_csr_noalloc(*d, B, C[: d[0]])
+            assert oracle_mod.rel_fro(w, C[: d[0]].cpu().numpy()) <= REL_FRO_TOL_FP32
