@@ -19,7 +19,8 @@
 //
 // In host code the name g_scratch is only a stand-in, not a device address.  The address the
 // kernels receive comes from cudaGetSymbolAddress, looked up once per device, with that device
-// current, by the first call made on it; that first call should be made outside any stream capture.
+// current, by the first call made on it, which also loads every kernel of this file; that first call should be made
+// outside any stream capture.
 //
 // No counterpart in the reference project.
 #include <cuda_runtime.h>
@@ -309,25 +310,8 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
     }
 }
 
-// What a device needs to know: looked up once.
-struct DeviceSetup {
-    float *scratch = nullptr;
-    void *state = nullptr;
-    int sm_count = 0;
-};
-constexpr int kMaxDevices = 64;
-DeviceSetup g_setup[kMaxDevices];
-std::mutex g_setup_mutex;
-
-template <int VEC, int CH, int G> cudaError_t launch_main(MainArgs a, int sm_count, cudaStream_t s)
+template <int VEC, int CH, int G> cudaError_t launch_main(MainArgs a, int sm_count, int per_sm, cudaStream_t s)
 {
-    static int per_sm = 0;  // same for every device of one model; queried once
-    if (per_sm == 0) {
-        int n = 0;
-        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, noalloc_main_kernel<VEC, CH, G>, kWarps * 32, 0);
-        if (e != cudaSuccess) return e;
-        per_sm = n > 0 ? n : 1;
-    }
     const uint32_t slabs = (a.N + 32 / G * VEC * CH - 1) / (32 / G * VEC * CH);
     const uint32_t wave = (uint32_t)(sm_count * per_sm) / slabs;  // one resident wave
     // rows per claim: about a buffer of nonzeros, at most one per lane; few rows are spread over all warps
@@ -340,6 +324,57 @@ template <int VEC, int CH, int G> cudaError_t launch_main(MainArgs a, int sm_cou
     const uint64_t want = a.nnz > a.split && chunk_blocks > row_blocks ? chunk_blocks : row_blocks;
     return cutespmm::launch_overlapped(noalloc_main_kernel<VEC, CH, G>, dim3((uint32_t)(want < wave ? (want ? want : 1) : (wave ? wave : 1)), slabs), kWarps * 32,
                                        0, s, a);
+}
+
+// Loads the kernel's code on the current device and asks how many of its blocks an SM holds.
+template <int VEC, int CH, int G> cudaError_t load_main(int *per_sm)
+{
+    cudaFuncAttributes attr{};
+    const cudaError_t e = cudaFuncGetAttributes(&attr, noalloc_main_kernel<VEC, CH, G>);
+    return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, noalloc_main_kernel<VEC, CH, G>, kWarps * 32, 0);
+}
+
+// The forms of the product, by whether the rows of B and C are 16-byte aligned and by width: four columns per lane (or one), and
+// several rows per warp for narrow products.
+struct Form {
+    uint32_t widest;
+    cudaError_t (*load)(int *per_sm);
+    cudaError_t (*launch)(MainArgs, int sm_count, int per_sm, cudaStream_t);
+};
+template <int VEC, int CH, int G> constexpr Form form(uint32_t widest) { return Form{widest, load_main<VEC, CH, G>, launch_main<VEC, CH, G>}; }
+constexpr int kWidths = 5;
+constexpr Form kForms[2][kWidths] = {
+    {form<1, 1, 4>(8), form<1, 1, 2>(16), form<1, 1, 1>(32), form<1, 2, 1>(64), form<1, 4, 1>(CUTESPMM_NOALLOC_MAX_N)},
+    {form<4, 1, 8>(16), form<4, 1, 4>(32), form<4, 1, 2>(64), form<4, 1, 1>(128), form<4, 2, 1>(CUTESPMM_NOALLOC_MAX_N)}};
+
+// What the calls on a device need to know, looked up by the first of them.  All of the kernels are loaded then, whatever the
+// first call's width: later calls load nothing and ask nothing, so they run inside a capture or with no device memory left, and a
+// call that is going to fail has queued nothing.
+struct DeviceSetup {
+    float *scratch = nullptr;
+    void *state = nullptr;
+    int sm_count = 0;
+    int per_sm[2][kWidths] = {};
+};
+constexpr int kMaxDevices = 64;
+DeviceSetup g_setup[kMaxDevices];
+std::mutex g_setup_mutex;
+
+cudaError_t look_up(int dev, DeviceSetup &d)
+{
+    cudaError_t e;
+    if ((e = cudaGetSymbolAddress(reinterpret_cast<void **>(&d.scratch), g_scratch)) != cudaSuccess ||
+        (e = cudaGetSymbolAddress(&d.state, g_state)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        return e;
+    cudaFuncAttributes attr{};
+    if ((e = cudaFuncGetAttributes(&attr, noalloc_list_kernel)) != cudaSuccess) return e;
+    for (int v4 = 0; v4 < 2; ++v4)
+        for (int w = 0; w < kWidths; ++w) {
+            if ((e = kForms[v4][w].load(&d.per_sm[v4][w])) != cudaSuccess) return e;
+            if (d.per_sm[v4][w] < 1) d.per_sm[v4][w] = 1;
+        }
+    return cudaSuccess;
 }
 
 int fail(int status, const std::string &msg)
@@ -376,19 +411,11 @@ extern "C" int cutespmm_spmm_csr_noalloc(uint32_t M, uint32_t K, uint32_t nnz, c
     DeviceSetup setup;
     {
         std::lock_guard<std::mutex> lock(g_setup_mutex);
-        if (!g_setup[dev].scratch) {  // first call on this device: resolve the symbol with this device current
-            float *ptr = nullptr;
-            void *state = nullptr;
-            if ((e = cudaGetSymbolAddress(reinterpret_cast<void **>(&ptr), g_scratch)) != cudaSuccess || !ptr ||
-                (e = cudaGetSymbolAddress(&state, g_state)) != cudaSuccess || !state)
-                return fail(CUTESPMM_ECUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
-            int sms = 0;
-            e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (e != cudaSuccess || sms <= 0)
-                return fail(CUTESPMM_ECUDA, std::string("cudaDeviceGetAttribute: ") + cudaGetErrorString(e));
-            g_setup[dev].sm_count = sms;
-            g_setup[dev].state = state;
-            g_setup[dev].scratch = ptr;
+        if (!g_setup[dev].scratch) {
+            DeviceSetup found;
+            if ((e = look_up(dev, found)) != cudaSuccess)
+                return fail(CUTESPMM_ECUDA, std::string("cutespmm_spmm_csr_noalloc, first call on the device: ") + cudaGetErrorString(e));
+            g_setup[dev] = found;
         }
         setup = g_setup[dev];
     }
@@ -404,15 +431,11 @@ extern "C" int cutespmm_spmm_csr_noalloc(uint32_t M, uint32_t K, uint32_t nnz, c
         e = cutespmm::launch_overlapped(noalloc_list_kernel, (uint32_t)(want < cap ? want : cap), 256, 0, s, rowPtr_dev, M, nnz, a.split,
                                         a.capacity);
     }
-    // four columns per lane where the rows of B and C are 16-byte aligned; narrow products put several rows on a warp
-    const bool v4 = !((reinterpret_cast<uintptr_t>(B_dev) | reinterpret_cast<uintptr_t>(C_dev)) & 15) && !((ldb | ldc | N) & 3);
     if (e == cudaSuccess) {
-        if (v4) e = N <= 16 ? launch_main<4, 1, 8>(a, setup.sm_count, s) : N <= 32 ? launch_main<4, 1, 4>(a, setup.sm_count, s)
-                  : N <= 64 ? launch_main<4, 1, 2>(a, setup.sm_count, s) : N <= 128 ? launch_main<4, 1, 1>(a, setup.sm_count, s)
-                                                                                   : launch_main<4, 2, 1>(a, setup.sm_count, s);
-        else e = N <= 8 ? launch_main<1, 1, 4>(a, setup.sm_count, s) : N <= 16 ? launch_main<1, 1, 2>(a, setup.sm_count, s)
-                : N <= 32 ? launch_main<1, 1, 1>(a, setup.sm_count, s) : N <= 64 ? launch_main<1, 2, 1>(a, setup.sm_count, s)
-                                                                              : launch_main<1, 4, 1>(a, setup.sm_count, s);
+        const int v4 = !((reinterpret_cast<uintptr_t>(B_dev) | reinterpret_cast<uintptr_t>(C_dev)) & 15) && !((ldb | ldc | N) & 3) ? 1 : 0;
+        int w = 0;
+        while (N > kForms[v4][w].widest) ++w;
+        e = kForms[v4][w].launch(a, setup.sm_count, setup.per_sm[v4][w], s);
     }
     if (e != cudaSuccess) cudaMemsetAsync(setup.state, 0, sizeof(State), s);  // a list without its product
     if (e != cudaSuccess) return fail(CUTESPMM_ECUDA, std::string("cutespmm_spmm_csr_noalloc launch: ") + cudaGetErrorString(e));

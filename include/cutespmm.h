@@ -234,8 +234,10 @@ int cutespmm_plan_csr_device(const cutespmm_plan_t *plan, uint32_t *rowPtr_dev, 
  *   (16.7 M nonzeros at N = 128).
  * All calls on a device share the scratch and its counters.  Calls that overlap on the same GPU race on them and their
  * results are undefined -- keep them on one stream or order them with events; they stay inside their own operands, and later
- * calls that overlap with none are not affected.  The first call on each device looks up the device address of the scratch
- * (cudaGetSymbolAddress) and the kernels' occupancy; make that first call outside any stream capture. */
+ * calls that overlap with none are not affected.  The first call on each device, of any
+ * size and width, looks up the device address of the scratch (cudaGetSymbolAddress) and loads every kernel this call uses
+ * at any width: make it outside any stream capture and before the host framework takes the device's memory.  Later
+ * calls load nothing. */
 #define CUTESPMM_NOALLOC_SCRATCH_BYTES (16u << 20)
 #define CUTESPMM_NOALLOC_SPLIT_NNZ 1024u
 #define CUTESPMM_NOALLOC_MAX_N 512u
