@@ -541,10 +541,13 @@ int cutespmm_internal_spmm_range(const cutespmm_plan *p, const float *B, uint64_
         const bool aligned = !(reinterpret_cast<uintptr_t>(Bw) & 15) && !(ldb & 3) && (!(nw & 3) || b_padded);
         if (!aligned && (list.tiles || list.chunks) && !rg && worth_padding(p->host, Bw, ldb, C + n0, ldc, nw, s)) {
             ldw = (nw + 3) / 4 * 4;
-            if (cutespmm_internal_pool_alloc(reinterpret_cast<void **>(&copy), p->host.K * ldw * sizeof(float), p->device, s) == cudaSuccess) {
-                if ((e = launch_pad_rows(Bw, ldb, copy, p->host.K, nw, p->sm_count, s)) != cudaSuccess) return fail_cuda(e, "padding the rows of B");
+            if (cutespmm_internal_pool_alloc(reinterpret_cast<void **>(&copy), p->host.K * ldw * sizeof(float), p->device, s, false) == cudaSuccess) {
+                if ((e = launch_pad_rows(Bw, ldb, copy, p->host.K, nw, p->sm_count, s)) != cudaSuccess) {
+                    cudaFreeAsync(copy, s);
+                    return fail_cuda(e, "padding the rows of B");
+                }
                 Bw = copy;
-            } else {  // no memory for the copy: the kernel reads B as it is
+            } else {  // no memory for the copy: the kernel reads B as it is, and the call waits for nothing
                 cudaGetLastError();
                 copy = nullptr;
                 ldw = ldb;

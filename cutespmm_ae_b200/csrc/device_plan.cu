@@ -99,12 +99,12 @@ struct Temp {  // stream-ordered scratch of one call
 
 }  // namespace
 
-cudaError_t cutespmm_internal_pool_alloc(void **p, uint64_t bytes, int dev, cudaStream_t s)
+cudaError_t cutespmm_internal_pool_alloc(void **p, uint64_t bytes, int dev, cudaStream_t s, bool may_wait)
 {
     cudaMemPool_t pool = nullptr;
     cudaError_t e = device_pool(dev, &pool);
     if (e != cudaSuccess) return e;
-    if ((e = cudaMallocFromPoolAsync(p, bytes, pool, s)) != cudaErrorMemoryAllocation) return e;
+    if ((e = cudaMallocFromPoolAsync(p, bytes, pool, s)) != cudaErrorMemoryAllocation || !may_wait) return e;
     cudaGetLastError();
     cudaStreamSynchronize(s);
     cudaMemPoolTrimTo(pool, 0);
@@ -332,7 +332,7 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
     };
     Carver sizes;
     carve_temp(sizes);
-    if ((e = cutespmm_internal_pool_alloc(&temp.p, sizes.used, dev, s)) != cudaSuccess) return fail_cuda_status(e, "scratch of the plan creation");
+    if ((e = cutespmm_internal_pool_alloc(&temp.p, sizes.used, dev, s, true)) != cudaSuccess) return fail_cuda_status(e, "scratch of the plan creation");
     Carver at;
     at.base = static_cast<char *>(temp.p);
     const uint64_t zeroed = carve_temp(at);
@@ -430,7 +430,7 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
     // a block the pool would not keep is the driver's: mapping it into the pool takes longer than cudaMalloc (R-MAT 2^24,
     // 3.7 GB: plan creation 130 ms longer)
     const bool pooled = need.used <= kPoolKeeps;
-    if ((e = pooled ? cutespmm_internal_pool_alloc(&p->d_block, need.used, dev, s) : cudaMalloc(&p->d_block, need.used)) != cudaSuccess)
+    if ((e = pooled ? cutespmm_internal_pool_alloc(&p->d_block, need.used, dev, s, true) : cudaMalloc(&p->d_block, need.used)) != cudaSuccess)
         return fail_cuda_status(e, "memory of the plan");
     p->block_bytes = need.used;
     if (pooled) note_live(dev, (int64_t)need.used);

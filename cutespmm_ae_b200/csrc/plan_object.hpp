@@ -131,8 +131,9 @@ int cutespmm_internal_usable_device(int *dev, int *sm_count);
 int cutespmm_internal_fetch_lists(const cutespmm_plan *p);
 int cutespmm_internal_fetch_views(const cutespmm_plan *p, std::vector<uint32_t> *ncols, std::vector<uint32_t> *acols);
 
-// Memory of the library's pool on `dev` in the order of stream s (cudaFreeAsync gives it back).
-cudaError_t cutespmm_internal_pool_alloc(void **p, uint64_t bytes, int dev, cudaStream_t s);
+// Memory of the library's pool on `dev` in the order of stream s (cudaFreeAsync gives it back).  may_wait: where there is none
+// left, wait for the stream, give back what the pool keeps and try again (plan creation, which waits anyway; never a product).
+cudaError_t cutespmm_internal_pool_alloc(void **p, uint64_t bytes, int dev, cudaStream_t s, bool may_wait);
 
 // cutespmm_spmm restricted to a range of work items (nullptr: everything).  b_padded: rows of B can be read up to N rounded up
 // to four columns.  capi.cu

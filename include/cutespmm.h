@@ -18,8 +18,8 @@
  *     was created; all GPU work is ordered on the stream the caller passes
  *     (a cudaStream_t cast to void*, NULL = the legacy default stream the
  *     reference uses, spmm.cu:171-174);
- *   - cutespmm_spmm performs no allocation: the scratch it needs belongs to
- *     the plan.
+ *   - cutespmm_spmm never waits for the device, and its scratch belongs to the
+ *     plan; the one thing it may take besides is a padded copy of B (see there).
  */
 #ifndef CUTESPMM_H
 #define CUTESPMM_H
@@ -179,7 +179,14 @@ int cutespmm_plan_decode_csr(const cutespmm_plan_t *plan, uint64_t *rowPtr, uint
  * (kernel.cu:119-288).  B: K x N device, row-major, leading dimension ldb >= N; C: M x N device,
  * ldc >= N.  Every row of C is written (rows without nonzeros become 0), so C needs no memset
  * (the reference relies on run.cu:43,49).  Any N >= 1.  The plan's device must be the current one
- * (CUTESPMM_EINVAL otherwise): a host that drives several GPUs calls cudaSetDevice before each plan. */
+ * (CUTESPMM_EINVAL otherwise): a host that drives several GPUs calls cudaSetDevice before each plan.
+ *
+ * Nothing waits for the device.  Where the rows of B are not 16-byte aligned (ldb or N not a multiple of four, B off the
+ * 16-byte grid) and the matrix names them often enough, the row kernel reads a copy of B with padded rows, of at most 512 MiB
+ * at a time (wider products go in column windows), which is taken from the library's stream-ordered pool (the one
+ * cutespmm_plan_create_device uses) and given back on the stream within the call.  Without memory for it, and
+ * while the stream is being captured, the kernel reads B as it is: the same result, more slowly.  A caller that wants no
+ * allocation at all keeps rows of B that are 16-byte aligned. */
 int cutespmm_spmm(const cutespmm_plan_t *plan, const float *B_dev, uint64_t ldb, float *C_dev,
                   uint64_t ldc, uint32_t N, void *stream);
 

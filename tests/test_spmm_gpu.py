@@ -494,3 +494,38 @@ def test_brick_spans(oracle_mod, make, N):
         assert oracle_mod.rel_fro(want, out[:A.M].cpu().numpy()) <= 1e-3
         assert torch.isnan(out[A.M]).all() and p.device_status() == 0
     assert cs.Plan.from_csr(A, path=cs.PATH_BRICK).launch_count(N) == {160: 2, 224: 2, 288: 2, 320: 2, 352: 2, 480: 2, 608: 2}.get(N, 1)
+
+
+def test_product_waits_for_nothing_without_memory_for_a_padded_copy(oracle_mod):
+    """Rows of B off the 16-byte grid are read through a padded copy where there is memory for it.  Where there is none
+    the product reads B as it is; it does not wait for the stream to find some, nor fail."""
+    rng = np.random.default_rng(11)
+    M, K, N, per_row = 20000, 330000, 301, 60  # a copy of 401 MB
+    A = g.CsrMatrix(M, K, torch.arange(0, M * per_row + 1, per_row), torch.from_numpy(rng.integers(0, K, M * per_row).astype(np.int32)),
+                    torch.from_numpy(rng.standard_normal(M * per_row).astype(np.float32)))
+    csr = A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda()
+    p = cs.Plan.from_device_csr(M, K, *csr, path=cs.PATH_ROWS)
+    B = torch.randn((K, N), generator=torch.Generator("cuda").manual_seed(12), device="cuda")
+    few = cs.Plan.from_device_csr(64, K, csr[0][:65], csr[1][:64 * per_row], csr[2][:64 * per_row], path=cs.PATH_ROWS)
+    few.spmm(B)  # not worth a copy: the kernel that reads B as it is has been loaded
+    C, want = torch.full((M, N), float("nan"), device="cuda"), p.spmm(B)
+    stalled = torch.cuda.Event()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    assert cs.lib.cutespmm_release_memory() == 0  # what the pool keeps
+    before = torch.cuda.mem_get_info()[0]
+    hog = torch.empty(before - (256 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        torch.cuda._sleep(1_000_000_000)  # half a second
+        stalled.record()
+        p.spmm(B, C)
+        assert not stalled.query()  # the call came back while the stream was still busy
+        torch.cuda.synchronize()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert oracle_mod.rel_fro(want.cpu().numpy(), C.cpu().numpy()) <= REL_FRO_TOL_FP32
+    rows = np.concatenate([np.arange(5), np.arange(M - 5, M)])
+    ref = oracle_mod.spmm_csr_rows(A.row_ptr, A.cols, A.vals, B.cpu().numpy(), rows)
+    assert oracle_mod.rel_fro(ref, C[torch.from_numpy(rows).cuda()].cpu().numpy()) <= REL_FRO_TOL_FP32
+    assert p.device_status() == 0
