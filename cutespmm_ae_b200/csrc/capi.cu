@@ -423,39 +423,6 @@ static bool use_brick(const cutespmm_plan *p, const float *B, uint64_t ldb, cons
     return brick_wanted(p, N) && brick_supports(N, ldb, ldc, B, C);
 }
 
-// Kernels of one column window of width nw (bit 0 row kernel, bit 1 brick kernel, bit 2 slab kernel).  The alignment of
-// the caller's pointers is unknown here: the aligned case is assumed.
-static int window_kernels(const cutespmm_plan *p, uint32_t nw)
-{
-    const HostPlan &h = p->host;
-    const bool brick = brick_wanted(p, nw) && nw % 32 == 0;
-    const bool slab = h.slab_panels && nw % 128 == 0;
-    const bool all_rows = (!brick && h.num_bricks) || (!slab && h.slab_panels);
-    int mask = (brick ? 2 : 0) | (slab ? 4 : 0);
-    const cutespmm_list_sizes &rows = all_rows ? p->every : p->own;
-    if (rows.tiles || rows.chunks) mask |= 1;
-    return mask;
-}
-
-int cutespmm_spmm_kernels(const cutespmm_plan_t *p, uint32_t N)
-{
-    if (!p || N == 0 || p->host.M == 0) return 0;
-    int mask = 0;
-    for (uint32_t n0 = 0; n0 < N; n0 += kScratchCols) mask |= window_kernels(p, N - n0 < kScratchCols ? N - n0 : kScratchCols);
-    return mask;
-}
-
-int cutespmm_spmm_launch_count(const cutespmm_plan_t *p, uint32_t N)
-{
-    if (!p || N == 0 || p->host.M == 0) return 0;
-    int total = 0;
-    for (uint32_t n0 = 0; n0 < N; n0 += kScratchCols) {
-        const int mask = window_kernels(p, N - n0 < kScratchCols ? N - n0 : kScratchCols);
-        total += (mask & 1) + (mask & 2 ? brick_launches(N - n0 < kScratchCols ? N - n0 : kScratchCols) : 0) + ((mask >> 2) & 1);
-    }
-    return total;
-}
-
 int cutespmm_spmm(const cutespmm_plan_t *p, const float *B, uint64_t ldb, float *C, uint64_t ldc, uint32_t N,
                   void *stream)
 {
@@ -479,19 +446,85 @@ static void note_stream(const cutespmm_plan *p, cudaStream_t s)
 // (1.8 GB: 4.6 -> 5.6 ms per product); wide products of large matrices go in narrower windows instead.  Even widths above 32 are read two columns per lane and gain nothing.  Not while the stream is being captured
 // (a graph should not own memory).
 constexpr uint64_t kMaxPadBytes = 512ull << 20;
-static bool worth_padding(const HostPlan &h, const float *B, uint64_t ldb, const float *C, uint64_t ldc, uint32_t N, cudaStream_t s)
+static bool worth_padding(const HostPlan &h, const float *B, uint64_t ldb, const float *C, uint64_t ldc, uint32_t N)
 {
     const bool two = !((reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 7) && !((ldb | ldc | N) & 1);
     if (two && N > 32) return false;
     const uint64_t gain = h.nnz * (N <= 64 ? 12 : N * 2 / 5), cost = 3000000 + h.K * N * 5 / 4;  // picoseconds
-    if (gain < cost || h.K * ((uint64_t)N + 3) * sizeof(float) > kMaxPadBytes) return false;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return cap == cudaStreamCaptureStatusNone;
+    return gain >= cost && h.K * ((uint64_t)N + 3) * sizeof(float) <= kMaxPadBytes;
 }
+
+static bool capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
+// What the next column window of a product runs, `left` columns from its end: B and C point at the window's first column.
+struct ColumnWindow {
+    uint32_t cols;
+    bool slab, brick;  // the tensor-core panels run their kernel (otherwise the row kernel takes every row)
+    bool all_rows;     // the row kernel walks its list over every row
+    bool rows;         // ... and that list has entries
+    bool pad;          // B is copied into padded rows first
+};
+// whole: not a range of the work items; may_copy() is asked only where a copy would be worth it.
+template <class MayCopy>
+static ColumnWindow column_window(const cutespmm_plan *p, const float *B, uint64_t ldb, const float *C, uint64_t ldc, uint32_t left, bool whole, bool b_padded,
+                                  MayCopy &&may_copy)
+{
+    const HostPlan &h = p->host;
+    ColumnWindow w{};
+    w.cols = left < kScratchCols ? left : kScratchCols;
+    // rows of B off the 16-byte grid: a window is narrowed until a padded copy of it may be made
+    if (((reinterpret_cast<uintptr_t>(B) & 15) || (ldb & 3)) && h.K * ((uint64_t)w.cols + 3) * sizeof(float) > kMaxPadBytes) {
+        const uint64_t fit = kMaxPadBytes / (h.K * sizeof(float)) / 128 * 128;
+        if (fit && fit < w.cols && worth_padding(h, B, ldb, C, ldc, (uint32_t)fit) && may_copy()) w.cols = (uint32_t)fit;
+    }
+    w.slab = h.slab_panels && slab_supports(w.cols, ldb, ldc, B, C);
+    w.brick = use_brick(p, B, ldb, C, ldc, w.cols);
+    // brick panels whose shape the brick kernel does not take (N not a multiple of 32, unaligned
+    // operands) are executed by the row kernel from its all-rows work list
+    w.all_rows = (!w.brick && h.num_bricks) || (!w.slab && h.slab_panels);
+    const cutespmm_list_sizes &list = w.all_rows ? p->every : p->own;
+    w.rows = list.tiles || list.chunks;
+    const bool aligned = !(reinterpret_cast<uintptr_t>(B) & 15) && !(ldb & 3) && (!(w.cols & 3) || b_padded);
+    w.pad = !aligned && w.rows && whole && worth_padding(h, B, ldb, C, ldc, w.cols) && may_copy();
+    return w;
+}
+
+// The windows of a product of N columns of contiguous operands that start on a 16-byte boundary.
+template <class Fn> static void for_each_window(const cutespmm_plan *p, uint32_t N, Fn &&fn)
+{
+    float *at = reinterpret_cast<float *>(uintptr_t(1) << 40);  // stands for both operands, never followed
+    ColumnWindow w{};
+    for (uint32_t n0 = 0; n0 < N; n0 += w.cols) {
+        w = column_window(p, at + n0, N, at + n0, N, N - n0, true, false, [] { return true; });
+        fn(w);
+    }
+}
+
+extern "C" {
+
+int cutespmm_spmm_kernels(const cutespmm_plan_t *p, uint32_t N)
+{
+    if (!p || N == 0 || p->host.M == 0) return 0;
+    int mask = 0;
+    for_each_window(p, N, [&](const ColumnWindow &w) { mask |= (w.rows ? 1 : 0) | (w.brick ? 2 : 0) | (w.slab ? 4 : 0); });
+    return mask;
+}
+
+int cutespmm_spmm_launch_count(const cutespmm_plan_t *p, uint32_t N)
+{
+    if (!p || N == 0 || p->host.M == 0) return 0;
+    int total = 0;
+    for_each_window(p, N, [&](const ColumnWindow &w) { total += (w.pad ? 1 : 0) + (w.rows ? 1 : 0) + (w.brick ? brick_launches(w.cols) : 0) + (w.slab ? 1 : 0); });
+    return total;
+}
+
+}  // extern "C"
 
 int cutespmm_internal_spmm_range(const cutespmm_plan *p, const float *B, uint64_t ldb, float *C, uint64_t ldc, uint32_t N, void *stream,
                                  const cutespmm_item_range *rg, bool b_padded)
@@ -511,35 +544,25 @@ int cutespmm_internal_spmm_range(const cutespmm_plan *p, const float *B, uint64_
         return fail(CUTESPMM_EINVAL, "the current CUDA device (" + std::to_string(cur) + ") is not the one the plan was created on (" +
                                          std::to_string(p->device) + "): call cudaSetDevice first");
     note_stream(p, s);
-    uint32_t nw = 0;
-    for (uint32_t n0 = 0; n0 < N; n0 += nw) {
-        nw = N - n0 < kScratchCols ? N - n0 : kScratchCols;
-        // rows of B off the 16-byte grid: a window is narrowed until a padded copy of it may be made
-        if (((reinterpret_cast<uintptr_t>(B) & 15) || (ldb & 3)) && p->host.K * ((uint64_t)nw + 3) * sizeof(float) > kMaxPadBytes) {
-            const uint64_t fit = kMaxPadBytes / (p->host.K * sizeof(float)) / 128 * 128;
-            if (fit && fit < nw && worth_padding(p->host, B, ldb, C, ldc, (uint32_t)fit, s)) nw = (uint32_t)fit;
-        }
+    ColumnWindow w{};
+    for (uint32_t n0 = 0; n0 < N; n0 += w.cols) {
+        const float *Bw = B + n0;
+        float *Cw = C + n0;
+        w = column_window(p, Bw, ldb, Cw, ldc, N - n0, rg == nullptr, b_padded, [&] { return !capturing(s); });
+        const uint32_t nw = w.cols;
         cudaError_t e;
-        const bool slab = p->host.slab_panels && slab_supports(nw, ldb, ldc, B + n0, C + n0);
-        if (slab && rg) return fail(CUTESPMM_EUNSUPPORTED, "a plan with slab panels runs whole");
-        if (slab) {
-            SlabArgs sa = slab_args(p, B + n0, ldb, C + n0, ldc, nw);
+        if (w.slab && rg) return fail(CUTESPMM_EUNSUPPORTED, "a plan with slab panels runs whole");
+        if (w.slab) {
+            SlabArgs sa = slab_args(p, Bw, ldb, Cw, ldc, nw);
             if ((e = launch_slab(sa, p->sm_count, s)) != cudaSuccess) return fail_cuda(e, "slab kernel launch");
         }
-        const bool brick = use_brick(p, B + n0, ldb, C + n0, ldc, nw);
-        if (brick) {
-            BrickArgs ba = brick_args(p, B + n0, ldb, C + n0, ldc, nw, rg);
+        if (w.brick) {
+            BrickArgs ba = brick_args(p, Bw, ldb, Cw, ldc, nw, rg);
             if ((e = launch_brick(ba, p->sm_count, s)) != cudaSuccess) return fail_cuda(e, "brick kernel launch");
         }
-        // brick panels whose shape the brick kernel does not take (N not a multiple of 32, unaligned
-        // operands) are executed by the row kernel from its all-rows work list
-        const bool all_rows = (!brick && p->host.num_bricks) || (!slab && p->host.slab_panels);
-        const float *Bw = B + n0;
         uint64_t ldw = ldb;
         float *copy = nullptr;
-        const cutespmm_list_sizes &list = all_rows ? p->every : p->own;
-        const bool aligned = !(reinterpret_cast<uintptr_t>(Bw) & 15) && !(ldb & 3) && (!(nw & 3) || b_padded);
-        if (!aligned && (list.tiles || list.chunks) && !rg && worth_padding(p->host, Bw, ldb, C + n0, ldc, nw, s)) {
+        if (w.pad) {
             ldw = (nw + 3) / 4 * 4;
             if (cutespmm_internal_pool_alloc(reinterpret_cast<void **>(&copy), p->host.K * ldw * sizeof(float), p->device, s, false) == cudaSuccess) {
                 if ((e = launch_pad_rows(Bw, ldb, copy, p->host.K, nw, p->sm_count, s)) != cudaSuccess) {
@@ -553,7 +576,7 @@ int cutespmm_internal_spmm_range(const cutespmm_plan *p, const float *B, uint64_
                 ldw = ldb;
             }
         }
-        RowsArgs ra = rows_args(p, all_rows, Bw, ldw, C + n0, ldc, nw, copy || b_padded, rg);
+        RowsArgs ra = rows_args(p, w.all_rows, Bw, ldw, Cw, ldc, nw, copy || b_padded, rg);
         e = launch_rows(ra, p->sm_count, s);
         if (copy) cudaFreeAsync(copy, s);
         if (e != cudaSuccess) return fail_cuda(e, "row kernel launch");

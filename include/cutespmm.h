@@ -252,11 +252,12 @@ int cutespmm_spmm_csr_noalloc(uint32_t M, uint32_t K, uint32_t nnz, const uint32
                               const uint32_t *cols_dev, const float *vals_dev, const float *B_dev, uint64_t ldb,
                               float *C_dev, uint64_t ldc, uint32_t N, void *stream);
 
-/* Number of kernels one cutespmm_spmm call launches for this plan and N. */
+/* Number of kernels one cutespmm_spmm call launches for this plan and N, the padding of B included, on contiguous operands
+ * (ldb = ldc = N) that start on a 16-byte boundary, outside a capture and with memory for the padded copy. */
 int cutespmm_spmm_launch_count(const cutespmm_plan_t *plan, uint32_t N);
 
 /* Which kernels those are: bit 0 the CUDA-core row kernel, bit 1 the tensor-core brick kernel, bit 2 the tcgen05 slab
- * kernel (16-byte aligned operands assumed).  A plan made with path auto runs products narrower than 64 columns on the
+ * kernel (on the same operands).  A plan made with path auto runs products narrower than 64 columns on the
  * row kernel alone, whatever its panels look like: there a row kernel with several rows of A per warp is the faster. */
 int cutespmm_spmm_kernels(const cutespmm_plan_t *plan, uint32_t N);
 

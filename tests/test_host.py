@@ -284,6 +284,17 @@ def test_kernels_of_a_product_by_width():
     assert auto.launch_count(32) == 1 and auto.launch_count(128) == 1 and auto.launch_count(1024) == 2
 
 
+def test_launch_count_covers_the_padded_copy_of_b():
+    """Widths no vector divides: where the matrix names rows of B often enough a kernel copies B into padded rows first, one
+    window at a time where the copy would be above 512 MiB; each window counts."""
+    mk = lambda A: cs.Plan.from_csr(A, path=cs.PATH_ROWS, host_only=True)
+    often, seldom, wide = mk(g.uniform_random(4000, 1000, 200, seed=3)), mk(g.uniform_random(4000, 1000, 4, seed=3)), mk(g.uniform_random(2000, 340000, 700, seed=3))
+    assert [often.launch_count(n) for n in (47, 48, 66, 515)] == [2, 1, 1, 4]  # 66: read two columns at a time, no copy
+    assert [seldom.launch_count(n) for n in (47, 48, 515)] == [1, 1, 2]
+    assert [wide.launch_count(n) for n in (301, 409, 412)] == [2, 4, 1]  # 409 columns are 556 MB: windows of 384 and 25
+    assert often.kernels(47) == "rows"
+
+
 def test_auto_keeps_small_matrices_on_the_row_kernel():
     """The default of path auto: dense panels go to the tensor-core kernel only when there are enough of them to fill
     its grid (4440); a small stencil stays on the row kernel, the 512 x 512 one does not."""
