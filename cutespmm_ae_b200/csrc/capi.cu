@@ -97,7 +97,7 @@ int cutespmm_plan_build_host(cutespmm_plan_t **plan, uint64_t M, uint64_t K, con
 }
 
 // What the row kernel needs to finish long rows inside the launch: per scratch slot the long row it belongs to (for
-// both work lists), one arrival counter per long row and column slab (zero between launches), and the scratch matrix.
+// both work lists), one arrival counter per long row of each list and column slab (zero between launches), and the scratch matrix.
 static cudaError_t reserve_long_row_state(cutespmm_plan *p, uint64_t &by, const char **what)
 {
     const HostPlan &h = p->host;
@@ -111,7 +111,7 @@ static cudaError_t reserve_long_row_state(cutespmm_plan *p, uint64_t &by, const 
     *what = "chunk owners";
     if ((e = upload(owners(h.chunks, h.long_rows), &p->d_chunk_owner, by)) != cudaSuccess) return e;
     if ((e = upload(owners(h.chunks_all, h.long_rows_all), &p->d_chunk_owner_all, by)) != cudaSuccess) return e;
-    const uint64_t counters = (uint64_t)std::max(h.long_rows.size(), h.long_rows_all.size()) * (kScratchCols / 32) * sizeof(uint32_t);
+    const uint64_t counters = (uint64_t)(h.long_rows.size() + h.long_rows_all.size()) * kArrivalSlabs * sizeof(uint32_t);
     if (counters) {
         *what = "arrival counters";
         if ((e = cudaMalloc(&p->d_arrivals, counters)) != cudaSuccess || (e = cudaMemset(p->d_arrivals, 0, counters)) != cudaSuccess) return e;
@@ -332,7 +332,7 @@ static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B,
     a.num_tiles = all_rows ? p->every.tiles : p->own.tiles;
     a.num_chunks = all_rows ? p->every.chunks : p->own.chunks;
     a.chunk_owner = static_cast<const uint32_t *>(all_rows ? p->d_chunk_owner_all : p->d_chunk_owner);
-    a.arrivals = p->d_arrivals;
+    a.arrivals = p->d_arrivals + (all_rows ? (uint64_t)p->own.long_rows * kArrivalSlabs : 0);
     a.split_nnz = h.opts.split_nnz;
     a.avg_row_nnz = (uint32_t)(h.nnz / std::max<uint64_t>(h.M, 1));
     a.short_chunks = item_sizes(h.nnz + kRowCost * h.M, h.nnz, h.M, 0, h.opts.split_nnz, h.opts.tile_nnz, h.adaptive_tiling).latency_bound ? 1u : 0u;
@@ -342,7 +342,8 @@ static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B,
     a.status = p->d_status;
     a.row_map = static_cast<const uint32_t *>(p->d_row_map);
     // Tiles are dealt as they are finished where there are long rows: launches of such a plan share the partial sums and must
-    // not overlap anyway; a plan without long rows may run on several streams at once and keeps nothing between launches.
+    // not overlap anyway (where they do, their results are undefined, but the counters end at zero all the same); a plan
+    // without long rows may run on several streams at once and keeps nothing between launches.
     a.counters = a.num_chunks && !rg ? p->d_status + kTileCounters : nullptr;
     a.early = h.values_on_device ? 0u : 1u;
     a.run_rows = h.run_rows;

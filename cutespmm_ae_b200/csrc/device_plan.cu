@@ -395,7 +395,7 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
 
     // ---- one block for everything ----
     const uint64_t col_words = h.brick_slots * kBrickCols + 96, rec_words = h.brick_slots * kBrickRecWords;
-    const uint64_t slots = std::max(p->own.chunks, p->every.chunks), longs = std::max(p->own.long_rows, p->every.long_rows);
+    const uint64_t slots = std::max(p->own.chunks, p->every.chunks), longs = (uint64_t)p->own.long_rows + p->every.long_rows;
     uint32_t *d_rp = nullptr, *d_owner = nullptr, *d_owner_all = nullptr, *d_bcols = nullptr, *d_brecs = nullptr, *d_first = nullptr, *d_last = nullptr, *d_ids = nullptr;
     Pair *d_pairs = nullptr;
     Tile *d_tiles = nullptr, *d_tiles_all = nullptr;
@@ -403,7 +403,7 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
     LongRow *d_longs = nullptr, *d_longs_all = nullptr;
     auto carve = [&](Carver &c) {
         c.take(p->d_status, 64);
-        c.take(p->d_arrivals, longs * (kScratchCols / 32));
+        c.take(p->d_arrivals, longs * kArrivalSlabs);
         const uint64_t zero = c.used;
         c.take(d_rp, (uint64_t)M + 1 + kRowPtrSlack);
         c.take(d_pairs, h.nnz + 2);

@@ -36,6 +36,7 @@ constexpr uint32_t kWideTileCost = 768, kMixedTileCost = 640;  // ... and with a
 constexpr uint32_t kMinChunkNnz = 32;             // smallest piece of a cut row
 constexpr uint32_t kMaxSplitNnz = 384;   // a row must fit a tile together with a part-filled one
 constexpr uint32_t kScratchCols = 512;  // widest N one launch handles; wider products run in column windows
+constexpr uint32_t kArrivalSlabs = kScratchCols / 32;  // arrival counters of a long row: one per column slab of the narrowest kind
 
 // One nonzero as the row kernel reads it: column index and fp32 bit pattern side by side (8 bytes,
 // one coalesced 64-bit load per lane).

@@ -11,7 +11,7 @@
 
 #include "plan.hpp"
 
-// The 256-byte status block: word 0 the status, words kTileCounters... the row kernel's counters (blocks done, tiles per slab).
+// The 256-byte status block: word 0 the status, words kTileCounters... the row kernel's counters (RowsArgs::counters).
 constexpr uint32_t kTileCounters = 16;
 
 // A contiguous range of the plan's work items (tiles and chunks of the row kernel -- of its own list and
@@ -63,7 +63,7 @@ struct cutespmm_plan {
     void *d_scols = nullptr, *d_srecs = nullptr, *d_srec_off = nullptr, *d_sfirst = nullptr, *d_slast = nullptr, *d_sids = nullptr;
     void *d_row_map = nullptr;
     void *d_chunk_owner = nullptr, *d_chunk_owner_all = nullptr;  // per scratch slot: its long row
-    uint32_t *d_arrivals = nullptr;                               // per long row and column slab: chunks finished
+    uint32_t *d_arrivals = nullptr;  // per long row (of the own list, then of the list of every row) and column slab: chunks finished
     float *d_scratch = nullptr;
     uint32_t *d_status = nullptr;
     // staging for the host-buffer call

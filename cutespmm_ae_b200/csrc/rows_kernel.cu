@@ -19,6 +19,7 @@
 #include <cstdint>
 
 #include "device_plan.hpp"
+#include "last_block.cuh"
 #include "plan.hpp"
 #include "ptx.cuh"
 #include "tile_stage.cuh"
@@ -327,9 +328,10 @@ __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
                 owner = __ldg(a.chunk_owner + ck.w);
                 lr = __ldg(a.long_rows + owner);
             }
-            uint32_t *cnt = a.arrivals + (uint64_t)owner * gridDim.y + blockIdx.y;
-            if (atomicAdd(cnt, 1u) == lr.z - lr.y - 1) {  // every chunk of this row and column slab has arrived
-                *cnt = 0;                                  // ready for the next launch
+            // the counter of this row and column slab runs through 0 .. chunks - 1 and wraps: it is back at zero for the next launch,
+            // also after launches of this list that overlapped (each adds as many as there are chunks, whatever its grid)
+            uint32_t *cnt = a.arrivals + (uint64_t)owner * kArrivalSlabs + blockIdx.y;
+            if (atomicInc(cnt, lr.z - lr.y - 1) == lr.z - lr.y - 1) {  // every chunk has arrived
                 __threadfence();
                 lr_row = lr.x; slot0 = lr.y; slot1 = lr.z;
             }
@@ -446,14 +448,10 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DYN, G))
         }
         tile_release<DYN>(ring, src, i, t, lane);  // the last warp to leave the stage refills it
     }
-    if (DYN) {  // the last block to leave puts the tile counters back for the next launch
+    if (DYN) {
         __syncthreads();
-        if (threadIdx.x == 0) {
-            const uint32_t blocks = gridDim.x * gridDim.y;
-            __threadfence();
-            if (atomicInc(a.counters, blocks - 1) == blocks - 1)
-                for (uint32_t y = 0; y < gridDim.y; ++y) a.counters[1 + y] = 0;
-        }
+        if (threadIdx.x == 0 && last_block_out(a.counters))
+            for (uint32_t y = 0; y < kDealtSlabs; ++y) a.counters[1 + y] = 0;
     }
 }
 
@@ -488,9 +486,9 @@ cudaError_t launch_rows_t(RowsArgs a, uint32_t slabs, int sm_count, cudaStream_t
     int n = 0;
     cudaError_t e;
     if constexpr (VEC == 4)
-        if (a.counters) {  // tiles dealt by a counter: where there are enough to deal
+        if (a.counters && slabs <= kDealtSlabs) {  // tiles dealt by a counter: where there are enough to deal
             if ((e = blocks_per_sm<VEC, CH, FULL, DEEP, G, true>(n)) != cudaSuccess) return e;
-            if (a.num_tiles >= 8ull * grid(n)) 
+            if (a.num_tiles >= 8ull * grid(n))
                 return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true>, dim3(grid(n), slabs), kWarps * 32, 0, s, a);
         }
     if ((e = blocks_per_sm<VEC, CH, FULL, DEEP, G, false>(n)) != cudaSuccess) return e;

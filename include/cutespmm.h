@@ -186,7 +186,12 @@ int cutespmm_plan_decode_csr(const cutespmm_plan_t *plan, uint64_t *rowPtr, uint
  * at a time (wider products go in column windows), which is taken from the library's stream-ordered pool (the one
  * cutespmm_plan_create_device uses) and given back on the stream within the call.  Without memory for it, and
  * while the stream is being captured, the kernel reads B as it is: the same result, more slowly.  A caller that wants no
- * allocation at all keeps rows of B that are 16-byte aligned. */
+ * allocation at all keeps rows of B that are 16-byte aligned.
+ *
+ * Products of one plan may overlap (on several streams, from several threads) where the plan has no long rows
+ * (cutespmm_plan_info_t::num_long_rows, and none among the tensor-core panels' rows).  The others share the plan's partial sums
+ * and counters and have to be ordered, on one stream or with events: what overlapping ones write is not defined, in any row
+ * of C, and nothing reports it; products queued after them are not affected. */
 int cutespmm_spmm(const cutespmm_plan_t *plan, const float *B_dev, uint64_t ldb, float *C_dev,
                   uint64_t ldc, uint32_t N, void *stream);
 

@@ -529,3 +529,43 @@ def test_product_waits_for_nothing_without_memory_for_a_padded_copy(oracle_mod):
     ref = oracle_mod.spmm_csr_rows(A.row_ptr, A.cols, A.vals, B.cpu().numpy(), rows)
     assert oracle_mod.rel_fro(ref, C[torch.from_numpy(rows).cuda()].cpu().numpy()) <= REL_FRO_TOL_FP32
     assert p.device_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["tiles_dealt", "two_lists"])
+def test_products_after_overlapping_ones_are_whole(oracle_mod, kind):
+    """Products of a plan with long rows that overlap on two streams are undefined, but what they leave behind is not: the
+    counters of arrived chunks and of dealt tiles are back at zero, whatever the widths (grids, column slabs, work lists)."""
+    rng = np.random.default_rng(15)
+    if kind == "tiles_dealt":
+        ln = rng.integers(0, 6, 900_000)
+        ln[rng.choice(ln.size, 300, replace=False)] = 900
+        rp = np.concatenate([[0], np.cumsum(ln)])
+        A = g.CsrMatrix(ln.size, 5000, torch.from_numpy(rp), torch.from_numpy(rng.integers(0, 5000, rp[-1]).astype(np.int32)),
+                        torch.from_numpy(rng.standard_normal(rp[-1]).astype(np.float32)))
+        kw, widths, tol = dict(path=cs.PATH_ROWS), (32, 300), REL_FRO_TOL_FP32
+    else:  # brick panels beside long rows: N = 128 runs the rows the bricks leave, N = 33 every row
+        S = g.stencil9(120)
+        rows = [S.cols[S.row_ptr[r] : S.row_ptr[r + 1]].numpy() for r in range(S.M)]
+        for r in range(40, S.M, 997):
+            rows[r] = np.sort(rng.choice(S.K, 400 + r % 300, replace=False))
+        rp = np.concatenate([[0], np.cumsum([len(c) for c in rows])])
+        A = g.CsrMatrix(S.M, S.K, torch.from_numpy(rp), torch.from_numpy(np.concatenate(rows).astype(np.int32)),
+                        torch.from_numpy(rng.standard_normal(rp[-1]).astype(np.float32)))
+        kw, widths, tol = dict(), (128, 33), REL_FRO_TOL
+    p = cs.Plan.from_device_csr(A.M, A.K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), **kw)
+    assert p.info()["num_long_rows"] > 0 and (kind == "tiles_dealt") == (p.info()["num_bricks"] == 0)
+    Bs = [g.dense_operand(A.K, N, 16, device="cuda") for N in widths]
+    Cs = [torch.empty((A.M, N), device="cuda") for N in widths]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for B, C, s in zip(Bs, Cs, streams):
+            p.spmm(B, C, stream=s)
+    torch.cuda.synchronize()
+    for B, C in zip(Bs, Cs):
+        want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.cpu().numpy(), A.M, A.K)
+        for _ in range(2):
+            C.fill_(float("nan"))
+            p.spmm(B, C)
+            assert oracle_mod.rel_fro(want, C.cpu().numpy()) <= tol
+    assert p.device_status() == 0
