@@ -333,7 +333,6 @@ static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B,
     a.num_chunks = all_rows ? p->every.chunks : p->own.chunks;
     a.chunk_owner = static_cast<const uint32_t *>(all_rows ? p->d_chunk_owner_all : p->d_chunk_owner);
     a.arrivals = p->d_arrivals + (all_rows ? (uint64_t)p->own.long_rows * kArrivalSlabs : 0);
-    a.split_nnz = h.opts.split_nnz;
     a.avg_row_nnz = (uint32_t)(h.nnz / std::max<uint64_t>(h.M, 1));
     a.short_chunks = item_sizes(h.nnz + kRowCost * h.M, h.nnz, h.M, 0, h.opts.split_nnz, h.opts.tile_nnz, h.adaptive_tiling).latency_bound ? 1u : 0u;
     a.B = B; a.C = C; a.scratch = p->d_scratch;

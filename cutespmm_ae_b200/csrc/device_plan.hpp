@@ -54,7 +54,7 @@ struct RowsArgs {
     uint32_t *arrivals;        // per long row of the list kArrivalSlabs counters: chunks finished so far (zero between launches)
     uint32_t *counters;        // balance of the blocks that left, then tiles dealt per column slab (kDealtSlabs of them); zero between
                                // launches.  nullptr: tiles in fixed turns
-    uint32_t num_tiles, num_chunks, split_nnz;
+    uint32_t num_tiles, num_chunks;
     uint32_t avg_row_nnz;      // nonzeros per row of the whole matrix (picks the kernel's tuning)
     uint32_t short_chunks;     // 1: a small job, its long rows are cut into pieces of tens of nonzeros
     const float *B;            // K x N window, leading dimension ldb
@@ -76,7 +76,6 @@ cudaError_t launch_block_rows(const RowsArgs &a, int sm_count, cudaStream_t s);
 cudaError_t launch_rows(const RowsArgs &a, int sm_count, cudaStream_t s);
 // dst: rows x (N rounded up to 4) floats, 16-byte aligned
 cudaError_t launch_pad_rows(const float *src, uint64_t ld_src, float *dst, uint64_t rows, uint32_t N, int sm_count, cudaStream_t s);
-int rows_kernel_count(const RowsArgs &a);
 
 // Arguments of the SDDMM kernel (sddmm_kernel.cu): out[j] = (scale ? value of nonzero j : 1) * <X[row of j], Y[column of j]>.
 struct SddmmArgs {

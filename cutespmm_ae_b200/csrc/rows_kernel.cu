@@ -534,8 +534,6 @@ cudaError_t launch_pad_rows(const float *src, uint64_t ld_src, float *dst, uint6
     return launch_overlapped(pad_rows_kernel, (uint32_t)(want < cap ? want : cap), 256, 0, s, src, ld_src, reinterpret_cast<float4 *>(dst), quads, N, rows);
 }
 
-int rows_kernel_count(const RowsArgs &a) { return (a.num_tiles || a.num_chunks) ? 1 : 0; }
-
 // Picks the widest vector the pointers, leading dimensions and N allow.
 cudaError_t launch_rows(const RowsArgs &args, int sm_count, cudaStream_t s)
 {
