@@ -292,27 +292,50 @@ void *named_stream(PyObject *o)
     return s ? s : reinterpret_cast<void *>(0x1);  // cudaStreamLegacy
 }
 
+// fn without the interpreter lock, as ctypes makes its calls: a launch that waits for room in its stream's queue must not hold
+// up other threads, and threads that drive a stream each run side by side.  The calls below take their arguments out of
+// Python first and hold references of their own to the tensors.
+template <class Fn> auto without_gil(Fn &&fn)
+{
+    struct Released {
+        PyThreadState *state = PyEval_SaveThread();
+        ~Released() { PyEval_RestoreThread(state); }
+    } released;
+    return fn();
+}
+
 PyObject *py_spmm(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     HANDLE_TH_ERRORS
     want_args(n, 6);  // plan, M, K, B, C or None, stream or None
-    return THPVariable_Wrap(run_spmm(static_cast<cutespmm_plan_t *>(pointer(a[0])), integer(a[1]), integer(a[2]), tensor(a[3], "B"),
-                                     tensor_or_none(a[4], "C"), named_stream(a[5])));
+    auto *plan = static_cast<cutespmm_plan_t *>(pointer(a[0]));
+    const int64_t M = integer(a[1]), K = integer(a[2]);
+    const Tensor B = tensor(a[3], "B"), C = tensor_or_none(a[4], "C");
+    void *s = named_stream(a[5]);
+    return THPVariable_Wrap(without_gil([&] { return run_spmm(plan, M, K, B, C, s); }));
     END_HANDLE_TH_ERRORS
 }
 PyObject *py_sddmm(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     HANDLE_TH_ERRORS
     want_args(n, 9);  // plan, M, K, nnz, X, Y, out or None, scale, stream or None
-    return THPVariable_Wrap(run_sddmm(static_cast<cutespmm_plan_t *>(pointer(a[0])), integer(a[1]), integer(a[2]), integer(a[3]), tensor(a[4], "X"),
-                                      tensor(a[5], "Y"), tensor_or_none(a[6], "out"), PyObject_IsTrue(a[7]) == 1, named_stream(a[8])));
+    auto *plan = static_cast<cutespmm_plan_t *>(pointer(a[0]));
+    const int64_t M = integer(a[1]), K = integer(a[2]), nnz = integer(a[3]);
+    const Tensor X = tensor(a[4], "X"), Y = tensor(a[5], "Y"), o = tensor_or_none(a[6], "out");
+    const bool scale = PyObject_IsTrue(a[7]) == 1;
+    void *s = named_stream(a[8]);
+    return THPVariable_Wrap(without_gil([&] { return run_sddmm(plan, M, K, nnz, X, Y, o, scale, s); }));
     END_HANDLE_TH_ERRORS
 }
 PyObject *py_set_values(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     HANDLE_TH_ERRORS
     want_args(n, 4);  // plan, nnz, vals, stream or None
-    run_set_values(static_cast<cutespmm_plan_t *>(pointer(a[0])), integer(a[1]), tensor(a[2], "vals"), Tensor(), named_stream(a[3]));
+    auto *plan = static_cast<cutespmm_plan_t *>(pointer(a[0]));
+    const int64_t nnz = integer(a[1]);
+    const Tensor vals = tensor(a[2], "vals");
+    void *s = named_stream(a[3]);
+    without_gil([&] { run_set_values(plan, nnz, vals, Tensor(), s); });
     Py_RETURN_NONE;
     END_HANDLE_TH_ERRORS
 }
@@ -321,7 +344,7 @@ PyObject *py_noalloc(PyObject *, PyObject *const *a, Py_ssize_t n)
     HANDLE_TH_ERRORS
     want_args(n, 8);  // M, K, row_ptr, cols, vals, B, C, stream or None
     const int64_t M = integer(a[0]), K = integer(a[1]);
-    const Tensor &rp = tensor(a[2], "row_ptr"), &cols = tensor(a[3], "cols"), &vals = tensor(a[4], "vals"), &B = tensor(a[5], "B"), &C = tensor(a[6], "C");
+    const Tensor rp = tensor(a[2], "row_ptr"), cols = tensor(a[3], "cols"), vals = tensor(a[4], "vals"), B = tensor(a[5], "B"), C = tensor(a[6], "C");
     auto is = [](const Tensor &t, at::ScalarType dt) { return t.is_cuda() && t.scalar_type() == dt; };
     TORCH_CHECK_VALUE(is(rp, at::kInt) && is(cols, at::kInt) && is(vals, at::kFloat) && is(B, at::kFloat) && is(C, at::kFloat),
                       "all operands must be CUDA tensors: row_ptr/cols int32, vals/B/C float32");
@@ -336,9 +359,11 @@ PyObject *py_noalloc(PyObject *, PyObject *const *a, Py_ssize_t n)
     TORCH_CHECK_VALUE(rp.device() == B.device() && cols.device() == B.device() && vals.device() == B.device() && C.device() == B.device(),
                       "all operands must live on one device");
     void *s = named_stream(a[7]);
-    check_status(cutespmm_spmm_csr_noalloc((uint32_t)M, (uint32_t)K, (uint32_t)cols.numel(), static_cast<const uint32_t *>(rp.const_data_ptr()),
-                                           static_cast<const uint32_t *>(cols.const_data_ptr()), in(vals), in(B), ld(B, K), out(C), ld(C, M), (uint32_t)N,
-                                           s ? s : stream_of(B)));
+    without_gil([&] {
+        check_status(cutespmm_spmm_csr_noalloc((uint32_t)M, (uint32_t)K, (uint32_t)cols.numel(), static_cast<const uint32_t *>(rp.const_data_ptr()),
+                                               static_cast<const uint32_t *>(cols.const_data_ptr()), in(vals), in(B), ld(B, K), out(C), ld(C, M),
+                                               (uint32_t)N, s ? s : stream_of(B)));
+    });
     Py_INCREF(a[6]);
     return a[6];
     END_HANDLE_TH_ERRORS
@@ -349,21 +374,28 @@ PyObject *py_op_spmm(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     HANDLE_TH_ERRORS
     want_args(n, 2);
-    return THPVariable_Wrap(call_spmm(integer(a[0]), tensor(a[1], "B")));
+    const int64_t id = integer(a[0]);
+    const Tensor B = tensor(a[1], "B");
+    return THPVariable_Wrap(without_gil([&] { return call_spmm(id, B); }));
     END_HANDLE_TH_ERRORS
 }
 PyObject *py_op_weighted(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     HANDLE_TH_ERRORS
     want_args(n, 3);
-    return THPVariable_Wrap(call_spmm_weighted(integer(a[0]), tensor(a[1], "w"), tensor(a[2], "B")));
+    const int64_t id = integer(a[0]);
+    const Tensor w = tensor(a[1], "w"), B = tensor(a[2], "B");
+    return THPVariable_Wrap(without_gil([&] { return call_spmm_weighted(id, w, B); }));
     END_HANDLE_TH_ERRORS
 }
 PyObject *py_op_sddmm(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     HANDLE_TH_ERRORS
     want_args(n, 4);
-    return THPVariable_Wrap(call_sddmm(integer(a[0]), tensor(a[1], "X"), tensor(a[2], "Y"), PyObject_IsTrue(a[3]) == 1));
+    const int64_t id = integer(a[0]);
+    const Tensor X = tensor(a[1], "X"), Y = tensor(a[2], "Y");
+    const bool scale = PyObject_IsTrue(a[3]) == 1;
+    return THPVariable_Wrap(without_gil([&] { return call_sddmm(id, X, Y, scale); }));
     END_HANDLE_TH_ERRORS
 }
 

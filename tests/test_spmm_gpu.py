@@ -569,3 +569,44 @@ def test_products_after_overlapping_ones_are_whole(oracle_mod, kind):
             p.spmm(B, C)
             assert oracle_mod.rel_fro(want, C.cpu().numpy()) <= tol
     assert p.device_status() == 0
+
+
+@pytest.mark.parametrize("call", ["spmm", "sddmm", "set_values", "noalloc", "operator"])
+def test_calls_leave_the_interpreter_to_other_threads(call):
+    """A call whose stream's queue is full waits in the driver until the GPU has made room.  It waits without the interpreter
+    lock: another thread goes on all the while."""
+    import threading
+    import time
+
+    from cutespmm_ae_b200 import torch_ops
+
+    A = g.uniform_random(64, 48, 4, seed=17)
+    csr = A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda()
+    plan = cs.Plan.from_device_csr(A.M, A.K, *csr, path=cs.PATH_ROWS)
+    op = torch_ops.SparseOperator(plan)
+    B, C, out = torch.randn(A.K, 32, device="cuda"), torch.randn(A.M, 32, device="cuda"), torch.empty(A.nnz, device="cuda")
+    run = {"spmm": lambda: plan.spmm(B, C), "sddmm": lambda: plan.sddmm(C, B, out), "set_values": lambda: plan.set_values(csr[2]),
+           "noalloc": lambda: cs.spmm_csr_noalloc(A.M, A.K, *csr, B, C), "operator": lambda: op(B)}[call]
+    run()
+    torch.cuda.synchronize()
+    stream, times = torch.cuda.Stream(), []
+
+    def fill():
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(1_000_000_000)  # half a second of GPU time
+            for _ in range(4000):  # more launches than a queue holds
+                t = time.perf_counter()
+                run()
+                times.append(time.perf_counter() - t)
+
+    worker = threading.Thread(target=fill)
+    longest, last = 0.0, time.perf_counter()
+    worker.start()
+    while worker.is_alive():
+        now = time.perf_counter()
+        longest, last = max(longest, now - last), now
+        time.sleep(0.001)
+    torch.cuda.synchronize()
+    assert max(times) > 0.2  # the queue did fill up
+    assert longest < 0.1 * max(times), (longest, max(times))
+    op.close()
