@@ -126,12 +126,17 @@ std::shared_ptr<OpState> get_op(int64_t id)
     return it->second;
 }
 
-// The plan of A^T, built through the Python object on first use.
-void need_transposed(OpState &op, bool with_order)
+// The plan of A^T (and the order), built through the Python object on first use; two threads that ask at once get the same one
+// (the object's lock).
+struct Transposed {
+    cutespmm_plan_t *plan;
+    Tensor order;
+};
+Transposed need_transposed(OpState &op, bool with_order)
 {
     {
         std::lock_guard<std::mutex> lock(g_ops_mutex);
-        if (op.transposed && (!with_order || op.order.defined())) return;
+        if (op.transposed && (!with_order || op.order.defined())) return {op.transposed, op.order};
     }
     PyGILState_STATE g = PyGILState_Ensure();
     PyObject *r = PyObject_CallFunction(op.build, "i", with_order ? 1 : 0);
@@ -143,7 +148,9 @@ void need_transposed(OpState &op, bool with_order)
     }
     Py_DECREF(r);
     PyGILState_Release(g);
-    TORCH_CHECK(op.transposed, "cutespmm: the plan of A^T could not be built");
+    std::lock_guard<std::mutex> lock(g_ops_mutex);
+    TORCH_CHECK(op.transposed && (!with_order || op.order.defined()), "cutespmm: the plan of A^T could not be built");
+    return {op.transposed, op.order};
 }
 
 Tensor unit_stride(const Tensor &t) { return t.dim() > 0 && t.stride(-1) == 1 ? t : t.contiguous(); }
@@ -156,8 +163,7 @@ Tensor op_spmm(int64_t id, const Tensor &B)
 Tensor op_spmm_transposed(int64_t id, const Tensor &G)
 {
     auto op = get_op(id);
-    need_transposed(*op, false);
-    return run_spmm(op->transposed, op->K, op->M, unit_stride(G), Tensor(), nullptr);
+    return run_spmm(need_transposed(*op, false).plan, op->K, op->M, unit_stride(G), Tensor(), nullptr);
 }
 Tensor op_spmm_weighted(int64_t id, const Tensor &w, const Tensor &B)
 {
@@ -168,9 +174,9 @@ Tensor op_spmm_weighted(int64_t id, const Tensor &w, const Tensor &B)
 Tensor op_spmm_weighted_transposed(int64_t id, const Tensor &w, const Tensor &G)
 {
     auto op = get_op(id);
-    need_transposed(*op, true);
-    run_set_values(op->transposed, op->nnz, w.contiguous(), op->order, nullptr);
-    return run_spmm(op->transposed, op->K, op->M, unit_stride(G), Tensor(), nullptr);
+    const Transposed t = need_transposed(*op, true);
+    run_set_values(t.plan, op->nnz, w.contiguous(), t.order, nullptr);
+    return run_spmm(t.plan, op->K, op->M, unit_stride(G), Tensor(), nullptr);
 }
 Tensor op_sddmm(int64_t id, const Tensor &X, const Tensor &Y, bool scale)
 {

@@ -21,6 +21,7 @@ permutation computed once) and dw = sddmm(dC, B).
 from __future__ import annotations
 
 import itertools
+import threading
 import weakref
 
 import numpy as np
@@ -58,6 +59,7 @@ class SparseOperator:
         self._plan_kwargs = plan_kwargs or {}
         self._transposed: Plan | None = None
         self._t_perm: torch.Tensor | None = None  # storage position in A of every stored position of A^T (int32)
+        self._t_lock = threading.RLock()  # around the two: backward passes of several threads may ask for them at once
         self.id = next(_ids)
         _plans[self.id] = self
         weakref.finalize(self, _plans.pop, self.id, None)
@@ -65,38 +67,42 @@ class SparseOperator:
         plan.__dict__.setdefault("_op_ids", []).append(self.id)
 
     def transposed(self) -> Plan:
-        if self._transposed is None:
-            self._make_transposed(False)
+        self._make_transposed(False)
         return self._transposed
 
     def _make_transposed(self, with_order: bool) -> None:
         """Builds what is missing of the plan of A^T and the order its stored positions have in A, and hands both to the
         native operators.  On the device where the plan's options and layout allow it."""
-        on_device = self._plan_kwargs.get("path", 0) != PATH_SLAB and not set(self._plan_kwargs) - {"path", "split_nnz", "tile_nnz", "min_brick_panels"}
-        csr = None
-        if on_device:
-            try:
-                csr = self.plan.csr_device()
-            except CuteSpmmError:  # rows reordered, or a host-only plan
-                csr = None
-        if csr is not None:
-            rp, cols, vals = csr
-            _, order = torch.sort(cols.to(torch.int64) & 0xFFFFFFFF, stable=True)
-            if self._transposed is None:
-                rows = torch.repeat_interleave(torch.arange(self.M, dtype=torch.int32, device=cols.device), (rp[1:] - rp[:-1]).to(torch.int64), output_size=self.nnz)
-                t_rp = torch.zeros(self.K + 1, dtype=torch.int64, device=cols.device)
-                torch.cumsum(torch.bincount(cols.to(torch.int64) & 0xFFFFFFFF, minlength=self.K), 0, out=t_rp[1:])
-                self._transposed = Plan.from_device_csr(self.K, self.M, t_rp.to(torch.int32), rows[order], vals[order], **self._plan_kwargs)
-            if with_order and self._t_perm is None:
-                self._t_perm = order.to(torch.int32)
-        else:
-            rp, cols, vals = self.plan.decode_csr()
-            if self._transposed is None:
-                t_rp, t_cols, t_vals = transpose_csr(self.M, self.K, rp, cols, vals)
-                self._transposed = Plan(self.K, self.M, t_rp, t_cols, t_vals, **self._plan_kwargs)
-            if with_order and self._t_perm is None:
-                self._t_perm = torch.from_numpy(np.argsort(np.asarray(cols, dtype=np.int64), kind="stable").astype(np.uint32).view(np.int32)).cuda()
-        _native.set_transposed(self.id, self._transposed._h.value, self._t_perm)
+        with self._t_lock:
+            if self._transposed is not None and (self._t_perm is not None or not with_order):
+                return
+            on_device = self._plan_kwargs.get("path", 0) != PATH_SLAB and not set(self._plan_kwargs) - {"path", "split_nnz", "tile_nnz", "min_brick_panels"}
+            csr = None
+            if on_device:
+                try:
+                    csr = self.plan.csr_device()
+                except CuteSpmmError:  # rows reordered, or a host-only plan
+                    csr = None
+            if csr is not None:
+                rp, cols, vals = csr
+                _, order = torch.sort(cols.to(torch.int64) & 0xFFFFFFFF, stable=True)
+                if self._transposed is None:
+                    rows = torch.repeat_interleave(torch.arange(self.M, dtype=torch.int32, device=cols.device), (rp[1:] - rp[:-1]).to(torch.int64), output_size=self.nnz)
+                    t_rp = torch.zeros(self.K + 1, dtype=torch.int64, device=cols.device)
+                    torch.cumsum(torch.bincount(cols.to(torch.int64) & 0xFFFFFFFF, minlength=self.K), 0, out=t_rp[1:])
+                    self._transposed = Plan.from_device_csr(self.K, self.M, t_rp.to(torch.int32), rows[order], vals[order], **self._plan_kwargs)
+                if with_order and self._t_perm is None:
+                    self._t_perm = order.to(torch.int32)
+                    if not torch.cuda.is_current_stream_capturing():
+                        torch.cuda.current_stream(cols.device).synchronize()  # the next user may be on another stream
+            else:
+                rp, cols, vals = self.plan.decode_csr()
+                if self._transposed is None:
+                    t_rp, t_cols, t_vals = transpose_csr(self.M, self.K, rp, cols, vals)
+                    self._transposed = Plan(self.K, self.M, t_rp, t_cols, t_vals, **self._plan_kwargs)
+                if with_order and self._t_perm is None:
+                    self._t_perm = torch.from_numpy(np.argsort(np.asarray(cols, dtype=np.int64), kind="stable").astype(np.uint32).view(np.int32)).cuda()
+            _native.set_transposed(self.id, self._transposed._h.value, self._t_perm)
 
     def __call__(self, B: torch.Tensor) -> torch.Tensor:
         if torch.compiler.is_compiling():
@@ -117,10 +123,11 @@ class SparseOperator:
         """New values for the same pattern (Plan.set_values), e.g. normalised `sddmm` scores as attention weights.  The
         plan of A^T, if a backward pass has built one, is dropped and rebuilt from the new values on next use."""
         self.plan.set_values(vals)
-        if self._transposed is not None:
-            _native.set_transposed(self.id, None, self._t_perm)
-            self._transposed.close()
-            self._transposed = None
+        with self._t_lock:
+            if self._transposed is not None:
+                _native.set_transposed(self.id, None, self._t_perm)
+                self._transposed.close()
+                self._transposed = None
 
     def close(self) -> None:
         _plans.pop(self.id, None)

@@ -108,3 +108,43 @@ def test_weighted_product_is_differentiable_in_the_weights_and_in_b():
                           (op.id, w.detach().clone().requires_grad_(True), B.detach().clone().requires_grad_(True)),
                           test_utils=("test_schema", "test_faketensor", "test_autograd_registration"))
     op.close()
+
+
+@pytest.mark.gpu
+def test_threads_that_need_the_transposed_plan_at_once_share_one(monkeypatch):
+    """The plan of A^T is built on first use, without the interpreter lock: of two threads that come to need it together
+    one builds it and the other waits for that one (a second plan would replace, and destroy, the one in use)."""
+    import threading
+    import time
+
+    A = g.rmat(9, 8, seed=41, values="uniform")
+    op = torch_ops.SparseOperator(cs.Plan.from_csr(A, path=cs.PATH_ROWS), plan_kwargs=dict(path=cs.PATH_ROWS))
+    built, make = [], cs.Plan.from_device_csr
+
+    def slowly(*a, **kw):
+        time.sleep(0.2)
+        built.append(make(*a, **kw))
+        return built[-1]
+
+    monkeypatch.setattr(cs.Plan, "from_device_csr", slowly)
+    G, out = g.dense_operand(A.M, 32, 42, device="cuda"), [None, None]
+    torch.cuda.synchronize()
+    start = threading.Barrier(2)
+
+    def multiply(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            start.wait()
+            out[i] = torch.ops.cutespmm.spmm_transposed(op.id, G)
+
+    threads = [threading.Thread(target=multiply, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert len(built) == 1
+    want = torch.zeros(A.K, A.M, device="cuda")
+    want[A.cols.long().cuda(), torch.repeat_interleave(torch.arange(A.M), A.row_ptr[1:] - A.row_ptr[:-1]).cuda()] = A.vals.cuda()
+    for C in out:
+        assert torch.allclose(C, want @ G, rtol=1e-4, atol=1e-4)
+    op.close()
