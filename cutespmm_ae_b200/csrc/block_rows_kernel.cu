@@ -115,13 +115,9 @@ __global__ void __launch_bounds__(kTileWarps * 32, 4) spmm_block_rows_kernel(Row
 
 template <int R, int G> cudaError_t launch_t(const RowsArgs &a, int sm_count, cudaStream_t s)
 {
-    static int per_sm = 0;  // same for every device of one model; queried once
-    if (per_sm == 0) {
-        int n = 0;
-        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, spmm_block_rows_kernel<R, G>, kTileWarps * 32, 0);
-        if (e != cudaSuccess) return e;
-        per_sm = n > 0 ? n : 1;
-    }
+    int per_sm = 0;
+    const cudaError_t e = blocks_per_sm<spmm_block_rows_kernel<R, G>>(per_sm, kTileWarps * 32);
+    if (e != cudaSuccess) return e;
     const uint32_t slabs = (a.N + 127) / 128, wave = (uint32_t)(sm_count * per_sm);
     uint32_t gx = a.num_tiles < wave ? a.num_tiles : wave;
     if (slabs > 1) gx = (gx + slabs - 1) / slabs;

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 namespace cutespmm {
@@ -13,7 +14,7 @@ namespace cutespmm {
 template <auto Kernel> cudaError_t allow_dynamic_smem(int bytes)
 {
     constexpr int kMaxDevices = 64;
-    static bool done[kMaxDevices] = {};
+    static std::atomic<bool> done[kMaxDevices] = {};  // several threads may come here at once: each sets the same
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -21,6 +22,19 @@ template <auto Kernel> cudaError_t allow_dynamic_smem(int bytes)
     e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess && dev >= 0 && dev < kMaxDevices) done[dev] = true;
     return e;
+}
+
+// Blocks of `threads` threads of a kernel that an SM holds: the same for every device of one model, so asked once per kernel.
+// Several threads may come here at once: each asks for and stores the same.
+template <auto Kernel> cudaError_t blocks_per_sm(int &n, int threads)
+{
+    static std::atomic<int> known{0};
+    if ((n = known) != 0) return cudaSuccess;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, Kernel, threads, 0);
+    if (e != cudaSuccess) return e;
+    if (n < 1) n = 1;
+    known = n;
+    return cudaSuccess;
 }
 
 // Launches a kernel whose blocks may be set up while the kernel in front of it on the stream still runs (the kernel calls

@@ -455,20 +455,6 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DYN, G))
     }
 }
 
-template <int VEC, int CH, bool FULL, bool DEEP, int G, bool DYN>
-cudaError_t blocks_per_sm(int &n)
-{
-    static int known = 0;  // same for every device of one model; queried once
-    if (known == 0) {
-        int got = 0;
-        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&got, spmm_rows_kernel<VEC, CH, FULL, DEEP, G, DYN>, kWarps * 32, 0);
-        if (e != cudaSuccess) return e;
-        known = got > 0 ? got : 1;
-    }
-    n = known;
-    return cudaSuccess;
-}
-
 template <int VEC, int CH, bool FULL, bool DEEP, int G = 1>
 cudaError_t launch_rows_t(RowsArgs a, uint32_t slabs, int sm_count, cudaStream_t s)
 {
@@ -487,11 +473,11 @@ cudaError_t launch_rows_t(RowsArgs a, uint32_t slabs, int sm_count, cudaStream_t
     cudaError_t e;
     if constexpr (VEC == 4)
         if (a.counters && slabs <= kDealtSlabs) {  // tiles dealt by a counter: where there are enough to deal
-            if ((e = blocks_per_sm<VEC, CH, FULL, DEEP, G, true>(n)) != cudaSuccess) return e;
+            if ((e = blocks_per_sm<spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true>>(n, kWarps * 32)) != cudaSuccess) return e;
             if (a.num_tiles >= 8ull * grid(n))
                 return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true>, dim3(grid(n), slabs), kWarps * 32, 0, s, a);
         }
-    if ((e = blocks_per_sm<VEC, CH, FULL, DEEP, G, false>(n)) != cudaSuccess) return e;
+    if ((e = blocks_per_sm<spmm_rows_kernel<VEC, CH, FULL, DEEP, G, false>>(n, kWarps * 32)) != cudaSuccess) return e;
     return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, false>, dim3(grid(n), slabs), kWarps * 32, 0, s, a);
 }
 

@@ -241,13 +241,9 @@ __global__ void __launch_bounds__(kTileWarps * 32, FLAT || V < 3 ? 4 : 3) sddmm_
 
 template <int LANES, int V, bool VEC4, bool FULL, bool FLAT> cudaError_t launch_sddmm_t(const SddmmArgs &a, int sm_count, cudaStream_t s)
 {
-    static int per_sm = 0;  // same for every device of one model; queried once
-    if (per_sm == 0) {
-        int n = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sddmm_kernel<LANES, V, VEC4, FULL, FLAT>, kTileWarps * 32, 0);
-        if (e != cudaSuccess) return e;
-        per_sm = n > 0 ? n : 1;
-    }
+    int per_sm = 0;
+    const cudaError_t e = blocks_per_sm<sddmm_kernel<LANES, V, VEC4, FULL, FLAT>>(per_sm, kTileWarps * 32);
+    if (e != cudaSuccess) return e;
     const uint32_t chunk_blocks = (a.num_chunks + kTileWarps - 1) / kTileWarps;
     uint32_t blocks = a.num_tiles > chunk_blocks ? a.num_tiles : chunk_blocks;
     const uint32_t cap = (uint32_t)(sm_count * per_sm);  // one resident wave
