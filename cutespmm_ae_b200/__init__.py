@@ -112,8 +112,23 @@ def _load() -> C.CDLL:
     return lib
 
 
+def _build_bind_if_stale() -> None:
+    """The binding on torch tensors is built where the library is, when the package is imported, so that no product compiles
+    anything.  A machine without torch or a compiler keeps what is there."""
+    if importlib.util.find_spec("torch") is None:
+        return
+    try:
+        if _build.bind_stale():
+            _build.build_bind()
+    except Exception as e:  # reported by the first call that needs the binding
+        global _bind_error
+        _bind_error = e
+
+
 lib = _load()
 _bind = None  # the native binding on torch tensors (csrc/torch_bind.cpp), loaded with the first call that needs it
+_bind_error = None
+_build_bind_if_stale()
 
 
 def _native():
@@ -121,7 +136,9 @@ def _native():
     if _bind is None:
         import torch  # noqa: F401 -- its libraries first
 
-        path = _build.build_bind()
+        path = _build.BIND
+        if _build.bind_stale():
+            raise RuntimeError(f"{path} is missing or does not belong to this torch: run python -m cutespmm_ae_b200._build") from _bind_error
         loader = importlib.machinery.ExtensionFileLoader("_torch_bind", str(path))
         mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_torch_bind", loader))
         loader.exec_module(mod)

@@ -83,12 +83,18 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
 
 def _bind_stamp() -> str:
-    import torch
+    import importlib.metadata
 
-    h = hashlib.sha256(torch.__version__.encode())
+    h = hashlib.sha256(importlib.metadata.version("torch").encode())
     for f in (BIND_SOURCE, HERE.parent / "include" / "cutespmm.h"):
         h.update(f.read_bytes())
     return h.hexdigest()
+
+
+def bind_stale() -> bool:
+    """True when the torch binding does not correspond to its source, the header and the installed torch.  Does not import torch."""
+    stamp_file = LIBDIR / (BIND.name + ".stamp")
+    return not (BIND.exists() and stamp_file.exists() and stamp_file.read_text() == _bind_stamp())
 
 
 def build_bind(force: bool = False) -> Path:
@@ -97,19 +103,21 @@ def build_bind(force: bool = False) -> Path:
 
     import torch
 
+    if not force and not bind_stale():
+        return BIND
     stamp_file = LIBDIR / (BIND.name + ".stamp")
     stamp = _bind_stamp()
-    if not force and BIND.exists() and stamp_file.exists() and stamp_file.read_text() == stamp:
-        return BIND
     build()
     troot = Path(torch.__file__).resolve().parent
     include = [troot / "include", troot / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"], CUDA_HOME / "include"]
+    part = LIBDIR / f"{BIND.name}.{os.getpid()}"  # whole before it bears the name: other processes may be loading it
     # libstdc++ by its shared name: a static copy would not unwind the exceptions torch's libraries throw
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", *[f"-isystem{d}" for d in include], "-o", str(BIND), str(BIND_SOURCE),
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", *[f"-isystem{d}" for d in include], "-o", str(part), str(BIND_SOURCE),
            f"-L{LIBDIR}", f"-L{troot / 'lib'}", "-l:" + LIB.name, "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-l:libstdc++.so.6", "-Wl,-rpath,$ORIGIN"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("building the torch binding failed:\n" + res.stderr)
+    part.replace(BIND)
     stamp_file.write_text(stamp)
     return BIND
 

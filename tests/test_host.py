@@ -305,3 +305,30 @@ def test_auto_keeps_small_matrices_on_the_row_kernel():
     assert cs.Plan.from_csr(small, host_only=True).info()["brick_panels"] == 0
     assert cs.Plan.from_csr(big, host_only=True).info()["brick_panels"] == big.M // 16
     assert cs.Plan.from_csr(small, host_only=True, path=cs.PATH_BRICK).info()["brick_panels"] == small.M // 16  # an explicit path is obeyed
+
+
+def test_torch_binding_is_built_at_import(tmp_path):
+    """Where the torch binding is missing it is built when the package is imported (a stand-in compiler here), so the first product
+    compiles nothing; where it cannot be built the package still imports and says why when the binding is needed."""
+    import os
+    import shutil
+    import subprocess
+    import sys
+
+    pkg = tmp_path / "cutespmm_ae_b200"
+    shutil.copytree(ROOT / "cutespmm_ae_b200", pkg, ignore=shutil.ignore_patterns("__pycache__", "_torch_bind.so*"))
+    shutil.copytree(ROOT / "include", tmp_path / "include")
+    compiler = tmp_path / "cxx"
+    compiler.write_text('#!/bin/sh\nwhile [ $# -gt 1 ]; do [ "$1" = -o ] && echo made > "$2"; shift; done\n')
+    compiler.chmod(0o755)
+    script = "import cutespmm_ae_b200 as cs; print(cs.__file__, cs._build.BIND.exists() and cs._build.BIND.read_text(), cs._build.bind_stale())"
+
+    def run(code, **env):
+        return subprocess.run([sys.executable, "-c", code], cwd=tmp_path, capture_output=True, text=True, env=os.environ | {"PYTHONPATH": str(tmp_path)} | env)
+
+    res = run(script + "\ncs._native()", CXX="/nonexistent/compiler")
+    assert res.stdout.split() == [str(pkg / "__init__.py"), "False", "True"]
+    assert res.returncode != 0 and "/nonexistent/compiler" in res.stderr and "_build" in res.stderr.splitlines()[-1]
+    res = run(script, CXX=str(compiler))
+    assert res.returncode == 0, res.stderr
+    assert res.stdout.split() == [str(pkg / "__init__.py"), "made", "False"]
