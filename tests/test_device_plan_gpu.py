@@ -204,3 +204,22 @@ def test_device_cut_work_lists_equal_the_host_builder_s(oracle_mod, M, lengths, 
     del pd
     again = cs.Plan.from_device_csr(A.M, A.K, *_dev(A), **kw)
     assert torch.equal(again.spmm(B), Ch)
+
+
+def test_release_memory_gives_back_what_dropped_plans_held():
+    """The memory of a dropped plan stays with the library for the next one until it is given back; living plans keep theirs."""
+    A = g.uniform_random(200_000, 50_000, 64, seed=8)  # 100 MB of packed nonzeros
+    arrays = _dev(A)
+    B = g.dense_operand(A.K, 16, 9, device="cuda")
+    keep, drop = (cs.Plan.from_device_csr(A.M, A.K, *arrays) for _ in range(2))
+    want = keep.spmm(B)
+    torch.cuda.synchronize()
+    size = drop.info()["device_bytes"]
+    drop.close()
+    torch.cuda.synchronize()
+    held = torch.cuda.mem_get_info()[0]
+    assert cs.lib.cutespmm_release_memory() == 0
+    assert torch.cuda.mem_get_info()[0] - held >= size // 2  # the pool gives back whole pages of its own size
+    assert torch.equal(keep.spmm(B), want)
+    assert torch.equal(cs.Plan.from_device_csr(A.M, A.K, *arrays).spmm(B), want)
+    assert cs.lib.cutespmm_release_memory() == 0
