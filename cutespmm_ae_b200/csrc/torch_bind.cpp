@@ -8,6 +8,7 @@
 // The plans themselves stay with the Python objects (Plan, SparseOperator); this file holds handles only.
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/library.h>
 #include <ATen/ops/empty.h>
@@ -16,6 +17,7 @@
 
 #include <memory>
 #include <mutex>
+#include <optional>
 #include <string>
 #include <unordered_map>
 
@@ -246,6 +248,10 @@ struct WeightedGrad : torch::autograd::Function<WeightedGrad> {
     {
         const int64_t id = ctx->saved_data["id"].toInt();
         const variable_list saved = ctx->get_saved_variables();
+        // the two have no gradients of their own: unless a graph of this pass is asked for (and has to name them), go past the
+        // kernels that say so
+        std::optional<at::AutoDispatchBelowADInplaceOrView> guard;
+        if (!c10::GradMode::is_enabled()) guard.emplace();
         return {Tensor(), ctx->needs_input_grad(0) ? call_sddmm(id, g[0], saved[1], false) : Tensor(),
                 ctx->needs_input_grad(1) ? call_spmm_weighted_transposed(id, saved[0], g[0]) : Tensor()};
     }
@@ -272,6 +278,9 @@ TORCH_LIBRARY_IMPL(cutespmm, Autograd, m)
     m.impl("spmm", [](int64_t id, const Tensor &B) { return SpmmGrad<false>::apply(id, B); });
     m.impl("spmm_transposed", [](int64_t id, const Tensor &G) { return SpmmGrad<true>::apply(id, G); });
     m.impl("spmm_weighted", [](int64_t id, const Tensor &w, const Tensor &B) { return WeightedGrad::apply(id, w, B); });
+    // without one of these a backward pass through them would go on with zeros and a warning
+    m.impl("spmm_weighted_transposed", torch::autograd::autogradNotImplementedFallback());
+    m.impl("sddmm", torch::autograd::autogradNotImplementedFallback());
 }
 
 // ---- the Python module -----------------------------------------------------------------------------------------------

@@ -148,3 +148,26 @@ def test_threads_that_need_the_transposed_plan_at_once_share_one(monkeypatch):
     for C in out:
         assert torch.allclose(C, want @ G, rtol=1e-4, atol=1e-4)
     op.close()
+
+
+@pytest.mark.gpu
+def test_what_has_no_gradient_refuses_a_backward_pass():
+    """The scores of `sddmm` and the gradients of the weighted product are not differentiable themselves: a backward pass
+    through them is refused, not answered with zeros.  The plain product can be differentiated again."""
+    A = g.uniform_random(60, 50, 5, seed=43)
+    op = torch_ops.SparseOperator(cs.Plan.from_csr(A, path=cs.PATH_ROWS), plan_kwargs=dict(path=cs.PATH_ROWS))
+    X, B = (g.dense_operand(n, 16, 44, device="cuda").requires_grad_() for n in (A.M, A.K))
+    w = torch.rand(A.nnz, device="cuda", requires_grad=True)
+    scores = op.sddmm(X, B)
+    with pytest.raises(RuntimeError):
+        scores.sum().backward()
+    (dB,) = torch.autograd.grad((op(B) ** 2).sum(), B, create_graph=True)
+    (ddB,) = torch.autograd.grad(dB.sum(), B)
+    dense = torch.zeros(A.M, A.K, device="cuda")
+    dense[torch.repeat_interleave(torch.arange(A.M), A.row_ptr[1:] - A.row_ptr[:-1]).cuda(), A.cols.long().cuda()] = A.vals.cuda()
+    assert torch.allclose(ddB, 2 * dense.T @ dense @ torch.ones_like(B), rtol=1e-4, atol=1e-4)
+    for i in range(2):  # dw, then dB
+        grads = torch.autograd.grad((op.weighted(w, B) ** 2).sum(), (w, B), create_graph=True)
+        with pytest.raises(RuntimeError):
+            grads[i].sum().backward()
+    op.close()
