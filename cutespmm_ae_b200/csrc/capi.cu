@@ -178,6 +178,9 @@ static int upload_plan(cutespmm_plan *p, int dev, int sm_count)
     if ((e = cudaMalloc(&p->d_status, 256)) != cudaSuccess || (e = cudaMemset(p->d_status, 0, 256)) != cudaSuccess)
         return fail_cuda(e, "status word");
     by += 256;
+    // Clearing memory returns before it is done, and a copy from pageable memory may; both are ordered with the default stream
+    // only, and the first product may be on one that does not wait for it.
+    if ((e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess) return fail_cuda(e, "uploading the plan");
     return CUTESPMM_OK;
 }
 

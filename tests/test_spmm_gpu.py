@@ -610,3 +610,17 @@ def test_calls_leave_the_interpreter_to_other_threads(call):
     assert max(times) > 0.2  # the queue did fill up
     assert longest < 0.1 * max(times), (longest, max(times))
     op.close()
+
+
+def test_first_product_on_another_stream_sees_a_finished_plan(oracle_mod):
+    """A plan made on the host is complete when the call returns, for streams too that do not wait for the default one."""
+    A = g.rmat(11, 8, seed=18, values="uniform")
+    B = g.dense_operand(A.K, 64, 19, device="cuda")
+    want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.cpu().numpy(), A.M, A.K)
+    side, C = torch.cuda.Stream(), torch.empty((A.M, 64), device="cuda")  # a stream of torch's does not wait for the default stream
+    torch.cuda.synchronize()
+    for _ in range(10):
+        p = cs.Plan.from_csr(A, path=cs.PATH_ROWS)
+        p.spmm(B, C, stream=side)
+        side.synchronize()
+        assert oracle_mod.rel_fro(want, C.cpu().numpy()) <= REL_FRO_TOL_FP32
