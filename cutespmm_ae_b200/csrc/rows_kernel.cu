@@ -95,7 +95,7 @@ __device__ __forceinline__ void accumulate(typename Vec<VEC>::T (&acc)[CH], cons
                                            const bool (&ok)[CH], int lane)
 {
     using V = typename Vec<VEC>::T;
-    // nonzeros in flight per step.  With float4 lanes in the 40-register tuning 8 was measured: no gain, spills; the
+    // nonzeros in flight per step.  Eight with float4 lanes in the shallow tuning spilled and gained nothing (at 40 registers); the
     // deep tuning and narrow lanes have the registers, and a deeper step shortens the chain of a latency-bound job
     constexpr int U = DEEP ? 8 / CH : ((CH == 1) ? (VEC == 4 ? 4 : 8) : 2);
     for (uint32_t j = j0; j < j1; j += 32) {

@@ -10,8 +10,8 @@
 // is a group of eight (four for N <= 16) lanes' work and a span of 16 to 128 columns, by N.  Rows of few
 // nonzeros are walked flat, 32 nonzeros per claim; wide products of longer rows take a warp per row, which
 // keeps its part of X in registers.  Every nonzero has its own output, so nothing is summed across work items.
-// Measured (R-MAT 2^18, 3.9 M nonzeros): N = 64 212 -> 111 us (a 128-column span before, half of it idle),
-// N = 32 199 -> 78 us, N = 128 186 -> 170 us.
+// Measured (R-MAT 2^18, 3.9 M nonzeros): N = 64 212 -> 103 us (a 128-column span before, half of it idle; now bound by the L1
+// data pipe, 67 % busy, and the loads behind it), N = 32 199 -> 78 us, N = 128 186 -> 167 us.
 #include <cuda_runtime.h>
 
 #include <cstdint>
