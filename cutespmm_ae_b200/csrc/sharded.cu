@@ -285,7 +285,7 @@ bool cut_row_blocks(cutespmm_plan *p, uint32_t N)
     // nothing, so a small call wants small blocks (23 MB each way: 0.77 ms in two blocks, 0.70 in five); a large one is bound by
     // what the link carries both ways at once, and every block costs about 40 us of hand-over between the copy engines and
     // its kernel (134 MB: 3.50 ms in eight blocks, 3.86 in sixteen).  At 49 MB the two are level: 1.41 ms in three blocks and 1.48
-    // (1.28 at best) in ten on one box, 1.55 and 1.43 on another; ten uploads and downloads alone take 1.2 ms there
+    // (1.28 at best) in ten on one machine (where ten uploads and downloads alone take 1.2), 1.55 and 1.43 on another
     int R = (int)(c_bytes <= (48u << 20) ? std::min<uint64_t>(10, c_bytes / (4u << 20)) : std::min<uint64_t>(cutespmm_plan::kMaxRowBlocks, c_bytes / (16u << 20)));
     if (R < 2) return false;
     // boundaries: near equal row counts, on 16-row panel boundaries, never inside a tile of either tile list
