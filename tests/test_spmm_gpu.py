@@ -516,7 +516,7 @@ def test_product_waits_for_nothing_without_memory_for_a_padded_copy(oracle_mod):
     before = torch.cuda.mem_get_info()[0]
     hog = torch.empty(before - (256 << 20), dtype=torch.uint8, device="cuda")
     try:
-        torch.cuda._sleep(1_000_000_000)  # half a second
+        torch.cuda._sleep(2_000_000_000)  # a second
         stalled.record()
         p.spmm(B, C)
         assert not stalled.query()  # the call came back while the stream was still busy
@@ -608,7 +608,7 @@ def test_calls_leave_the_interpreter_to_other_threads(call):
         time.sleep(0.001)
     torch.cuda.synchronize()
     assert max(times) > 0.2  # the queue did fill up
-    assert longest < 0.1 * max(times), (longest, max(times))
+    assert longest < 0.5 * max(times), (longest, max(times))  # all of it where the lock is held, a few milliseconds where not
     op.close()
 
 
