@@ -622,9 +622,8 @@ int cutespmm_sddmm(const cutespmm_plan_t *p, const float *X, uint64_t ldx, const
     a.X = X; a.Y = Y; a.ldx = ldx; a.ldy = ldy; a.out = out; a.N = N;
     a.scale = scale_by_values ? 1u : 0u;
     a.early = h.values_on_device ? 0u : 1u;
-    a.avg_row_nnz = (uint32_t)(h.nnz / std::max<uint64_t>(h.M, 1));
     a.status = p->d_status;
-    a.vec4 = !((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15) && !((ldx | ldy) & 3) ? 1u : 0u;
+    a.vec4 = !((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15) && !((ldx | ldy) & 3) && (ldx | ldy) < (1ull << 30) ? 1u : 0u;
     cudaError_t e = launch_sddmm(a, p->sm_count, s);
     return e == cudaSuccess ? CUTESPMM_OK : fail_cuda(e, "SDDMM kernel launch");
 }

@@ -6,12 +6,16 @@
 // TC-GNN's forward_ef, TC-GNN_ATC23/TCGNN_conv/TCGNN.cpp:265, and its own kernels do not have it), and
 // the gradient of SpMM with respect to the values of A (dA = SDDMM(dC, B)).  Like the row kernel it is
 // bound by gathering rows of Y, and it is built on the same skeleton: the block's tiles arrive in shared
-// memory by TMA, warps claim work as they go, chunks of long rows are dealt over the blocks first.  A nonzero
-// is a group of eight (four for N <= 16) lanes' work and a span of 16 to 128 columns, by N.  Rows of few
-// nonzeros are walked flat, 32 nonzeros per claim; wide products of longer rows take a warp per row, which
-// keeps its part of X in registers.  Every nonzero has its own output, so nothing is summed across work items.
-// Measured (R-MAT 2^18, 3.9 M nonzeros): N = 64 212 -> 103 us (a 128-column span before, half of it idle; now bound by the L1
-// data pipe, 67 % busy, and the loads behind it), N = 32 199 -> 78 us, N = 128 186 -> 167 us.
+// memory by TMA, warps claim work as they go, chunks of long rows are dealt over the blocks first.  A nonzero is a group of
+// eight (four for N <= 16) lanes' work and a span of 16 to 128 columns, by N.  A warp claims 32 nonzeros whatever their rows
+// and its groups walk a run of them each, a row of X in registers for as long as it lasts.  Every nonzero has its own output,
+// so nothing is summed across work items.
+// Bound by the latency of the gathers (32 warps per SM, 16 to 32 registers of Y in flight each) and the instructions around
+// them; gathers alone would take 50 us on R-MAT 2^18 (3.9 M nonzeros) at N = 64 (20 TB/s out of L2, measured).  Before, every
+// nonzero loaded its row of X again and wide products of longer rows took a warp per row: R-MAT 2^18 at N = 16 / 32 / 64 / 128
+// 48.0 / 74.8 / 106 / 168 -> 43.0 / 57.1 / 83.3 / 139 us, elasticity40 N = 64 106 -> 80.7, 60 000 x 32 per row N = 64 50.6 ->
+// 39.5.  Tried: the next batch's rows of Y in flight beside this one's (83 -> 86 us), the next claim looked up meanwhile (86), 40
+// and 48 warps per SM with fewer rows in flight (90, 96), the tiles' rows of X prefetched into L2 (87).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -25,7 +29,6 @@ namespace cutespmm {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr uint32_t kRowsFromNnz = 16;  // nonzeros per row from which a wide product takes a warp per row
 
 // LANES lanes share a nonzero and cover a span of 4 * V * LANES columns of its row of Y: as V float4 each (VEC4), lane sub
 // at float4 number sub, sub + LANES, ..., or as 4 V single columns where the rows are not 16-byte aligned.  FULL: N is a
@@ -33,7 +36,8 @@ constexpr uint32_t kRowsFromNnz = 16;  // nonzeros per row from which a wide pro
 template <int LANES, int V, bool VEC4, bool FULL> struct Span {
     static constexpr int kCols = 4 * V * LANES;
     static constexpr int kGroups = 32 / LANES;                        // nonzeros per load instruction
-    static constexpr int kSteps = V >= 4 ? 2 : (V == 1 ? 4 : 8 / V);  // ... and load steps in flight per warp
+    static constexpr unsigned kGroupStarts = LANES == 8 ? 0x01010101u : 0x11111111u;  // the first lane of every group
+    static constexpr int kSteps = 2;                                  // ... and load steps in flight per warp that walks a row
 
     static __device__ __forceinline__ void load(float4 (&v)[V], const float *row, uint32_t c0, uint32_t N, int sub)
     {
@@ -59,17 +63,25 @@ template <int LANES, int V, bool VEC4, bool FULL> struct Span {
         }
     }
 
+    // Row r of X or Y.  Four columns per lane: `ld` is below 2^30 (SddmmArgs::vec4), so the stride in bytes is 32 bits wide and an
+    // address is one 32 x 32 + 64-bit multiply-add.
+    static __device__ __forceinline__ const float *row_of(const float *base, uint32_t r, uint64_t ld)
+    {
+        if (VEC4) return reinterpret_cast<const float *>(reinterpret_cast<const char *>(base) + (uint64_t)r * (uint32_t)(ld * 4));
+        return base + r * ld;
+    }
+
+    // Even and odd columns are added up separately, two at a time (one instruction each), and then together.
     static __device__ __forceinline__ float dot(const float4 (&x)[V], const float4 (&y)[V])
     {
-        float s = 0.f;
+        uint64_t s = 0;
 #pragma unroll
         for (int i = 0; i < V; ++i) {
-            s = fmaf(x[i].x, y[i].x, s);
-            s = fmaf(x[i].y, y[i].y, s);
-            s = fmaf(x[i].z, y[i].z, s);
-            s = fmaf(x[i].w, y[i].w, s);
+            s = ptx::fma2(ptx::pack2(x[i].x, x[i].y), ptx::pack2(y[i].x, y[i].y), s);
+            s = ptx::fma2(ptx::pack2(x[i].z, x[i].w), ptx::pack2(y[i].z, y[i].w), s);
         }
-        return s;
+        const float2 e = ptx::unpack2(s);
+        return e.x + e.y;
     }
 
     // STEPS load steps, starting at nonzero k of the item: the span c0 of X[row] (in x) against the same span of the rows of
@@ -85,7 +97,7 @@ template <int LANES, int V, bool VEC4, bool FULL> struct Span {
         for (int u = 0; u < STEPS; ++u) {
             const uint32_t mine = k + u * kGroups + grp;
             pr[u] = pair_at(min(mine, cnt - 1));  // positions past the end repeat the last pair (a cache hit) and are not stored
-            load(y[u], a.Y + (uint64_t)pr[u].x * a.ldy, c0, a.N, sub);
+            load(y[u], row_of(a.Y, pr[u].x, a.ldy), c0, a.N, sub);
         }
 #pragma unroll
         for (int u = 0; u < STEPS; ++u) {
@@ -111,56 +123,69 @@ template <int LANES, int V, bool VEC4, bool FULL> struct Span {
         if (k < cnt) step<kSteps / 2>(a, x, pair_at, k, cnt, out, c0, first, lane);
     }
 
-    // n <= 32 nonzeros whose pairs are pairs[k] (shared memory), the k-th in row `row` of lane k: both rows are loaded.
-    // The kFlat sums a lane ends up with are added over the lanes of its group by halving: at each level a lane hands
-    // half of its sums to its partner and keeps the other half, so a step costs one shuffle instead of one per level, and
-    // the lanes of a group hold different nonzeros' results at the end.
-    static __device__ __forceinline__ void flat(const SddmmArgs &a, uint32_t row, const uint2 *pairs, uint32_t n, float *out, uint32_t c0, bool first, int lane)
+    // 32 nonzeros, lane k's in row `row` and column `col`.  Group g takes nonzeros g * LANES ... one after the other and keeps
+    // its row of X in registers (x, loaded by the caller where KEEP): bit k of `turn` says that nonzero k is the first its
+    // group sees of its row.  The sums of a group's nonzeros are added over its lanes by halving: at each level a lane hands
+    // half of its sums to its partner and keeps the other half, first inside every batch of kFly nonzeros whose rows of Y are in
+    // flight together, then over the batches.  That is LANES - 1 shuffles for LANES sums, and a lane is left with the result of
+    // nonzero result_of(lane).
+    static constexpr int kFly = V == 1 ? LANES : V == 2 ? 4 : 2;  // 16 to 32 registers of Y
+    static constexpr int kBatches = LANES / kFly;
+    static __device__ __forceinline__ uint32_t result_of(int lane)
     {
-        constexpr int kFlat = V == 1 ? 4 : V == 2 ? 2 : 1;  // load steps in flight: 16 to 32 registers of X and of Y
-        const int sub = lane % LANES, grp = lane / LANES;
-        for (uint32_t k = 0; k < n; k += kGroups * kFlat) {
-            float4 x[kFlat][V], y[kFlat][V];
+        const int sub = lane % LANES;
+        return (uint32_t)(lane - sub + sub % kBatches * kFly + sub / kBatches);
+    }
+    template <int CNT> static __device__ __forceinline__ void halve(float *s, int &o, int sub)
+    {
 #pragma unroll
-            for (int u = 0; u < kFlat; ++u) {
-                const uint32_t from = min(k + u * kGroups + grp, n - 1);  // positions past the end repeat the last one and are not stored
-                load(x[u], a.X + (uint64_t)__shfl_sync(kFull, row, (int)from) * a.ldx, c0, a.N, sub);
-                load(y[u], a.Y + (uint64_t)pairs[from].x * a.ldy, c0, a.N, sub);
-            }
-            float s[kFlat];
+        for (int left = CNT / 2; left > 0; left /= 2, o /= 2) {
+            const bool upper = sub & o;
 #pragma unroll
-            for (int u = 0; u < kFlat; ++u) s[u] = dot(x[u], y[u]);
-            uint32_t mine = 0;   // which of the group's steps this lane ends up with
-            bool spare = false;  // another lane holds the same
-            int left = kFlat;
-#pragma unroll
-            for (int o = LANES / 2; o > 0; o >>= 1) {
-                const bool upper = sub & o;
-                if (left > 1) {
-                    left /= 2;
-#pragma unroll
-                    for (int i = 0; i < left; ++i) {
-                        const float keep = upper ? s[i + left] : s[i], give = upper ? s[i] : s[i + left];
-                        s[i] = keep + __shfl_xor_sync(kFull, give, o);
-                    }
-                    if (upper) mine += left;
-                } else {
-                    s[0] += __shfl_xor_sync(kFull, s[0], o);
-                    spare |= upper;
-                }
-            }
-            mine = k + mine * kGroups + grp;
-            if (mine < n && !spare) {
-                float v = s[0];
-                if (a.scale) v *= __uint_as_float(pairs[mine].y);
-                out[mine] = first ? v : out[mine] + v;
+            for (int i = 0; i < left; ++i) {
+                const float keep = upper ? s[i + left] : s[i], give = upper ? s[i] : s[i + left];
+                s[i] = keep + __shfl_xor_sync(kFull, give, o);
             }
         }
     }
+    template <bool KEEP>
+    static __device__ __forceinline__ float flat(const SddmmArgs &a, float4 (&x)[V], uint32_t row, unsigned turn, uint32_t col, uint32_t c0, int lane)
+    {
+        const int sub = lane % LANES, k0 = lane - sub;
+        float sums[kBatches];
+        int o = LANES / 2;
+#pragma unroll
+        for (int b = 0; b < kBatches; ++b) {
+            float4 y[kFly][V];
+            float s[kFly];
+#pragma unroll
+            for (int u = 0; u < kFly; ++u) load(y[u], row_of(a.Y, __shfl_sync(kFull, col, b * kFly + u, LANES), a.ldy), c0, a.N, sub);
+#pragma unroll
+            for (int u = 0; u < kFly; ++u) {
+                const int q = b * kFly + u;
+                if constexpr (!KEEP)
+                    if (turn & (kGroupStarts << q)) {  // the same for every lane
+                        const uint32_t r = __shfl_sync(kFull, row, q, LANES);
+                        if (turn >> (k0 + q) & 1u) load(x, row_of(a.X, r, a.ldx), c0, a.N, sub);
+                    }
+                s[u] = dot(x, y[u]);
+            }
+            o = LANES / 2;
+            halve<kFly>(s, o, sub);
+            sums[b] = s[0];
+        }
+        halve<kBatches>(sums, o, sub);
+        return sums[0];
+    }
 };
 
-template <int LANES, int V, bool VEC4, bool FULL, bool FLAT>
-__global__ void __launch_bounds__(kTileWarps * 32, FLAT || V < 3 ? 4 : 3) sddmm_kernel(SddmmArgs a)
+// Nonzeros are walked flat, 32 per claim, except where a wide product's rows are not 16-byte aligned: its single-column loads keep a
+// warp per row (60 000 x 32 per row N = 101 104 us, flat 130; up to 64 columns flat is faster there too: N = 63 74 -> 72, stencil512
+// 143 -> 88.5).
+template <int V, bool VEC4> constexpr bool kFlat = VEC4 || V < 3;
+
+template <int LANES, int V, bool VEC4, bool FULL>
+__global__ void __launch_bounds__(kTileWarps * 32, kFlat<V, VEC4> ? 4 : 3) sddmm_kernel(SddmmArgs a)
 {
     using S = Span<LANES, V, VEC4, FULL>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % LANES;
@@ -180,14 +205,19 @@ __global__ void __launch_bounds__(kTileWarps * 32, FLAT || V < 3 ? 4 : 3) sddmm_
             const uint4 ck = __ldg(chunks + c);  // row, j0, j1, slot
             for (uint32_t c0 = 0; c0 < a.N; c0 += S::kCols) {
                 float4 x[V];
-                S::load(x, a.X + (uint64_t)ck.x * a.ldx, c0, a.N, sub);
-                uint2 nxt = make_uint2(0u, 0u);
-                if (ck.y + lane < ck.z) nxt = __ldg(pairs + ck.y + lane);
+                S::load(x, S::row_of(a.X, ck.x, a.ldx), c0, a.N, sub);
+                uint2 nxt = __ldg(pairs + min(ck.y + lane, ck.z - 1));  // lanes past the end repeat the last one and store nothing
                 for (uint32_t j = ck.y; j < ck.z; j += 32) {
                     const uint2 cur = nxt;
-                    if (j + 32 + lane < ck.z) nxt = __ldg(pairs + j + 32 + lane);
-                    auto pair_at = [&](uint32_t k) { return make_uint2(__shfl_sync(kFull, cur.x, (int)k), __shfl_sync(kFull, cur.y, (int)k)); };
-                    S::items(a, x, pair_at, min(32u, ck.z - j), a.out + j, c0, c0 == 0, lane);
+                    if (j + 32 < ck.z) nxt = __ldg(pairs + min(j + 32 + lane, ck.z - 1));
+                    const uint32_t n = min(32u, ck.z - j);
+                    float v = S::template flat<true>(a, x, 0u, 0u, cur.x, c0, lane);
+                    const uint32_t mine = S::result_of(lane);
+                    const float scale = __uint_as_float(__shfl_sync(kFull, cur.y, (int)mine));
+                    if (mine < n) {
+                        if (a.scale) v *= scale;
+                        a.out[j + mine] = c0 == 0 ? v : a.out[j + mine] + v;
+                    }
                 }
             }
         }
@@ -204,21 +234,39 @@ __global__ void __launch_bounds__(kTileWarps * 32, FLAT || V < 3 ? 4 : 3) sddmm_
         const TileStage &st = ring.stage[s];
         const uint4 d = st.desc;
         const uint32_t rb = d.x & ~3u, jb = d.z & ~1u;
-        if constexpr (FLAT) {
-            // A warp claims 32 nonzeros at a time whatever their rows: lane i looks the row of the i-th up in the staged row
-            // pointers and the groups load both rows, X and Y.  Neighbouring groups mostly name the same row of X (one
-            // request for all of them).
+        if constexpr (kFlat<V, VEC4>) {
+            // A warp claims 32 nonzeros at a time whatever their rows; lane i looks the row of the i-th up in the staged row pointers.
             const uint32_t cnt = d.w - d.z;
             for (;;) {
                 const uint32_t k0 = tile_claim_rows(ring, s, 32u, lane);
                 if (k0 >= cnt) break;
-                const uint32_t n = min(32u, cnt - k0), j = d.z + min(k0 + lane, cnt - 1);
-                uint32_t lo = d.x, hi = d.y;  // the row r with row_ptr[r] <= j < row_ptr[r + 1]
-                while (hi - lo > 1) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (st.row_ptr[mid - rb] <= j) lo = mid; else hi = mid;
+                const uint32_t n = min(32u, cnt - k0), j = d.z + min(k0 + lane, cnt - 1);  // lanes past the end repeat the last nonzero and store nothing
+                uint32_t row = d.x, hi = d.y;  // the row with row_ptr[row] <= j < row_ptr[row + 1]
+                while (hi - row > 1) {
+                    const uint32_t mid = (row + hi) >> 1;
+                    if (st.row_ptr[mid - rb] <= j) row = mid; else hi = mid;
                 }
-                for (uint32_t c0 = 0; c0 < a.N; c0 += S::kCols) S::flat(a, lo, st.pairs + (d.z - jb + k0), n, a.out + d.z + k0, c0, c0 == 0, lane);
+                const uint2 cur = st.pairs[j - jb];
+                const uint32_t mine = S::result_of(lane);
+                const float scale = __uint_as_float(__shfl_sync(kFull, cur.y, (int)mine));
+                const uint32_t before = __shfl_up_sync(kFull, row, 1);
+                const unsigned turn = __ballot_sync(kFull, row != before) | S::kGroupStarts;
+                // the rows of X that a group meets on its way arrive in L1 beside its first loads (R-MAT 2^18 N = 64: 89.6 -> 83.3 us)
+                if constexpr (VEC4)
+                    if (row != before && lane % LANES) {
+                        const float *p = S::row_of(a.X, row, a.ldx);
+#pragma unroll
+                        for (int i = 0; i < V; ++i) ptx::prefetch_l1(p + 4 * LANES * i);
+                    }
+                for (uint32_t c0 = 0; c0 < a.N; c0 += S::kCols) {
+                    float4 x[V];
+                    float v = S::template flat<false>(a, x, row, turn, cur.x, c0, lane);
+                    if (mine < n) {
+                        float *out = a.out + d.z + k0 + mine;
+                        if (a.scale) v *= scale;
+                        *out = c0 == 0 ? v : *out + v;
+                    }
+                }
             }
         } else {
             for (;;) {
@@ -230,7 +278,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, FLAT || V < 3 ? 4 : 3) sddmm_
                 auto pair_at = [&](uint32_t k) { return row_pairs[k]; };  // the lanes of a group read one address
                 for (uint32_t c0 = 0; c0 < a.N; c0 += S::kCols) {
                     float4 x[V];
-                    S::load(x, a.X + (uint64_t)r * a.ldx, c0, a.N, sub);
+                    S::load(x, S::row_of(a.X, r, a.ldx), c0, a.N, sub);
                     S::items(a, x, pair_at, j1 - j0, a.out + j0, c0, c0 == 0, lane);
                 }
             }
@@ -239,30 +287,21 @@ __global__ void __launch_bounds__(kTileWarps * 32, FLAT || V < 3 ? 4 : 3) sddmm_
     }
 }
 
-template <int LANES, int V, bool VEC4, bool FULL, bool FLAT> cudaError_t launch_sddmm_t(const SddmmArgs &a, int sm_count, cudaStream_t s)
+template <int LANES, int V, bool VEC4, bool FULL> cudaError_t launch_sddmm_t(const SddmmArgs &a, int sm_count, cudaStream_t s)
 {
     int per_sm = 0;
-    const cudaError_t e = blocks_per_sm<sddmm_kernel<LANES, V, VEC4, FULL, FLAT>>(per_sm, kTileWarps * 32);
+    const cudaError_t e = blocks_per_sm<sddmm_kernel<LANES, V, VEC4, FULL>>(per_sm, kTileWarps * 32);
     if (e != cudaSuccess) return e;
     const uint32_t chunk_blocks = (a.num_chunks + kTileWarps - 1) / kTileWarps;
     uint32_t blocks = a.num_tiles > chunk_blocks ? a.num_tiles : chunk_blocks;
     const uint32_t cap = (uint32_t)(sm_count * per_sm);  // one resident wave
     if (blocks > cap) blocks = cap;
-    return launch_overlapped(sddmm_kernel<LANES, V, VEC4, FULL, FLAT>, blocks, kTileWarps * 32, 0, s, a);
+    return launch_overlapped(sddmm_kernel<LANES, V, VEC4, FULL>, blocks, kTileWarps * 32, 0, s, a);
 }
 template <int LANES, int V> cudaError_t launch_sddmm_v(const SddmmArgs &a, int sm_count, cudaStream_t s)
 {
-    if (!a.vec4) return launch_sddmm_t<LANES, V, false, false, false>(a, sm_count, s);  // twice the scalar loads: X stays in registers
-    const bool full = a.N % (4 * V * LANES) == 0;
-    // Nonzeros flat, or a warp per row.  A row's chain of latencies (claim, pointers, X, Y, sums) is what a warp per row
-    // costs, a second load per nonzero what the flat form costs.  Flat wins up to 64 columns everywhere (R-MAT 2^18 at N = 64:
-    // 125 -> 111 us, stencil512 at N = 32: 86 -> 55 us); beyond, two loads of up to 512 bytes per nonzero fill the L1 data
-    // pipe, and rows of 16 and more nonzeros repay their latencies (N = 128, flat against rows: 8 per row 47 / 53 us, 16 per
-    // row 78 / 71 us, elasticity40 186 / 152 us, R-MAT 2^18 170 / 190 us).
-    if constexpr (V >= 3)
-        if (a.avg_row_nnz >= kRowsFromNnz)
-            return full ? launch_sddmm_t<LANES, V, true, true, false>(a, sm_count, s) : launch_sddmm_t<LANES, V, true, false, false>(a, sm_count, s);
-    return full ? launch_sddmm_t<LANES, V, true, true, true>(a, sm_count, s) : launch_sddmm_t<LANES, V, true, false, true>(a, sm_count, s);
+    if (!a.vec4) return launch_sddmm_t<LANES, V, false, false>(a, sm_count, s);
+    return a.N % (4 * V * LANES) == 0 ? launch_sddmm_t<LANES, V, true, true>(a, sm_count, s) : launch_sddmm_t<LANES, V, true, false>(a, sm_count, s);
 }
 
 }  // namespace

@@ -32,6 +32,25 @@ def test_sddmm_matches_oracle_for_any_width(oracle_mod, N, scale):
     assert rel(want, out.cpu().numpy()) <= TOL
 
 
+@pytest.mark.parametrize("N", [16, 17, 32, 33, 64, 65, 96, 97, 130])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_sddmm_where_rows_end_inside_a_run_of_nonzeros(oracle_mod, N, shift):
+    """A warp takes 32 nonzeros, a group of lanes eight (four) of them: rows that end in front of, on and behind those borders,
+    empty rows between them, a tile whose last claim is one nonzero; aligned operands and operands off the 16-byte grid."""
+    lengths = [1, 7, 8, 9, 0, 0, 3, 4, 5, 31, 32, 33, 0, 1, 1, 1, 1, 2, 63, 64, 65, 0, 129, 255, 257, 1]
+    row_ptr = torch.cat([torch.zeros(1, dtype=torch.int64), torch.cumsum(torch.tensor(lengths * 3), 0)])
+    M, nnz, K = len(lengths) * 3, int(row_ptr[-1]), 301
+    cols = torch.arange(nnz, dtype=torch.int64).mul(97).remainder(K).to(torch.int32)
+    vals = g.dense_operand(nnz, 1, 71).flatten()
+    p = cs.Plan.from_device_csr(M, K, row_ptr.to(torch.int32).cuda(), cols.cuda(), vals.cuda(), path=cs.PATH_ROWS)
+    X, Y = g.dense_operand(M, N + shift, 72).cuda()[:, shift:], g.dense_operand(K, N + shift, 73).cuda()[:, shift:]
+    out = torch.full((nnz + 1,), float("nan"), device="cuda")  # nothing is written behind the last nonzero
+    p.sddmm(X, Y, out[:nnz], scale_by_values=True)
+    want = oracle_mod.sddmm_csr(row_ptr, cols, vals, X.cpu().contiguous().numpy(), Y.cpu().contiguous().numpy())
+    # two fp32 sums of N <= 130 products in different orders
+    assert rel(want, out[:nnz].cpu().numpy()) <= TOL and torch.isnan(out[nnz])
+
+
 @pytest.mark.parametrize("make,path", [(lambda: g.stencil9(64), cs.PATH_AUTO), (lambda: g.elasticity3d(8, 3, 4), cs.PATH_BRICK),
                                         (lambda: g.uniform_random(300, 200, 5, seed=41), cs.PATH_ROWS)])
 def test_sddmm_on_every_plan_flavour_and_strided_operands(oracle_mod, make, path):
