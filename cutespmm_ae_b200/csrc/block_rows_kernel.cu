@@ -6,6 +6,8 @@
 // (tile_stage.cuh); a run that a tile boundary cuts is computed in two parts.  The reference has no counterpart (its bricks
 // share loads between the rows of a panel on the tensor cores, kernel.cu:119-288).
 // Here the pipe is 58 % busy and instruction issue 70 %.
+// Rows of B off the 16-byte grid are read one column per load, the lanes' columns interleaved (elasticity40 N = 63 60.5 -> 51 us, N = 203
+// 222 -> 165, N = 334 654 -> 360; before, after a padded copy of B or one row at a time).
 // Row kernel -> here: elasticity40 N = 32 35.1 -> 25.7 us, N = 27 48.7 -> 34.2; elasticity20 N = 128 20.4 -> 12.8.
 #include <cuda_runtime.h>
 
@@ -27,16 +29,24 @@ __device__ __forceinline__ void fma4(float4 &a, float v, const float4 &b)
     a.x = fmaf(v, b.x, a.x); a.y = fmaf(v, b.y, a.y); a.z = fmaf(v, b.z, a.z); a.w = fmaf(v, b.w, a.w);
 }
 
+// Four columns of a row of B: one load where rows are 16-byte aligned, otherwise four of columns L apart (a load instruction
+// reads neighbouring columns), `cols` of the slab's columns from the lane's first on.
+template <int L, bool ALIGNED> __device__ __forceinline__ float4 load4(const float *row, bool ok, uint32_t cols)
+{
+    if (ALIGNED) return ok ? __ldg(reinterpret_cast<const float4 *>(row)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    return make_float4(ok ? __ldg(row) : 0.f, L < cols ? __ldg(row + L) : 0.f, 2 * L < cols ? __ldg(row + 2 * L) : 0.f, 3 * L < cols ? __ldg(row + 3 * L) : 0.f);
+}
+
 // U columns of a run, the pairs of its rows at first[0 .. R-1] + i: U rows of B in flight.  TAIL: only the first cnt count.
-template <int R, int U, bool TAIL>
+template <int R, int U, bool TAIL, int L, bool ALIGNED>
 __device__ __forceinline__ void run_step(float4 (&acc)[R], const uint2 *pairs, const uint32_t (&first)[R], uint32_t i, uint32_t cnt, const float *bl, uint32_t ldb,
-                                         bool ok)
+                                         bool ok, uint32_t cols)
 {
     float4 b[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         const uint32_t c = pairs[first[0] + i + (TAIL ? min((uint32_t)u, cnt - 1) : u)].x;
-        b[u] = ok ? __ldg(reinterpret_cast<const float4 *>(bl + (uint64_t)c * ldb)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        b[u] = load4<L, ALIGNED>(bl + (uint64_t)c * ldb, ok, cols);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
@@ -46,13 +56,14 @@ __device__ __forceinline__ void run_step(float4 (&acc)[R], const uint2 *pairs, c
         }
 }
 
-template <int R, int G>
+template <int R, int G, bool ALIGNED>
 __global__ void __launch_bounds__(kTileWarps * 32, 4) spmm_block_rows_kernel(RowsArgs a)
 {
     constexpr int L = 32 / G, U = kUnroll;
     const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
-    const uint32_t col0 = blockIdx.y * 128 + sub * 4;
+    const uint32_t col0 = blockIdx.y * 128 + (ALIGNED ? sub * 4 : sub);  // a lane's columns: four from here on, or every L-th
     const bool ok = col0 < a.N;
+    const uint32_t cols = ok ? a.N - col0 : 0u;
     const float *bl = a.B + col0;
     const uint32_t ldb = (uint32_t)a.ldb;
 
@@ -89,22 +100,23 @@ __global__ void __launch_bounds__(kTileWarps * 32, 4) spmm_block_rows_kernel(Row
 #pragma unroll
                 for (int k = 0; k < R; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
                 uint32_t j = 0;
-                for (; j + U <= len; j += U) run_step<R, U, false>(acc, st.pairs, first, j, U, bl, ldb, ok);
+                for (; j + U <= len; j += U) run_step<R, U, false, L, ALIGNED>(acc, st.pairs, first, j, U, bl, ldb, ok, cols);
                 if (const uint32_t rem = len - j) {
-                    if (rem > U / 2) run_step<R, U, true>(acc, st.pairs, first, j, rem, bl, ldb, ok);
-                    else run_step<R, U / 2, true>(acc, st.pairs, first, j, rem, bl, ldb, ok);
+                    if (rem > U / 2) run_step<R, U, true, L, ALIGNED>(acc, st.pairs, first, j, rem, bl, ldb, ok, cols);
+                    else run_step<R, U / 2, true, L, ALIGNED>(acc, st.pairs, first, j, rem, bl, ldb, ok, cols);
                 }
 #pragma unroll
                 for (int k = 0; k < R; ++k) {
                     if (r0 + k < lo || r0 + k >= hi || !ok) continue;
                     float *p = a.C + (uint64_t)(r0 + k) * a.ldc + col0;
-                    if (!a.c_scalar) {
+                    if (ALIGNED && !a.c_scalar) {
                         __stcs(reinterpret_cast<float4 *>(p), acc[k]);
                     } else {
+                        constexpr int D = ALIGNED ? 1 : L;
                         __stcs(p, acc[k].x);
-                        if (col0 + 1 < a.N) __stcs(p + 1, acc[k].y);
-                        if (col0 + 2 < a.N) __stcs(p + 2, acc[k].z);
-                        if (col0 + 3 < a.N) __stcs(p + 3, acc[k].w);
+                        if (D < cols) __stcs(p + D, acc[k].y);
+                        if (2 * D < cols) __stcs(p + 2 * D, acc[k].z);
+                        if (3 * D < cols) __stcs(p + 3 * D, acc[k].w);
                     }
                 }
             }
@@ -114,31 +126,32 @@ __global__ void __launch_bounds__(kTileWarps * 32, 4) spmm_block_rows_kernel(Row
     }
 }
 
-template <int R, int G> cudaError_t launch_t(const RowsArgs &a, int sm_count, cudaStream_t s)
+template <int R, int G, bool ALIGNED> cudaError_t launch_t(const RowsArgs &a, int sm_count, cudaStream_t s)
 {
     int per_sm = 0;
-    const cudaError_t e = blocks_per_sm<spmm_block_rows_kernel<R, G>>(per_sm, kTileWarps * 32);
+    const cudaError_t e = blocks_per_sm<spmm_block_rows_kernel<R, G, ALIGNED>>(per_sm, kTileWarps * 32);
     if (e != cudaSuccess) return e;
     const uint32_t slabs = (a.N + 127) / 128, wave = (uint32_t)(sm_count * per_sm);
     uint32_t gx = a.num_tiles < wave ? a.num_tiles : wave;
     if (slabs > 1) gx = (gx + slabs - 1) / slabs;
-    return launch_overlapped(spmm_block_rows_kernel<R, G>, dim3(gx, slabs), kTileWarps * 32, 0, s, a);
+    return launch_overlapped(spmm_block_rows_kernel<R, G, ALIGNED>, dim3(gx, slabs), kTileWarps * 32, 0, s, a);
 }
-template <int R> cudaError_t launch_r(const RowsArgs &a, int sm_count, cudaStream_t s)
+template <int R, bool ALIGNED> cudaError_t launch_r(const RowsArgs &a, int sm_count, cudaStream_t s)
 {
-    if (a.N <= 16) return launch_t<R, 8>(a, sm_count, s);
-    if (a.N <= 32) return launch_t<R, 4>(a, sm_count, s);
-    if (a.N <= 64) return launch_t<R, 2>(a, sm_count, s);
-    return launch_t<R, 1>(a, sm_count, s);
+    if (a.N <= 16) return launch_t<R, 8, ALIGNED>(a, sm_count, s);
+    if (a.N <= 32) return launch_t<R, 4, ALIGNED>(a, sm_count, s);
+    if (a.N <= 64) return launch_t<R, 2, ALIGNED>(a, sm_count, s);
+    return launch_t<R, 1, ALIGNED>(a, sm_count, s);
 }
 
 }  // namespace
 
-// Called by launch_rows for operands it reads four columns per lane (a.c_scalar is set), a list without chunks and a plan
-// whose rows come in runs of a.run_rows.
-cudaError_t launch_block_rows(const RowsArgs &a, int sm_count, cudaStream_t s)
+// Called by launch_rows for a list without chunks and a plan whose rows come in runs of a.run_rows.  aligned: B is read four
+// columns per load.
+cudaError_t launch_block_rows(const RowsArgs &a, bool aligned, int sm_count, cudaStream_t s)
 {
-    return a.run_rows == 3 ? launch_r<3>(a, sm_count, s) : launch_r<2>(a, sm_count, s);
+    if (aligned) return a.run_rows == 3 ? launch_r<3, true>(a, sm_count, s) : launch_r<2, true>(a, sm_count, s);
+    return a.run_rows == 3 ? launch_r<3, false>(a, sm_count, s) : launch_r<2, false>(a, sm_count, s);
 }
 
 }  // namespace cutespmm

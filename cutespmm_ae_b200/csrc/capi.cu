@@ -336,6 +336,7 @@ static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B,
     a.num_chunks = all_rows ? p->every.chunks : p->own.chunks;
     a.chunk_owner = static_cast<const uint32_t *>(all_rows ? p->d_chunk_owner_all : p->d_chunk_owner);
     a.arrivals = p->d_arrivals + (all_rows ? (uint64_t)p->own.long_rows * kArrivalSlabs : 0);
+    a.dense_panels = h.num_bricks ? 1u : 0u;
     a.avg_row_nnz = (uint32_t)(h.nnz / std::max<uint64_t>(h.M, 1));
     a.short_chunks = item_sizes(h.nnz + kRowCost * h.M, h.nnz, h.M, 0, h.opts.split_nnz, h.opts.tile_nnz, h.adaptive_tiling).latency_bound ? 1u : 0u;
     a.B = B; a.C = C; a.scratch = p->d_scratch;
@@ -440,21 +441,28 @@ static void note_stream(const cutespmm_plan *p, cudaStream_t s)
     if (s != nullptr && s != cudaStreamLegacy && !p->used_elsewhere.load(std::memory_order_relaxed)) p->used_elsewhere = true;
 }
 
-// Rows of B that are not 16-byte aligned (N not a multiple of four columns, a view) cost the row kernel four times the
-// load instructions, each for a quarter of the bytes, and there is no form for several rows per warp.  Where the matrix
-// names a row of B often enough it pays to copy B once into rows of N rounded up to four (the copy lives on the stream):
-// measured, the row kernel gains about 12 ps per nonzero up to 64 columns and 0.4 ps per nonzero and column beyond (R-MAT
-// 2^18 N = 47: 186 -> 139 us, uniform 7 per row N = 201: 211 -> 125 us), the copy costs a launch and 8 bytes per element at
-// 6.4 TB/s.  Copies above kMaxPadBytes are not made: the pool would give them back at every synchronisation and map them anew
-// (1.8 GB: 4.6 -> 5.6 ms per product); wide products of large matrices go in narrower windows instead.  Even widths above 32 are read two columns per lane and gain nothing.  Not while the stream is being captured
-// (a graph should not own memory).
+// Rows of B that are not 16-byte aligned (N not a multiple of four columns, a view) are read one or two columns per lane and load.
+// Copying B once into rows of N rounded up to four first (the copy lives on the stream) costs a launch, 1.25 ps per element of the
+// copy and, as C is written column by column then, 1.6 ps per element of C; with the kernels for unaligned rows as they are it
+// pays in two ranges only (us without / with the copy):
+//   20 or 25 to 31 columns, short rows: the copy lets a warp take four rows with one load each; 6 ps per nonzero (7 per row
+//     N = 31 26.0 / 21.2, stencil512 52.5 / 37.9, elasticity40 N = 22 35.5 / 31.7; 4 per row N = 27 37.9 / 46.4: not there);
+//   33 to 64 and above 384 columns, rows long enough: 0.1 ps per nonzero and column (64 per row N = 47 37.0 / 35.1, N = 511
+//     258 / 234; N = 259 177 / 218; 7 per row N = 47 32.6 / 33.9).
+// Even widths above 32 are read two columns per lane and gain nothing.  Copies above kMaxPadBytes are not made: the pool would
+// give them back at every synchronisation and map them anew (1.8 GB: 4.6 -> 5.6 ms per product).  Not while the stream is being
+// captured (a graph should not own memory).
 constexpr uint64_t kMaxPadBytes = 512ull << 20;
-static bool worth_padding(const HostPlan &h, const float *B, uint64_t ldb, const float *C, uint64_t ldc, uint32_t N)
+static bool worth_padding(const cutespmm_plan *p, const cutespmm_list_sizes &list, const float *B, uint64_t ldb, const float *C, uint64_t ldc, uint32_t N)
 {
+    const HostPlan &h = p->host;
     const bool two = !((reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 7) && !((ldb | ldc | N) & 1);
-    if (two && N > 32) return false;
-    const uint64_t gain = h.nnz * (N <= 64 ? 12 : N * 2 / 5), cost = 3000000 + h.K * N * 5 / 4;  // picoseconds
-    return gain >= cost && h.K * ((uint64_t)N + 3) * sizeof(float) <= kMaxPadBytes;
+    if ((two && N > 32) || h.K * ((uint64_t)N + 3) * sizeof(float) > kMaxPadBytes) return false;
+    if (N <= 32) {
+        if (N < (h.run_rows ? 20u : 25u) || list.chunks || h.nnz >= 24 * h.M) return false;
+        return h.nnz * 6 >= 3000000 + h.K * N * 5 / 4;  // picoseconds
+    }
+    return (N <= 64 || N > 384) && h.nnz * N / 10 >= 3000000 + N * (h.K * 13 + h.M * 16) / 10;
 }
 
 static bool capturing(cudaStream_t s)
@@ -481,11 +489,6 @@ static ColumnWindow column_window(const cutespmm_plan *p, const float *B, uint64
     const HostPlan &h = p->host;
     ColumnWindow w{};
     w.cols = left < kScratchCols ? left : kScratchCols;
-    // rows of B off the 16-byte grid: a window is narrowed until a padded copy of it may be made
-    if (((reinterpret_cast<uintptr_t>(B) & 15) || (ldb & 3)) && h.K * ((uint64_t)w.cols + 3) * sizeof(float) > kMaxPadBytes) {
-        const uint64_t fit = kMaxPadBytes / (h.K * sizeof(float)) / 128 * 128;
-        if (fit && fit < w.cols && worth_padding(h, B, ldb, C, ldc, (uint32_t)fit) && may_copy()) w.cols = (uint32_t)fit;
-    }
     w.slab = h.slab_panels && slab_supports(w.cols, ldb, ldc, B, C);
     w.brick = use_brick(p, B, ldb, C, ldc, w.cols);
     // brick panels whose shape the brick kernel does not take (N not a multiple of 32, unaligned
@@ -494,7 +497,7 @@ static ColumnWindow column_window(const cutespmm_plan *p, const float *B, uint64
     const cutespmm_list_sizes &list = w.all_rows ? p->every : p->own;
     w.rows = list.tiles || list.chunks;
     const bool aligned = !(reinterpret_cast<uintptr_t>(B) & 15) && !(ldb & 3) && (!(w.cols & 3) || b_padded);
-    w.pad = !aligned && w.rows && whole && worth_padding(h, B, ldb, C, ldc, w.cols) && may_copy();
+    w.pad = !aligned && w.rows && whole && worth_padding(p, list, B, ldb, C, ldc, w.cols) && may_copy();
     return w;
 }
 

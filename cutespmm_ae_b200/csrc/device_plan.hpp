@@ -78,6 +78,7 @@ struct RowsArgs {
     uint32_t N;
     uint32_t num_rows;         // of the whole matrix
     uint32_t run_rows;         // rows come in aligned runs of this many (2 or 3) with the same columns; 0: they do not
+    uint32_t dense_panels;     // 1: some panels of 16 rows are dense enough for the tensor cores: neighbouring rows share columns
     uint32_t early;            // 1: the plan's arrays never change, its first tiles can be fetched before the kernel in front is done
     uint32_t b_padded;         // 1: a row of B can be read up to N rounded up to four columns
     uint32_t slab_cols;        // set by launch_rows: columns per slab of blocks (a multiple of 4)
@@ -86,7 +87,7 @@ struct RowsArgs {
     const uint32_t *row_map;   // reordered plan: row r of the work lists is row row_map[r] of C (nullptr: identity)
 };
 
-cudaError_t launch_block_rows(const RowsArgs &a, int sm_count, cudaStream_t s);
+cudaError_t launch_block_rows(const RowsArgs &a, bool aligned, int sm_count, cudaStream_t s);
 cudaError_t launch_rows(const RowsArgs &a, int sm_count, cudaStream_t s);
 // dst: rows x (N rounded up to 4) floats, 16-byte aligned
 cudaError_t launch_pad_rows(const float *src, uint64_t ld_src, float *dst, uint64_t rows, uint32_t N, int sm_count, cudaStream_t s);

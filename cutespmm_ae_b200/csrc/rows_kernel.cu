@@ -8,8 +8,9 @@
 // (one float4 each at N = 128, so a row of B is one coalesced 512-byte request), the row's
 // (column, value) pairs are read from the block's staged tile in shared memory (tile_stage.cuh; one
 // broadcast read per nonzero), and the products are accumulated in fp32 registers in storage order.
-// For narrow products (N <= 64) a warp splits into groups of N/4 lanes and owns that many rows at
-// once.  The eight warps of a block claim the rows of one scheduling tile as they go, so rows that
+// For narrow products (N <= 64) a warp splits into groups of lanes and owns that many rows at
+// once.  Rows of B that are not 16-byte aligned are read one or two columns per lane and load, the lanes'
+// columns interleaved, with as many loads in flight as the registers hold.  The eight warps of a block claim the rows of one scheduling tile as they go, so rows that
 // share columns (stencils, block structure) meet in L1.  C rows are written once with streaming
 // stores; nothing is read-modify-written: a long row is cut into chunks whose partial sums go to a
 // scratch matrix and are added, in slot order, by whichever warp finishes the row's last chunk (one
@@ -34,12 +35,15 @@ namespace {
 //   DEEP = true   8 rows in flight, 4 blocks per SM: fewer dependent steps per row, better for long rows and when
 //                 the whole job is a single wave of tiles and the time is a handful of latencies.
 template <bool DEEP> struct Tuning {
-    static constexpr int kUnroll = DEEP ? 8 : 4;
     // 48 registers, 40 warps per SM (the lane-group kernels spill 200 bytes at 40 registers and 48 warps: R-MAT 2^17 N = 64
     // 55.8 -> 50.8 us, 800 000 rows of 4 at N = 32 74 -> 65, R-MAT 2^20 N = 128 662 -> 647); the narrow kernels that deal
     // tiles by a counter have long rows to hide and keep 48 warps (R-MAT 2^20 N = 32: 266 us, 281 with 40)
     static constexpr int min_blocks(bool dyn, int G) { return DEEP ? 4 : dyn && G >= 4 ? 6 : 5; }
 };
+// Rows of B in flight per warp (or group): 16 (deep: 32) registers of B, eight rows at most.  Two column groups of two columns stay
+// at four rows: with eight the deep form spills (4096 x 4096 with 16 per row at N = 66 3.8 -> 4.6 us).
+template <int VEC, int CH, bool DEEP>
+constexpr int kRowsInFlight = VEC == 2 && CH == 2 ? 4 : (DEEP ? 32 : 16) / (VEC * CH) < 8 ? (DEEP ? 32 : 16) / (VEC * CH) : 8;
 constexpr int kWarps = kTileWarps;
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -97,7 +101,7 @@ __device__ __forceinline__ void accumulate(typename Vec<VEC>::T (&acc)[CH], cons
     using V = typename Vec<VEC>::T;
     // nonzeros in flight per step.  Eight with float4 lanes in the shallow tuning spilled and gained nothing (at 40 registers); the
     // deep tuning and narrow lanes have the registers, and a deeper step shortens the chain of a latency-bound job
-    constexpr int U = DEEP ? 8 / CH : ((CH == 1) ? (VEC == 4 ? 4 : 8) : 2);
+    constexpr int U = kRowsInFlight<VEC, CH, DEEP>;
     for (uint32_t j = j0; j < j1; j += 32) {
         const uint32_t n = min(32u, j1 - j);
         uint2 pr = make_uint2(0u, 0u);
@@ -140,7 +144,7 @@ __device__ __forceinline__ void accumulate(typename Vec<VEC>::T (&acc)[CH], cons
 // acc[ch] += sum of val * B[col][lane's columns] over `cnt` staged (column, value) pairs, UU rows of B in flight.
 // TAIL: cnt may be smaller than UU; the surplus positions load the row of the last pair again (an L1 hit) and
 // are left out of the sum.
-template <int VEC, int CH, bool FULL, int UU, bool TAIL>
+template <int VEC, int CH, int L, bool FULL, int UU, bool TAIL>
 __device__ __forceinline__ void row_group(typename Vec<VEC>::T (&acc)[CH], const uint2 *pairs_smem, uint32_t cnt, const float *__restrict__ bl,
                                           uint32_t ldb32, const bool (&ok)[CH])
 {
@@ -154,7 +158,7 @@ __device__ __forceinline__ void row_group(typename Vec<VEC>::T (&acc)[CH], const
         const float *row = bl + (uint64_t)pr.x * ldb32;
 #pragma unroll
         for (int ch = 0; ch < CH; ++ch) {
-            if (FULL || ok[ch]) b[u][ch] = ldg_b(reinterpret_cast<const V *>(row + ch * 32 * VEC));
+            if (FULL || ok[ch]) b[u][ch] = ldg_b(reinterpret_cast<const V *>(row + ch * L * VEC));
             else zero_vec(b[u][ch]);
         }
     }
@@ -192,7 +196,7 @@ __device__ __forceinline__ void accumulate_group(typename Vec<VEC>::T (&acc)[CH]
                 const float *row = bl + (uint64_t)c * ldb32;
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch) {
-                    if (FULL || ok[ch]) b[u][ch] = ldg_b(reinterpret_cast<const V *>(row + ch * 32 * VEC));
+                    if (FULL || ok[ch]) b[u][ch] = ldg_b(reinterpret_cast<const V *>(row + ch * L * VEC));
                     else zero_vec(b[u][ch]);
                 }
             }
@@ -234,7 +238,7 @@ __device__ __forceinline__ void accumulate_shared(typename Vec<VEC>::T (&acc)[CH
                 const float *row = bl + (uint64_t)c * ldb32;
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch) {  // positions past the end load nothing and add nothing
-                    if (at < n && (FULL || ok[ch])) b[u][ch] = ldg_b(reinterpret_cast<const V *>(row + ch * 32 * VEC));
+                    if (at < n && (FULL || ok[ch])) b[u][ch] = ldg_b(reinterpret_cast<const V *>(row + ch * (32 / G) * VEC));
                     else zero_vec(b[u][ch]);
                 }
             }
@@ -248,15 +252,18 @@ __device__ __forceinline__ void accumulate_shared(typename Vec<VEC>::T (&acc)[CH
 
 // acc = the sum over the groups of a warp, pairwise in a fixed tree (the result depends on nothing but the group size), in
 // every lane.
-template <int L> __device__ __forceinline__ void add_groups(float4 &acc)
+__device__ __forceinline__ float4 from_lane(const float4 &a, int off)
+{
+    return make_float4(__shfl_xor_sync(kFull, a.x, off), __shfl_xor_sync(kFull, a.y, off), __shfl_xor_sync(kFull, a.z, off), __shfl_xor_sync(kFull, a.w, off));
+}
+__device__ __forceinline__ float2 from_lane(const float2 &a, int off) { return make_float2(__shfl_xor_sync(kFull, a.x, off), __shfl_xor_sync(kFull, a.y, off)); }
+__device__ __forceinline__ float from_lane(const float &a, int off) { return __shfl_xor_sync(kFull, a, off); }
+template <int L, class V, int CH> __device__ __forceinline__ void add_groups(V (&acc)[CH])
 {
 #pragma unroll
-    for (int off = L; off < 32; off <<= 1) {
-        acc.x += __shfl_xor_sync(kFull, acc.x, off);
-        acc.y += __shfl_xor_sync(kFull, acc.y, off);
-        acc.z += __shfl_xor_sync(kFull, acc.z, off);
-        acc.w += __shfl_xor_sync(kFull, acc.w, off);
-    }
+    for (int off = L; off < 32; off <<= 1)
+#pragma unroll
+        for (int ch = 0; ch < CH; ++ch) add_vec(acc[ch], from_lane(acc[ch], off));
 }
 
 // What the chunk part of the kernel needs.  The pointers bl / scratch / C already point at this lane's first column.
@@ -286,7 +293,7 @@ __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
     const bool lead = P == 1 ? lane == 0 : sub == 0;
     bool ok[CH];
 #pragma unroll
-    for (int ch = 0; ch < CH; ++ch) ok[ch] = FULL || (a.col0 + ch * 32 * VEC < a.N);
+    for (int ch = 0; ch < CH; ++ch) ok[ch] = FULL || (a.col0 + ch * L * VEC < a.N);
     // chunk (group) c goes to block c mod gridDim.x: spread over the SMs, and the warps of a block that got none
     // start on the block's tile at once (rows of a tile are claimed as they go, so they take over the others' share)
     const uint32_t gw = warp * gridDim.x + blockIdx.x, nw = gridDim.x * kWarps;
@@ -309,16 +316,16 @@ __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
         if constexpr (G == 1) {
             accumulate<VEC, CH, FULL, DEEP>(acc, a.pairs, ck.y, ck.z, a.bl, a.ldb, ok, lane);
         } else if constexpr (!SHARE) {
-            accumulate_group<VEC, CH, FULL, Tuning<DEEP>::kUnroll, L>(acc, a.pairs, ck.y, ck.z, a.bl, (uint32_t)a.ldb, ok, sub, ((1u << L) - 1u) << (grp * L));
+            accumulate_group<VEC, CH, FULL, kRowsInFlight<VEC, CH, DEEP>, L>(acc, a.pairs, ck.y, ck.z, a.bl, (uint32_t)a.ldb, ok, sub, ((1u << L) - 1u) << (grp * L));
         } else {
-            accumulate_shared<VEC, CH, FULL, Tuning<DEEP>::kUnroll, G>(acc, a.pairs, ck.y, ck.z, a.bl, (uint32_t)a.ldb, ok, lane, grp);
-            add_groups<L>(acc[0]);
+            accumulate_shared<VEC, CH, FULL, kRowsInFlight<VEC, CH, DEEP>, G>(acc, a.pairs, ck.y, ck.z, a.bl, (uint32_t)a.ldb, ok, lane, grp);
+            add_groups<L>(acc);
         }
         if (P == 1 ? (G == 1 || grp == 0) : have) {
             float *out = a.scratch + (uint64_t)ck.w * a.ld_scratch;
 #pragma unroll
             for (int ch = 0; ch < CH; ++ch)
-                if (FULL || ok[ch]) __stcg(reinterpret_cast<V *>(out + ch * 32 * VEC), acc[ch]);
+                if (FULL || ok[ch]) __stcg(reinterpret_cast<V *>(out + ch * L * VEC), acc[ch]);
         }
         __threadfence();  // this lane's part of the slot is visible device-wide before the arrival is counted
         __syncwarp();
@@ -342,21 +349,21 @@ __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
         for (int q = 0; q < P; ++q) {
             const uint32_t s0 = __shfl_sync(kFull, slot0, q * L), s1 = __shfl_sync(kFull, slot1, q * L), row = __shfl_sync(kFull, lr_row, q * L);
             if (s1 > s0) {  // the same for every lane of the warp
-                constexpr int R = (VEC * CH >= 8) ? 4 : 8;  // slots in flight
+                constexpr int R = VEC * CH >= 8 || CH >= 4 ? 4 : 8;  // slots in flight
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch) zero_vec(acc[ch]);
 #pragma unroll R
                 for (uint32_t k = s0 + grp; k < s1; k += G) {
 #pragma unroll
                     for (int ch = 0; ch < CH; ++ch)
-                        if (FULL || ok[ch]) add_vec(acc[ch], __ldcg(reinterpret_cast<const V *>(a.scratch + (uint64_t)k * a.ld_scratch + ch * 32 * VEC)));
+                        if (FULL || ok[ch]) add_vec(acc[ch], __ldcg(reinterpret_cast<const V *>(a.scratch + (uint64_t)k * a.ld_scratch + ch * L * VEC)));
                 }
-                if constexpr (G > 1) add_groups<L>(acc[0]);
+                if constexpr (G > 1) add_groups<L>(acc);
                 if (G == 1 || grp == 0) {
                     float *crow = a.C + (uint64_t)row * a.ldc;
 #pragma unroll
                     for (int ch = 0; ch < CH; ++ch)
-                        if (FULL || ok[ch]) store_row<FULL>(crow + ch * 32 * VEC, acc[ch], a.c_scalar, a.N - a.col0 - ch * 32 * VEC);
+                        if (FULL || ok[ch]) store_row<FULL>(crow + ch * L * VEC, acc[ch], a.c_scalar, a.N - a.col0 - ch * L * VEC);
                 }
             }
         }
@@ -364,14 +371,13 @@ __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
     }
 }
 
-// G = rows of A (or chunks) a warp works on at the same time.  G = 1: the 32 lanes span 32*VEC*CH columns of B.
-// G = 2, 4, 8 (narrow products, N <= 64, float4 lanes): the warp is G groups of 32/G lanes, a group spans the whole
-// row of B and owns a row of A of its own, so a warp keeps G times as many gathers in flight and no lane idles.
+// G = rows of A (or chunks) a warp works on at the same time: it is G groups of L = 32/G lanes, and a group spans L * VEC * CH
+// columns, CH groups of L * VEC neighbouring ones.  G > 1 (narrow products): a group spans the whole row of B and owns a row of A
+// of its own, so a warp keeps G times as many gathers in flight and few lanes idle.
 template <int VEC, int CH, bool FULL, bool DEEP, int G, bool DYN>
 __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DYN, G)) spmm_rows_kernel(RowsArgs a)
 {
     using V = typename Vec<VEC>::T;
-    static_assert(G == 1 || (VEC == 4 && CH == 1), "row groups are for float4 lanes and one column group");
     constexpr int L = 32 / G;  // lanes of a group
     const int lane = threadIdx.x & 31;
     const int grp = G == 1 ? 0 : lane / L, sub = G == 1 ? lane : lane % L;
@@ -379,7 +385,7 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DYN, G))
     const uint32_t end = min(a.N, (blockIdx.y + 1) * a.slab_cols);       // ... and the end of the block's slab
     bool ok[CH];
 #pragma unroll
-    for (int ch = 0; ch < CH; ++ch) ok[ch] = FULL || (col0 + ch * 32 * VEC < end);
+    for (int ch = 0; ch < CH; ++ch) ok[ch] = FULL || (col0 + ch * L * VEC < end);
     const float *bl = a.B + col0;
     const uint32_t ldb32 = (uint32_t)a.ldb;  // < 2^32 (checked by the caller): one 32x32->64 multiply per address
     const uint2 *pairs = reinterpret_cast<const uint2 *>(a.pairs);
@@ -429,20 +435,20 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DYN, G))
                 V acc[CH];
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch) zero_vec(acc[ch]);
-                constexpr int U = (CH == 1) ? Tuning<DEEP>::kUnroll : Tuning<DEEP>::kUnroll / 2;  // rows of B in flight per group and step
+                constexpr int U = kRowsInFlight<VEC, CH, DEEP>;  // rows of B in flight per group and step
                 uint32_t j = j0 - jb, jend = j1 - jb;  // positions in the staged pair slice
-                for (; j + U <= jend; j += U) row_group<VEC, CH, FULL, U, false>(acc, st.pairs + j, U, bl, ldb32, ok);
+                for (; j + U <= jend; j += U) row_group<VEC, CH, L, FULL, U, false>(acc, st.pairs + j, U, bl, ldb32, ok);
                 // what is left of the row (fewer than U nonzeros) goes as one more group, so that its loads are in flight
                 // together instead of one after the other: positions past the end repeat the row's last pair and are not added
                 if (const uint32_t rem = jend - j) {
-                    if (rem > U / 2) row_group<VEC, CH, FULL, U, true>(acc, st.pairs + j, rem, bl, ldb32, ok);
-                    else row_group<VEC, CH, FULL, U / 2, true>(acc, st.pairs + j, rem, bl, ldb32, ok);
+                    if (rem > U / 2) row_group<VEC, CH, L, FULL, U, true>(acc, st.pairs + j, rem, bl, ldb32, ok);
+                    else row_group<VEC, CH, L, FULL, U / 2, true>(acc, st.pairs + j, rem, bl, ldb32, ok);
                 }
                 const uint32_t r_out = a.row_map ? __ldg(a.row_map + r) : r;  // a reordered plan writes the row to its place in the caller's C
                 float *out = a.C + (uint64_t)r_out * a.ldc + col0;
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch)
-                    if (FULL || ok[ch]) store_row<FULL>(out + ch * 32 * VEC, acc[ch], a.c_scalar != 0, end - col0 - ch * 32 * VEC);
+                    if (FULL || ok[ch]) store_row<FULL>(out + ch * L * VEC, acc[ch], a.c_scalar != 0, end - col0 - ch * L * VEC);
             }
             if constexpr (G > 1) __syncwarp();
         }
@@ -468,15 +474,15 @@ cudaError_t launch_rows_t(RowsArgs a, uint32_t slabs, int sm_count, cudaStream_t
     // Slabs get equal shares of the grid, so a small job's are of equal width (uniform 15727 x 13804 at N = 260: 33.4 us as 256 + 4
     // columns, 24.5 as 132 + 128); large ones are bound by the gathers' bytes and keep whole lines (170003 x 99991 at N = 384:
     // 225 us as 256 + 128, 256 as 192 + 192).
-    a.slab_cols = (uint64_t)a.num_tiles <= (uint64_t)sm_count * 6 ? ((a.N + slabs - 1) / slabs + 3) & ~3u : 32 / G * VEC * CH;
+    // Rows off the 16-byte grid have no whole lines to keep (64 per row N = 334 207 -> 152 us).
+    a.slab_cols = VEC < 4 || (uint64_t)a.num_tiles <= (uint64_t)sm_count * 6 ? ((a.N + slabs - 1) / slabs + 3) & ~3u : 32 / G * VEC * CH;
     int n = 0;
     cudaError_t e;
-    if constexpr (VEC == 4)
-        if (a.counters && slabs <= kDealtSlabs) {  // tiles dealt by a counter: where there are enough to deal
-            if ((e = blocks_per_sm<spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true>>(n, kWarps * 32)) != cudaSuccess) return e;
-            if (a.num_tiles >= 8ull * grid(n))
-                return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true>, dim3(grid(n), slabs), kWarps * 32, 0, s, a);
-        }
+    if (a.counters && slabs <= kDealtSlabs) {  // tiles dealt by a counter: where there are enough to deal
+        if ((e = blocks_per_sm<spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true>>(n, kWarps * 32)) != cudaSuccess) return e;
+        if (a.num_tiles >= 8ull * grid(n))
+            return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true>, dim3(grid(n), slabs), kWarps * 32, 0, s, a);
+    }
     if ((e = blocks_per_sm<spmm_rows_kernel<VEC, CH, FULL, DEEP, G, false>>(n, kWarps * 32)) != cudaSuccess) return e;
     return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, false>, dim3(grid(n), slabs), kWarps * 32, 0, s, a);
 }
@@ -521,6 +527,7 @@ cudaError_t launch_pad_rows(const float *src, uint64_t ld_src, float *dst, uint6
 }
 
 // Picks the widest vector the pointers, leading dimensions and N allow.
+constexpr uint32_t kLongRows = 24;  // nonzeros per row from which fewer, wider groups win on rows off the 16-byte grid
 cudaError_t launch_rows(const RowsArgs &args, int sm_count, cudaStream_t s)
 {
     RowsArgs a = args;
@@ -536,8 +543,8 @@ cudaError_t launch_rows(const RowsArgs &args, int sm_count, cudaStream_t s)
     // fewer runs than a block per SM has lane groups keep the row kernel: they need the rows to fill the machine
     // (elasticity12 at N = 64: 4.1 us, 4.3 by runs).
     const uint64_t groups = (uint64_t)sm_count * kWarps * (N <= 16 ? 8 : N <= 32 ? 4 : N <= 64 ? 2 : 1);
-    if (a.run_rows && v4 && a.num_chunks == 0 && !a.row_map && a.num_rows / a.run_rows * ((N + 127) / 128) >= groups)
-        return launch_block_rows(a, sm_count, s);
+    if (a.run_rows && a.num_chunks == 0 && !a.row_map && a.num_rows / a.run_rows * ((N + 127) / 128) >= groups)
+        return launch_block_rows(a, v4, sm_count, s);
     // deep: at most one resident wave of tiles, or long rows (R-MAT 2^24 with 300 nonzeros per row 2.19 against 2.38 ms, with 21
     // 1.88 against 1.93; with 15 R-MAT 2^20 0.652 against 0.647 and 3.4 per row 1.50 against 1.48 in favour of shallow).  Two
     // column groups per lane halve the rows in flight, and deep pays from shorter rows on: N = 256, R-MAT 2^18 (15 per row) 275
@@ -554,29 +561,61 @@ cudaError_t launch_rows(const RowsArgs &args, int sm_count, cudaStream_t s)
         return full(w) ? launch_rows_t<VEC, CH, true, false>(a, slabs, sm_count, s)             \
                             : launch_rows_t<VEC, CH, false, false>(a, slabs, sm_count, s);     \
     } while (0)
-    if (v4 && N <= 64) {  // narrow products: G rows of A per warp, a group of 32/G float4 lanes spans the row of B
-#define CUTESPMM_GROUPS(G)                                                                              \
-    do {                                                                                                \
-        if (deep) return full(128 / G) ? launch_rows_t<4, 1, true, true, G>(a, 1, sm_count, s)         \
-                                        : launch_rows_t<4, 1, false, true, G>(a, 1, sm_count, s);       \
-        return full(128 / G) ? launch_rows_t<4, 1, true, false, G>(a, 1, sm_count, s)                  \
-                              : launch_rows_t<4, 1, false, false, G>(a, 1, sm_count, s);                \
+    // narrow products: G rows of A per warp, a group of 32/G lanes spans the row of B
+#define CUTESPMM_GROUPS(VEC, CH, G)                                                                        \
+    do {                                                                                                   \
+        constexpr uint32_t w = 32 / G * VEC * CH;                                                          \
+        if (deep) return full(w) ? launch_rows_t<VEC, CH, true, true, G>(a, 1, sm_count, s)                \
+                                 : launch_rows_t<VEC, CH, false, true, G>(a, 1, sm_count, s);              \
+        return full(w) ? launch_rows_t<VEC, CH, true, false, G>(a, 1, sm_count, s)                         \
+                       : launch_rows_t<VEC, CH, false, false, G>(a, 1, sm_count, s);                       \
     } while (0)
-        if (N <= 16) CUTESPMM_GROUPS(8);
-        if (N <= 32) CUTESPMM_GROUPS(4);
-        CUTESPMM_GROUPS(2);
-#undef CUTESPMM_GROUPS
+    if (v4) {
+        if (N <= 16) CUTESPMM_GROUPS(4, 1, 8);
+        if (N <= 32) CUTESPMM_GROUPS(4, 1, 4);
+        if (N <= 64) CUTESPMM_GROUPS(4, 1, 2);
     }
     if (v4) {
         if (N > 128) CUTESPMM_GO(4, 2);
         CUTESPMM_GO(4, 1);
     }
+    // Rows off the 16-byte grid: two columns per load where they lie on the 8-byte grid, one otherwise, the lanes' columns
+    // interleaved.  A warp covers up to 256 columns (before: 64 of them, with two rows in flight: R-MAT 2^20 N = 203 3501 -> 1485 us,
+    // N = 511 12990 -> 3984, stencil512 N = 101 133 -> 96.6) and takes several rows up to 64 (one before; N = 7 R-MAT 2^17 47.4 -> 29.0,
+    // 64 per row 22.3 -> 17.4, which took a padded copy of B until then).  How many, by what was measured (us, more groups / fewer):
+    //   few_rows    fewer rows than warps: one row per warp (4096 x 16 per row N = 27 3.6 / 3.0);
+    //   few_groups  long rows and no chunks, or a small job: N = 47 64 per row 41.7 / 37.0, R-MAT 2^14 17.2 / 14.4; against them
+    //               stencil512 53.9 / 82, R-MAT 2^17 67.4 / 70.6;
+    //   runs_long   long rows, chunks among them: N = 7 R-MAT 2^17 35.3 / 29.0, stencil512 15.8 / 21.8; N = 27 34.0 / 27.0 with 64
+    //               per row, 37.9 / 43.6 with 4;
+    //   dense_panels  neighbouring rows share columns, and their gathers hit L1: N = 13 stencil512 19.5 / 26.3, 7 per row 17.3 / 14.6.
+    const bool few_rows = a.num_rows < (uint32_t)sm_count * 40;
+    const bool runs_long = a.num_chunks || a.avg_row_nnz >= kLongRows;
+    const bool few_groups = a.num_rows < (uint32_t)sm_count * 160 || (!a.num_chunks && a.avg_row_nnz >= kLongRows);
     if (v2 && N > 32) {
+        if (N > 128) CUTESPMM_GO(2, 4);
         if (N > 64) CUTESPMM_GO(2, 2);
-        CUTESPMM_GO(2, 1);
+        if (few_groups) CUTESPMM_GO(2, 1);
+        CUTESPMM_GROUPS(2, 2, 2);
     }
-    if (N > 32) CUTESPMM_GO(1, 2);
-    CUTESPMM_GO(1, 1);
+    if (N > 128) CUTESPMM_GO(1, 8);
+    if (N > 64) CUTESPMM_GO(1, 4);
+    if (N > 32) {
+        if (few_groups) CUTESPMM_GO(1, 2);
+        CUTESPMM_GROUPS(1, 4, 2);
+    }
+    if (few_rows) CUTESPMM_GO(1, 1);
+    if (N > 16) {
+        if (runs_long) CUTESPMM_GROUPS(1, 2, 2);
+        CUTESPMM_GROUPS(1, 4, 4);
+    }
+    if (N > 8) {
+        if (a.dense_panels) CUTESPMM_GROUPS(1, 4, 8);
+        CUTESPMM_GROUPS(1, 2, 4);
+    }
+    if (runs_long) CUTESPMM_GROUPS(1, 1, 4);
+    CUTESPMM_GROUPS(1, 2, 8);
+#undef CUTESPMM_GROUPS
 #undef CUTESPMM_GO
 }
 

@@ -467,8 +467,37 @@ def test_rows_in_runs_of_the_same_columns(oracle_mod, run, N):
                 assert torch.isnan(out[A.M]).all() and p.device_status() == 0
 
 
+@pytest.mark.parametrize("shape", ["few", "short", "long", "chunks", "band"])
+@pytest.mark.parametrize("N", [1, 8, 9, 16, 17, 24, 31, 32, 33, 34, 63, 64, 65, 127, 129, 250, 257, 509])
+def test_operands_off_the_16_byte_grid(oracle_mod, shape, N):
+    """One form of the row kernel per width, alignment (4 or 8 bytes) and kind of matrix: few rows, short rows, long rows, rows cut
+    into chunks, neighbouring rows with the same columns.  B and C are views into wider arrays, so nothing beside C's columns may
+    be written; the aligned form's result is the same sum (chunks: in another order)."""
+    rng = np.random.default_rng(N)
+    M, K = {"few": (300, 700), "band": (96 * 96, 96 * 96)}.get(shape, (24001, 997))
+    if shape == "band":
+        A = g.stencil9(96, 96, 5)
+    else:
+        ln = rng.integers(0, 13, M) if shape != "long" else rng.integers(20, 40, M)
+        if shape == "chunks":
+            ln[rng.integers(0, M, 40)] = rng.integers(100, 2500, 40)
+        rp = np.concatenate([[0], np.cumsum(ln)])
+        A = g.CsrMatrix(M, K, torch.from_numpy(rp), torch.from_numpy(rng.integers(0, K, rp[-1]).astype(np.int32)), torch.from_numpy(rng.standard_normal(rp[-1]).astype(np.float32)))
+    plan = cs.Plan.from_device_csr(A.M, A.K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), **({"min_brick_panels": 1} if shape == "band" else {"path": cs.PATH_ROWS}))
+    B = g.dense_operand(A.K, N, 6)
+    want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.numpy(), A.M, A.K)
+    for shift, wide in ((1, N + 2 + N % 2), (2, N + 4 + N % 2)):  # 4- and 8-byte aligned rows
+        Bd = torch.full((A.K, wide), float("nan"), device="cuda")
+        Cd = torch.full((A.M, wide), float("nan"), device="cuda")
+        Bd[:, shift:shift + N] = B.cuda()
+        plan.spmm(Bd[:, shift:shift + N], Cd[:, shift:shift + N])
+        got = Cd[:, shift:shift + N].cpu().numpy()
+        assert oracle_mod.rel_fro(want, got) <= REL_FRO_TOL_FP32  # two fp32 sums in (almost) the same order
+        assert torch.isnan(Cd[:, :shift]).all() and torch.isnan(Cd[:, shift + N:]).all() and plan.device_status() == 0
+
+
 def test_wide_unaligned_products_of_large_matrices_go_in_windows(oracle_mod):
-    """A padded copy of B above 512 MiB is made window by window; rows in runs take the run kernel in every window."""
+    """Columns of B that a padded copy of 512 MiB would not hold; rows in runs take the run kernel in every window of 512."""
     A = g.elasticity3d(48, 3, 9)  # 331776 rows: 409 columns are 543 MB
     N = 409
     p = cs.Plan.from_device_csr(A.M, A.K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS)
