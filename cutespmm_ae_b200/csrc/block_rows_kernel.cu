@@ -7,7 +7,10 @@
 // share loads between the rows of a panel on the tensor cores, kernel.cu:119-288).
 // Here the pipe is 58 % busy and instruction issue 70 %.
 // Rows of B off the 16-byte grid are read one column per load, the lanes' columns interleaved (elasticity40 N = 63 60.5 -> 51 us, N = 203
-// 222 -> 165, N = 334 654 -> 360; before, after a padded copy of B or one row at a time).
+// 222 -> 165; before, after a padded copy of B or one row at a time).
+// Products wider than 128 columns go in slabs of equal width, and a block walks its tile once per slab, so that nobody waits for a
+// narrow last slab's blocks and the tile's rows of B are near for all of them (elasticity40 N = 300 284 -> 199 us, N = 132 130 -> 119,
+// N = 511 478 -> 335; slabs side by side in the grid before).  Jobs of less than a wave of tiles spread the slabs over blocks.
 // Row kernel -> here: elasticity40 N = 32 35.1 -> 25.7 us, N = 27 48.7 -> 34.2; elasticity20 N = 128 20.4 -> 12.8.
 #include <cuda_runtime.h>
 
@@ -61,10 +64,6 @@ __global__ void __launch_bounds__(kTileWarps * 32, 4) spmm_block_rows_kernel(Row
 {
     constexpr int L = 32 / G, U = kUnroll;
     const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
-    const uint32_t col0 = blockIdx.y * 128 + (ALIGNED ? sub * 4 : sub);  // a lane's columns: four from here on, or every L-th
-    const bool ok = col0 < a.N;
-    const uint32_t cols = ok ? a.N - col0 : 0u;
-    const float *bl = a.B + col0;
     const uint32_t ldb = (uint32_t)a.ldb;
 
     __shared__ TileRing ring;
@@ -87,9 +86,16 @@ __global__ void __launch_bounds__(kTileWarps * 32, 4) spmm_block_rows_kernel(Row
         const uint32_t rb = d.x & ~3u, jb = d.z & ~1u, run0 = d.x / R, runs = (d.y + R - 1) / R - run0;
         for (;;) {
             const uint32_t claimed = tile_claim_rows(ring, s, (uint32_t)G, lane);
-            if (claimed >= runs) break;
-            const uint32_t run = claimed + grp;
-            if (run < runs) {
+            // a wide product's block walks its tile once per slab of columns
+            const uint32_t walk = G == 1 ? claimed / runs : 0u, slab0 = (G == 1 ? blockIdx.y + walk * gridDim.y : 0u) * a.slab_cols;
+            if (G == 1 ? slab0 >= a.N : claimed >= runs) break;
+            const uint32_t run = G == 1 ? claimed - walk * runs : claimed + grp;
+            if (G == 1 || run < runs) {
+                const uint32_t col0 = slab0 + (ALIGNED ? sub * 4 : sub);  // a lane's columns: four from here on, or every L-th
+                const uint32_t end = min(a.N, slab0 + a.slab_cols);       // the slab's end
+                const bool ok = col0 < end;
+                const uint32_t cols = ok ? end - col0 : 0u;
+                const float *bl = a.B + col0;
                 const uint32_t r0 = (run0 + run) * R, lo = max(r0, d.x), hi = min(r0 + R, d.y);
                 // rows of the run outside the tile stand in for a row inside it; they are not stored
                 uint32_t first[R];
@@ -126,15 +132,15 @@ __global__ void __launch_bounds__(kTileWarps * 32, 4) spmm_block_rows_kernel(Row
     }
 }
 
-template <int R, int G, bool ALIGNED> cudaError_t launch_t(const RowsArgs &a, int sm_count, cudaStream_t s)
+template <int R, int G, bool ALIGNED> cudaError_t launch_t(RowsArgs a, int sm_count, cudaStream_t s)
 {
     int per_sm = 0;
     const cudaError_t e = blocks_per_sm<spmm_block_rows_kernel<R, G, ALIGNED>>(per_sm, kTileWarps * 32);
     if (e != cudaSuccess) return e;
     const uint32_t slabs = (a.N + 127) / 128, wave = (uint32_t)(sm_count * per_sm);
-    uint32_t gx = a.num_tiles < wave ? a.num_tiles : wave;
-    if (slabs > 1) gx = (gx + slabs - 1) / slabs;
-    return launch_overlapped(spmm_block_rows_kernel<R, G, ALIGNED>, dim3(gx, slabs), kTileWarps * 32, 0, s, a);
+    const bool spread = a.num_tiles < wave;  // slabs beside each other in the grid
+    a.slab_cols = ((a.N + slabs - 1) / slabs + 3) & ~3u;
+    return launch_overlapped(spmm_block_rows_kernel<R, G, ALIGNED>, spread ? dim3((a.num_tiles + slabs - 1) / slabs, slabs) : dim3(wave), kTileWarps * 32, 0, s, a);
 }
 template <int R, bool ALIGNED> cudaError_t launch_r(const RowsArgs &a, int sm_count, cudaStream_t s)
 {

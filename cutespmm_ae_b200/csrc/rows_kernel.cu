@@ -471,11 +471,13 @@ cudaError_t launch_rows_t(RowsArgs a, uint32_t slabs, int sm_count, cudaStream_t
         const uint64_t gx = ((work < want ? work : want) + slabs - 1) / slabs;
         return (uint32_t)(gx ? gx : 1);
     };
-    // Slabs get equal shares of the grid, so a small job's are of equal width (uniform 15727 x 13804 at N = 260: 33.4 us as 256 + 4
-    // columns, 24.5 as 132 + 128); large ones are bound by the gathers' bytes and keep whole lines (170003 x 99991 at N = 384:
-    // 225 us as 256 + 128, 256 as 192 + 192).
-    // Rows off the 16-byte grid have no whole lines to keep (64 per row N = 334 207 -> 152 us).
-    a.slab_cols = VEC < 4 || (uint64_t)a.num_tiles <= (uint64_t)sm_count * 6 ? ((a.N + slabs - 1) / slabs + 3) & ~3u : 32 / G * VEC * CH;
+    // Slabs get equal shares of the grid, so they are of equal width where whole lines gain less than that: in small jobs (uniform
+    // 15727 x 13804 at N = 260: 33.4 us as 256 + 4 columns, 24.5 as 132 + 128), where the last one would be less than half full
+    // (64 per row N = 320 198 -> 150 us, stencil512 N = 260 277 -> 228, 7 per row N = 288 192 -> 185; 32 per row N = 448 238 as 256 +
+    // 192, 268 as 224 + 224) and off the 16-byte grid, which has no whole lines to keep (64 per row N = 334 207 -> 152 us).
+    constexpr uint32_t w = 32 / G * VEC * CH;
+    const bool equal = VEC < 4 || (uint64_t)a.num_tiles <= (uint64_t)sm_count * 6 || a.N - (slabs - 1) * w < w / 2;
+    a.slab_cols = equal ? ((a.N + slabs - 1) / slabs + 3) & ~3u : w;
     int n = 0;
     cudaError_t e;
     if (a.counters && slabs <= kDealtSlabs) {  // tiles dealt by a counter: where there are enough to deal

@@ -496,6 +496,19 @@ def test_operands_off_the_16_byte_grid(oracle_mod, shape, N):
         assert torch.isnan(Cd[:, :shift]).all() and torch.isnan(Cd[:, shift + N:]).all() and plan.device_status() == 0
 
 
+@pytest.mark.parametrize("N", [128, 129, 132, 256, 260, 388, 509])
+def test_wide_products_of_rows_in_runs_walk_a_tile_once_per_slab(oracle_mod, N):
+    """More tiles than a wave of blocks: slabs of equal width, one after the other over each tile; the last one may be narrower."""
+    A = g.elasticity3d(32, 3, 9)
+    p = cs.Plan.from_device_csr(A.M, A.K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS)
+    B = g.dense_operand(A.K, N, 7)
+    out = torch.full((A.M + 1, N), float("nan"), device="cuda")
+    p.spmm(B.cuda(), out[:A.M])
+    want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.numpy(), A.M, A.K)
+    assert oracle_mod.rel_fro(want, out[:A.M].cpu().numpy()) <= REL_FRO_TOL_FP32
+    assert torch.isnan(out[A.M]).all() and p.device_status() == 0
+
+
 def test_wide_unaligned_products_of_large_matrices_go_in_windows(oracle_mod):
     """Columns of B that a padded copy of 512 MiB would not hold; rows in runs take the run kernel in every window of 512."""
     A = g.elasticity3d(48, 3, 9)  # 331776 rows: 409 columns are 543 MB
