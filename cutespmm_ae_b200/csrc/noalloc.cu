@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <algorithm>
 #include <mutex>
 #include <string>
 
@@ -122,7 +123,8 @@ struct MainArgs {
     const float *vals, *B;
     float *C, *scratch;
     uint64_t ldb, ldc;
-    uint32_t M, K, nnz, N, lds, split, capacity, claim;  // capacity: chunks the scratch and the list hold for this call
+    uint32_t M, K, nnz, N, lds, split, capacity, claim, claim_uneven;  // capacity: chunks the scratch and the list hold for this call
+    bool whole_steps;  // whole steps of sound columns go without a check per nonzero
 };
 
 // The product.  A warp is G groups of 32/G lanes; a group spans a slab of 32/G * VEC * CH columns.  First the listed chunks
@@ -134,7 +136,7 @@ struct MainArgs {
 // gathers; no unit of the SM is above 55 % busy) and by the tail, a fifth of the warps' time: warps that find no rows left wait for
 // the others.  U rows of B are in flight per group, 40 warps per SM (U = 8 with 32 warps was 171 against 160 us below, then).
 // R-MAT 2^18, 3.9 M nonzeros, N = 64: 815 -> 160 us (before: a warp per row and per 1024-nonzero chunk, single-column
-// loads, three kernels one after the other) -> 150 (joins_batch); R-MAT 2^16 N = 16 474 -> 29, uniform4096 N = 32 25.6 -> 7.5
+// loads, three kernels one after the other) -> 150 (joins_batch) -> 125 (claim sizes, whole steps); R-MAT 2^16 N = 16 474 -> 29, uniform4096 N = 32 25.6 -> 7.5
 // (back to back, with overlapping launches), stencil512 N = 128 169 -> 139.
 template <int VEC, int CH, int G>
 __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a)
@@ -142,6 +144,7 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
     using V = typename Vec<VEC>::T;
     constexpr int L = 32 / G, U = (VEC == 4 ? 4 : 8) / CH;  // rows of B in flight per group
     static_assert(U >= 2 && (G == 1 || CH == 1), "groups span one vector per lane");
+    constexpr bool kWhole = VEC == 1 || G <= 4;  // launch_main
     __shared__ uint2 bufs[kWarps][kBuf];
     __shared__ uint32_t starts[kWarps][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / L, sub = lane % L;
@@ -153,15 +156,41 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
     for (int ch = 0; ch < CH; ++ch) ok[ch] = col0 + ch * L * VEC < a.N;
     const float *bl = a.B + col0;
 
-    auto stage = [&](uint32_t j, uint32_t n) {  // nonzeros [j, j + n) to the warp's buffer; a column that is not below K counts nothing
+    // nonzeros [j, j + n) to the warp's buffer; a column that is not below K counts nothing.  True: all of them are below K, and
+    // whole steps are wanted.
+    auto stage = [&](uint32_t j, uint32_t n) {
+        bool sound = true;
         for (uint32_t t = lane; t < n; t += 32) {
             const uint32_t c = __ldg(a.cols + j + t);
             buf[t] = make_uint2(c < a.K ? c : kNoCol, __float_as_uint(__ldg(a.vals + j + t)));
+            if (kWhole) sound &= c < a.K;
         }
+        return kWhole && a.whole_steps && __all_sync(kFull, sound);
     };
-    // acc += the staged nonzeros from, from + step, ... below end
-    auto gather = [&](V(&acc)[CH], uint32_t from, uint32_t end, uint32_t step) {
-        for (uint32_t k = from; k < end; k += U * step) {
+    // acc += the staged nonzeros from, from + step, ... below end; whole steps of sound columns need no check (and a 32-bit stride)
+    auto gather = [&](V(&acc)[CH], uint32_t from, uint32_t end, uint32_t step, bool sound) {
+        uint32_t k = from;
+        if (kWhole && sound) {
+            const uint32_t ldb = (uint32_t)a.ldb;
+            for (; k + (U - 1) * step < end; k += U * step) {
+                uint2 pr[U];
+                V x[U][CH];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    pr[u] = buf[k + u * step];
+#pragma unroll
+                    for (int ch = 0; ch < CH; ++ch) {
+                        if (ok[ch]) x[u][ch] = __ldg(reinterpret_cast<const V *>(bl + (uint64_t)pr[u].x * ldb + ch * L * VEC));
+                        else zero(x[u][ch]);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int ch = 0; ch < CH; ++ch) fma_to(acc[ch], __uint_as_float(pr[u].y), x[u][ch]);
+            }
+        }
+        for (; k < end; k += U * step) {
             float v[U];
             V x[U][CH];
 #pragma unroll
@@ -199,9 +228,9 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
         for (uint32_t j = j0; j < j1; j += kBuf) {
             const uint32_t n = min(kBuf, j1 - j);
             __syncwarp();
-            stage(j, n);
+            const bool sound = stage(j, n);
             __syncwarp();
-            gather(acc, grp, n, G);
+            gather(acc, grp, n, G, sound);
         }
         over_groups(acc);
     };
@@ -244,12 +273,13 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
         }
     }
 
+    const uint32_t take = chunks ? a.claim_uneven : a.claim;
     for (;;) {
         uint32_t first = 0;
-        if (lane == 0) first = atomicAdd(&g_state.next_row[blockIdx.y], a.claim);
+        if (lane == 0) first = atomicAdd(&g_state.next_row[blockIdx.y], take);
         first = __shfl_sync(kFull, first, 0);
         if (first >= a.M) break;
-        const uint32_t cnt = min(a.claim, a.M - first);
+        const uint32_t cnt = min(take, a.M - first);
         RowRange g{0u, 0u};
         if ((uint32_t)lane < cnt) g = load_range(a.rowPtr, (uint64_t)first + lane, a.nnz);
         const RowRange before{__shfl_up_sync(kFull, g.j0, 1), __shfl_up_sync(kFull, g.j1, 1)};
@@ -274,7 +304,7 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
             const uint32_t i1 = miss ? __ffs(miss) - 1 : 32u;
             const uint32_t end = __shfl_sync(kFull, g.j1, (int)i1 - 1);
             __syncwarp();
-            stage(j0, end - j0);
+            const bool sound = stage(j0, end - j0);
             if ((uint32_t)lane >= i0 && (uint32_t)lane < i1) start[lane] = g.j0 - j0;
             if ((uint32_t)lane + 1 == i1) start[i1] = g.j1 - j0;
             __syncwarp();
@@ -285,7 +315,7 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
                 if (G > 1 && to - from > kShared) continue;
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch) zero(acc[ch]);
-                gather(acc, from, to, 1);
+                gather(acc, from, to, 1, sound);
                 store((uint64_t)first + i, acc);
             }
             if constexpr (G > 1) {
@@ -295,7 +325,7 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
                     const uint32_t i = __ffs(shared) - 1;
 #pragma unroll
                     for (int ch = 0; ch < CH; ++ch) zero(acc[ch]);
-                    gather(acc, start[i] + grp, start[i + 1], G);
+                    gather(acc, start[i] + grp, start[i + 1], G, sound);
                     over_groups(acc);
                     if (grp == 0) store((uint64_t)first + i, acc);
                 }
@@ -316,12 +346,19 @@ template <int VEC, int CH, int G> cudaError_t launch_main(MainArgs a, int sm_cou
 {
     const uint32_t slabs = (a.N + 32 / G * VEC * CH - 1) / (32 / G * VEC * CH);
     const uint32_t wave = (uint32_t)(sm_count * per_sm) / slabs;  // one resident wave
-    // rows per claim: about a buffer of nonzeros, at most one per lane; few rows are spread over all warps
-    const uint64_t fill = (uint64_t)kBuf * a.M / (a.nnz + 1) + 1, spread = (uint64_t)a.M / ((uint64_t)wave * kWarps) + 1;
-    uint64_t claim = fill < spread ? fill : spread;
-    if (claim < (uint64_t)G) claim = G;
-    if (claim > 32) claim = 32;
-    a.claim = (uint32_t)claim;
+    // Rows per claim: about a buffer of nonzeros; where a warp's share is two such claims, halves of it (stencil512 N = 8: 23 rows twice
+    // 26.4 us, 29 and a half-empty second round 31.5).  Where there are long rows, others are likely to be of hundreds of nonzeros:
+    // a quarter of a buffer then, or the warps that meet several of those end last (R-MAT 2^18 N = 64: 18 rows per claim 148 us,
+    // 4 rows 125; claims that shrink towards the end leave 148: the heavy ones come first).
+    const uint64_t fill = std::min<uint64_t>((uint64_t)kBuf * a.M / (a.nnz + 1) + 1, 32), per_warp = (uint64_t)a.M / ((uint64_t)wave * kWarps) + 1;
+    const uint64_t rounds = (per_warp + fill - 1) / fill;
+    a.claim = (uint32_t)std::max<uint64_t>(rounds == 2 ? (per_warp + 1) / 2 : std::min(fill, per_warp), G);
+    a.claim_uneven = (uint32_t)std::max<uint64_t>(std::min<uint64_t>(fill / 4, per_warp), G);
+    // Whole steps pay in rows of several of them (32 per row N = 32 30.7 -> 28.8, R-MAT 2^18 N = 256 638 -> 355, 4 per row N = 32 39 -> 45:
+    // not there) and not with eight groups, whose rows end at different steps (64 per row N = 8 25 -> 36); single columns per lane
+    // always gain (64 per row N = 47 81 -> 47, 4 per row 95 -> 75).
+    a.whole_steps = a.ldb < (1ull << 32) && (VEC == 1 || (G <= 4 && a.nnz >= 6ull * CH * a.M));
+    const uint64_t claim = a.claim;
     const uint64_t row_blocks = ((uint64_t)a.M + claim * kWarps - 1) / (claim * kWarps), chunk_blocks = (2ull * a.nnz / a.split + kWarps - 1) / kWarps;
     const uint64_t want = a.nnz > a.split && chunk_blocks > row_blocks ? chunk_blocks : row_blocks;
     return cutespmm::launch_overlapped(noalloc_main_kernel<VEC, CH, G>, dim3((uint32_t)(want < wave ? (want ? want : 1) : (wave ? wave : 1)), slabs), kWarps * 32,
@@ -427,7 +464,7 @@ extern "C" int cutespmm_spmm_csr_noalloc(uint32_t M, uint32_t K, uint32_t nnz, c
     uint64_t split = nnz > (2u << 20) ? 256 : 128;
     auto slots_of = [&](uint64_t len) { return 2ull * ((nnz + len - 1) / len) + 2; };
     while (slots_of(split) * lds > kScratchFloats || slots_of(split) > kListSlots) split *= 2;
-    MainArgs a{rowPtr_dev, cols_dev, vals_dev, B_dev, C_dev, setup.scratch, ldb, ldc, M, K, nnz, N, lds, (uint32_t)split, (uint32_t)slots_of(split), 1};
+    MainArgs a{rowPtr_dev, cols_dev, vals_dev, B_dev, C_dev, setup.scratch, ldb, ldc, M, K, nnz, N, lds, (uint32_t)split, (uint32_t)slots_of(split), 1, 1, false};
     if (nnz > split) {
         const uint64_t want = ((uint64_t)M + 255) / 256, cap = (uint64_t)setup.sm_count * 8;
         e = cutespmm::launch_overlapped(noalloc_list_kernel, (uint32_t)(want < cap ? want : cap), 256, 0, s, rowPtr_dev, M, nnz, a.split,

@@ -140,6 +140,32 @@ def test_noalloc_at_the_edges_of_every_width(oracle_mod, N):
     assert oracle_mod.rel_fro(want, C[:A.M].cpu().numpy()) <= REL_FRO_TOL_FP32
 
 
+@pytest.mark.parametrize("N", [7, 16, 31, 32, 64, 65, 128, 250, 256, 512])
+@pytest.mark.parametrize("longest", [40, 400])
+def test_noalloc_rows_of_whole_steps_beside_a_column_that_counts_nothing(oracle_mod, N, longest):
+    """Rows long enough for whole steps, every remainder of one among them, with and without rows that are cut into chunks (which
+    choose the claim); a column that is not below K sends the nonzeros staged with it through the checked steps, and the rows of
+    B nobody names hold infinities."""
+    rng = np.random.default_rng(N + longest)
+    M, K = 3000, 500
+    ln = rng.integers(0, 40, M)
+    ln[:41] = np.arange(41)
+    ln[100:103] = longest
+    rp = np.concatenate([[0], np.cumsum(ln)])
+    cols, vals = rng.integers(1, K, rp[-1]).astype(np.int32), rng.standard_normal(rp[-1]).astype(np.float32)
+    B = g.dense_operand(K, N, 100)
+    B[0] = float("inf")
+    for unsound in (False, True):
+        c, v = cols.copy(), vals.copy()
+        if unsound:
+            at = rng.choice(rp[-1], 25, replace=False)
+            c[at], v[at] = K + 5, 0.0  # for the oracle: nothing times a row that is there
+        want = oracle_mod.spmm_csr(rp, np.where(c < K, c, 1), v, B.numpy(), M, K)
+        C = torch.full((M, N), float("nan"), device="cuda")
+        cs.spmm_csr_noalloc(M, K, torch.from_numpy(rp.astype(np.int32)).cuda(), torch.from_numpy(c).cuda(), torch.from_numpy(vals).cuda(), B.cuda(), C)
+        assert oracle_mod.rel_fro(want, C.cpu().numpy()) <= REL_FRO_TOL_FP32
+
+
 @pytest.mark.parametrize("N", [1, 16, 33, 64, 128, 132, 256])
 def test_noalloc_with_row_pointers_that_go_down(oracle_mod, N):
     """Row ends that decrease among rows that a warp takes together: every row is the sum over its own range, cut to the
