@@ -354,10 +354,12 @@ template <int VEC, int CH, int G> cudaError_t launch_main(MainArgs a, int sm_cou
     const uint64_t rounds = (per_warp + fill - 1) / fill;
     a.claim = (uint32_t)std::max<uint64_t>(rounds == 2 ? (per_warp + 1) / 2 : std::min(fill, per_warp), G);
     a.claim_uneven = (uint32_t)std::max<uint64_t>(std::min<uint64_t>(fill / 4, per_warp), G);
-    // Whole steps pay in rows of several of them (32 per row N = 32 30.7 -> 28.8, R-MAT 2^18 N = 256 638 -> 355, 4 per row N = 32 39 -> 45:
-    // not there) and not with eight groups, whose rows end at different steps (64 per row N = 8 25 -> 36); single columns per lane
-    // always gain (64 per row N = 47 81 -> 47, 4 per row 95 -> 75).
-    a.whole_steps = a.ldb < (1ull << 32) && (VEC == 1 || (G <= 4 && a.nnz >= 6ull * CH * a.M));
+    // Whole steps pay in rows of several of them (32 per row N = 32 30.7 -> 28.8, R-MAT 2^18 N = 256 638 -> 355; 4 per row N = 32 39 -> 45:
+    // not there), later where B does not stay in L2 (735 000 x 10 per row N = 32, 71 MB, 135 -> 151 us; stencil512 N = 64, 67 MB, 80 -> 74), and
+    // not with eight groups, whose rows end at different steps (64 per row N = 8 25 -> 36); single columns per lane always gain (64
+    // per row N = 47 81 -> 47, 4 per row 95 -> 75).
+    const uint64_t least = (uint64_t)a.K * a.N * sizeof(float) > (64ull << 20) ? 12 : 6;
+    a.whole_steps = a.ldb < (1ull << 32) && (VEC == 1 || (G <= 4 && a.nnz >= least * CH * a.M));
     const uint64_t claim = a.claim;
     const uint64_t row_blocks = ((uint64_t)a.M + claim * kWarps - 1) / (claim * kWarps), chunk_blocks = (2ull * a.nnz / a.split + kWarps - 1) / kWarps;
     const uint64_t want = a.nnz > a.split && chunk_blocks > row_blocks ? chunk_blocks : row_blocks;
