@@ -444,24 +444,30 @@ static void note_stream(const cutespmm_plan *p, cudaStream_t s)
 // Rows of B that are not 16-byte aligned (N not a multiple of four columns, a view) are read one or two columns per lane and load.
 // Copying B once into rows of N rounded up to four first (the copy lives on the stream) costs a launch, 1.25 ps per element of the
 // copy and, as C is written column by column then, 1.6 ps per element of C; with the kernels for unaligned rows as they are it
-// pays in two ranges only (us without / with the copy):
+// pays in these ranges only (us without / with the copy):
 //   20 or 25 to 31 columns, short rows: the copy lets a warp take four rows with one load each; 6 ps per nonzero (7 per row
-//     N = 31 26.0 / 21.2, stencil512 52.5 / 37.9, elasticity40 N = 22 35.5 / 31.7; 4 per row N = 27 37.9 / 46.4: not there);
+//     N = 31 26.0 / 21.2, stencil512 52.5 / 37.9, elasticity40 N = 22 35.5 / 31.7; 4 per row N = 27 37.9 / 46.4: not there); graphs
+//     with long rows from 17 columns on, 4 ps, where the copy stays in L2 (R-MAT 2^18 N = 27 92.2 / 80.8, 2^20 322 / 422);
 //   33 to 64 and above 384 columns, rows long enough: 0.1 ps per nonzero and column (64 per row N = 47 37.0 / 35.1, N = 511
-//     258 / 234; N = 259 177 / 218; 7 per row N = 47 32.6 / 33.9).
+//     258 / 234; N = 259 177 / 218; 7 per row N = 47 32.6 / 33.9);
+//   65 to 256 columns of mid-sized graphs with long rows, 0.2 ps per nonzero and column against a copy that stays in L2 (R-MAT 2^15
+//     with 19 per row N = 135 72.2 / 55.2, 2^16 102 / 89.0; 2^14 25.6 / 27.9 and 2^17 156 / 167: not there).
 // Even widths above 32 are read two columns per lane and gain nothing.  Copies above kMaxPadBytes are not made: the pool would
 // give them back at every synchronisation and map them anew (1.8 GB: 4.6 -> 5.6 ms per product).  Not while the stream is being
 // captured (a graph should not own memory).
-constexpr uint64_t kMaxPadBytes = 512ull << 20;
+constexpr uint64_t kMaxPadBytes = 512ull << 20, kNearBytes = 64ull << 20;
 static bool worth_padding(const cutespmm_plan *p, const cutespmm_list_sizes &list, const float *B, uint64_t ldb, const float *C, uint64_t ldc, uint32_t N)
 {
     const HostPlan &h = p->host;
     const bool two = !((reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 7) && !((ldb | ldc | N) & 1);
     if ((two && N > 32) || h.K * ((uint64_t)N + 3) * sizeof(float) > kMaxPadBytes) return false;
     if (N <= 32) {
-        if (N < (h.run_rows ? 20u : 25u) || list.chunks || h.nnz >= 24 * h.M) return false;
-        return h.nnz * 6 >= 3000000 + h.K * N * 5 / 4;  // picoseconds
+        if (N < (list.chunks ? 17u : h.run_rows ? 20u : 25u) || (!list.chunks && h.nnz >= 24 * h.M)) return false;
+        if (list.chunks && h.K * ((uint64_t)N + 3) * sizeof(float) > kNearBytes) return false;
+        return h.nnz * (list.chunks ? 4 : 6) >= 3000000 + h.K * N * 5 / 4;  // picoseconds
     }
+    if (N > 64 && N <= 256 && list.chunks && h.K * ((uint64_t)N + 3) * sizeof(float) <= kNearBytes)
+        return h.nnz * std::max(N, 100u) / 5 >= 6000000 + N * (h.K * 8 + h.M * 12) / 10;
     return (N <= 64 || N > 384) && h.nnz * N / 10 >= 3000000 + N * (h.K * 13 + h.M * 16) / 10;
 }
 

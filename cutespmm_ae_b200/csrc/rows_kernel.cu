@@ -44,6 +44,7 @@ template <bool DEEP> struct Tuning {
 // at four rows: with eight the deep form spills (4096 x 4096 with 16 per row at N = 66 3.8 -> 4.6 us).
 template <int VEC, int CH, bool DEEP>
 constexpr int kRowsInFlight = VEC == 2 && CH == 2 ? 4 : (DEEP ? 32 : 16) / (VEC * CH) < 8 ? (DEEP ? 32 : 16) / (VEC * CH) : 8;
+constexpr uint32_t kSharedRow = 16;  // nonzeros from which the groups of a warp share a row (32: the same within 1 %, 64: 2-5 % slower)
 constexpr int kWarps = kTileWarps;
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -141,10 +142,10 @@ __device__ __forceinline__ void accumulate(typename Vec<VEC>::T (&acc)[CH], cons
     }
 }
 
-// acc[ch] += sum of val * B[col][lane's columns] over `cnt` staged (column, value) pairs, UU rows of B in flight.
+// acc[ch] += sum of val * B[col][lane's columns] over `cnt` staged (column, value) pairs, every STEP-th, UU rows of B in flight.
 // TAIL: cnt may be smaller than UU; the surplus positions load the row of the last pair again (an L1 hit) and
 // are left out of the sum.
-template <int VEC, int CH, int L, bool FULL, int UU, bool TAIL>
+template <int VEC, int CH, int L, bool FULL, int UU, bool TAIL, int STEP = 1>
 __device__ __forceinline__ void row_group(typename Vec<VEC>::T (&acc)[CH], const uint2 *pairs_smem, uint32_t cnt, const float *__restrict__ bl,
                                           uint32_t ldb32, const bool (&ok)[CH])
 {
@@ -153,7 +154,7 @@ __device__ __forceinline__ void row_group(typename Vec<VEC>::T (&acc)[CH], const
     V b[UU][CH];
 #pragma unroll
     for (int u = 0; u < UU; ++u) {
-        const uint2 pr = pairs_smem[TAIL ? min((uint32_t)u, cnt - 1) : (uint32_t)u];  // all lanes read one address: broadcast
+        const uint2 pr = pairs_smem[(TAIL ? min((uint32_t)u, cnt - 1) : (uint32_t)u) * STEP];  // all lanes read one address: broadcast
         v[u] = __uint_as_float(pr.y);
         const float *row = bl + (uint64_t)pr.x * ldb32;
 #pragma unroll
@@ -168,6 +169,20 @@ __device__ __forceinline__ void row_group(typename Vec<VEC>::T (&acc)[CH], const
 #pragma unroll
             for (int ch = 0; ch < CH; ++ch) fma_vec(acc[ch], v[u], b[u][ch]);
         }
+}
+
+// The same over any number of pairs, U rows of B in flight.  What is left of them (fewer than U) goes as one more group, so that its
+// loads are in flight together instead of one after the other: positions past the end repeat the last pair and are not added.
+template <int VEC, int CH, int L, bool FULL, int U, int STEP>
+__device__ __forceinline__ void row_walk(typename Vec<VEC>::T (&acc)[CH], const uint2 *pairs_smem, uint32_t cnt, const float *__restrict__ bl, uint32_t ldb32,
+                                         const bool (&ok)[CH])
+{
+    uint32_t j = 0;
+    for (; j + U <= cnt; j += U) row_group<VEC, CH, L, FULL, U, false, STEP>(acc, pairs_smem + j * STEP, U, bl, ldb32, ok);
+    if (const uint32_t rem = cnt - j) {
+        if (rem > U / 2) row_group<VEC, CH, L, FULL, U, true, STEP>(acc, pairs_smem + j * STEP, rem, bl, ldb32, ok);
+        else row_group<VEC, CH, L, FULL, U / 2, true, STEP>(acc, pairs_smem + j * STEP, rem, bl, ldb32, ok);
+    }
 }
 
 // The same sum for a group of L = 32/G lanes that walks a chunk on its own (G > 1).  The group fetches L pairs with one
@@ -426,6 +441,46 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DYN, G))
         const TileStage &st = ring.stage[s];
         const uint4 d = st.desc;
         const uint32_t rb = d.x & ~3u, jb = d.z & ~1u;
+        constexpr int U = kRowsInFlight<VEC, CH, DEEP>;  // rows of B in flight per group and step
+        if constexpr (G > 1 && DYN) {
+            // Graphs with long rows, many tiles: the rows of a tile are of very different lengths, and one of hundreds of nonzeros is
+            // a chain of as many steps for its group while the tile has too few rows to go round.  The groups of a warp share
+            // such a row, group g takes nonzeros g, g + G, ... (R-MAT 2^20 N = 8 / 16 / 32 / 64 210 / 212 / 266 / 367 us -> 187 / 176 / 250 / 357).
+            auto store = [&](uint32_t r, V(&acc)[CH]) {
+                const uint32_t r_out = a.row_map ? __ldg(a.row_map + r) : r;
+                float *out = a.C + (uint64_t)r_out * a.ldc + col0;
+#pragma unroll
+                for (int ch = 0; ch < CH; ++ch)
+                    if (FULL || ok[ch]) store_row<FULL>(out + ch * L * VEC, acc[ch], a.c_scalar != 0, end - col0 - ch * L * VEC);
+            };
+            for (;;) {
+                const uint32_t first = tile_claim_rows(ring, s, (uint32_t)G, lane) + d.x;
+                if (first >= d.y) break;
+                const uint32_t r = first + grp;  // the group's own row
+                uint32_t at = 0, cnt = 0;        // its nonzeros in the staged pair slice
+                if (r < d.y) {
+                    at = st.row_ptr[r - rb] - jb;
+                    cnt = st.row_ptr[r - rb + 1] - jb - at;
+                }
+                V acc[CH];
+                if (r < d.y && cnt <= kSharedRow) {
+#pragma unroll
+                    for (int ch = 0; ch < CH; ++ch) zero_vec(acc[ch]);
+                    row_walk<VEC, CH, L, FULL, U, 1>(acc, st.pairs + at, cnt, bl, ldb32, ok);
+                    store(r, acc);
+                }
+                for (unsigned shared = __ballot_sync(kFull, cnt > kSharedRow && sub == 0); shared; shared &= shared - 1) {
+                    const int from = __ffs(shared) - 1;  // the first lane of the group whose row it is
+                    const uint32_t n = __shfl_sync(kFull, cnt, from), start = __shfl_sync(kFull, at, from);
+#pragma unroll
+                    for (int ch = 0; ch < CH; ++ch) zero_vec(acc[ch]);
+                    row_walk<VEC, CH, L, FULL, U, G>(acc, st.pairs + start + grp, (n - grp + G - 1) / G, bl, ldb32, ok);
+                    __syncwarp();
+                    add_groups<L>(acc);
+                    if (grp == from / L) store(first + grp, acc);
+                }
+            }
+        } else
         for (;;) {
             uint32_t r = tile_claim_rows(ring, s, (uint32_t)G, lane) + d.x;
             if (r >= d.y) break;
@@ -435,7 +490,6 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DYN, G))
                 V acc[CH];
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch) zero_vec(acc[ch]);
-                constexpr int U = kRowsInFlight<VEC, CH, DEEP>;  // rows of B in flight per group and step
                 uint32_t j = j0 - jb, jend = j1 - jb;  // positions in the staged pair slice
                 for (; j + U <= jend; j += U) row_group<VEC, CH, L, FULL, U, false>(acc, st.pairs + j, U, bl, ldb32, ok);
                 // what is left of the row (fewer than U nonzeros) goes as one more group, so that its loads are in flight
