@@ -452,15 +452,19 @@ static void note_stream(const cutespmm_plan *p, cudaStream_t s)
 //     258 / 234; N = 259 177 / 218; 7 per row N = 47 32.6 / 33.9);
 //   65 to 256 columns of mid-sized graphs with long rows, 0.2 ps per nonzero and column against a copy that stays in L2 (R-MAT 2^15
 //     with 19 per row N = 135 72.2 / 55.2, 2^16 102 / 89.0; 2^14 25.6 / 27.9 and 2^17 156 / 167: not there).
+//   rows of 150 and more nonzeros at every width, in windows of columns where the copy would be too large, by 12 ps per nonzero up to
+//     64 columns and 0.4 ps per nonzero and column beyond (300 per row N = 15 84.0 / 67.1, N = 301 776 / 685, 4000 x 200 per row N = 7
+//     43 / 12; 120 per row N = 7 21.5 / 30.0).
 // Even widths above 32 are read two columns per lane and gain nothing.  Copies above kMaxPadBytes are not made: the pool would
 // give them back at every synchronisation and map them anew (1.8 GB: 4.6 -> 5.6 ms per product).  Not while the stream is being
 // captured (a graph should not own memory).
-constexpr uint64_t kMaxPadBytes = 512ull << 20, kNearBytes = 64ull << 20;
+constexpr uint64_t kMaxPadBytes = 512ull << 20, kNearBytes = 64ull << 20, kVeryLongRows = 150;
 static bool worth_padding(const cutespmm_plan *p, const cutespmm_list_sizes &list, const float *B, uint64_t ldb, const float *C, uint64_t ldc, uint32_t N)
 {
     const HostPlan &h = p->host;
     const bool two = !((reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 7) && !((ldb | ldc | N) & 1);
     if ((two && N > 32) || h.K * ((uint64_t)N + 3) * sizeof(float) > kMaxPadBytes) return false;
+    if (h.nnz >= kVeryLongRows * h.M) return h.nnz * (N <= 64 ? 12 : N * 2 / 5) >= 3000000 + h.K * N * 5 / 4;
     if (N <= 32) {
         if (N < (list.chunks ? 17u : h.run_rows ? 20u : 25u) || (!list.chunks && h.nnz >= 24 * h.M)) return false;
         if (list.chunks && h.K * ((uint64_t)N + 3) * sizeof(float) > kNearBytes) return false;
@@ -495,6 +499,12 @@ static ColumnWindow column_window(const cutespmm_plan *p, const float *B, uint64
     const HostPlan &h = p->host;
     ColumnWindow w{};
     w.cols = left < kScratchCols ? left : kScratchCols;
+    const cutespmm_list_sizes &every = h.num_bricks || h.slab_panels ? p->every : p->own;
+    // very long rows: a window is narrowed until a padded copy of it may be made
+    if (h.nnz >= kVeryLongRows * h.M && ((reinterpret_cast<uintptr_t>(B) & 15) || (ldb & 3)) && h.K * ((uint64_t)w.cols + 3) * sizeof(float) > kMaxPadBytes) {
+        const uint64_t fit = kMaxPadBytes / (h.K * sizeof(float)) / 128 * 128;
+        if (fit && fit < w.cols && worth_padding(p, every, B, ldb, C, ldc, (uint32_t)fit) && may_copy()) w.cols = (uint32_t)fit;
+    }
     w.slab = h.slab_panels && slab_supports(w.cols, ldb, ldc, B, C);
     w.brick = use_brick(p, B, ldb, C, ldc, w.cols);
     // brick panels whose shape the brick kernel does not take (N not a multiple of 32, unaligned

@@ -496,6 +496,36 @@ def test_operands_off_the_16_byte_grid(oracle_mod, shape, N):
         assert torch.isnan(Cd[:, :shift]).all() and torch.isnan(Cd[:, shift + N:]).all() and plan.device_status() == 0
 
 
+@pytest.fixture(scope="module")
+def many_tiles():
+    """Tiles enough to be dealt by a counter, a few rows cut into chunks, and rows of every length around those a warp shares."""
+    rng = np.random.default_rng(17)
+    M, K = 330000, 20000
+    ln = rng.integers(0, 26, M)
+    ln[rng.choice(M, 2000, replace=False)] = rng.integers(27, 257, 2000)
+    ln[:9] = (15, 16, 17, 18, 31, 32, 33, 255, 256)
+    ln[5000:5003] = (257, 600, 1500)
+    rp = np.concatenate([[0], np.cumsum(ln)])
+    A = g.CsrMatrix(M, K, torch.from_numpy(rp), torch.from_numpy(rng.integers(0, K, rp[-1]).astype(np.int32)), torch.from_numpy(rng.standard_normal(rp[-1]).astype(np.float32)))
+    p = cs.Plan.from_device_csr(M, K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS)
+    assert p.info()["num_chunks"] and p.info()["num_tiles"] >= 8 * 6 * torch.cuda.get_device_properties(0).multi_processor_count
+    return A, p
+
+
+@pytest.mark.parametrize("N", [5, 8, 16, 27, 32, 47, 64, 81])
+def test_rows_that_the_groups_of_a_warp_share(oracle_mod, many_tiles, N):
+    """Long rows of a tile in narrow products of large matrices, aligned, off the 16-byte grid and after a padded copy of B."""
+    A, p = many_tiles
+    B = g.dense_operand(A.K, N, 8)
+    want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.numpy(), A.M, A.K)
+    Bd = B.cuda()
+    first = p.spmm(Bd)
+    assert oracle_mod.rel_fro(want, first.cpu().numpy()) <= REL_FRO_TOL_FP32
+    for _ in range(3):  # whoever takes a row, its sum is the same
+        assert torch.equal(p.spmm(Bd), first)
+    assert p.device_status() == 0
+
+
 @pytest.mark.parametrize("N", [128, 129, 132, 256, 260, 388, 509])
 def test_wide_products_of_rows_in_runs_walk_a_tile_once_per_slab(oracle_mod, N):
     """More tiles than a wave of blocks: slabs of equal width, one after the other over each tile; the last one may be narrower."""
