@@ -27,9 +27,18 @@ namespace {
 
 constexpr int kUnroll = 6;  // rows of B in flight per group: 4 / 6 / 8 took 27.2 / 25.7 / 28.5 us on elasticity40 at N = 32
 
-__device__ __forceinline__ void fma4(float4 &a, float v, const float4 &b)
+// a += v * b.  TWO: two columns per instruction, each rounded like fmaf (the kernel is bound by instruction issue: elasticity40 N = 32
+// 24.4 -> 23.4 us, N = 64 39.6 -> 38.6; with single-column loads the register pairs cost as much as they save).
+template <bool TWO> __device__ __forceinline__ void fma4(float4 &a, float v, const float4 &b)
 {
-    a.x = fmaf(v, b.x, a.x); a.y = fmaf(v, b.y, a.y); a.z = fmaf(v, b.z, a.z); a.w = fmaf(v, b.w, a.w);
+    if (TWO) {
+        const uint64_t vv = ptx::pack2(v, v);
+        const float2 lo = ptx::unpack2(ptx::fma2(vv, ptx::pack2(b.x, b.y), ptx::pack2(a.x, a.y)));
+        const float2 hi = ptx::unpack2(ptx::fma2(vv, ptx::pack2(b.z, b.w), ptx::pack2(a.z, a.w)));
+        a = make_float4(lo.x, lo.y, hi.x, hi.y);
+    } else {
+        a.x = fmaf(v, b.x, a.x); a.y = fmaf(v, b.y, a.y); a.z = fmaf(v, b.z, a.z); a.w = fmaf(v, b.w, a.w);
+    }
 }
 
 // Four columns of a row of B: one load where rows are 16-byte aligned, otherwise four of columns L apart (a load instruction
@@ -55,7 +64,7 @@ __device__ __forceinline__ void run_step(float4 (&acc)[R], const uint2 *pairs, c
     for (int u = 0; u < U; ++u)
         if (!TAIL || (uint32_t)u < cnt) {
 #pragma unroll
-            for (int k = 0; k < R; ++k) fma4(acc[k], __uint_as_float(pairs[first[k] + i + u].y), b[u]);
+            for (int k = 0; k < R; ++k) fma4<ALIGNED>(acc[k], __uint_as_float(pairs[first[k] + i + u].y), b[u]);
         }
 }
 
