@@ -102,6 +102,7 @@ struct SddmmArgs {
     float *out;                          // one value per nonzero, in the plan's storage order
     uint32_t N;
     uint32_t scale;                      // 1: multiply by the stored value of A
+    uint32_t short_rows;                 // 1: fewer than four nonzeros per row (picks the kernel's form)
     uint32_t early;                      // 1: the plan's arrays never change (RowsArgs::early)
     uint32_t vec4;                       // 1: X, Y and their leading dimensions (below 2^30) allow 16-byte loads
     uint32_t *status;                    // device status word: set to 1 when a bounded wait gives up

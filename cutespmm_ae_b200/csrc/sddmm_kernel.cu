@@ -33,7 +33,8 @@ constexpr unsigned kFull = 0xffffffffu;
 // LANES lanes share a nonzero and cover a span of 4 * V * LANES columns of its row of Y: as V float4 each (VEC4), lane sub
 // at float4 number sub, sub + LANES, ..., or as 4 V single columns where the rows are not 16-byte aligned.  FULL: N is a
 // multiple of the span.
-template <int LANES, int V, bool VEC4, bool FULL> struct Span {
+// EACH: a row of X is loaded beside every row of Y, for matrices whose rows are so short that a group hardly meets one twice.
+template <int LANES, int V, bool VEC4, bool FULL, bool EACH> struct Span {
     static constexpr int kCols = 4 * V * LANES;
     static constexpr int kGroups = 32 / LANES;                        // nonzeros per load instruction
     static constexpr unsigned kGroupStarts = LANES == 8 ? 0x01010101u : 0x11111111u;  // the first lane of every group
@@ -129,7 +130,7 @@ template <int LANES, int V, bool VEC4, bool FULL> struct Span {
     // half of its sums to its partner and keeps the other half, first inside every batch of kFly nonzeros whose rows of Y are in
     // flight together, then over the batches.  That is LANES - 1 shuffles for LANES sums, and a lane is left with the result of
     // nonzero result_of(lane).
-    static constexpr int kFly = V == 1 ? LANES : V == 2 ? 4 : 2;  // 16 to 32 registers of Y
+    static constexpr int kFly = EACH ? (V == 1 ? 4 : 2) : V == 1 ? LANES : V == 2 ? 4 : 2;  // 16 to 32 registers of Y (EACH: and as many of X)
     static constexpr int kBatches = LANES / kFly;
     static __device__ __forceinline__ uint32_t result_of(int lane)
     {
@@ -156,19 +157,22 @@ template <int LANES, int V, bool VEC4, bool FULL> struct Span {
         int o = LANES / 2;
 #pragma unroll
         for (int b = 0; b < kBatches; ++b) {
-            float4 y[kFly][V];
+            float4 y[kFly][V], xs[EACH && !KEEP ? kFly : 1][V];
             float s[kFly];
 #pragma unroll
-            for (int u = 0; u < kFly; ++u) load(y[u], row_of(a.Y, __shfl_sync(kFull, col, b * kFly + u, LANES), a.ldy), c0, a.N, sub);
+            for (int u = 0; u < kFly; ++u) {
+                if constexpr (EACH && !KEEP) load(xs[u], row_of(a.X, __shfl_sync(kFull, row, b * kFly + u, LANES), a.ldx), c0, a.N, sub);
+                load(y[u], row_of(a.Y, __shfl_sync(kFull, col, b * kFly + u, LANES), a.ldy), c0, a.N, sub);
+            }
 #pragma unroll
             for (int u = 0; u < kFly; ++u) {
                 const int q = b * kFly + u;
-                if constexpr (!KEEP)
+                if constexpr (!KEEP && !EACH)
                     if (turn & (kGroupStarts << q)) {  // the same for every lane
                         const uint32_t r = __shfl_sync(kFull, row, q, LANES);
                         if (turn >> (k0 + q) & 1u) load(x, row_of(a.X, r, a.ldx), c0, a.N, sub);
                     }
-                s[u] = dot(x, y[u]);
+                s[u] = dot(EACH && !KEEP ? xs[EACH && !KEEP ? u : 0] : x, y[u]);
             }
             o = LANES / 2;
             halve<kFly>(s, o, sub);
@@ -184,10 +188,10 @@ template <int LANES, int V, bool VEC4, bool FULL> struct Span {
 // 143 -> 88.5).
 template <int V, bool VEC4> constexpr bool kFlat = VEC4 || V < 3;
 
-template <int LANES, int V, bool VEC4, bool FULL>
+template <int LANES, int V, bool VEC4, bool FULL, bool EACH>
 __global__ void __launch_bounds__(kTileWarps * 32, kFlat<V, VEC4> ? 4 : 3) sddmm_kernel(SddmmArgs a)
 {
-    using S = Span<LANES, V, VEC4, FULL>;
+    using S = Span<LANES, V, VEC4, FULL, EACH>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % LANES;
     const uint2 *pairs = reinterpret_cast<const uint2 *>(a.pairs);
     __shared__ TileRing ring;
@@ -252,7 +256,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, kFlat<V, VEC4> ? 4 : 3) sddmm
                 const uint32_t before = __shfl_up_sync(kFull, row, 1);
                 const unsigned turn = __ballot_sync(kFull, row != before) | S::kGroupStarts;
                 // the rows of X that a group meets on its way arrive in L1 beside its first loads (R-MAT 2^18 N = 64: 89.6 -> 83.3 us)
-                if constexpr (VEC4)
+                if constexpr (VEC4 && !EACH)
                     if (row != before && lane % LANES) {
                         const float *p = S::row_of(a.X, row, a.ldx);
 #pragma unroll
@@ -287,20 +291,25 @@ __global__ void __launch_bounds__(kTileWarps * 32, kFlat<V, VEC4> ? 4 : 3) sddmm
     }
 }
 
-template <int LANES, int V, bool VEC4, bool FULL> cudaError_t launch_sddmm_t(const SddmmArgs &a, int sm_count, cudaStream_t s)
+template <int LANES, int V, bool VEC4, bool FULL, bool EACH = false> cudaError_t launch_sddmm_t(const SddmmArgs &a, int sm_count, cudaStream_t s)
 {
     int per_sm = 0;
-    const cudaError_t e = blocks_per_sm<sddmm_kernel<LANES, V, VEC4, FULL>>(per_sm, kTileWarps * 32);
+    const cudaError_t e = blocks_per_sm<sddmm_kernel<LANES, V, VEC4, FULL, EACH>>(per_sm, kTileWarps * 32);
     if (e != cudaSuccess) return e;
     const uint32_t chunk_blocks = (a.num_chunks + kTileWarps - 1) / kTileWarps;
     uint32_t blocks = a.num_tiles > chunk_blocks ? a.num_tiles : chunk_blocks;
     const uint32_t cap = (uint32_t)(sm_count * per_sm);  // one resident wave
     if (blocks > cap) blocks = cap;
-    return launch_overlapped(sddmm_kernel<LANES, V, VEC4, FULL>, blocks, kTileWarps * 32, 0, s, a);
+    return launch_overlapped(sddmm_kernel<LANES, V, VEC4, FULL, EACH>, blocks, kTileWarps * 32, 0, s, a);
 }
 template <int LANES, int V> cudaError_t launch_sddmm_v(const SddmmArgs &a, int sm_count, cudaStream_t s)
 {
     if (!a.vec4) return launch_sddmm_t<LANES, V, false, false>(a, sm_count, s);
+    // Rows of two or three nonzeros: 200 000 x 3 per row N = 16 / 32 / 64 12.8 / 22.9 / 34.0 us with X kept, 11.3 / 19.0 / 32.8 with X
+    // loaded each time (before the walk by runs 12.3 / 19.2 / 30.2); 4 per row N = 32 33.2 with X kept, 38.8 before.
+    if constexpr (V <= 2)
+        if (a.short_rows)
+            return a.N % (4 * V * LANES) == 0 ? launch_sddmm_t<LANES, V, true, true, true>(a, sm_count, s) : launch_sddmm_t<LANES, V, true, false, true>(a, sm_count, s);
     return a.N % (4 * V * LANES) == 0 ? launch_sddmm_t<LANES, V, true, true>(a, sm_count, s) : launch_sddmm_t<LANES, V, true, false>(a, sm_count, s);
 }
 

@@ -51,6 +51,23 @@ def test_sddmm_where_rows_end_inside_a_run_of_nonzeros(oracle_mod, N, shift):
     assert rel(want, out[:nnz].cpu().numpy()) <= TOL and torch.isnan(out[nnz])
 
 
+@pytest.mark.parametrize("N", [7, 16, 20, 32, 33, 64, 100])
+def test_sddmm_of_rows_of_few_nonzeros(oracle_mod, N):
+    """Fewer than four nonzeros per row: a row of X is loaded for each; long rows among them, empty ones and a last claim of one."""
+    rng = np.random.default_rng(N)
+    ln = rng.integers(0, 5, 4000)
+    ln[[3, 700]] = (300, 33)
+    rp = np.concatenate([[0], np.cumsum(ln)])
+    M, K, nnz = 4000, 900, int(rp[-1])
+    cols, vals = torch.from_numpy(rng.integers(0, K, nnz).astype(np.int32)), g.dense_operand(nnz, 1, 74).flatten()
+    p = cs.Plan.from_device_csr(M, K, torch.from_numpy(rp.astype(np.int32)).cuda(), cols.cuda(), vals.cuda(), path=cs.PATH_ROWS)
+    X, Y = g.dense_operand(M, N, 75), g.dense_operand(K, N, 76)
+    out = torch.full((nnz + 1,), float("nan"), device="cuda")
+    p.sddmm(X.cuda(), Y.cuda(), out[:nnz], scale_by_values=True)
+    want = oracle_mod.sddmm_csr(rp, cols, vals, X.numpy(), Y.numpy())
+    assert rel(want, out[:nnz].cpu().numpy()) <= TOL and torch.isnan(out[nnz])
+
+
 @pytest.mark.parametrize("make,path", [(lambda: g.stencil9(64), cs.PATH_AUTO), (lambda: g.elasticity3d(8, 3, 4), cs.PATH_BRICK),
                                         (lambda: g.uniform_random(300, 200, 5, seed=41), cs.PATH_ROWS)])
 def test_sddmm_on_every_plan_flavour_and_strided_operands(oracle_mod, make, path):
