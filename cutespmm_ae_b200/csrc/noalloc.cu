@@ -27,7 +27,6 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <algorithm>
 #include <mutex>
 #include <string>
 
@@ -62,8 +61,10 @@ static __device__ uint32_t g_arrivals[kListSlots * kMaxSlabs];  // per first slo
 // All zero between calls: the last block of a call's main kernel puts it back, and the host where that kernel could not be
 // launched behind the list.  (Clearing it on the stream in front of every call instead gives up the overlap of launches: 65 000
 // nonzeros at N = 32 7.5 -> 10.3 us, R-MAT 2^16 N = 16 30.9 -> 32.9.)
-struct State {
-    uint32_t chunks, overflow, balance, pad;
+struct alignas(16) State {
+    uint32_t chunks, overflow;
+    uint32_t mid_nnz;  // nonzeros in rows of more than MainArgs::mid that are not listed
+    uint32_t balance;
     uint32_t next_row[kMaxSlabs];
 };
 static __device__ State g_state;
@@ -76,16 +77,21 @@ __device__ __forceinline__ RowRange load_range(const uint32_t *__restrict__ rowP
 // Lists the chunks of the rows longer than `split`.  One pass over the row pointers (4 us at 2^18 rows); which slots a row
 // gets depends on the order of arrival, the order its chunks are added in does not.  A row that does not fit the list (row
 // pointers that claim more nonzeros than there are) raises `overflow`: the main kernel then computes long rows whole.
-__global__ void __launch_bounds__(256) noalloc_list_kernel(const uint32_t *__restrict__ rowPtr, uint32_t M, uint32_t nnz, uint32_t split,
-                                                           uint32_t capacity)
+// mid: not 0 where the main kernel wants to know how many nonzeros the other rows of more than `mid` hold.
+__global__ void __launch_bounds__(kWarps * 32) noalloc_list_kernel(const uint32_t *__restrict__ rowPtr, uint32_t M, uint32_t nnz, uint32_t split,
+                                                                   uint32_t capacity, uint32_t mid)
 {
     ptx::grid_wait();
     ptx::grid_release();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    uint32_t in_mid = 0;
     for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < M; r += stride) {
         const RowRange g = load_range(rowPtr, r, nnz);
         const uint32_t len = g.j1 - g.j0;
-        if (len <= split) continue;
+        if (len <= split) {
+            if (len > mid) in_mid += len;
+            continue;
+        }
         const uint32_t n = (uint32_t)(((uint64_t)len + split - 1) / split);
         const uint32_t slot0 = n <= capacity ? atomicAdd(&g_state.chunks, n) : 0u;
         if (n > capacity || slot0 > capacity - n) {
@@ -97,6 +103,15 @@ __global__ void __launch_bounds__(256) noalloc_list_kernel(const uint32_t *__res
             g_list[slot0 + i] = make_uint4((uint32_t)r, j, min(g.j1 - j, split) + j, slot0);
         }
         for (uint32_t y = 0; y < kMaxSlabs; ++y) g_arrivals[slot0 * kMaxSlabs + y] = 0;
+    }
+    if (!mid) return;
+    __shared__ uint32_t per_warp[kWarps];
+    in_mid = __reduce_add_sync(kFull, in_mid);
+    if (threadIdx.x % 32 == 0) per_warp[threadIdx.x / 32] = in_mid;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        in_mid = __reduce_add_sync(kFull, threadIdx.x < kWarps ? per_warp[threadIdx.x] : 0u);
+        if (threadIdx.x == 0 && in_mid) atomicAdd(&g_state.mid_nnz, in_mid);
     }
 }
 
@@ -123,7 +138,8 @@ struct MainArgs {
     const float *vals, *B;
     float *C, *scratch;
     uint64_t ldb, ldc;
-    uint32_t M, K, nnz, N, lds, split, capacity, claim, claim_uneven;  // capacity: chunks the scratch and the list hold for this call
+    uint32_t M, K, nnz, N, lds, split, capacity;  // capacity: chunks the scratch and the list hold for this call
+    uint32_t claim, claim_uneven, mid;  // rows per claim, the same where rows of more than `mid` hold much of the matrix, set by launch_main
     bool whole_steps;  // whole steps of sound columns go without a check per nonzero
 };
 
@@ -237,8 +253,8 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
 
     ptx::grid_wait();
     ptx::grid_release();
-    const bool overflow = g_state.overflow != 0;
-    const uint32_t chunks = overflow ? 0u : min(g_state.chunks, a.capacity);
+    const bool overflow = g_state.overflow != 0, uneven = g_state.mid_nnz > a.nnz / 8;
+    const uint32_t chunks = overflow ? 0u : min(g_state.chunks, a.capacity), take = chunks && uneven ? a.claim_uneven : a.claim;
     for (uint32_t c = warp * gridDim.x + blockIdx.x; c < chunks; c += gridDim.x * kWarps) {
         const uint4 ck = g_list[c];
         // a call that overlaps this one may have written the list: what it names has to lie inside this call's arrays
@@ -273,7 +289,6 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
         }
     }
 
-    const uint32_t take = chunks ? a.claim_uneven : a.claim;
     for (;;) {
         uint32_t first = 0;
         if (lane == 0) first = atomicAdd(&g_state.next_row[blockIdx.y], take);
@@ -338,6 +353,7 @@ __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a
     if (threadIdx.x == 0 && cutespmm::last_block_out(&g_state.balance)) {
         g_state.chunks = 0;
         g_state.overflow = 0;
+        g_state.mid_nnz = 0;
         for (uint32_t y = 0; y < kMaxSlabs; ++y) g_state.next_row[y] = 0;
     }
 }
@@ -347,9 +363,13 @@ template <int VEC, int CH, int G> cudaError_t launch_main(MainArgs a, int sm_cou
     const uint32_t slabs = (a.N + 32 / G * VEC * CH - 1) / (32 / G * VEC * CH);
     const uint32_t wave = (uint32_t)(sm_count * per_sm) / slabs;  // one resident wave
     // Rows per claim: about a buffer of nonzeros; where a warp's share is two such claims, halves of it (stencil512 N = 8: 23 rows twice
-    // 26.4 us, 29 and a half-empty second round 31.5).  Where there are long rows, others are likely to be of hundreds of nonzeros:
-    // a quarter of a buffer then, or the warps that meet several of those end last (R-MAT 2^18 N = 64: 18 rows per claim 148 us,
-    // 4 rows 125; claims that shrink towards the end leave 148: the heavy ones come first).
+    // 26.4 us, 29 and a half-empty second round 31.5).  Where an eighth of the nonzeros sits in rows of more than twice the mean
+    // that are not listed, beside rows that are, a quarter of a buffer, or the warps that meet several of those end last (R-MAT 2^18
+    // N = 64: 18 rows per claim 148 us, 4 rows 125; claims that shrink towards the end leave 148: the heavy ones come first).  A few
+    // long rows alone are no reason, they are summed before the claims: quarters took 49.1 / 56.5 us against 28.8 / 41.7 at N = 16 /
+    // 32 with 400 000 rows of 4 and one of 2000, 199 against 96 with a million rows at N = 32.  R-MAT graphs hold 17 % and more of
+    // their nonzeros in such rows; counting them takes the list kernel 0.3 us, which is left out where both claims are the same.
+    // (Each warp going by the rows of its last claim instead: R-MAT 2^16 N = 64 44 -> 64.)
     const uint64_t fill = std::min<uint64_t>((uint64_t)kBuf * a.M / (a.nnz + 1) + 1, 32), per_warp = (uint64_t)a.M / ((uint64_t)wave * kWarps) + 1;
     const uint64_t rounds = (per_warp + fill - 1) / fill;
     a.claim = (uint32_t)std::max<uint64_t>(rounds == 2 ? (per_warp + 1) / 2 : std::min(fill, per_warp), G);
@@ -360,9 +380,16 @@ template <int VEC, int CH, int G> cudaError_t launch_main(MainArgs a, int sm_cou
     // per row N = 47 81 -> 47, 4 per row 95 -> 75).
     const uint64_t least = (uint64_t)a.K * a.N * sizeof(float) > (64ull << 20) ? 12 : 6;
     a.whole_steps = a.ldb < (1ull << 32) && (VEC == 1 || (G <= 4 && a.nnz >= least * CH * a.M));
+    a.mid = a.claim == a.claim_uneven ? 0u : (uint32_t)std::max<uint64_t>(2ull * a.nnz / a.M, 32);
     const uint64_t claim = a.claim;
     const uint64_t row_blocks = ((uint64_t)a.M + claim * kWarps - 1) / (claim * kWarps), chunk_blocks = (2ull * a.nnz / a.split + kWarps - 1) / kWarps;
     const uint64_t want = a.nnz > a.split && chunk_blocks > row_blocks ? chunk_blocks : row_blocks;
+    if (a.nnz > a.split) {
+        const uint64_t rows = ((uint64_t)a.M + kWarps * 32 - 1) / (kWarps * 32), cap = (uint64_t)sm_count * 8;
+        const cudaError_t e = cutespmm::launch_overlapped(noalloc_list_kernel, (uint32_t)(rows < cap ? rows : cap), kWarps * 32, 0, s, a.rowPtr, a.M, a.nnz, a.split,
+                                                          a.capacity, a.mid);
+        if (e != cudaSuccess) return e;
+    }
     return cutespmm::launch_overlapped(noalloc_main_kernel<VEC, CH, G>, dim3((uint32_t)(want < wave ? (want ? want : 1) : (wave ? wave : 1)), slabs), kWarps * 32,
                                        0, s, a);
 }
@@ -466,18 +493,11 @@ extern "C" int cutespmm_spmm_csr_noalloc(uint32_t M, uint32_t K, uint32_t nnz, c
     uint64_t split = nnz > (2u << 20) ? 256 : 128;
     auto slots_of = [&](uint64_t len) { return 2ull * ((nnz + len - 1) / len) + 2; };
     while (slots_of(split) * lds > kScratchFloats || slots_of(split) > kListSlots) split *= 2;
-    MainArgs a{rowPtr_dev, cols_dev, vals_dev, B_dev, C_dev, setup.scratch, ldb, ldc, M, K, nnz, N, lds, (uint32_t)split, (uint32_t)slots_of(split), 1, 1, false};
-    if (nnz > split) {
-        const uint64_t want = ((uint64_t)M + 255) / 256, cap = (uint64_t)setup.sm_count * 8;
-        e = cutespmm::launch_overlapped(noalloc_list_kernel, (uint32_t)(want < cap ? want : cap), 256, 0, s, rowPtr_dev, M, nnz, a.split,
-                                        a.capacity);
-    }
-    if (e == cudaSuccess) {
-        const int v4 = !((reinterpret_cast<uintptr_t>(B_dev) | reinterpret_cast<uintptr_t>(C_dev)) & 15) && !((ldb | ldc | N) & 3) ? 1 : 0;
-        int w = 0;
-        while (N > kForms[v4][w].widest) ++w;
-        e = kForms[v4][w].launch(a, setup.sm_count, setup.per_sm[v4][w], s);
-    }
+    MainArgs a{rowPtr_dev, cols_dev, vals_dev, B_dev, C_dev, setup.scratch, ldb, ldc, M, K, nnz, N, lds, (uint32_t)split, (uint32_t)slots_of(split), 1, 1, 0, false};
+    const int v4 = !((reinterpret_cast<uintptr_t>(B_dev) | reinterpret_cast<uintptr_t>(C_dev)) & 15) && !((ldb | ldc | N) & 3) ? 1 : 0;
+    int w = 0;
+    while (N > kForms[v4][w].widest) ++w;
+    e = kForms[v4][w].launch(a, setup.sm_count, setup.per_sm[v4][w], s);
     if (e != cudaSuccess) cudaMemsetAsync(setup.state, 0, sizeof(State), s);  // a list without its product
     if (e != cudaSuccess) return fail(CUTESPMM_ECUDA, std::string("cutespmm_spmm_csr_noalloc launch: ") + cudaGetErrorString(e));
     return CUTESPMM_OK;

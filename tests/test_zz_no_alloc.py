@@ -212,6 +212,44 @@ def test_noalloc_calls_after_overlapping_ones_are_whole(oracle_mod):
             assert oracle_mod.rel_fro(w, C[: d[0]].cpu().numpy()) <= REL_FRO_TOL_FP32
 
 
+def _best_us(call):
+    best = float("inf")
+    for _ in range(6):
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        for _ in range(10):
+            call()
+        end.record()
+        end.synchronize()
+        best = min(best, start.elapsed_time(end) * 100)
+    return best
+
+
+@pytest.mark.parametrize("N", [16, 32])
+def test_noalloc_a_long_row_leaves_the_others_their_time(oracle_mod, N):
+    """Rows of four nonzeros, one of them replaced by a long one: the rows are claimed as without it (1.01 to 1.05 times the time;
+    1.8 to 2.1 with claims of a quarter of the rows).  Rows of a hundred nonzeros beside long ones take those claims."""
+    rng = np.random.default_rng(107)
+    M, K = 1_000_000, 50_000
+    times = []
+    for kind in ("even", "one long", "many of a hundred"):
+        ln = np.full(M, 4)
+        if kind != "even":
+            ln[M // 3] = 3000
+        if kind == "many of a hundred":
+            ln[rng.choice(M, 10_000, replace=False)] = 100  # a fifth of the nonzeros
+        rp = np.concatenate([[0], np.cumsum(ln)])
+        cols, vals = rng.integers(0, K, rp[-1]).astype(np.int32), rng.standard_normal(rp[-1]).astype(np.float32)
+        dev = torch.from_numpy(rp.astype(np.int32)).cuda(), torch.from_numpy(cols).cuda(), torch.from_numpy(vals).cuda()
+        B = g.dense_operand(K, N, 108, device="cuda")
+        C = torch.full((M, N), float("nan"), device="cuda")
+        cs.spmm_csr_noalloc(M, K, *dev, B, C)
+        want = oracle_mod.spmm_csr(torch.from_numpy(rp), torch.from_numpy(cols), torch.from_numpy(vals), B.cpu().numpy(), M, K)
+        assert oracle_mod.rel_fro(want, C.cpu().numpy()) <= REL_FRO_TOL_FP32, kind
+        times.append(_best_us(lambda: cs.spmm_csr_noalloc(M, K, *dev, B, C)))
+    assert times[1] <= 1.4 * times[0], times
+
+
 _FIRST_CALLS = """
 import statistics, time
 import torch
