@@ -344,6 +344,7 @@ static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B,
     a.N = N;
     a.status = p->d_status;
     a.row_map = static_cast<const uint32_t *>(p->d_row_map);
+    a.uneven = a.num_chunks && h.uneven ? 1u : 0u;
     // Tiles are dealt as they are finished where there are long rows: launches of such a plan share the partial sums and must
     // not overlap anyway (where they do, their results are undefined, but the counters end at zero all the same); a plan
     // without long rows may run on several streams at once and keeps nothing between launches.

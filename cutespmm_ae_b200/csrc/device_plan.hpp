@@ -70,6 +70,7 @@ struct RowsArgs {
                                // launches.  nullptr: tiles in fixed turns
     uint32_t num_tiles, num_chunks;
     uint32_t avg_row_nnz;      // nonzeros per row of the whole matrix (picks the kernel's tuning)
+    uint32_t uneven;           // 1: the list has chunks, and the other rows are of very different lengths, too (is_uneven)
     uint32_t short_chunks;     // 1: a small job, its long rows are cut into pieces of tens of nonzeros
     const float *B;            // K x N window, leading dimension ldb
     float *C;                  // M x N window, leading dimension ldc
@@ -167,8 +168,8 @@ struct BuildTotals {  // one per plan creation, read by the host after the count
     uint32_t tiles;
     uint32_t chunks, long_rows, brick_panels, brick_slots;  // in the order of the per-segment counters
     uint32_t brick_nnz_max, brick_cols_max;
-    uint32_t uneven;  // bit 0: some odd row has other columns than the row in front of it, bit 1: some row not divisible by 3
-    unsigned long long bricks, brick_cost, long_nnz;
+    uint32_t unlike;  // bit 0: some odd row has other columns than the row in front of it, bit 1: some row not divisible by 3
+    unsigned long long bricks, brick_cost, long_nnz, mid_nnz;
 };
 struct ListArgs {
     uint32_t M, num_segments;

@@ -326,6 +326,16 @@ void choose_panel_paths(HostPlan &p, const std::vector<uint32_t> &panel_ncols)
     }
 }
 
+bool find_uneven(const HostPlan &p)
+{
+    uint64_t mid_nnz = 0;
+    for (uint64_t r = 0; r < p.M; ++r) {
+        const uint32_t len = p.row_ptr[r + 1] - p.row_ptr[r];
+        if (mid_row(len, p.nnz, p.M)) mid_nnz += len;
+    }
+    return is_uneven(mid_nnz, p.nnz);
+}
+
 uint32_t find_row_runs(const HostPlan &p)
 {
     if (p.M < 2 || p.nnz == 0) return 0;
@@ -419,6 +429,7 @@ int build_host_plan(HostPlan &p, uint64_t M, uint64_t K, const uint64_t *rowPtr,
     if (p.opts.reorder == CUTESPMM_REORDER_SIMILAR_ROWS) group_similar_rows(p);
 
     p.run_rows = find_row_runs(p);
+    p.uneven = find_uneven(p);
     const std::vector<uint32_t> panel_ncols = analyze_panels(p);
 
     choose_panel_paths(p, panel_ncols);

@@ -91,6 +91,11 @@ CUTESPMM_HD inline ItemSizes item_sizes(uint64_t total, uint64_t nnz, uint64_t M
     }
     return s;
 }
+// Rows are of very different lengths: an eighth of the nonzeros (mid_nnz) sits in rows of more than twice the mean and more than 32,
+// those beyond kDefaultSplitNnz left out, which are cut up anyway.  R-MAT graphs of up to 24 edges per node and side hold 13 to 50 %
+// there.  A few long rows in a matrix of short ones do not make it uneven, whatever they hold.
+CUTESPMM_HD inline bool mid_row(uint32_t len, uint64_t nnz, uint64_t M) { return len > 32 && len <= kDefaultSplitNnz && len * M > 2 * nnz; }
+CUTESPMM_HD inline bool is_uneven(uint64_t mid_nnz, uint64_t nnz) { return mid_nnz > nnz / 8; }
 // nonzeros per chunk of a row of `len` nonzeros that is being cut
 CUTESPMM_HD inline uint32_t piece_length(const ItemSizes &s, uint32_t len)
 {
@@ -157,6 +162,7 @@ struct HostPlan {
     std::vector<Chunk> chunks;
     std::vector<LongRow> long_rows;
 
+    bool uneven = false;                 // rows of very different lengths (is_uneven)
     uint32_t run_rows = 0;               // rows come in aligned runs of 3 or 2 with the same columns (0: they do not)
 
     // ---- panel analysis (HRPB-compatible view) ----
@@ -211,6 +217,9 @@ int build_host_plan(HostPlan &p, uint64_t M, uint64_t K, const uint64_t *rowPtr,
 
 // The options of a plan that is built on the device, checked and with the defaults filled in (p.opts, p.adaptive_tiling).
 int check_device_options(HostPlan &p, uint64_t M, uint64_t K, const cutespmm_options_t *opts, std::string &err);
+
+// HostPlan::uneven of a matrix whose row pointers are on the host.
+bool find_uneven(const HostPlan &p);
 
 // HostPlan::run_rows of a matrix whose pairs are on the host.
 uint32_t find_row_runs(const HostPlan &p);

@@ -640,14 +640,17 @@ cudaError_t launch_rows(const RowsArgs &args, int sm_count, cudaStream_t s)
     // N = 511 12990 -> 3984, stencil512 N = 101 133 -> 96.6) and takes several rows up to 64 (one before; N = 7 R-MAT 2^17 47.4 -> 29.0,
     // 64 per row 22.3 -> 17.4, which took a padded copy of B until then).  How many, by what was measured (us, more groups / fewer):
     //   few_rows    fewer rows than warps: one row per warp (4096 x 16 per row N = 27 3.6 / 3.0);
-    //   few_groups  long rows and no chunks, or a small job: N = 47 64 per row 41.7 / 37.0, R-MAT 2^14 17.2 / 14.4; against them
+    //   few_groups  rows evenly long, or a small job: N = 47 64 per row 41.7 / 37.0, R-MAT 2^14 17.2 / 14.4; against them
     //               stencil512 53.9 / 82, R-MAT 2^17 67.4 / 70.6;
-    //   runs_long   long rows, chunks among them: N = 7 R-MAT 2^17 35.3 / 29.0, stencil512 15.8 / 21.8; N = 27 34.0 / 27.0 with 64
+    //   few_long    long rows among even ones, in pieces of 256 that nothing evens out: the piece is the longest chain, and one row per
+    //               warp walks it fastest (400 000 x 4 and one of 2000 N = 47 / 63 92 / 74, 133 / 86);
+    //   runs_long   rows long, evenly or not: N = 7 R-MAT 2^17 35.3 / 29.0, stencil512 15.8 / 21.8; N = 27 34.0 / 27.0 with 64
     //               per row, 37.9 / 43.6 with 4;
     //   dense_panels  neighbouring rows share columns, and their gathers hit L1: N = 13 stencil512 19.5 / 26.3, 7 per row 17.3 / 14.6.
     const bool few_rows = a.num_rows < (uint32_t)sm_count * 40;
-    const bool runs_long = a.num_chunks || a.avg_row_nnz >= kLongRows;
-    const bool few_groups = a.num_rows < (uint32_t)sm_count * 160 || (!a.num_chunks && a.avg_row_nnz >= kLongRows);
+    const bool runs_long = a.uneven || a.avg_row_nnz >= kLongRows;
+    const bool few_long = a.num_chunks && !a.uneven && !a.short_chunks && a.num_tiles < (uint32_t)sm_count * 48;
+    const bool few_groups = few_long || a.num_rows < (uint32_t)sm_count * 160 || (!a.uneven && a.avg_row_nnz >= kLongRows);
     if (v2 && N > 32) {
         if (N > 128) CUTESPMM_GO(2, 4);
         if (N > 64) CUTESPMM_GO(2, 2);

@@ -526,6 +526,53 @@ def test_rows_that_the_groups_of_a_warp_share(oracle_mod, many_tiles, N):
     assert p.device_status() == 0
 
 
+def _rows_of(ln, K, seed):
+    """A matrix of given row lengths, and its CSR arrays on the GPU."""
+    rng = np.random.default_rng(seed)
+    rp = np.concatenate([[0], np.cumsum(ln)])
+    A = g.CsrMatrix(len(ln), K, torch.from_numpy(rp), torch.from_numpy(rng.integers(0, K, rp[-1]).astype(np.int32)), torch.from_numpy(rng.standard_normal(rp[-1]).astype(np.float32)))
+    return A, (A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda())
+
+
+def _best_us(call):
+    best = float("inf")
+    for _ in range(6):
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        for _ in range(10):
+            call()
+        end.record()
+        end.synchronize()
+        best = min(best, start.elapsed_time(end) * 100)
+    return best
+
+
+@pytest.mark.parametrize("made", ["device", "host", "file"])
+@pytest.mark.parametrize("M, per_row, N", [(60_000, 32, 47), (400_000, 4, 63)])
+def test_a_long_row_leaves_the_others_their_kernel(oracle_mod, tmp_path, made, M, per_row, N):
+    """Rows off the 16-byte grid: one long row among even ones costs its own pieces (1.1 and 1.25 times the time; 1.9 times where it
+    decides which kernel all rows take), whoever made the plan."""
+    times = []
+    for hub in (False, True):
+        ln = np.full(M, per_row)
+        if hub:
+            ln[M // 3] = 1000
+        A, csr = _rows_of(ln, M, 21)
+        p = cs.Plan.from_device_csr(M, M, *csr) if made == "device" else cs.Plan.from_csr(A)
+        if made == "file":
+            p.save(str(tmp_path / "plan"))
+            p = cs.Plan.load(str(tmp_path / "plan"))
+        B, C = g.dense_operand(M, N, 22, device="cuda"), torch.empty((M, N), device="cuda")
+        p.spmm(B, C)
+        if hub:
+            rows = np.concatenate([np.arange(5), np.arange(M // 3 - 2, M // 3 + 3), np.arange(M - 5, M)])
+            want = oracle_mod.spmm_csr_rows(A.row_ptr, A.cols, A.vals, B.cpu().numpy(), rows)
+            assert oracle_mod.rel_fro(want, C[torch.from_numpy(rows).cuda()].cpu().numpy()) <= REL_FRO_TOL_FP32
+        times.append(_best_us(lambda: p.spmm(B, C)))
+        assert p.device_status() == 0
+    assert times[1] <= 1.5 * times[0], times
+
+
 @pytest.mark.parametrize("N", [128, 129, 132, 256, 260, 388, 509])
 def test_wide_products_of_rows_in_runs_walk_a_tile_once_per_slab(oracle_mod, N):
     """More tiles than a wave of blocks: slabs of equal width, one after the other over each tile; the last one may be narrower."""
