@@ -322,6 +322,12 @@ int cutespmm_plan_decode_csr(const cutespmm_plan_t *p, uint64_t *rowPtr, uint32_
     return CUTESPMM_OK;
 }
 
+// A small job: its long rows are cut into pieces of tens of nonzeros.
+static bool short_pieces(const HostPlan &h)
+{
+    return item_sizes(h.nnz + kRowCost * h.M, h.nnz, h.M, 0, h.opts.split_nnz, h.opts.tile_nnz, h.adaptive_tiling).latency_bound;
+}
+
 static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B, uint64_t ldb, float *C, uint64_t ldc,
                           uint32_t N, bool b_padded, const cutespmm_item_range *rg = nullptr)
 {
@@ -338,7 +344,7 @@ static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B,
     a.arrivals = p->d_arrivals + (all_rows ? (uint64_t)p->own.long_rows * kArrivalSlabs : 0);
     a.dense_panels = h.num_bricks ? 1u : 0u;
     a.avg_row_nnz = (uint32_t)(h.nnz / std::max<uint64_t>(h.M, 1));
-    a.short_chunks = item_sizes(h.nnz + kRowCost * h.M, h.nnz, h.M, 0, h.opts.split_nnz, h.opts.tile_nnz, h.adaptive_tiling).latency_bound ? 1u : 0u;
+    a.short_chunks = short_pieces(h) ? 1u : 0u;
     a.B = B; a.C = C; a.scratch = p->d_scratch;
     a.ldb = ldb; a.ldc = ldc; a.ld_scratch = kScratchCols;
     a.N = N;
@@ -445,13 +451,17 @@ static void note_stream(const cutespmm_plan *p, cudaStream_t s)
 // Rows of B that are not 16-byte aligned (N not a multiple of four columns, a view) are read one or two columns per lane and load.
 // Copying B once into rows of N rounded up to four first (the copy lives on the stream) costs a launch, 1.25 ps per element of the
 // copy and, as C is written column by column then, 1.6 ps per element of C; with the kernels for unaligned rows as they are it
-// pays in these ranges only (us without / with the copy):
+// pays in these ranges only (us without / with the copy; "graphs": rows cut into pieces, and uneven ones):
 //   20 or 25 to 31 columns, short rows: the copy lets a warp take four rows with one load each; 6 ps per nonzero (7 per row
 //     N = 31 26.0 / 21.2, stencil512 52.5 / 37.9, elasticity40 N = 22 35.5 / 31.7; 4 per row N = 27 37.9 / 46.4: not there); graphs
-//     with long rows from 17 columns on, 4 ps, where the copy stays in L2 (R-MAT 2^18 N = 27 92.2 / 80.8, 2^20 322 / 422);
+//     from 17 columns on, 4 ps, where the copy stays in L2 (R-MAT 2^18 N = 27 92.2 / 80.8, 2^20 322 / 422);
 //   33 to 64 and above 384 columns, rows long enough: 0.1 ps per nonzero and column (64 per row N = 47 37.0 / 35.1, N = 511
 //     258 / 234; N = 259 177 / 218; 7 per row N = 47 32.6 / 33.9);
-//   65 to 256 columns of mid-sized graphs with long rows, 0.2 ps per nonzero and column against a copy that stays in L2 (R-MAT 2^15
+//   9 to 64 columns (9 to 32 where all rows are long) of jobs whose rows are even but for a few in pieces of 256: four columns per load
+//     are the quickest at walking such a piece, 12 ps (400 000 x 4 and one of 1000 N = 15 35.3 / 25.1, N = 31 57.4 / 37.7, N = 47
+//     62.3 / 51.7, N = 7 20.4 / 21.6; 60 000 x 32 and one of 1000 N = 15 29.3 / 25.0, N = 47 41.6 / 48.1).  Not where there are tiles
+//     enough to be dealt, which hides the piece (two million x 4 and one of 3000 N = 47 206 / 231);
+//   65 to 256 columns of mid-sized graphs, 0.2 ps per nonzero and column against a copy that stays in L2 (R-MAT 2^15
 //     with 19 per row N = 135 72.2 / 55.2, 2^16 102 / 89.0; 2^14 25.6 / 27.9 and 2^17 156 / 167: not there).
 //   rows of 150 and more nonzeros at every width, in windows of columns where the copy would be too large, by 12 ps per nonzero up to
 //     64 columns and 0.4 ps per nonzero and column beyond (300 per row N = 15 84.0 / 67.1, N = 301 776 / 685, 4000 x 200 per row N = 7
@@ -459,19 +469,21 @@ static void note_stream(const cutespmm_plan *p, cudaStream_t s)
 // Even widths above 32 are read two columns per lane and gain nothing.  Copies above kMaxPadBytes are not made: the pool would
 // give them back at every synchronisation and map them anew (1.8 GB: 4.6 -> 5.6 ms per product).  Not while the stream is being
 // captured (a graph should not own memory).
-constexpr uint64_t kMaxPadBytes = 512ull << 20, kNearBytes = 64ull << 20, kVeryLongRows = 150;
+constexpr uint64_t kMaxPadBytes = 512ull << 20, kNearBytes = 64ull << 20, kVeryLongRows = 150, kFewTiles = 7104;  // tiles: 8 x 148 x 6, launch_rows_t
 static bool worth_padding(const cutespmm_plan *p, const cutespmm_list_sizes &list, const float *B, uint64_t ldb, const float *C, uint64_t ldc, uint32_t N)
 {
     const HostPlan &h = p->host;
     const bool two = !((reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 7) && !((ldb | ldc | N) & 1);
     if ((two && N > 32) || h.K * ((uint64_t)N + 3) * sizeof(float) > kMaxPadBytes) return false;
     if (h.nnz >= kVeryLongRows * h.M) return h.nnz * (N <= 64 ? 12 : N * 2 / 5) >= 3000000 + h.K * N * 5 / 4;
+    const bool graph = list.chunks && h.uneven, long_rows = h.nnz >= 24 * h.M;
+    if (list.chunks && !graph && !short_pieces(h) && list.tiles < kFewTiles && N > 8 && N <= (long_rows ? 32u : 64u)) return h.nnz * 12 >= 3000000 + h.K * N * 5 / 4;  // picoseconds
     if (N <= 32) {
-        if (N < (list.chunks ? 17u : h.run_rows ? 20u : 25u) || (!list.chunks && h.nnz >= 24 * h.M)) return false;
-        if (list.chunks && h.K * ((uint64_t)N + 3) * sizeof(float) > kNearBytes) return false;
-        return h.nnz * (list.chunks ? 4 : 6) >= 3000000 + h.K * N * 5 / 4;  // picoseconds
+        if (N < (graph ? 17u : h.run_rows ? 20u : 25u) || (!graph && long_rows)) return false;
+        if (graph && h.K * ((uint64_t)N + 3) * sizeof(float) > kNearBytes) return false;
+        return h.nnz * (graph ? 4 : 6) >= 3000000 + h.K * N * 5 / 4;
     }
-    if (N > 64 && N <= 256 && list.chunks && h.K * ((uint64_t)N + 3) * sizeof(float) <= kNearBytes)
+    if (N > 64 && N <= 256 && graph && h.K * ((uint64_t)N + 3) * sizeof(float) <= kNearBytes)
         return h.nnz * std::max(N, 100u) / 5 >= 6000000 + N * (h.K * 8 + h.M * 12) / 10;
     return (N <= 64 || N > 384) && h.nnz * N / 10 >= 3000000 + N * (h.K * 13 + h.M * 16) / 10;
 }

@@ -328,12 +328,13 @@ void choose_panel_paths(HostPlan &p, const std::vector<uint32_t> &panel_ncols)
 
 bool find_uneven(const HostPlan &p)
 {
-    uint64_t mid_nnz = 0;
+    uint64_t mid_nnz = 0, long_nnz = 0;
     for (uint64_t r = 0; r < p.M; ++r) {
         const uint32_t len = p.row_ptr[r + 1] - p.row_ptr[r];
-        if (mid_row(len, p.nnz, p.M)) mid_nnz += len;
+        if (len > kDefaultSplitNnz) long_nnz += len;
+        else if (mid_row(len, p.nnz, p.M)) mid_nnz += len;
     }
-    return is_uneven(mid_nnz, p.nnz);
+    return is_uneven(mid_nnz, long_nnz, p.nnz);
 }
 
 uint32_t find_row_runs(const HostPlan &p)

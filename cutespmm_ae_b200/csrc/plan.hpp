@@ -92,10 +92,11 @@ CUTESPMM_HD inline ItemSizes item_sizes(uint64_t total, uint64_t nnz, uint64_t M
     return s;
 }
 // Rows are of very different lengths: an eighth of the nonzeros (mid_nnz) sits in rows of more than twice the mean and more than 32,
-// those beyond kDefaultSplitNnz left out, which are cut up anyway.  R-MAT graphs of up to 24 edges per node and side hold 13 to 50 %
-// there.  A few long rows in a matrix of short ones do not make it uneven, whatever they hold.
+// those beyond kDefaultSplitNnz left out, which are cut up anyway, or a quarter in the latter (long_nnz).  R-MAT graphs of up to 20
+// edges per node and side hold 25 to 43 % in the former, denser ones 50 to 78 % in the latter.  A few long rows in a matrix of short
+// ones do not make it uneven.
 CUTESPMM_HD inline bool mid_row(uint32_t len, uint64_t nnz, uint64_t M) { return len > 32 && len <= kDefaultSplitNnz && len * M > 2 * nnz; }
-CUTESPMM_HD inline bool is_uneven(uint64_t mid_nnz, uint64_t nnz) { return mid_nnz > nnz / 8; }
+CUTESPMM_HD inline bool is_uneven(uint64_t mid_nnz, uint64_t long_nnz, uint64_t nnz) { return mid_nnz > nnz / 8 || long_nnz > nnz / 4; }
 // nonzeros per chunk of a row of `len` nonzeros that is being cut
 CUTESPMM_HD inline uint32_t piece_length(const ItemSizes &s, uint32_t len)
 {

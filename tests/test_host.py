@@ -295,6 +295,28 @@ def test_launch_count_covers_the_padded_copy_of_b():
     assert often.kernels(47) == "rows"
 
 
+def _even_rows(M, K, per_row, hub=0):
+    ln = np.full(M, per_row)
+    if hub:
+        ln[M // 3] = hub
+    rp = np.concatenate([[0], np.cumsum(ln)]).astype(np.uint64)
+    return cs.Plan(M, K, rp, (np.arange(rp[-1]) * 97 % K).astype(np.uint32), np.ones(rp[-1], np.float32), path=cs.PATH_ROWS, host_only=True)
+
+
+def test_a_few_long_rows_and_the_padded_copy_of_b():
+    """One row in pieces among even ones does not make them a graph: where the others take a copy they still do, and narrow products
+    of large jobs take one for the piece's sake.  Graphs, of few or of many nonzeros per row, go by their own rule."""
+    even, hub = _even_rows(400_000, 100_000, 4), _even_rows(400_000, 100_000, 4, hub=1000)
+    assert [even.launch_count(n) for n in (7, 15, 27, 31, 47)] == [1, 1, 2, 2, 1]
+    assert [hub.launch_count(n) for n in (7, 15, 27, 31, 47)] == [1, 2, 2, 2, 2]
+    assert [_even_rows(60_000, 60_000, 32, hub=1000).launch_count(n) for n in (7, 15, 27, 47)] == [1, 2, 2, 1]
+    assert [_even_rows(100_000, 100_000, 7, hub=1000).launch_count(n) for n in (7, 15, 23, 47)] == [1, 1, 1, 1]  # a small job: short pieces
+    assert [_even_rows(1_500_000, 50_000, 4, hub=3000).launch_count(n) for n in (15, 47)] == [1, 1]  # tiles enough to be dealt
+    for edges in (8, 40):
+        graph = cs.Plan.from_csr(g.rmat(15, edges, seed=3), path=cs.PATH_ROWS, host_only=True)
+        assert [graph.launch_count(n) for n in (7, 15, 27)] == [1, 1, 1 + (edges == 40)]
+
+
 def test_auto_keeps_small_matrices_on_the_row_kernel():
     """The default of path auto: dense panels go to the tensor-core kernel only when there are enough of them to fill
     its grid (4440); a small stencil stays on the row kernel, the 512 x 512 one does not."""
