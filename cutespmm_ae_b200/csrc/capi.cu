@@ -455,8 +455,11 @@ static void note_stream(const cutespmm_plan *p, cudaStream_t s)
 //   20 or 25 to 31 columns, short rows: the copy lets a warp take four rows with one load each; 6 ps per nonzero (7 per row
 //     N = 31 26.0 / 21.2, stencil512 52.5 / 37.9, elasticity40 N = 22 35.5 / 31.7; 4 per row N = 27 37.9 / 46.4: not there); graphs
 //     from 17 columns on, 4 ps, where the copy stays in L2 (R-MAT 2^18 N = 27 92.2 / 80.8, 2^20 322 / 422);
-//   33 to 64 and above 384 columns, rows long enough: 0.1 ps per nonzero and column (64 per row N = 47 37.0 / 35.1, N = 511
-//     258 / 234; N = 259 177 / 218; 7 per row N = 47 32.6 / 33.9);
+//   33 to 64 and above 256 columns (graphs: above 384), rows long enough: 0.1 ps per nonzero and column (64 per row N = 47 37.0 / 35.1,
+//     N = 511 258 / 234; 100 000 x 28 of 2000 columns N = 301 260 / 239, 60 000 x 48 N = 383 396 / 338; 7 per row N = 47 32.6 / 33.9);
+//   65 to 256 columns, no graph, 36 and more per row: 0.0625 ps (60 000 x 100 N = 65 / 135 / 201 / 255 160 / 141, 266 / 240, 303 / 287,
+//     387 / 361, 300 000 x 40 of 20 000 columns N = 135 552 / 475; 30 000 x 60 of 300 000 columns N = 135 138 / 179: not there;
+//     100 000 x 28 of 2000 N = 201 136 / 149: not there);
 //   9 to 64 columns (9 to 32 where all rows are long) of jobs whose rows are even but for a few in pieces of 256: four columns per load
 //     are the quickest at walking such a piece, 12 ps (400 000 x 4 and one of 1000 N = 15 35.3 / 25.1, N = 31 57.4 / 37.7, N = 47
 //     62.3 / 51.7, N = 7 20.4 / 21.6; 60 000 x 32 and one of 1000 N = 15 29.3 / 25.0, N = 47 41.6 / 48.1).  Not where there are tiles
@@ -485,7 +488,9 @@ static bool worth_padding(const cutespmm_plan *p, const cutespmm_list_sizes &lis
     }
     if (N > 64 && N <= 256 && graph && h.K * ((uint64_t)N + 3) * sizeof(float) <= kNearBytes)
         return h.nnz * std::max(N, 100u) / 5 >= 6000000 + N * (h.K * 8 + h.M * 12) / 10;
-    return (N <= 64 || N > 384) && h.nnz * N / 10 >= 3000000 + N * (h.K * 13 + h.M * 16) / 10;
+    const bool wide = N > 64 && N <= (graph ? 384 : 256);
+    if (wide && (graph || h.nnz < 36 * h.M)) return false;
+    return h.nnz * N / (wide ? 16 : 10) >= 3000000 + N * (h.K * 13 + h.M * 16) / 10;
 }
 
 static bool capturing(cudaStream_t s)

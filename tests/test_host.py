@@ -317,6 +317,18 @@ def test_a_few_long_rows_and_the_padded_copy_of_b():
         assert [graph.launch_count(n) for n in (7, 15, 27)] == [1, 1, 1 + (edges == 40)]
 
 
+def test_wide_products_of_long_even_rows_take_a_padded_copy_of_b():
+    """Odd widths above 64: rows of dozens of nonzeros gain more than the copy of B and the narrower stores of C cost."""
+    widths = (65, 135, 201, 255, 301, 383, 409)
+    assert [_even_rows(60_000, 60_000, 100).launch_count(n) for n in widths] == [2] * 7
+    assert [_even_rows(100_000, 10_000, 60).launch_count(n) for n in widths] == [2] * 7
+    assert [_even_rows(100_000, 2000, 28).launch_count(n) for n in widths] == [1, 1, 1, 1, 2, 2, 2]  # rows too short up to 256
+    assert [_even_rows(30_000, 300_000, 60).launch_count(n) for n in widths] == [1] * 7  # each row of B used too seldom
+    assert [_even_rows(100_000, 100_000, 7).launch_count(n) for n in widths] == [1] * 7
+    graph = cs.Plan.from_csr(g.rmat(16, 40, seed=3), path=cs.PATH_ROWS, host_only=True)
+    assert [graph.launch_count(n) for n in (135, 301, 383, 409)] == [2, 1, 1, 2]
+
+
 def test_auto_keeps_small_matrices_on_the_row_kernel():
     """The default of path auto: dense panels go to the tensor-core kernel only when there are enough of them to fill
     its grid (4440); a small stencil stays on the row kernel, the 512 x 512 one does not."""
