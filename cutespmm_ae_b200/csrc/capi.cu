@@ -452,8 +452,11 @@ static void note_stream(const cutespmm_plan *p, cudaStream_t s)
 // Copying B once into rows of N rounded up to four first (the copy lives on the stream) costs a launch, 1.25 ps per element of the
 // copy and, as C is written column by column then, 1.6 ps per element of C; with the kernels for unaligned rows as they are it
 // pays in these ranges only (us without / with the copy; "graphs": rows cut into pieces, and uneven ones):
-//   20 or 25 to 31 columns, short rows: the copy lets a warp take four rows with one load each; 6 ps per nonzero (7 per row
-//     N = 31 26.0 / 21.2, stencil512 52.5 / 37.9, elasticity40 N = 22 35.5 / 31.7; 4 per row N = 27 37.9 / 46.4: not there); graphs
+//   25 (rows in runs: 20) to 31 columns, short rows: the copy lets a warp take four rows with one load each; 6 ps per nonzero (7 per
+//     row N = 31 26.0 / 21.2, stencil512 52.5 / 37.9, elasticity40 N = 22 35.5 / 31.7; 4 per row N = 27 37.9 / 46.4: not there), from 29
+//     columns on 10 ps below 16 per row (100 000 x 7 N = 29 / 31 15.8 / 15.0, 16.6 / 15.2; 30 000 x 20 13.1 / 13.6: not there);
+//   9 to 24 columns, 6 to 23 per row, no dense panels, 5 ps: 200 000 x 10 of 20 000 columns N = 15 / 23 25.3 / 18.7, 31.5 / 25.9, 300 000 x
+//     7 of 20 000 N = 23 36.9 / 30.7 (of 300 000 N = 22 35.7 / 37.0: not there; 4 per row, of 100 000, N = 22 29.2 / 31.5); graphs
 //     from 17 columns on, 4 ps, where the copy stays in L2 (R-MAT 2^18 N = 27 92.2 / 80.8, 2^20 322 / 422);
 //   33 to 64 and above 256 columns (graphs: above 384), rows long enough: 0.1 ps per nonzero and column (64 per row N = 47 37.0 / 35.1,
 //     N = 511 258 / 234; 100 000 x 28 of 2000 columns N = 301 260 / 239, 60 000 x 48 N = 383 396 / 338; 7 per row N = 47 32.6 / 33.9);
@@ -482,9 +485,19 @@ static bool worth_padding(const cutespmm_plan *p, const cutespmm_list_sizes &lis
     const bool graph = list.chunks && h.uneven, long_rows = h.nnz >= 24 * h.M;
     if (list.chunks && !graph && !short_pieces(h) && list.tiles < kFewTiles && N > 8 && N <= (long_rows ? 32u : 64u)) return h.nnz * 12 >= 3000000 + h.K * N * 5 / 4;  // picoseconds
     if (N <= 32) {
-        if (N < (graph ? 17u : h.run_rows ? 20u : 25u) || (!graph && long_rows)) return false;
-        if (graph && h.K * ((uint64_t)N + 3) * sizeof(float) > kNearBytes) return false;
-        return h.nnz * (graph ? 4 : 6) >= 3000000 + h.K * N * 5 / 4;
+        uint32_t gain = 6;
+        if (graph) {
+            if (N < 17 || h.K * ((uint64_t)N + 3) * sizeof(float) > kNearBytes) return false;
+            gain = 4;
+        } else if (long_rows || N < (h.run_rows ? 20u : 9u)) {
+            return false;
+        } else if (!h.run_rows && N < 25) {
+            if (h.num_bricks || h.nnz < 6 * h.M) return false;
+            gain = 5;
+        } else if (!h.run_rows && N > 28 && h.nnz < 16 * h.M) {
+            gain = 10;
+        }
+        return h.nnz * gain >= 3000000 + h.K * N * 5 / 4;
     }
     if (N > 64 && N <= 256 && graph && h.K * ((uint64_t)N + 3) * sizeof(float) <= kNearBytes)
         return h.nnz * std::max(N, 100u) / 5 >= 6000000 + N * (h.K * 8 + h.M * 12) / 10;

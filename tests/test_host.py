@@ -329,6 +329,17 @@ def test_wide_products_of_long_even_rows_take_a_padded_copy_of_b():
     assert [graph.launch_count(n) for n in (135, 301, 383, 409)] == [2, 1, 1, 2]
 
 
+def test_narrow_products_of_short_even_rows_take_a_padded_copy_of_b():
+    """Odd widths up to 31, no rows in runs: both sides of the rule in rows of B, nonzeros per row and columns."""
+    widths = (7, 8, 9, 15, 23, 27, 29, 31)
+    counts = lambda *a: [_even_rows(*a).launch_count(n) for n in widths]
+    assert counts(200_000, 20_000, 10) == counts(300_000, 20_000, 7) == [1, 1, 2, 2, 2, 2, 2, 2]
+    assert counts(100_000, 100_000, 7) == [1, 1, 1, 1, 1, 1, 2, 2]
+    assert counts(300_000, 300_000, 7) == [1, 1, 2, 2, 1, 1, 2, 2]
+    assert counts(400_000, 100_000, 4) == [1, 1, 1, 1, 1, 2, 2, 2]
+    assert counts(30_000, 30_000, 20) == counts(20_000, 20_000, 60) == [1] * 8
+
+
 def test_auto_keeps_small_matrices_on_the_row_kernel():
     """The default of path auto: dense panels go to the tensor-core kernel only when there are enough of them to fill
     its grid (4440); a small stencil stays on the row kernel, the 512 x 512 one does not."""
