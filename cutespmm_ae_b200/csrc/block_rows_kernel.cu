@@ -10,7 +10,8 @@
 // 222 -> 165; before, after a padded copy of B or one row at a time).
 // Products wider than 128 columns go in slabs of equal width, and a block walks its tile once per slab, so that nobody waits for a
 // narrow last slab's blocks and the tile's rows of B are near for all of them (elasticity40 N = 300 284 -> 199 us, N = 132 130 -> 119,
-// N = 511 478 -> 335; slabs side by side in the grid before).  Jobs of less than a wave of tiles spread the slabs over blocks.
+// N = 511 478 -> 335; slabs side by side in the grid before, two blocks more than a wave where there were three).  Jobs of a few
+// waves of tiles spread the slabs over blocks (launch_t).
 // Row kernel -> here: elasticity40 N = 32 35.1 -> 25.7 us, N = 27 48.7 -> 34.2; elasticity20 N = 128 20.4 -> 12.8.
 #include <cuda_runtime.h>
 
@@ -146,10 +147,14 @@ template <int R, int G, bool ALIGNED> cudaError_t launch_t(RowsArgs a, int sm_co
     int per_sm = 0;
     const cudaError_t e = blocks_per_sm<spmm_block_rows_kernel<R, G, ALIGNED>>(per_sm, kTileWarps * 32);
     if (e != cudaSuccess) return e;
-    const uint32_t slabs = (a.N + 127) / 128, wave = (uint32_t)(sm_count * per_sm);
-    const bool spread = a.num_tiles < wave;  // slabs beside each other in the grid
+    const uint32_t slabs = (a.N + 127) / 128, wave = (uint32_t)(sm_count * per_sm), per_slab = wave / slabs ? wave / slabs : 1;
+    // Up to four waves of tiles the slabs lie beside each other in the grid, in one wave of blocks: a block that walks whole tiles has
+    // too few of them (walk / grid: elasticity21 N = 132 / 256 / 512 22.9 / 18.7 us, 24.3 / 19.7, 45.2 / 38.1, elasticity28 N = 300 / 512 68.5 /
+    // 64.5, 95 / 85.7, but N = 132 39.4 / 41.6; from there on elasticity33 N = 260 93.9 / 101, elasticity40 176 / 201).
+    const bool spread = a.num_tiles < 4 * wave;
     a.slab_cols = ((a.N + slabs - 1) / slabs + 3) & ~3u;
-    return launch_overlapped(spmm_block_rows_kernel<R, G, ALIGNED>, spread ? dim3((a.num_tiles + slabs - 1) / slabs, slabs) : dim3(wave), kTileWarps * 32, 0, s, a);
+    return launch_overlapped(spmm_block_rows_kernel<R, G, ALIGNED>, spread ? dim3(a.num_tiles < per_slab ? a.num_tiles : per_slab, slabs) : dim3(wave), kTileWarps * 32,
+                             0, s, a);
 }
 template <int R, bool ALIGNED> cudaError_t launch_r(const RowsArgs &a, int sm_count, cudaStream_t s)
 {

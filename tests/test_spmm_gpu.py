@@ -575,7 +575,7 @@ def test_a_long_row_leaves_the_others_their_kernel(oracle_mod, tmp_path, made, M
 
 @pytest.mark.parametrize("N", [128, 129, 132, 256, 260, 388, 509])
 def test_wide_products_of_rows_in_runs_walk_a_tile_once_per_slab(oracle_mod, N):
-    """More tiles than a wave of blocks: slabs of equal width, one after the other over each tile; the last one may be narrower."""
+    """Five waves of tiles: slabs of equal width, one after the other over each tile; the last one may be narrower."""
     A = g.elasticity3d(32, 3, 9)
     p = cs.Plan.from_device_csr(A.M, A.K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS)
     B = g.dense_operand(A.K, N, 7)
@@ -584,6 +584,33 @@ def test_wide_products_of_rows_in_runs_walk_a_tile_once_per_slab(oracle_mod, N):
     want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.numpy(), A.M, A.K)
     assert oracle_mod.rel_fro(want, out[:A.M].cpu().numpy()) <= REL_FRO_TOL_FP32
     assert torch.isnan(out[A.M]).all() and p.device_status() == 0
+
+
+@pytest.mark.parametrize("N", [129, 132, 256, 260, 384, 388, 509, 512])
+@pytest.mark.parametrize("n", [13, 21])
+def test_wide_products_of_rows_in_runs_with_the_slabs_in_the_grid(oracle_mod, n, N):
+    """Fewer than four waves of tiles, less than one and one and a half: a block takes every few tiles of one slab."""
+    A = g.elasticity3d(n, 3, 9)
+    p = cs.Plan.from_device_csr(A.M, A.K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS)
+    B = g.dense_operand(A.K, N, 7)
+    out = torch.full((A.M + 1, N), float("nan"), device="cuda")
+    p.spmm(B.cuda(), out[:A.M])
+    want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.numpy(), A.M, A.K)
+    assert oracle_mod.rel_fro(want, out[:A.M].cpu().numpy()) <= REL_FRO_TOL_FP32
+    assert torch.isnan(out[A.M]).all() and p.device_status() == 0
+
+
+@pytest.mark.parametrize("N", [256, 512])
+def test_slabs_of_rows_in_runs_fill_the_machine(N):
+    """1.1 and 1.5 waves of tiles: in blocks that walk whole tiles both are two rounds per slab, and the larger matrix takes 1.03 and 1.01
+    times as long per row at 256 and 512 columns; with the slabs in the grid 0.85 and 0.93."""
+    times = []
+    for n in (19, 21):
+        A = g.elasticity3d(n, 3, 9)
+        p = cs.Plan.from_device_csr(A.M, A.K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS)
+        B, C = g.dense_operand(A.K, N, 7, device="cuda"), torch.empty((A.M, N), device="cuda")
+        times.append(_best_us(lambda: p.spmm(B, C)) / A.M)
+    assert times[1] <= 0.97 * times[0], times
 
 
 def test_wide_unaligned_products_of_large_matrices_go_in_windows(oracle_mod):
