@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "device_plan.hpp"
 #include "last_block.cuh"
@@ -389,9 +390,14 @@ __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
 // G = rows of A (or chunks) a warp works on at the same time: it is G groups of L = 32/G lanes, and a group spans L * VEC * CH
 // columns, CH groups of L * VEC neighbouring ones.  G > 1 (narrow products): a group spans the whole row of B and owns a row of A
 // of its own, so a warp keeps G times as many gathers in flight and few lanes idle.
-template <int VEC, int CH, bool FULL, bool DEEP, int G, bool DYN>
-__global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DYN, G)) spmm_rows_kernel(RowsArgs a)
+// Which tiles a block gets: every gridDim.x-th, the next one of a counter, or that with the long rows of a tile shared by the groups.
+enum Deal { kFixed, kDealt, kShared };
+
+template <int VEC, int CH, bool FULL, bool DEEP, int G, Deal DEAL>
+__global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DEAL != kFixed, G)) spmm_rows_kernel(RowsArgs a)
 {
+    constexpr bool DYN = DEAL != kFixed;
+    static_assert(DEAL != kShared || G > 1, "rows are shared between groups");
     using V = typename Vec<VEC>::T;
     constexpr int L = 32 / G;  // lanes of a group
     const int lane = threadIdx.x & 31;
@@ -442,8 +448,8 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DYN, G))
         const uint4 d = st.desc;
         const uint32_t rb = d.x & ~3u, jb = d.z & ~1u;
         constexpr int U = kRowsInFlight<VEC, CH, DEEP>;  // rows of B in flight per group and step
-        if constexpr (G > 1 && DYN) {
-            // Graphs with long rows, many tiles: the rows of a tile are of very different lengths, and one of hundreds of nonzeros is
+        if constexpr (DEAL == kShared) {
+            // Graphs with rows of very different lengths, many tiles: the rows of a tile are of very different lengths, and one of hundreds of nonzeros is
             // a chain of as many steps for its group while the tile has too few rows to go round.  The groups of a warp share
             // such a row, group g takes nonzeros g, g + G, ... (R-MAT 2^20 N = 8 / 16 / 32 / 64 210 / 212 / 266 / 367 us -> 187 / 176 / 250 / 357).
             auto store = [&](uint32_t r, V(&acc)[CH]) {
@@ -532,15 +538,31 @@ cudaError_t launch_rows_t(RowsArgs a, uint32_t slabs, int sm_count, cudaStream_t
     constexpr uint32_t w = 32 / G * VEC * CH;
     const bool equal = VEC < 4 || (uint64_t)a.num_tiles <= (uint64_t)sm_count * 6 || a.N - (slabs - 1) * w < w / 2;
     a.slab_cols = equal ? ((a.N + slabs - 1) / slabs + 3) & ~3u : w;
-    int n = 0;
-    cudaError_t e;
-    if (a.counters && slabs <= kDealtSlabs) {  // tiles dealt by a counter: where there are enough to deal
-        if ((e = blocks_per_sm<spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true>>(n, kWarps * 32)) != cudaSuccess) return e;
-        if (a.num_tiles >= 8ull * grid(n))
-            return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, true>, dim3(grid(n), slabs), kWarps * 32, 0, s, a);
+    cudaError_t e = cudaSuccess;
+    auto launched = [&](auto deal) {  // tiles are dealt where there are enough of them
+        constexpr Deal D = decltype(deal)::value;
+        int n = 0;
+        if ((e = blocks_per_sm<spmm_rows_kernel<VEC, CH, FULL, DEEP, G, D>>(n, kWarps * 32)) != cudaSuccess) return true;
+        if (D != kFixed && a.num_tiles < 8ull * grid(n)) return false;
+        e = launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, D>, dim3(grid(n), slabs), kWarps * 32, 0, s, a);
+        return true;
+    };
+    // Sharing pays in graphs of a dozen nonzeros per row and more; short rows are claimed more slowly by the kernels that can share (us
+    // dealt / shared: R-MAT 2^20 with 15 per row N = 8 / 16 / 32 209 / 185, 211 / 175, 264 / 249, 2^19 with 28 199 / 183, 181 / 166, 213 /
+    // 197; 2^20 with 7 136 / 145, 134 / 136, 155 / 162; two million x 4 and one of 3000 N = 16 / 32 / 64 78.5 / 84, 105 / 112, 168 / 186,
+    // but N = 8 78.5 / 73.3).  Off the 16-byte grid the claims are a smaller part of the time: always shared there (two million x 4
+    // N = 48 219, 232 after a padded copy and dealt; R-MAT 2^20 with 7 per row N = 16 / 48 159 / 297, before 216 / 365).
+    const bool share = VEC < 4 || (a.uneven ? a.avg_row_nnz >= kWideTileRowNnz : a.N <= 8);
+    if (a.counters && slabs <= kDealtSlabs) {
+        if constexpr (G > 1) {
+            if (share && launched(std::integral_constant<Deal, kShared>{})) return e;
+        }
+        if constexpr (G == 1 || VEC == 4) {
+            if ((G == 1 || !share) && launched(std::integral_constant<Deal, kDealt>{})) return e;
+        }
     }
-    if ((e = blocks_per_sm<spmm_rows_kernel<VEC, CH, FULL, DEEP, G, false>>(n, kWarps * 32)) != cudaSuccess) return e;
-    return launch_overlapped(spmm_rows_kernel<VEC, CH, FULL, DEEP, G, false>, dim3(grid(n), slabs), kWarps * 32, 0, s, a);
+    launched(std::integral_constant<Deal, kFixed>{});
+    return e;
 }
 
 // dst (rows x quads float4, 16-byte aligned) = src (rows x N, leading dimension ld_src), padding zeroed.  Bound by memory
