@@ -671,7 +671,7 @@ int cutespmm_sddmm(const cutespmm_plan_t *p, const float *X, uint64_t ldx, const
     a.num_chunks = all ? p->every.chunks : p->own.chunks;
     a.X = X; a.Y = Y; a.ldx = ldx; a.ldy = ldy; a.out = out; a.N = N;
     a.scale = scale_by_values ? 1u : 0u;
-    a.short_rows = h.nnz < 4 * h.M ? 1u : 0u;
+    a.short_rows = h.nnz < 4 * h.filled_rows ? 1u : 0u;
     a.early = h.values_on_device ? 0u : 1u;
     a.status = p->d_status;
     a.vec4 = !((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15) && !((ldx | ldy) & 3) && (ldx | ldy) < (1ull << 30) ? 1u : 0u;

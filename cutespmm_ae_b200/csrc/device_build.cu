@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(kCensusThreads) panel_census_kernel(const uint
 
 // ---- what the whole matrix looks like --------------------------------------------------------------------------------
 // A thread per row.  (1) The nonzeros in rows longer than kDefaultSplitNnz, which item_sizes decides by, and in those that make a
-// matrix uneven (mid_row).  (2) Whether rows come in runs of the same columns (find_row_runs, plan.cpp): a row is compared with the row in
+// matrix uneven (mid_row), and the rows that have any.  (2) Whether rows come in runs of the same columns (find_row_runs, plan.cpp): a row is compared with the row in
 // front; what is ruled out already is not looked at again, which for most matrices is everything after each block's first
 // rows, so the grid is one block per SM at most and a warp reports once.  Positions are clamped to nnz (nobody has checked
 // the row pointers yet).  cols may be missing: no runs are looked for then.
@@ -496,13 +496,14 @@ __global__ void __launch_bounds__(1024) row_survey_kernel(const uint32_t *__rest
     volatile uint32_t *unlike = &totals->unlike;
     const uint32_t nnz = __ldg(row_ptr + M), lane = threadIdx.x & 31;
     const uint32_t never = (M % 2 ? 1u : 0u) | (M % 3 ? 2u : 0u);
-    uint32_t in_long = 0, in_mid = 0;
+    uint32_t in_long = 0, in_mid = 0, filled = 0;
     for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); b < M; b += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t known = cols ? __shfl_sync(kFullMask, *unlike | never, 0) : 3u;
         const uint64_t r = b + lane;
         const uint32_t asks = r < M ? ((r % 2 ? 1u : 0u) | (r % 3 ? 2u : 0u)) & ~known : 0u;
         const uint32_t j = min(__ldg(row_ptr + min(r, (uint64_t)M)), nnz), e = min(__ldg(row_ptr + min(r + 1, (uint64_t)M)), nnz);
         const uint32_t len = e > j ? e - j : 0u;
+        filled += r < M && len != 0;
         if (len > kDefaultSplitNnz) in_long += len;
         else if (mid_row(len, nnz, M)) in_mid += len;
         uint32_t found = 0;
@@ -515,18 +516,22 @@ __global__ void __launch_bounds__(1024) row_survey_kernel(const uint32_t *__rest
         found = __reduce_or_sync(kFullMask, found);
         if (found && lane == 0) atomicOr(&totals->unlike, found);
     }
-    __shared__ uint32_t warps[2][32];
+    __shared__ uint32_t warps[3][32];
     in_long = __reduce_add_sync(kFullMask, in_long);
     in_mid = __reduce_add_sync(kFullMask, in_mid);
+    filled = __reduce_add_sync(kFullMask, filled);
     if (lane == 0) {
         warps[0][threadIdx.x >> 5] = in_long;
         warps[1][threadIdx.x >> 5] = in_mid;
+        warps[2][threadIdx.x >> 5] = filled;
     }
     __syncthreads();
     if (threadIdx.x >= 32) return;
     in_long = __reduce_add_sync(kFullMask, warps[0][lane]);
     in_mid = __reduce_add_sync(kFullMask, warps[1][lane]);
+    filled = __reduce_add_sync(kFullMask, warps[2][lane]);
     if (lane == 0) {
+        if (filled) atomicAdd(&totals->filled_rows, filled);
         if (in_long) atomicAdd(&totals->long_nnz, (unsigned long long)in_long);
         if (in_mid) atomicAdd(&totals->mid_nnz, (unsigned long long)in_mid);
     }

@@ -366,6 +366,7 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
         return fail_cuda_status(e, "reading the row pointers");
     h.nnz = t.nnz;
     h.uneven = is_uneven(t.mid_nnz, t.long_nnz, t.nnz);
+    h.filled_rows = t.filled_rows;
     h.run_rows = M < 2 || !t.nnz ? 0 : M % 3 == 0 && !(t.unlike & 2) ? 3 : M % 2 == 0 && !(t.unlike & 1) ? 2 : 0;
     if (t.bad_rows || (M == 0 && t.nnz)) return fail_status(CUTESPMM_EINVAL, "rowPtr must start at 0 and be non-decreasing");
     if (h.nnz && (!cols_dev || !vals_dev)) return fail_status(CUTESPMM_EINVAL, "cols/vals is NULL");

@@ -103,7 +103,7 @@ struct SddmmArgs {
     float *out;                          // one value per nonzero, in the plan's storage order
     uint32_t N;
     uint32_t scale;                      // 1: multiply by the stored value of A
-    uint32_t short_rows;                 // 1: fewer than four nonzeros per row (picks the kernel's form)
+    uint32_t short_rows;                 // 1: fewer than four nonzeros per row that has any (picks the kernel's form)
     uint32_t early;                      // 1: the plan's arrays never change (RowsArgs::early)
     uint32_t vec4;                       // 1: X, Y and their leading dimensions (below 2^30) allow 16-byte loads
     uint32_t *status;                    // device status word: set to 1 when a bounded wait gives up
@@ -168,6 +168,7 @@ struct BuildTotals {  // one per plan creation, read by the host after the count
     uint32_t tiles;
     uint32_t chunks, long_rows, brick_panels, brick_slots;  // in the order of the per-segment counters
     uint32_t brick_nnz_max, brick_cols_max;
+    uint32_t filled_rows;  // rows that have nonzeros
     uint32_t unlike;  // bit 0: some odd row has other columns than the row in front of it, bit 1: some row not divisible by 3
     unsigned long long bricks, brick_cost, long_nnz, mid_nnz;
 };

@@ -326,15 +326,17 @@ void choose_panel_paths(HostPlan &p, const std::vector<uint32_t> &panel_ncols)
     }
 }
 
-bool find_uneven(const HostPlan &p)
+void survey_rows(HostPlan &p)
 {
-    uint64_t mid_nnz = 0, long_nnz = 0;
+    uint64_t mid_nnz = 0, long_nnz = 0, filled = 0;
     for (uint64_t r = 0; r < p.M; ++r) {
         const uint32_t len = p.row_ptr[r + 1] - p.row_ptr[r];
+        if (len) ++filled;
         if (len > kDefaultSplitNnz) long_nnz += len;
         else if (mid_row(len, p.nnz, p.M)) mid_nnz += len;
     }
-    return is_uneven(mid_nnz, long_nnz, p.nnz);
+    p.uneven = is_uneven(mid_nnz, long_nnz, p.nnz);
+    p.filled_rows = filled;
 }
 
 uint32_t find_row_runs(const HostPlan &p)
@@ -430,7 +432,7 @@ int build_host_plan(HostPlan &p, uint64_t M, uint64_t K, const uint64_t *rowPtr,
     if (p.opts.reorder == CUTESPMM_REORDER_SIMILAR_ROWS) group_similar_rows(p);
 
     p.run_rows = find_row_runs(p);
-    p.uneven = find_uneven(p);
+    survey_rows(p);
     const std::vector<uint32_t> panel_ncols = analyze_panels(p);
 
     choose_panel_paths(p, panel_ncols);

@@ -164,6 +164,7 @@ struct HostPlan {
     std::vector<LongRow> long_rows;
 
     bool uneven = false;                 // rows of very different lengths (is_uneven)
+    uint64_t filled_rows = 0;            // rows that have nonzeros
     uint32_t run_rows = 0;               // rows come in aligned runs of 3 or 2 with the same columns (0: they do not)
 
     // ---- panel analysis (HRPB-compatible view) ----
@@ -219,8 +220,8 @@ int build_host_plan(HostPlan &p, uint64_t M, uint64_t K, const uint64_t *rowPtr,
 // The options of a plan that is built on the device, checked and with the defaults filled in (p.opts, p.adaptive_tiling).
 int check_device_options(HostPlan &p, uint64_t M, uint64_t K, const cutespmm_options_t *opts, std::string &err);
 
-// HostPlan::uneven of a matrix whose row pointers are on the host.
-bool find_uneven(const HostPlan &p);
+// HostPlan::uneven and ::filled_rows of a matrix whose row pointers are on the host.
+void survey_rows(HostPlan &p);
 
 // HostPlan::run_rows of a matrix whose pairs are on the host.
 uint32_t find_row_runs(const HostPlan &p);

@@ -205,7 +205,7 @@ int cutespmm_plan_load(cutespmm_plan_t **plan, const char *path, int host_only)
     }
     p->note_list_sizes();
     h.run_rows = find_row_runs(h);
-    h.uneven = find_uneven(h);
+    survey_rows(h);
     if (!host_only) {
         const int st = cutespmm_internal_upload_plan(p);
         if (st != CUTESPMM_OK) {

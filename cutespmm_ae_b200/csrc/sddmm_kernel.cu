@@ -305,8 +305,11 @@ template <int LANES, int V, bool VEC4, bool FULL, bool EACH = false> cudaError_t
 template <int LANES, int V> cudaError_t launch_sddmm_v(const SddmmArgs &a, int sm_count, cudaStream_t s)
 {
     if (!a.vec4) return launch_sddmm_t<LANES, V, false, false>(a, sm_count, s);
-    // Rows of two or three nonzeros: 200 000 x 3 per row N = 16 / 32 / 64 12.8 / 22.9 / 34.0 us with X kept, 11.3 / 19.0 / 32.8 with X
+    // Rows of two or three nonzeros, empty ones apart (a quarter of 400 000 rows with 12 each N = 32 / 64 25.9 / 47.7 us with X loaded each
+    // time, 23.1 / 43.4 with X kept): 200 000 x 3 per row N = 16 / 32 / 64 12.8 / 22.9 / 34.0 us with X kept, 11.3 / 19.0 / 32.8 with X
     // loaded each time (before the walk by runs 12.3 / 19.2 / 30.2); 4 per row N = 32 33.2 with X kept, 38.8 before.
+    // At 64 columns the walk by runs stays 3 % behind the form before it on the first of these matrices (K = M: 25.9 -> 26.7 us) and is 3 %
+    // ahead with 800 000 x 3 of 50 000 columns (77.8 -> 75.3; X kept 27.7 and 74.4, the groups' nonzeros dealt in turn 26.7 and 78.2).
     if constexpr (V <= 2)
         if (a.short_rows)
             return a.N % (4 * V * LANES) == 0 ? launch_sddmm_t<LANES, V, true, true, true>(a, sm_count, s) : launch_sddmm_t<LANES, V, true, false, true>(a, sm_count, s);

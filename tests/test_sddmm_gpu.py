@@ -51,6 +51,24 @@ def test_sddmm_where_rows_end_inside_a_run_of_nonzeros(oracle_mod, N, shift):
     assert rel(want, out[:nnz].cpu().numpy()) <= TOL and torch.isnan(out[nnz])
 
 
+@pytest.mark.parametrize("made", ["device", "host", "file"])
+@pytest.mark.parametrize("N", [16, 33, 64])
+def test_sddmm_of_a_matrix_of_mostly_empty_rows(oracle_mod, tmp_path, made, N):
+    """Twelve nonzeros in every fourth row: three per row on the average, but X is kept along a row."""
+    M, K = 8000, 500
+    ln = np.where(np.arange(M) % 4 == 1, 12, 0)
+    rp = torch.from_numpy(np.concatenate([[0], np.cumsum(ln)]))
+    rng = np.random.default_rng(N)
+    A = g.CsrMatrix(M, K, rp, torch.from_numpy(rng.integers(0, K, int(rp[-1])).astype(np.int32)), torch.from_numpy(rng.standard_normal(int(rp[-1])).astype(np.float32)))
+    p = cs.Plan.from_device_csr(M, K, rp.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS) if made == "device" else cs.Plan.from_csr(A, path=cs.PATH_ROWS)
+    if made == "file":
+        p.save(str(tmp_path / "plan"))
+        p = cs.Plan.load(str(tmp_path / "plan"))
+    X, Y = g.dense_operand(M, N, 81, device="cuda"), g.dense_operand(K, N, 82, device="cuda")
+    want = oracle_mod.sddmm_csr(A.row_ptr, A.cols, A.vals, X.cpu().numpy(), Y.cpu().numpy())
+    assert rel(want, p.sddmm(X, Y, scale_by_values=True).cpu().numpy()) <= TOL
+
+
 @pytest.mark.parametrize("N", [7, 16, 20, 32, 33, 64, 100])
 def test_sddmm_of_rows_of_few_nonzeros(oracle_mod, N):
     """Fewer than four nonzeros per row: a row of X is loaded for each; long rows among them, empty ones and a last claim of one."""
