@@ -466,7 +466,8 @@ static void note_stream(const cutespmm_plan *p, cudaStream_t s)
 //   9 to 64 columns (9 to 32 where all rows are long) of jobs whose rows are even but for a few in pieces of 256: four columns per load
 //     are the quickest at walking such a piece, 12 ps (400 000 x 4 and one of 1000 N = 15 35.3 / 25.1, N = 31 57.4 / 37.7, N = 47
 //     62.3 / 51.7, N = 7 20.4 / 21.6; 60 000 x 32 and one of 1000 N = 15 29.3 / 25.0, N = 47 41.6 / 48.1).  Not where there are tiles
-//     enough to be dealt, which hides the piece (two million x 4 and one of 3000 N = 47 206 / 231);
+//     enough to be dealt, which hides the piece (two million x 4 and one of 3000 N = 47 206 / 231), unless all rows are long (500 000 x
+//     32 and one of 3000 N = 32 195 / 174, N = 13 142 / 153);
 //   65 to 256 columns of mid-sized graphs, 0.2 ps per nonzero and column against a copy that stays in L2 (R-MAT 2^15
 //     with 19 per row N = 135 72.2 / 55.2, 2^16 102 / 89.0; 2^14 25.6 / 27.9 and 2^17 156 / 167: not there).
 //   rows of 150 and more nonzeros at every width, in windows of columns where the copy would be too large, by 12 ps per nonzero up to
@@ -483,7 +484,7 @@ static bool worth_padding(const cutespmm_plan *p, const cutespmm_list_sizes &lis
     if ((two && N > 32) || h.K * ((uint64_t)N + 3) * sizeof(float) > kMaxPadBytes) return false;
     if (h.nnz >= kVeryLongRows * h.M) return h.nnz * (N <= 64 ? 12 : N * 2 / 5) >= 3000000 + h.K * N * 5 / 4;
     const bool graph = list.chunks && h.uneven, long_rows = h.nnz >= 24 * h.M;
-    if (list.chunks && !graph && !short_pieces(h) && list.tiles < kFewTiles && N > 8 && N <= (long_rows ? 32u : 64u)) return h.nnz * 12 >= 3000000 + h.K * N * 5 / 4;  // picoseconds
+    if (list.chunks && !graph && !short_pieces(h) && (list.tiles < kFewTiles || (long_rows && N > 16)) && N > 8 && N <= (long_rows ? 32u : 64u)) return h.nnz * 12 >= 3000000 + h.K * N * 5 / 4;  // picoseconds
     if (N <= 32) {
         uint32_t gain = 6;
         if (graph) {

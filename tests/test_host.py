@@ -312,6 +312,7 @@ def test_a_few_long_rows_and_the_padded_copy_of_b():
     assert [_even_rows(60_000, 60_000, 32, hub=1000).launch_count(n) for n in (7, 15, 27, 47)] == [1, 2, 2, 1]
     assert [_even_rows(100_000, 100_000, 7, hub=1000).launch_count(n) for n in (7, 15, 23, 47)] == [1, 1, 1, 1]  # a small job: short pieces
     assert [_even_rows(1_500_000, 50_000, 4, hub=3000).launch_count(n) for n in (15, 47)] == [1, 1]  # tiles enough to be dealt
+    assert [_even_rows(200_000, 50_000, 32, hub=3000).launch_count(n) for n in (13, 23, 31)] == [1, 2, 2]  # ... but where all rows are long
     for edges in (8, 40):
         graph = cs.Plan.from_csr(g.rmat(15, edges, seed=3), path=cs.PATH_ROWS, host_only=True)
         assert [graph.launch_count(n) for n in (7, 15, 27)] == [1, 1, 1 + (edges == 40)]
