@@ -111,7 +111,7 @@ static cudaError_t reserve_long_row_state(cutespmm_plan *p, uint64_t &by, const 
     *what = "chunk owners";
     if ((e = upload(owners(h.chunks, h.long_rows), &p->d_chunk_owner, by)) != cudaSuccess) return e;
     if ((e = upload(owners(h.chunks_all, h.long_rows_all), &p->d_chunk_owner_all, by)) != cudaSuccess) return e;
-    const uint64_t counters = (uint64_t)(h.long_rows.size() + h.long_rows_all.size()) * kArrivalSlabs * sizeof(uint32_t);
+    const uint64_t counters = (uint64_t)(h.long_rows.size() + h.long_rows_all.size()) * kArrivalStride * sizeof(uint32_t);
     if (counters) {
         *what = "arrival counters";
         if ((e = cudaMalloc(&p->d_arrivals, counters)) != cudaSuccess || (e = cudaMemset(p->d_arrivals, 0, counters)) != cudaSuccess) return e;
@@ -341,7 +341,7 @@ static RowsArgs rows_args(const cutespmm_plan *p, bool all_rows, const float *B,
     a.num_tiles = all_rows ? p->every.tiles : p->own.tiles;
     a.num_chunks = all_rows ? p->every.chunks : p->own.chunks;
     a.chunk_owner = static_cast<const uint32_t *>(all_rows ? p->d_chunk_owner_all : p->d_chunk_owner);
-    a.arrivals = p->d_arrivals + (all_rows ? (uint64_t)p->own.long_rows * kArrivalSlabs : 0);
+    a.arrivals = p->d_arrivals + (all_rows ? (uint64_t)p->own.long_rows * kArrivalStride : 0);
     a.dense_panels = h.num_bricks ? 1u : 0u;
     a.avg_row_nnz = (uint32_t)(h.nnz / std::max<uint64_t>(h.M, 1));
     a.short_chunks = short_pieces(h) ? 1u : 0u;

@@ -405,7 +405,7 @@ int cutespmm_plan_create_device(cutespmm_plan_t **plan, uint64_t M64, uint64_t K
     LongRow *d_longs = nullptr, *d_longs_all = nullptr;
     auto carve = [&](Carver &c) {
         c.take(p->d_status, 64);
-        c.take(p->d_arrivals, longs * kArrivalSlabs);
+        c.take(p->d_arrivals, longs * kArrivalStride);
         const uint64_t zero = c.used;
         c.take(d_rp, (uint64_t)M + 1 + kRowPtrSlack);
         c.take(d_pairs, h.nnz + 2);

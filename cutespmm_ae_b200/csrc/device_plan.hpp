@@ -55,8 +55,6 @@ cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, dim3 block, 
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
-constexpr uint32_t kDealtSlabs = 2;  // column slabs of a launch that deals its tiles by counters: four columns per lane at 512 columns
-
 // Arguments of the row-gather kernel.
 struct RowsArgs {
     const uint32_t *row_ptr;   // M+1 offsets into pairs
@@ -65,8 +63,8 @@ struct RowsArgs {
     const void *chunks;        // num_chunks x {row, j0, j1, slot}
     const void *long_rows;     // the whole list of long rows {row of C, slot0, slot1, -}, indexed by chunk_owner
     const uint32_t *chunk_owner;  // per scratch slot: index of the long row the chunk belongs to
-    uint32_t *arrivals;        // per long row of the list kArrivalSlabs counters: chunks finished so far (zero between launches)
-    uint32_t *counters;        // balance of the blocks that left, then tiles dealt per column slab (kDealtSlabs of them); zero between
+    uint32_t *arrivals;        // per long row of the list, kArrivalStride apart, kRowSlabs counters: chunks finished so far (zero between launches)
+    uint32_t *counters;        // balance of the blocks that left, then tiles dealt per column slab (kRowSlabs of them); zero between
                                // launches.  nullptr: tiles in fixed turns
     uint32_t num_tiles, num_chunks;
     uint32_t avg_row_nnz;      // nonzeros per row of the whole matrix (picks the kernel's tuning)

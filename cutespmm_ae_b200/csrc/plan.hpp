@@ -36,7 +36,11 @@ constexpr uint32_t kWideTileCost = 768, kMixedTileCost = 640;  // ... and with a
 constexpr uint32_t kMinChunkNnz = 32;             // smallest piece of a cut row
 constexpr uint32_t kMaxSplitNnz = 384;   // a row must fit a tile together with a part-filled one
 constexpr uint32_t kScratchCols = 512;  // widest N one launch handles; wider products run in column windows
-constexpr uint32_t kArrivalSlabs = kScratchCols / 32;  // arrival counters of a long row: one per column slab of the narrowest kind
+constexpr uint32_t kRowSlabs = kScratchCols / 256;  // column slabs of a launch of the row kernel, which span 256 columns wherever one is not enough
+// Words from one long row's arrival counters, one per column slab, to the next one's: two rows share a 128-byte line, packed 16 rows
+// would (R-MAT 2^17 N = 64 47.4 -> 47.6 us, 2^16 28.4 -> 28.5).
+constexpr uint32_t kArrivalStride = 16;
+static_assert(kRowSlabs <= kArrivalStride);
 
 // One nonzero as the row kernel reads it: column index and fp32 bit pattern side by side (8 bytes,
 // one coalesced 64-bit load per lane).

@@ -8,10 +8,12 @@
 // (one float4 each at N = 128, so a row of B is one coalesced 512-byte request), the row's
 // (column, value) pairs are read from the block's staged tile in shared memory (tile_stage.cuh; one
 // broadcast read per nonzero), and the products are accumulated in fp32 registers in storage order.
-// For narrow products (N <= 64) a warp splits into groups of lanes and owns that many rows at
-// once.  Rows of B that are not 16-byte aligned are read one or two columns per lane and load, the lanes'
-// columns interleaved, with as many loads in flight as the registers hold.  The eight warps of a block claim the rows of one scheduling tile as they go, so rows that
-// share columns (stencils, block structure) meet in L1.  C rows are written once with streaming
+// For narrow products (N <= 64) a warp splits into G groups of lanes and owns that many rows at
+// once.  In storage order, too, except that graphs of many tiles share rows of more than 16 nonzeros between the groups
+// (Deal::kShared): such a row is G partial sums, of every G-th nonzero each, added in a fixed tree, as a piece of a long row is.
+// Rows of B that are not 16-byte aligned are read one or two columns per lane and load, the lanes'
+// columns interleaved, with as many loads in flight as the registers hold.  The eight warps of a block claim the rows of one
+// scheduling tile as they go, so rows that share columns (stencils, block structure) meet in L1.  C rows are written once with streaming
 // stores; nothing is read-modify-written: a long row is cut into chunks whose partial sums go to a
 // scratch matrix and are added, in slot order, by whichever warp finishes the row's last chunk (one
 // counter per long row), in the same launch.
@@ -38,7 +40,7 @@ namespace {
 template <bool DEEP> struct Tuning {
     // 48 registers, 40 warps per SM (the lane-group kernels spill 200 bytes at 40 registers and 48 warps: R-MAT 2^17 N = 64
     // 55.8 -> 50.8 us, 800 000 rows of 4 at N = 32 74 -> 65, R-MAT 2^20 N = 128 662 -> 647); the narrow kernels that deal
-    // tiles by a counter have long rows to hide and keep 48 warps (R-MAT 2^20 N = 32: 266 us, 281 with 40)
+    // tiles by a counter have long rows to hide and keep 48 warps (R-MAT 2^20 N = 32, rows not shared: 266 us, 281 with 40)
     static constexpr int min_blocks(bool dyn, int G) { return DEEP ? 4 : dyn && G >= 4 ? 6 : 5; }
 };
 // Rows of B in flight per warp (or group): 16 (deep: 32) registers of B, eight rows at most.  Two column groups of two columns stay
@@ -353,7 +355,7 @@ __device__ __forceinline__ void run_chunks(const ChunkArgs &a)
             }
             // the counter of this row and column slab runs through 0 .. chunks - 1 and wraps: it is back at zero for the next launch,
             // also after launches of this list that overlapped (each adds as many as there are chunks, whatever its grid)
-            uint32_t *cnt = a.arrivals + (uint64_t)owner * kArrivalSlabs + blockIdx.y;
+            uint32_t *cnt = a.arrivals + (uint64_t)owner * kArrivalStride + blockIdx.y;
             if (atomicInc(cnt, lr.z - lr.y - 1) == lr.z - lr.y - 1) {  // every chunk has arrived
                 __threadfence();
                 lr_row = lr.x; slot0 = lr.y; slot1 = lr.z;
@@ -449,9 +451,9 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DEAL != 
         const uint32_t rb = d.x & ~3u, jb = d.z & ~1u;
         constexpr int U = kRowsInFlight<VEC, CH, DEEP>;  // rows of B in flight per group and step
         if constexpr (DEAL == kShared) {
-            // Graphs with rows of very different lengths, many tiles: the rows of a tile are of very different lengths, and one of hundreds of nonzeros is
-            // a chain of as many steps for its group while the tile has too few rows to go round.  The groups of a warp share
-            // such a row, group g takes nonzeros g, g + G, ... (R-MAT 2^20 N = 8 / 16 / 32 / 64 210 / 212 / 266 / 367 us -> 187 / 176 / 250 / 357).
+            // The rows of a tile are of very different lengths, and one of hundreds of nonzeros is a chain of as many steps for its group
+            // while the tile has too few rows to go round.  The groups of a warp share such a row, group g takes nonzeros g, g + G,
+            // ... (R-MAT 2^20 N = 8 / 16 / 32 / 64 210 / 212 / 266 / 367 us -> 187 / 176 / 250 / 357).
             auto store = [&](uint32_t r, V(&acc)[CH]) {
                 const uint32_t r_out = a.row_map ? __ldg(a.row_map + r) : r;
                 float *out = a.C + (uint64_t)r_out * a.ldc + col0;
@@ -517,13 +519,14 @@ __global__ void __launch_bounds__(kWarps * 32, Tuning<DEEP>::min_blocks(DEAL != 
     if (DYN) {
         __syncthreads();
         if (threadIdx.x == 0 && last_block_out(a.counters))
-            for (uint32_t y = 0; y < kDealtSlabs; ++y) a.counters[1 + y] = 0;
+            for (uint32_t y = 0; y < kRowSlabs; ++y) a.counters[1 + y] = 0;
     }
 }
 
 template <int VEC, int CH, bool FULL, bool DEEP, int G = 1>
 cudaError_t launch_rows_t(RowsArgs a, uint32_t slabs, int sm_count, cudaStream_t s)
 {
+    if (slabs > kRowSlabs) return cudaErrorInvalidConfiguration;  // counters per slab: arrived chunks, dealt tiles
     const uint64_t chunk_blocks = ((uint64_t)a.num_chunks + kWarps - 1) / kWarps;
     const uint64_t work = a.num_tiles > chunk_blocks ? a.num_tiles : chunk_blocks;
     auto grid = [&](int per_sm) {  // about one resident wave over all slabs
@@ -553,7 +556,7 @@ cudaError_t launch_rows_t(RowsArgs a, uint32_t slabs, int sm_count, cudaStream_t
     // but N = 8 78.5 / 73.3).  Off the 16-byte grid the claims are a smaller part of the time: always shared there (two million x 4
     // N = 48 219, 232 after a padded copy and dealt; R-MAT 2^20 with 7 per row N = 16 / 48 159 / 297, before 216 / 365).
     const bool share = VEC < 4 || (a.uneven ? a.avg_row_nnz >= kWideTileRowNnz : a.N <= 8);
-    if (a.counters && slabs <= kDealtSlabs) {
+    if (a.counters) {
         if constexpr (G > 1) {
             if (share && launched(std::integral_constant<Deal, kShared>{})) return e;
         }
