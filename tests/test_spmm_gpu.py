@@ -498,13 +498,15 @@ def test_operands_off_the_16_byte_grid(oracle_mod, shape, N):
 
 @pytest.fixture(scope="module")
 def many_tiles():
-    """Tiles enough to be dealt by a counter, a few rows cut into chunks, and rows of every length around those a warp shares."""
+    """Tiles enough to be dealt by a counter, a few rows cut into chunks, and rows of every length around those a warp shares: a fifth
+    of the nonzeros in rows of more than twice the mean, a dozen and more per row."""
     rng = np.random.default_rng(17)
     M, K = 330000, 20000
     ln = rng.integers(0, 26, M)
-    ln[rng.choice(M, 2000, replace=False)] = rng.integers(27, 257, 2000)
+    ln[rng.choice(M, 8000, replace=False)] = rng.integers(33, 257, 8000)
     ln[:9] = (15, 16, 17, 18, 31, 32, 33, 255, 256)
     ln[5000:5003] = (257, 600, 1500)
+    assert ln.mean() >= 12 and ln[(ln > max(32, 2 * ln.mean())) & (ln <= 256)].sum() > ln.sum() / 8
     rp = np.concatenate([[0], np.cumsum(ln)])
     A = g.CsrMatrix(M, K, torch.from_numpy(rp), torch.from_numpy(rng.integers(0, K, rp[-1]).astype(np.int32)), torch.from_numpy(rng.standard_normal(rp[-1]).astype(np.float32)))
     p = cs.Plan.from_device_csr(M, K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS)
@@ -523,6 +525,38 @@ def test_rows_that_the_groups_of_a_warp_share(oracle_mod, many_tiles, N):
     assert oracle_mod.rel_fro(want, first.cpu().numpy()) <= REL_FRO_TOL_FP32
     for _ in range(3):  # whoever takes a row, its sum is the same
         assert torch.equal(p.spmm(Bd), first)
+    assert p.device_status() == 0
+
+
+@pytest.mark.parametrize("shift", [1, 2])  # rows on the 4- and the 8-byte grid
+@pytest.mark.parametrize("N", [7, 13, 20, 34, 50, 66, 130, 300, 301])
+def test_dealt_tiles_off_the_16_byte_grid(oracle_mod, many_tiles, N, shift):
+    """Every form that reads one or two columns per load, with the tiles dealt by a counter; nothing beside the columns is touched."""
+    A, p = many_tiles
+    wide = N + 4 + N % 2
+    B = g.dense_operand(A.K, N, 9)
+    Bd, Cd = torch.full((A.K, wide), float("nan"), device="cuda"), torch.full((A.M, wide), float("nan"), device="cuda")
+    Bd[:, shift:shift + N] = B.cuda()
+    p.spmm(Bd[:, shift:shift + N], Cd[:, shift:shift + N])
+    first = Cd[:, shift:shift + N].clone()
+    rows = np.concatenate([np.arange(40), np.arange(4990, 5010), np.arange(A.M // 2, A.M // 2 + 2000), np.arange(A.M - 40, A.M)])
+    want = oracle_mod.spmm_csr_rows(A.row_ptr, A.cols, A.vals, B.numpy(), rows)
+    assert oracle_mod.rel_fro(want, first[torch.from_numpy(rows).cuda()].cpu().numpy()) <= REL_FRO_TOL_FP32
+    assert torch.isfinite(first).all() and torch.isnan(Cd[:, :shift]).all() and torch.isnan(Cd[:, shift + N:]).all()
+    Cd.fill_(float("nan"))
+    p.spmm(Bd[:, shift:shift + N], Cd[:, shift:shift + N])
+    assert torch.equal(Cd[:, shift:shift + N], first) and p.device_status() == 0
+
+
+@pytest.mark.parametrize("N", [13, 32])
+def test_rows_that_the_groups_share_of_a_reordered_plan(oracle_mod, many_tiles, N):
+    """The sums of shared rows go through the row map to the caller's rows."""
+    A, _ = many_tiles
+    p = cs.Plan.from_csr(A, path=cs.PATH_ROWS, reorder="similar")
+    assert p.info()["num_tiles"] >= 8 * 6 * torch.cuda.get_device_properties(0).multi_processor_count
+    B = g.dense_operand(A.K, N, 10)
+    want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B.numpy(), A.M, A.K)
+    assert oracle_mod.rel_fro(want, p.spmm(B.cuda()).cpu().numpy()) <= REL_FRO_TOL_FP32
     assert p.device_status() == 0
 
 
@@ -634,14 +668,19 @@ def test_slabs_of_rows_in_runs_fill_the_machine(N):
     assert times[1] <= 0.97 * times[0], times
 
 
-def test_wide_unaligned_products_of_large_matrices_go_in_windows(oracle_mod):
-    """Columns of B that a padded copy of 512 MiB would not hold; rows in runs take the run kernel in every window of 512."""
-    A = g.elasticity3d(48, 3, 9)  # 331776 rows: 409 columns are 543 MB
+@pytest.mark.parametrize("make, launches", [
+    (lambda: g.uniform_random(2000, 340000, 700, seed=3), 4),  # windows of 384 and 25 columns, a padded copy for each
+    (lambda: g.elasticity3d(48, 3, 9), 1),                     # rows in runs: read as they are, whole
+])
+def test_wide_unaligned_products_of_large_matrices(oracle_mod, make, launches):
+    """Columns of B that a padded copy of 512 MiB would not hold (543 and 556 MB)."""
+    A = make()
     N = 409
-    p = cs.Plan.from_device_csr(A.M, A.K, A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda(), path=cs.PATH_ROWS)
+    p = cs.Plan.from_device_csr(A.M, A.K, A.row_ptr.to(torch.int32).cuda(), A.cols.to(torch.int32).cuda(), A.vals.cuda(), path=cs.PATH_ROWS)
+    assert p.launch_count(N) == launches
     B = torch.randn((A.K, N), generator=torch.Generator("cuda").manual_seed(3), device="cuda")
     C = p.spmm(B)
-    for cols in (slice(0, 8), slice(380, 388), slice(401, 409)):  # both sides of the window edges
+    for cols in (slice(0, 8), slice(380, 388), slice(401, 409)):  # both sides of the window's edge
         want = oracle_mod.spmm_csr(A.row_ptr, A.cols, A.vals, B[:, cols].contiguous().cpu().numpy(), A.M, A.K)
         assert oracle_mod.rel_fro(want, C[:, cols].cpu().numpy()) <= 2e-6
     assert p.device_status() == 0
@@ -667,13 +706,15 @@ def test_product_waits_for_nothing_without_memory_for_a_padded_copy(oracle_mod):
     """Rows of B off the 16-byte grid are read through a padded copy where there is memory for it.  Where there is none
     the product reads B as it is; it does not wait for the stream to find some, nor fail."""
     rng = np.random.default_rng(11)
-    M, K, N, per_row = 20000, 330000, 301, 60  # a copy of 401 MB
+    M, K, N, per_row = 20000, 330000, 301, 160  # a copy of 401 MB
     A = g.CsrMatrix(M, K, torch.arange(0, M * per_row + 1, per_row), torch.from_numpy(rng.integers(0, K, M * per_row).astype(np.int32)),
                     torch.from_numpy(rng.standard_normal(M * per_row).astype(np.float32)))
     csr = A.row_ptr.to(torch.int32).cuda(), A.cols.cuda(), A.vals.cuda()
     p = cs.Plan.from_device_csr(M, K, *csr, path=cs.PATH_ROWS)
+    assert p.launch_count(N) == 2  # the copy and the product
     B = torch.randn((K, N), generator=torch.Generator("cuda").manual_seed(12), device="cuda")
     few = cs.Plan.from_device_csr(64, K, csr[0][:65], csr[1][:64 * per_row], csr[2][:64 * per_row], path=cs.PATH_ROWS)
+    assert few.launch_count(N) == 1
     few.spmm(B)  # not worth a copy: the kernel that reads B as it is has been loaded
     C, want = torch.full((M, N), float("nan"), device="cuda"), p.spmm(B)
     stalled = torch.cuda.Event()
