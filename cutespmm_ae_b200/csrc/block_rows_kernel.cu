@@ -5,7 +5,7 @@
 // fp32, storage order: a row's result is the row kernel's, bit for bit.  Tiles and their staging are the row kernel's too
 // (tile_stage.cuh); a run that a tile boundary cuts is computed in two parts.  The reference has no counterpart (its bricks
 // share loads between the rows of a panel on the tensor cores, kernel.cu:119-288).
-// Here the pipe is 58 % busy and instruction issue 70 %.
+// Here the pipe is 62 % busy and instruction issue 60 % (70 % with one column per multiply-add); the rest is the gathers' latency.
 // Rows of B off the 16-byte grid are read one column per load, the lanes' columns interleaved (elasticity40 N = 63 60.5 -> 51 us, N = 203
 // 222 -> 165; before, after a padded copy of B or one row at a time).
 // Products wider than 128 columns go in slabs of equal width, and a block walks its tile once per slab, so that nobody waits for a

@@ -149,11 +149,10 @@ struct MainArgs {
 // rows r, r + stride, ... of a power-law graph, whose long rows sit at indices with few one-bits, to the same few warps --
 // and stages their nonzeros, up to kBuf at a time, in shared memory with one coalesced pass, columns checked; its groups
 // then take a row each (and a long one together).  Bound by the chain of latencies of a claim (counter, row pointers, columns,
-// gathers; no unit of the SM is above 55 % busy) and by the tail, a fifth of the warps' time: warps that find no rows left wait for
-// the others.  U rows of B are in flight per group, 40 warps per SM (U = 8 with 32 warps was 171 against 160 us below, then).
+// gathers): instruction issue is 63 % busy, the L1 data pipe 45 %.  U rows of B are in flight per group, 40 warps per SM (U = 8 with 32 warps was 171 against 160 us below, then).
 // R-MAT 2^18, 3.9 M nonzeros, N = 64: 815 -> 160 us (before: a warp per row and per 1024-nonzero chunk, single-column
-// loads, three kernels one after the other) -> 150 (joins_batch) -> 125 (claim sizes, whole steps); R-MAT 2^16 N = 16 474 -> 29, uniform4096 N = 32 25.6 -> 7.5
-// (back to back, with overlapping launches), stencil512 N = 128 169 -> 139.
+// loads, three kernels one after the other) -> 150 (joins_batch) -> 125 (claim sizes, whole steps); R-MAT
+// 2^16 N = 16 474 -> 29, uniform4096 N = 32 25.6 -> 7.5 (back to back, with overlapping launches), stencil512 N = 128 169 -> 139.
 template <int VEC, int CH, int G>
 __global__ void __launch_bounds__(kWarps * 32, 5) noalloc_main_kernel(MainArgs a)
 {

@@ -182,11 +182,13 @@ int cutespmm_plan_decode_csr(const cutespmm_plan_t *plan, uint64_t *rowPtr, uint
  * (CUTESPMM_EINVAL otherwise): a host that drives several GPUs calls cudaSetDevice before each plan.
  *
  * Nothing waits for the device.  Where the rows of B are not 16-byte aligned (ldb or N not a multiple of four, B off the
- * 16-byte grid) and the matrix names them often enough, the row kernel reads a copy of B with padded rows, of at most 512 MiB
- * at a time (wider products go in column windows), which is taken from the library's stream-ordered pool (the one
+ * 16-byte grid), the row kernel reads a copy of B with padded rows if that is quicker for the matrix and the width (it names the rows
+ * of B often enough; cutespmm_spmm_launch_count counts the copy), of at most 512 MiB (products of matrices with 150 nonzeros per row
+ * and more go in column windows that narrow).  The copy is taken from the library's stream-ordered pool (the one
  * cutespmm_plan_create_device uses) and given back on the stream within the call.  Without memory for it, and
- * while the stream is being captured, the kernel reads B as it is: the same result, more slowly.  A caller that wants no
- * allocation at all keeps rows of B that are 16-byte aligned.
+ * while the stream is being captured, the kernel reads B as it is, more slowly; the two may add a row's products in another
+ * order, and agree to the rounding of fp32 sums.  A caller that wants no allocation at all keeps rows of B that are 16-byte
+ * aligned.
  *
  * Products of one plan may overlap (on several streams, from several threads) where the plan has no long rows
  * (cutespmm_plan_info_t::num_long_rows, and none among the tensor-core panels' rows).  The others share the plan's partial sums
